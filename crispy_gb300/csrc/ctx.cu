@@ -295,7 +295,10 @@ int crispy_ctx_trim(crispy_ctx* ctx) {
     for (DevBuf* b : {&k.seq, &k.off, &k.len, &k.t, &k.gstart, &k.gent, &k.ent, &k.cntmax,
                       &k.hinfo, &k.keys, &k.keys_alt, &k.vals, &k.vals_alt, &k.pairs, &k.dists,
                       &k.counter, &k.mmin, &k.smin, &k.work, &k.sort_tmp, &k.tstart, &k.tgent,
-                      &k.tent, &k.bcnt, &k.tgentL, &k.nsec, &k.t0, &k.offp, &k.perm, &k.sq})
+                      &k.tent, &k.bcnt, &k.tgentL, &k.nsec, &k.t0, &k.offp, &k.perm, &k.sq,
+                      &k.f_packed, &k.f_hist, &k.f_map, &k.f_sig, &k.f_excess, &k.f_perm, &k.f_t,
+                      &k.f_hkey, &k.f_nh, &k.f_heavy, &k.f_pend, &k.f_need, &k.f_cmin, &k.f_ctl,
+                      &k.f_items, &k.f_cand, &k.f_sorted, &k.f_rows, &k.f_distinct, &k.f_meta, &k.f_repeats})
         release(ctx, *b);
     release_host(k.h_spill_pairs);
     release_host(k.h_spill_dists);
@@ -314,7 +317,7 @@ int crispy_ctx_trim(crispy_ctx* ctx) {
                       &pj.counters, &pj.primer, &pj.tmp, &pj.stage_len, &pj.stage_off})
         release(ctx, *b);
     pj.ready = false;
-    k.ready = false;
+    k.ready = k.ent_ready = k.f_ready = false;
     g.ready = false;
     return CRISPY_OK;
 }

@@ -93,6 +93,20 @@ struct KmerJob {
     DevBuf keys, keys_alt, vals, vals_alt, pairs, dists, counter, mmin, smin, work;
     DevBuf sq;                       // K = 8 same-key pass: queued H sums per block and lane slot
     DevBuf sort_tmp;
+    // Level entries and tile streams (the tile kernels' operands) are built
+    // by the first run that needs them; so are the packed reads and the
+    // signatures of the candidate filter (kmer_filter.cu).
+    bool ent_ready = false;
+    bool f_ready = false;
+    int f_dims = 0;                  // signature dimensions (4 bits each)
+    int f_stride = 0;                // words per packed read
+    int f_dstride = 0;               // distinct K-mers' room per read
+    DevBuf f_packed, f_hist, f_map, f_sig, f_excess, f_distinct, f_meta, f_repeats;
+    DevBuf f_perm, f_t, f_hkey, f_nh, f_heavy, f_pend;   // K = 8, by position
+    DevBuf f_need, f_cmin, f_ctl, f_items, f_cand, f_sorted, f_rows;
+    pinned_vector<int32_t> h_pend;
+    std::vector<int4> h_items;
+    int64_t f_pairs = 0, f_found = 0;   // last run: pairs bounded, candidates left
 };
 
 // Device-resident genDist job: 2-bit packed reads.
@@ -233,6 +247,12 @@ struct CohortJob {
     crispy_sink sink = nullptr;   // genDist chunks of this job (gen_run_cohort)
     void* user = nullptr;
 };
+// The candidate filter of the batched k-mer run (kmer_filter.cu).
+bool kmer_filter_applies(const KmerJob& j, float thr);
+int kmer_filter_build(crispy_ctx* ctx, float thr);
+size_t kmer_filter_bytes(const int32_t* len, int n, int k);
+int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int sd, int64_t* total,
+                     bool* gave_up);
 int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::vector<int64_t>& counts);
 // The k-mer bound pass's tuned splits as JSON objects, each preceded by ", ".
 std::string kmer_tune_json();

@@ -56,6 +56,7 @@
 #include <string>
 
 #include "internal.h"
+#include "kmer_emit.h"
 
 namespace crispy {
 namespace {
@@ -806,51 +807,6 @@ __device__ __forceinline__ void csa(uint32_t& h, uint32_t& l, uint32_t a, uint32
     const uint32_t u = l ^ a;
     h = (l & a) | (u & b);
     l = u ^ b;
-}
-
-__device__ __forceinline__ uint64_t stage_key(int r, int c, int n, int A, int sd) {
-    // kmerCUDA.cu:79-111 + Trag_reverse_eq (kmerMain.cpp:205-216): stages
-    // enumerate the upper triangle of the stageDim grid row-major; inside a
-    // stage the host scan is row-major (kmerMain.cpp:175-195).
-    const int64_t sx = r / A, sy = c / A;
-    const int64_t s = sx * sd - sx * (sx - 1) / 2 + (sy - sx);
-    return ((uint64_t)s * (uint64_t)n + (uint64_t)r) * (uint64_t)n + (uint64_t)c;
-}
-
-// Survivor emission with one atomic per warp.  All 32 lanes call it.
-// (r, c) are positions in the job's read order; with a read order (perm !=
-// nullptr, K = 8) they map back to the caller's read IDs, the pair is
-// reordered so that the lower ID comes first, and only pairs whose lower ID
-// lies in [olo, ohi) are kept (the stage rows of one pass).
-__device__ __forceinline__ void emit(unsigned long long* counter, uint64_t* keys, uint32_t* vals,
-                                     int64_t cap, int n, int A, int sd, const int32_t* perm,
-                                     int olo, int ohi, bool pass, int r, int c, int m, int mn,
-                                     int base_pos = 0, uint64_t tag = 0, unsigned long long* jcount = nullptr) {
-    if (perm != nullptr && pass) {
-        const int pr = __ldg(perm + r), pc = __ldg(perm + c);
-        r = min(pr, pc);
-        c = max(pr, pc);
-        pass = r >= olo && r < ohi;
-    }
-    const unsigned pm = __ballot_sync(0xffffffffu, pass);
-    if (!pm) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    const int leader = __ffs(pm) - 1;
-    if (lane == leader) {
-        base = atomicAdd(counter, (unsigned long long)__popc(pm));
-        if (jcount) atomicAdd(jcount, (unsigned long long)__popc(pm));
-    }
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (pass) {
-        const unsigned long long idx = base + __popc(pm & ((1u << lane) - 1u));
-        if (idx < (unsigned long long)cap) {
-            keys[idx] = tag | stage_key(r - base_pos, c - base_pos, n, A, sd);
-            // kmerKernel.cu:47: 1.0f - (float)matches / min(T1, T2), IEEE
-            const float d = __fsub_rn(1.0f, __fdiv_rn((float)m, (float)mn));
-            vals[idx] = __float_as_uint(d);
-        }
-    }
 }
 
 __device__ __forceinline__ uint32_t hash_slot(uint32_t key) {
@@ -2588,9 +2544,9 @@ int kmer_groups(crispy_ctx* ctx, const int32_t* t) {
     return CRISPY_OK;
 }
 
-// Per-read layout of a K-mer job from the read lengths (host metadata and
-// the device buffers sized for it); the reads themselves come next.  K = 8
-// jobs get their group layout at rebuild, in the read order built there.
+// Per-read metadata of a K-mer job from the read lengths; the reads
+// themselves come next, and their k-mer structures with the first run that
+// needs them (kmer_build_entries, kmer_filter_build).
 int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
     if (n > CRISPY_MAX_NUM_READS) return fail(ctx, CRISPY_E_UNSUPPORTED, "numReads %d > %d", n, CRISPY_MAX_NUM_READS);
     if (k < 1 || k > 8) return fail(ctx, CRISPY_E_UNSUPPORTED, "K = %d outside 1..8", k);
@@ -2611,8 +2567,22 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
         j.max_t = std::max(j.max_t, j.h_t[r]);
     }
     j.ngroups = (n + 31) / 32;
-    j.split = 0;
-    if (tile_rows_for(k) == kRows128) {
+    j.ent_ready = j.f_ready = false;
+    CRISPY_TRY(ensure(ctx, j.off, (size_t)n * 8));
+    CRISPY_TRY(ensure(ctx, j.t0, (size_t)n * 4));
+    CRISPY_CK(ctx, cudaMemcpyAsync(j.t0.ptr, j.h_t.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
+    return CRISPY_OK;
+}
+
+int kmer_order(crispy_ctx* ctx);
+
+// Group layout of the tile kernels' operands (K = 8: the read order first).
+// split < 0: the split this read set gets by itself.
+int kmer_entry_layout(crispy_ctx* ctx, int split) {
+    KmerJob& j = ctx->kmer;
+    const int n = j.n, k = j.k;
+    j.split = std::max(0, split);
+    if (tile_rows_for(k) == kRows128 && split < 0) {
         // section 0's share of the dense entries in 1/256 (0: one section,
         // no bound pass): CRISPY_KMER_SPLIT, else the tuned split of this
         // read set, else the default
@@ -2625,7 +2595,6 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
             }
         }
     }
-    CRISPY_TRY(ensure(ctx, j.off, (size_t)n * 8));
     CRISPY_TRY(ensure(ctx, j.t, (size_t)n * 4));
     CRISPY_TRY(ensure(ctx, j.gstart, (size_t)(j.ngroups + 1) * 8));
     CRISPY_TRY(ensure(ctx, j.gent, (size_t)j.ngroups * 4));
@@ -2634,18 +2603,15 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
     CRISPY_TRY(ensure(ctx, j.bcnt, (size_t)n * 128));
     CRISPY_TRY(ensure(ctx, j.tstart, (size_t)(j.ngroups + 1) * 8));
     CRISPY_TRY(ensure(ctx, j.tgent, (size_t)j.ngroups * 4));
-    if (j.split) {
+    if (j.split || k == 8) {
         CRISPY_TRY(ensure(ctx, j.tgentL, (size_t)j.ngroups * 4));
         CRISPY_TRY(ensure(ctx, j.nsec, (size_t)n * 8));
     }
     if (k != 8) return kmer_groups(ctx, j.h_t.data());
-    CRISPY_TRY(ensure(ctx, j.tgentL, (size_t)j.ngroups * 4));
-    CRISPY_TRY(ensure(ctx, j.nsec, (size_t)n * 8));
-    CRISPY_TRY(ensure(ctx, j.t0, (size_t)n * 4));
     CRISPY_TRY(ensure(ctx, j.offp, (size_t)n * 8));
     CRISPY_TRY(ensure(ctx, j.perm, (size_t)n * 4));
-    CRISPY_CK(ctx, cudaMemcpyAsync(j.t0.ptr, j.h_t.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    return CRISPY_OK;
+    j.hkeys_ordered = false;
+    return kmer_order(ctx);
 }
 
 // K = 8 read order (kmer_hkey_kernel): the sorted order as perm (position ->
@@ -2735,18 +2701,27 @@ int crispy_kmer_prepare_from_pre(crispy_ctx* ctx, const crispy_raw* raw, int k) 
     return crispy_kmer_rebuild(ctx);
 }
 
-// Rebuild the level entries, multiplicities and K = 8 keys from the reads
-// already resident on the device (no host transfer of reads).
+// The k-mer structures are built again from the reads already resident on
+// the device (no host transfer of reads): the next run builds those it needs.
 int crispy_kmer_rebuild(crispy_ctx* ctx) {
     if (!ctx) return CRISPY_E_INPUT;
     KmerJob& j = ctx->kmer;
     if (!j.ready) return fail(ctx, CRISPY_E_STATE, "kmer_rebuild before kmer_prepare");
     cudaSetDevice(ctx->device);
+    j.ent_ready = j.f_ready = false;
+    j.nsurv = 0;
+    // the caller's host buffers are its own again
+    CRISPY_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    return CRISPY_OK;
+}
+
+// Level entries, multiplicities, K = 8 keys and the tile streams.
+static int kmer_build_entries(crispy_ctx* ctx, int split = -1) {
+    KmerJob& j = ctx->kmer;
+    if (j.ent_ready) return CRISPY_OK;
+    CRISPY_TRY(kmer_entry_layout(ctx, split));
     cudaStream_t s = ctx->stream;
     const int n = j.n, k = j.k;
-    // K = 8: entries and streams are laid out in the read order
-    j.hkeys_ordered = false;
-    if (k == 8) CRISPY_TRY(kmer_order(ctx));
     const int64_t* loff = k == 8 ? j.offp.as<int64_t>() : j.off.as<int64_t>();
     CRISPY_CK(ctx, cudaMemsetAsync(j.ent.ptr, 0xFF, (size_t)std::max<int64_t>(j.nent, 4) * 4, s));
     const uint32_t K4 = 1u << (2 * k);
@@ -2846,7 +2821,7 @@ int crispy_kmer_rebuild(crispy_ctx* ctx) {
     CRISPY_CK(ctx, cudaMemcpyAsync(j.h_cntmax.data(), j.cntmax.ptr, (size_t)n * 8,
                                    cudaMemcpyDeviceToHost, s));
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
-    j.nsurv = 0;
+    j.ent_ready = true;
     return CRISPY_OK;
 }
 
@@ -2866,6 +2841,12 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     ctx->stats = crispy_stats{};
     ctx->ev_kmer.used = 0;
     CRISPY_CK(ctx, cudaEventRecord(ctx->t_begin, s));
+    // the batched form bounds every pair on the tensor cores and counts the
+    // candidates exactly, where that pays (kmer_filter.cu); the tile kernels
+    // below take everything else, and a run whose candidates are too many
+    bool filter = mode == CRISPY_MODE_BATCHED && sample == 0 && kmer_filter_applies(j, thr);
+    j.f_pairs = j.f_found = 0;
+    if (filter) CRISPY_TRY(kmer_filter_build(ctx, thr));
     const int sd = (n + A - 1) / A;
     const int64_t nstages = (int64_t)sd * (sd + 1) / 2;
 
@@ -2881,20 +2862,9 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     const int levels = dense_levels_for(K);
     const int rows_blk = tile_rows_for(K);   // row reads per tile block
     const int nrg = (n + rows_blk - 1) / rows_blk;
-    std::vector<uint8_t> dense(j.ngroups, 0);
+    std::vector<uint8_t> dense;
     bool any_dense = false;
-    for (int rg = 0; rg < nrg; ++rg) {
-        int64_t high = 0;
-        for (int r = rg * rows_blk; r < std::min(n, rg * rows_blk + rows_blk); ++r) high += j.h_cntmax[n + r];
-        if (levels == 0 || high > kHashMaxKeys) {
-            for (int r = rg * rows_blk; r < std::min(n, rg * rows_blk + rows_blk); r += 32) dense[r >> 5] = 1;
-            any_dense = true;
-        }
-    }
     const bool fast = levels > 0;
-    CRISPY_TRY(ensure(ctx, j.work, (size_t)j.ngroups + 16));
-    CRISPY_CK(ctx, cudaMemcpyAsync(j.work.ptr, dense.data(), j.ngroups, cudaMemcpyHostToDevice, s));
-
     const uint32_t K4 = 1u << (2 * K);
     const int B = std::max(8, bits_for((uint64_t)j.max_t));
     TileFn tile = K == 8 ? tile8_fn_for(B) : rows_blk == kRows128 ? tile128_fn_for(B) : tile_fn_for(B);
@@ -2902,41 +2872,76 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     const size_t tsmem = !fast ? 0 : K == 8 ? kSmem8     // one plane + guards
                                              : ((size_t)levels * K4 + 32) * (rows_blk / 8);   // planes + guards
     const size_t dsmem = (size_t)((K4 + 1) / 2) * 4;
-    if (fast) CRISPY_CK(ctx, cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
     // K = 8 batched: the H-only kernel over all row groups plus the two-phase
     // kernel over each row group's same-key column range (the H keys must be
     // in order along the positions, as the read order makes them)
     // (CRISPY_KMER_K8_SPLIT=0 selects the one-kernel form, the same
     // survivors: the two-phase kernel over every column)
-    const char* split_env = std::getenv("CRISPY_KMER_K8_SPLIT");
-    const bool split8 = fast && K == 8 && mode == CRISPY_MODE_BATCHED && j.hkeys_ordered &&
-                        !(split_env && std::strcmp(split_env, "0") == 0);
-    TileFn tile_h = split8 ? tile8h_fn_for(B) : nullptr;
-    if (split8) CRISPY_CK(ctx, cudaFuncSetAttribute(tile_h, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
     // the same-key ranges of the split: the kernel that queues its L sums
-    // (CRISPY_KMER_K8_QUEUE=0 selects the two-phase kernel)
-    const char* queue_env = std::getenv("CRISPY_KMER_K8_QUEUE");
-    const bool queue8 = split8 && !(queue_env && std::strcmp(queue_env, "0") == 0);
-    TileFn tile_s = queue8 ? tile8s_fn_for(B) : tile;
-    if (queue8) CRISPY_CK(ctx, cudaFuncSetAttribute(tile_s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
-    CRISPY_CK(ctx, cudaFuncSetAttribute(kmer_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+    // (CRISPY_KMER_K8_QUEUE=0 selects the two-phase kernel).
+    // K = 8 jobs hold their reads in the read order: the kernels run over
+    // positions, emit() maps them back to read IDs.
+    bool split8 = false, queue8 = false;
+    TileFn tile_h = nullptr, tile_s = tile;
+    const int32_t* perm = nullptr;
+    const int64_t* loff = j.off.as<int64_t>();
+    auto setup_tiles = [&]() -> int {
+        CRISPY_TRY(kmer_build_entries(ctx));
+        dense.assign(j.ngroups, 0);
+        for (int rg = 0; rg < nrg; ++rg) {
+            int64_t high = 0;
+            for (int r = rg * rows_blk; r < std::min(n, rg * rows_blk + rows_blk); ++r) high += j.h_cntmax[n + r];
+            if (levels == 0 || high > kHashMaxKeys) {
+                for (int r = rg * rows_blk; r < std::min(n, rg * rows_blk + rows_blk); r += 32) dense[r >> 5] = 1;
+                any_dense = true;
+            }
+        }
+        CRISPY_TRY(ensure(ctx, j.work, (size_t)j.ngroups + 16));
+        CRISPY_CK(ctx, cudaMemcpyAsync(j.work.ptr, dense.data(), j.ngroups, cudaMemcpyHostToDevice, s));
+        if (fast) CRISPY_CK(ctx, cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+        const char* split_env = std::getenv("CRISPY_KMER_K8_SPLIT");
+        split8 = fast && K == 8 && mode == CRISPY_MODE_BATCHED && j.hkeys_ordered &&
+                 !(split_env && std::strcmp(split_env, "0") == 0);
+        if (split8) {
+            tile_h = tile8h_fn_for(B);
+            CRISPY_CK(ctx, cudaFuncSetAttribute(tile_h, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
+        }
+        const char* queue_env = std::getenv("CRISPY_KMER_K8_QUEUE");
+        queue8 = split8 && !(queue_env && std::strcmp(queue_env, "0") == 0);
+        if (queue8) {
+            tile_s = tile8s_fn_for(B);
+            CRISPY_CK(ctx, cudaFuncSetAttribute(tile_s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
+        }
+        CRISPY_CK(ctx, cudaFuncSetAttribute(kmer_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+        if (K == 8) {
+            perm = j.perm.as<int32_t>();
+            loff = j.offp.as<int64_t>();
+        }
+        return CRISPY_OK;
+    };
+    if (!filter) CRISPY_TRY(setup_tiles());
 
-    // K = 8 jobs hold their reads in the read order built at rebuild: the
-    // kernels run over positions, emit() maps them back to read IDs.
-    const int32_t* perm = K == 8 ? j.perm.as<int32_t>() : nullptr;
-    const int64_t* loff = K == 8 ? j.offp.as<int64_t>() : j.off.as<int64_t>();
     // One pass over the pairs whose lower read ID lies in [olo, ohi):
     // survivors (up to cap) as sort keys in j.keys / j.vals, their count in
     // *total.  Without a read order the kernels cover the rows [olo, ohi);
     // with one they cover every row and emit() keeps the range.
     auto run_pass = [&](int olo, int ohi, int64_t cap, int64_t* total_out) -> int {
-        const int rlo = perm ? 0 : olo, rhi = perm ? n : ohi;
         CRISPY_TRY(ensure(ctx, j.keys, (size_t)cap * 8));
         CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)cap * 8));
         CRISPY_TRY(ensure(ctx, j.vals, (size_t)cap * 4));
         CRISPY_TRY(ensure(ctx, j.vals_alt, (size_t)cap * 4));
         CRISPY_TRY(ensure(ctx, j.counter, 64));
         CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
+        if (filter) {
+            bool gave_up = false;
+            CRISPY_TRY(kmer_filter_pass(ctx, olo, ohi, cap, A, sd, total_out, &gave_up));
+            if (!gave_up) return CRISPY_OK;
+            filter = false;
+            j.f_pairs = 0;
+            CRISPY_TRY(setup_tiles());
+            CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
+        }
+        const int rlo = perm ? 0 : olo, rhi = perm ? n : ohi;
 
         TileArgs ta{};
         ta.ent = j.ent.as<uint32_t>(); ta.gstart = j.gstart.as<int64_t>(); ta.gent = j.gent.as<int32_t>();
@@ -3240,7 +3245,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         // processed in ranges whose survivors fit; stage order is row-major
         // over stage rows, so each range's sorted pairs append in order to
         // one pinned host list (the count is known from the first pass).
-        if (!perm && A % rows_blk != 0) return fail(ctx, CRISPY_E_OOM, "survivor list exceeds the device share");
+        if (K != 8 && A % rows_blk != 0) return fail(ctx, CRISPY_E_OOM, "survivor list exceeds the device share");
         CRISPY_TRY(ensure_host(ctx, j.h_spill_pairs, (size_t)total * 8));
         if (dists) CRISPY_TRY(ensure_host(ctx, j.h_spill_dists, (size_t)total * 4));
         // expected survivors per stage row, proportional to its pairs
@@ -3294,15 +3299,10 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     return CRISPY_OK;
 }
 
-// Stream layout and level entries again, for the job's current split.
-static int kmer_relayout(crispy_ctx* ctx) {
-    KmerJob& j = ctx->kmer;
-    if (j.split) {
-        CRISPY_TRY(ensure(ctx, j.tgentL, (size_t)j.ngroups * 4));
-        CRISPY_TRY(ensure(ctx, j.nsec, (size_t)j.n * 8));
-    }
-    CRISPY_TRY(kmer_groups(ctx, j.h_t.data()));
-    return crispy_kmer_rebuild(ctx);
+// Stream layout and level entries again, for another split.
+static int kmer_relayout(crispy_ctx* ctx, int split) {
+    ctx->kmer.ent_ready = false;
+    return kmer_build_entries(ctx, split);
 }
 
 // The split of this read set: the tuned one, or -- from its second batched
@@ -3322,8 +3322,7 @@ static int kmer_tune_split(crispy_ctx* ctx, float thr) {
     if (best < 0) {
         float best_ms = 1e30f, dflt_ms = 0;
         for (int c : kSplitCandidates) {
-            j.split = c;
-            CRISPY_TRY(kmer_relayout(ctx));
+            CRISPY_TRY(kmer_relayout(ctx, c));
             float ms = 1e30f;
             for (int rep = 0; rep < 2; ++rep) {
                 float m = 0;
@@ -3337,11 +3336,27 @@ static int kmer_tune_split(crispy_ctx* ctx, float thr) {
         g_ktuned[fp] = KmerTuneEntry{j.n, j.k, best, best_ms, dflt_ms,
                                      (int)((j.n + kRows128 * kKmerTuneStride - 1) / (kRows128 * kKmerTuneStride))};
     }
-    if (j.split != best) {
-        j.split = best;
-        CRISPY_TRY(kmer_relayout(ctx));
-    }
+    if (!j.ent_ready || j.split != best) CRISPY_TRY(kmer_relayout(ctx, best));
     return CRISPY_OK;
+}
+
+// Read sets whose batched runs the candidate filter took twice or more, for
+// crispy_tune_report: the filter's dimensions and what it left, and the split
+// the tile kernels would start from.
+struct KmerFilterNote {
+    int n, k, dims, runs;
+    int64_t pairs, found;
+};
+static std::map<std::string, KmerFilterNote> g_kfilter;   // guarded by g_ktune_mu
+
+static void kmer_note_filter(const KmerJob& j) {
+    int64_t sum = 0;
+    for (int r = 0; r < j.n; ++r) sum += j.h_t[r];
+    const std::string key = key_of({(uint64_t)j.n, (uint64_t)j.k, (uint64_t)sum, (uint64_t)j.max_t});
+    std::lock_guard<std::mutex> g(g_ktune_mu);
+    if (g_kfilter.size() >= 256 && !g_kfilter.count(key)) g_kfilter.clear();
+    KmerFilterNote& e = g_kfilter[key];
+    e = KmerFilterNote{j.n, j.k, j.f_dims, e.runs + 1, j.f_pairs, j.f_found};
 }
 
 int crispy_kmer_run(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* npairs) {
@@ -3349,10 +3364,12 @@ int crispy_kmer_run(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* np
     KmerJob& j = ctx->kmer;
     if (!j.ready) return fail(ctx, CRISPY_E_STATE, "kmer_run before kmer_prepare");
     cudaSetDevice(ctx->device);
-    if (mode == CRISPY_MODE_BATCHED && ctx->kmer_tune && tile_rows_for(j.k) == kRows128 &&
-        j.n >= kKmerTuneMinReads && kmer_autotune_enabled() && !kmer_split_env(nullptr))
-        CRISPY_TRY(kmer_tune_split(ctx, thr));
-    return kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr);
+    const bool tunable = mode == CRISPY_MODE_BATCHED && ctx->kmer_tune && tile_rows_for(j.k) == kRows128 &&
+                         j.n >= kKmerTuneMinReads && kmer_autotune_enabled() && !kmer_split_env(nullptr);
+    if (tunable && !kmer_filter_applies(j, thr)) CRISPY_TRY(kmer_tune_split(ctx, thr));
+    CRISPY_TRY(kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr));
+    if (tunable && j.f_pairs > 0) kmer_note_filter(j);
+    return CRISPY_OK;
 }
 
 int crispy_kmer_fetch(crispy_ctx* ctx, int32_t* pairs, float* dists, int64_t cap, int64_t* count) {
@@ -3439,6 +3456,16 @@ std::string kmer_tune_json() {
                  kv.second.ms_default);
         out += item;
     }
+    for (auto& kv : g_kfilter) {
+        if (kv.second.runs < 2) continue;
+        char item[256];
+        snprintf(item, sizeof item,
+                 ", {\"stage\": \"kmer\", \"kernel\": \"kmer_filter_kernel\", \"reads\": %d, \"k\": %d, "
+                 "\"split\": %d, \"dims\": %d, \"pairs\": %lld, \"candidates\": %lld}",
+                 kv.second.n, kv.second.k, kSplitDefault, kv.second.dims, (long long)kv.second.pairs,
+                 (long long)kv.second.found);
+        out += item;
+    }
     return out;
 }
 
@@ -3451,6 +3478,7 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
     const int levels = dense_levels_for(K);
     if (levels <= 0) return fail(ctx, CRISPY_E_UNSUPPORTED, "cohort: no shared-memory planes for K %d", K);
     cudaSetDevice(ctx->device);
+    CRISPY_TRY(kmer_build_entries(ctx));
     cudaStream_t s = ctx->stream;
     ctx->stats = crispy_stats{};
     ctx->ev_kmer.used = 0;

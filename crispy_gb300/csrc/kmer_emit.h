@@ -1,0 +1,58 @@
+// kmer_emit.h -- device helpers shared by the k-mer kernels (kmer.cu,
+// kmer_filter.cu): stage order keys and survivor emission.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace crispy {
+namespace {
+
+__device__ __forceinline__ uint64_t stage_key(int r, int c, int n, int A, int sd) {
+    // kmerCUDA.cu:79-111 + Trag_reverse_eq (kmerMain.cpp:205-216): stages
+    // enumerate the upper triangle of the stageDim grid row-major; inside a
+    // stage the host scan is row-major (kmerMain.cpp:175-195).
+    const int64_t sx = r / A, sy = c / A;
+    const int64_t s = sx * sd - sx * (sx - 1) / 2 + (sy - sx);
+    return ((uint64_t)s * (uint64_t)n + (uint64_t)r) * (uint64_t)n + (uint64_t)c;
+}
+
+// Survivor emission with one atomic per warp.  All 32 lanes call it.
+// (r, c) are positions in the job's read order; with a read order (perm !=
+// nullptr, K = 8) they map back to the caller's read IDs, the pair is
+// reordered so that the lower ID comes first, and only pairs whose lower ID
+// lies in [olo, ohi) are kept (the stage rows of one pass).
+__device__ __forceinline__ void emit(unsigned long long* counter, uint64_t* keys, uint32_t* vals,
+                                     int64_t cap, int n, int A, int sd, const int32_t* perm,
+                                     int olo, int ohi, bool pass, int r, int c, int m, int mn,
+                                     int base_pos = 0, uint64_t tag = 0, unsigned long long* jcount = nullptr) {
+    if (perm != nullptr && pass) {
+        const int pr = __ldg(perm + r), pc = __ldg(perm + c);
+        r = min(pr, pc);
+        c = max(pr, pc);
+        pass = r >= olo && r < ohi;
+    }
+    const unsigned pm = __ballot_sync(0xffffffffu, pass);
+    if (!pm) return;
+    const int lane = threadIdx.x & 31;
+    unsigned long long base = 0;
+    const int leader = __ffs(pm) - 1;
+    if (lane == leader) {
+        base = atomicAdd(counter, (unsigned long long)__popc(pm));
+        if (jcount) atomicAdd(jcount, (unsigned long long)__popc(pm));
+    }
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (pass) {
+        const unsigned long long idx = base + __popc(pm & ((1u << lane) - 1u));
+        if (idx < (unsigned long long)cap) {
+            keys[idx] = tag | stage_key(r - base_pos, c - base_pos, n, A, sd);
+            // kmerKernel.cu:47: 1.0f - (float)matches / min(T1, T2), IEEE
+            const float d = __fsub_rn(1.0f, __fdiv_rn((float)m, (float)mn));
+            vals[idx] = __float_as_uint(d);
+        }
+    }
+}
+
+}  // namespace
+}  // namespace crispy

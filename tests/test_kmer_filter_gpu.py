@@ -1,0 +1,90 @@
+"""The tensor-core candidate filter of the batched k-mer run (K >= 5, cut
+<= 0.3) against the oracle: pairs, order and distances bit for bit.
+
+Sizes sit at the edges of the 128-row panels, the 224-column tiles and the
+256-dimension chunks of the signatures (resident and streamed rows); reads
+with folded counts beyond 36 (homopolymers), reads in no length order, reads
+without a k-mer, K = 8 reads with and without an H half, and sets whose
+candidates outgrow their buffer, which the tile kernels then take.
+"""
+import numpy as np
+import pytest
+
+import crispy_gb300 as cg
+import oracle
+from crispy_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _reads(n, seed, k=6, root=260, dist="normal", a=250, b=15, cents=None):
+    spec = synth.ReadSetSpec(n + n // 8 + 8, cents or max(2, n // 20), root, dist, a, b, k, seed)
+    return synth.make_read_set(spec)[:n]
+
+
+def _check(engine, monkeypatch, reads, k, thr):
+    buf, offs, lens = synth.pack_reads(reads)
+    got = {}
+    for on in ("1", "0"):
+        monkeypatch.setenv("CRISPY_KMER_FILTER", on)
+        engine.kmer_prepare(buf, offs, lens, k)
+        cnt = engine.kmer_run(thr, cg.MODE_BATCHED, True)
+        got[on] = engine.kmer_fetch(cnt, True)
+    op, od = oracle.kmer_all(buf, offs, lens, k, thr)
+    for pairs, d in got.values():
+        assert np.array_equal(pairs, op)
+        assert np.array_equal(d.view(np.uint32), od.view(np.uint32))
+    return len(op)
+
+
+@pytest.mark.parametrize("n", [10, 127, 128, 129, 223, 225, 449, 1025])
+def test_filter_tile_edges(engine, monkeypatch, n):
+    assert _check(engine, monkeypatch, _reads(n, 900 + n), 6, 0.2) > 0
+
+
+@pytest.mark.parametrize("k", [5, 6, 7, 8])
+@pytest.mark.parametrize("thr", [0.0, 0.1, 0.2, 0.3])
+def test_filter_k_and_cut(engine, monkeypatch, k, thr):
+    reads = _reads(700, 910 + k, k=k, root=520, dist="uniform", a=300, b=500)
+    _check(engine, monkeypatch, reads, k, thr)
+
+
+@pytest.mark.parametrize("length", [40, 128, 400, 700, 1100, 2048])
+def test_filter_signature_lengths(engine, monkeypatch, length):
+    # one chunk of 256 dimensions to the most (4,096, streamed)
+    reads = _reads(300, 920 + length, root=2100, dist="uniform", a=max(20, length - 30), b=length)
+    assert _check(engine, monkeypatch, reads, 6, 0.2) > 0
+
+
+@pytest.mark.parametrize("k", [6, 8])
+def test_filter_repeats_and_order(engine, monkeypatch, k):
+    rng = np.random.default_rng(k)
+    reads = _reads(260, 930, k=k)
+    for i in range(60):     # runs of one base: folded counts far beyond 36
+        s = bytearray(reads[i])
+        run = 40 + 3 * (i % 30)
+        s[20:20 + run] = b"ACGT"[i % 4:i % 4 + 1] * run
+        reads.append(bytes(s))
+    reads += [b"A" * (300 + i) for i in range(6)] + [b"CT" * (150 + i) for i in range(6)]
+    reads += [b"ACGTACG"[:k - 1 + (i & 1)] for i in range(2)]
+    reads = [reads[i] for i in rng.permutation(len(reads))]
+    assert _check(engine, monkeypatch, reads, k, 0.2) > 0
+
+
+def test_filter_heavy_h_reads(engine, monkeypatch):
+    # K = 8 reads rich in T and C: pairs of different H keys can pass
+    rng = np.random.default_rng(5)
+    reads = _reads(200, 940, k=8)
+    base = rng.choice(np.frombuffer(b"TC", np.uint8), 260).tobytes()
+    for i in range(80):
+        s = bytearray(base)
+        for p in rng.integers(0, 260, 3):
+            s[p] = b"TC"[rng.integers(0, 2)]
+        reads.append(bytes(s[:200 + i // 2]))
+    assert _check(engine, monkeypatch, synth.preprocess_order(reads), 8, 0.25) > 0
+
+
+def test_filter_gives_up(engine, monkeypatch):
+    # one centroid: nearly every pair is a candidate, more than the buffer holds
+    reads = _reads(1800, 950, cents=1)
+    assert _check(engine, monkeypatch, reads, 6, 0.3) > 300000
