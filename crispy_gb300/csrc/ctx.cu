@@ -298,7 +298,7 @@ int crispy_ctx_trim(crispy_ctx* ctx) {
                       &k.tent, &k.bcnt, &k.tgentL, &k.nsec, &k.t0, &k.offp, &k.perm, &k.sq,
                       &k.f_packed, &k.f_hist, &k.f_map, &k.f_sig, &k.f_excess, &k.f_perm, &k.f_t,
                       &k.f_hkey, &k.f_nh, &k.f_heavy, &k.f_pend, &k.f_need, &k.f_cmin, &k.f_ctl,
-                      &k.f_items, &k.f_cand, &k.f_sorted, &k.f_rows, &k.f_distinct, &k.f_meta, &k.f_repeats})
+                      &k.f_items, &k.f_cand, &k.f_candidx, &k.f_sorted, &k.f_rows, &k.f_distinct, &k.f_meta, &k.f_repeats})
         release(ctx, *b);
     release_host(k.h_spill_pairs);
     release_host(k.h_spill_dists);

@@ -103,9 +103,10 @@ struct KmerJob {
     int f_dstride = 0;               // distinct K-mers' room per read
     DevBuf f_packed, f_hist, f_map, f_sig, f_excess, f_distinct, f_meta, f_repeats;
     DevBuf f_perm, f_t, f_hkey, f_nh, f_heavy, f_pend;   // K = 8, by position
-    DevBuf f_need, f_cmin, f_ctl, f_items, f_cand, f_sorted, f_rows;
+    DevBuf f_need, f_cmin, f_ctl, f_items, f_cand, f_candidx, f_sorted, f_rows;
     pinned_vector<int32_t> h_pend;
     std::vector<int4> h_items;
+    std::vector<int> h_segs;
     int64_t f_pairs = 0, f_found = 0;   // last run: pairs bounded, candidates left
 };
 

@@ -400,33 +400,38 @@ constexpr int kCols = 224;                 // column positions of a tile: two ac
 constexpr int kChunkA = kRows * 128;       // 256 dimensions of a tile's rows (bytes)
 constexpr int kChunkB = kCols * 128;
 constexpr int kResidentChunks = 4;         // rows stay in shared memory up to 1,024 dimensions
-constexpr int kMaxStages = 6;
-constexpr int kCandBuf = 256;              // candidates a warp holds before it writes them out
-constexpr int kFilterThreads = 192;        // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+constexpr int kMaxDepth = 3;               // stages of each of the two rings
+constexpr int kCluster = 2;                // blocks that share the columns' boxes (TMA multicast)
+constexpr int kCandBuf = 96;               // candidates a warp holds before it writes them out
+constexpr int kEpilogueWarps = 12;         // for each quarter of the TMEM lanes:
+constexpr int kEpiPer = kEpilogueWarps / 4;
+constexpr int kEpiSteps = (kCols / 32 + kEpiPer - 1) / kEpiPer;
+constexpr int kFilterThreads = 96 + 32 * kEpilogueWarps;   // warp 0 TMA, warps 1-2 MMA, then the epilogue
 constexpr size_t kSmemLimit = 227 * 1024;
-constexpr unsigned long long kWaitNs = 2000000000ull;
+constexpr long long kWaitCycles = 4000000000ll;   // about two seconds
 
 struct FilterArgs {
-    const int4* items;    // (panel, first column tile, end column tile, -)
-    int nitems;
+    const int4* items;    // (panel group, first column tile, end column tile, -)
+    const int* segs;      // first item of each segment, and the end
+    int nsegs;
     int chunks;           // 256-dimension chunks of a signature
-    int stages;
+    int depth;            // stages of a ring
     int n;
     const float* need;
     const float* cmin;
     const uint16_t* excess;
-    uint64_t* cand;        // row << 40 | column << 20 | index among the row's candidates
-    uint32_t* rowcnt;      // candidates per row
+    uint2* cand;          // (row, column)
     unsigned long long cap;
     int round;
     FilterCtl* ctl;
 };
 
 struct Bars {
-    uint64_t full[kMaxStages], empty[kMaxStages];
+    uint64_t full[2 * kMaxDepth], empty[2 * kMaxDepth];
     uint64_t a_full, a_empty;
     uint64_t acc_full[2], acc_empty[2];
     uint64_t drain;
+    uint32_t held[kEpilogueWarps];   // candidates in each warp's buffer
     uint32_t tmem;
     uint32_t abort;
 };
@@ -451,18 +456,14 @@ __device__ __forceinline__ bool bar_try(uint64_t* b, uint32_t parity) {
         : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ unsigned long long now_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// A wait that gives up after kWaitNs, or once another warp of the block has:
-// the block then leaves its loops and reports a timeout.
+// A wait that gives up after kWaitCycles, or once another warp of the block
+// has: the block then leaves its loops and reports a timeout.
 __device__ __noinline__ bool bar_wait_slow(uint64_t* b, uint32_t parity, Bars* bars, FilterCtl* ctl) {
-    const unsigned long long t0 = now_ns();
-    while (!bar_try(b, parity)) {
+    const long long t0 = clock64();
+    for (uint32_t i = 1; !bar_try(b, parity); ++i) {
+        if (i & 31u) continue;
         if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) return false;
-        if (now_ns() - t0 > kWaitNs) {
+        if (clock64() - t0 > kWaitCycles) {
             *reinterpret_cast<volatile uint32_t*>(&bars->abort) = 1u;
             atomicOr(&ctl->timeout, 1u);
             return false;
@@ -478,6 +479,26 @@ __device__ __forceinline__ void tma_load(const CUtensorMap* map, uint32_t dst, i
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)) : "memory");
+}
+// The same box into every block of the cluster (the same offset there, and
+// the same barrier of each).
+__device__ __forceinline__ void tma_load_all(const CUtensorMap* map, uint32_t dst, int x, int y, uint64_t* bar,
+                                             uint16_t mask) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
+        "[%0], [%1, {%2, %3}], [%4], %5;"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)), "h"(mask) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // K-major operand, 128-byte swizzle: 8-row groups of 1,024 bytes.
@@ -501,6 +522,11 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  ::"r"(smem_addr(bar)) : "memory");
 }
 
+__device__ __forceinline__ void mma_commit_all(uint64_t* bar, uint16_t mask) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_addr(bar)), "h"(mask) : "memory");
+}
+
 #define TMEM_LD32(v, addr)                                                                                   \
     asm volatile(                                                                                            \
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                            \
@@ -513,18 +539,22 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
           "=f"(v[29]), "=f"(v[30]), "=f"(v[31])                                                              \
         : "r"(addr))
 
+// Waits for the warp's TMEM loads; the values pass through, so that nothing
+// reads them before the wait.
+#define TMEM_WAIT32(v)                                                                                       \
+    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                            \
+        : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),    \
+          "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),           \
+          "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),         \
+          "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),         \
+          "+f"(v[29]), "+f"(v[30]), "+f"(v[31])                                                              \
+        :: "memory")
+
 __device__ __forceinline__ void tmem_fill32(uint32_t addr, uint32_t x) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
         "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};"
         ::"r"(addr), "r"(x) : "memory");
-}
-
-// A candidate, with its index among its row's candidates of the round.
-__device__ __forceinline__ void cand_put(const FilterArgs& a, unsigned long long at, uint32_t row, uint32_t col) {
-    if (at >= a.cap) return;
-    const uint32_t k = atomicAdd(a.rowcnt + row, 1u);
-    a.cand[at] = ((uint64_t)row << 40) | ((uint64_t)col << 20) | k;
 }
 
 // Candidates of one warp: kept in shared memory, written out in runs.
@@ -534,11 +564,69 @@ __device__ __forceinline__ void cand_flush(const FilterArgs& a, const uint2* buf
     if (lane == 0) base = atomicAdd(&a.ctl->cand[a.round], (unsigned long long)count);
     base = __shfl_sync(0xffffffffu, base, 0);
     for (int i = lane; i < count; i += 32)
-        cand_put(a, base + i, buf[i].x, buf[i].y);
+        if (base + i < a.cap) a.cand[base + i] = buf[i];
 }
 
-// One persistent block per SM over a fixed share of the items.  An item is
-// 128 row positions (a panel) against a run of 224-column tiles.  The rows'
+__device__ __forceinline__ float max3(float x, float y, float z) {
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(x), "f"(y), "f"(z));
+    return m;
+}
+
+// One 32 x 32 block of bounds: lane = row, v = 32 columns from c0 on.
+__device__ __forceinline__ void take_candidates(const FilterArgs& a, const float (&v)[32], float thr, int row,
+                                                int c0, uint2* buf, uint32_t* held, int lane) {
+    float mx[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        mx[g] = max3(v[8 * g], v[8 * g + 1], v[8 * g + 2]);
+        mx[g] = max3(mx[g], v[8 * g + 3], v[8 * g + 4]);
+        mx[g] = max3(mx[g], v[8 * g + 5], fmaxf(v[8 * g + 6], v[8 * g + 7]));
+    }
+    const bool hit = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) >= thr;
+    if (!__any_sync(0xffffffffu, hit)) return;
+    if (hit) {
+        uint32_t mask = 0;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            if (mx[g] >= thr) {
+#pragma unroll
+                for (int e = 8 * g; e < 8 * g + 8; ++e) mask |= v[e] >= thr ? 1u << e : 0u;
+            }
+        }
+        if (c0 + 32 > a.n) mask &= c0 < a.n ? (1u << (a.n - c0)) - 1u : 0u;
+        const int d = row - c0;        // only columns beyond the row
+        if (d >= 0) mask &= d >= 31 ? 0u : ~0u << (d + 1);
+        const uint32_t mine = (uint32_t)__popc(mask);
+        if (mine > 0) {
+            const uint32_t at = atomicAdd(held, mine);
+            unsigned long long out = 0;
+            if (at + mine > (uint32_t)kCandBuf) {   // no room: the rest goes straight out
+                const uint32_t room = at < (uint32_t)kCandBuf ? (uint32_t)kCandBuf - at : 0u;
+                out = atomicAdd(&a.ctl->cand[a.round], (unsigned long long)(mine - room));
+            }
+            for (uint32_t k = at; mask; mask &= mask - 1, ++k) {
+                const uint2 p = make_uint2((uint32_t)row, (uint32_t)(c0 + __ffs(mask) - 1));
+                if (k < (uint32_t)kCandBuf) buf[k] = p;
+                else if (out < a.cap) a.cand[out++] = p;
+            }
+        }
+    }
+    __syncwarp();
+    const uint32_t n = *reinterpret_cast<volatile uint32_t*>(held);
+    if (n > (uint32_t)kCandBuf / 2) {
+        cand_flush(a, buf, (int)min(n, (uint32_t)kCandBuf), lane);
+        __syncwarp();
+        if (lane == 0) *held = 0;
+        __syncwarp();
+    }
+}
+
+// One persistent block per SM.  All tiles, panel after panel, are cut into
+// segments of equal length, and each cluster takes every so-many-th segment:
+// the same number of tiles for everyone, from several places of the triangle
+// (items of 64 tiles dealt in turn left the SMs idle for 14 % of the run).
+// An item is 128 row positions (a panel) against a run of 224-column tiles.  The rows'
 // signatures stay in shared memory for the whole item (up to 1,024
 // dimensions; longer signatures stream rows and columns together), the
 // columns' pass through a ring of 128-byte-wide TMA boxes.  One thread
@@ -549,7 +637,7 @@ __device__ __forceinline__ void cand_flush(const FilterArgs& a, const uint2* buf
 // Bound: the 4-bit MMA rate (a 128 x 224 tile of 768 dimensions is 1,344
 // cycles at 16,384 multiply-adds a cycle); the compare costs about 20
 // instructions per 32 x 32 values unless one of them is a candidate.
-template <bool kResident>
+template <bool kResident, int kCluster>
 __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const FilterArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -559,17 +647,22 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     const int bytes_a = kResident ? a.chunks * kChunkA : 0;
     constexpr int kStage = kResident ? kChunkB : kChunkA + kChunkB;
     const uint32_t ring = smem0 + bytes_a;
-    uint8_t* tail = smem + bytes_a + a.stages * kStage;
+    uint8_t* tail = smem + bytes_a + 2 * a.depth * kStage;
     uint2* cbuf = reinterpret_cast<uint2*>(tail);
-    Bars* bars = reinterpret_cast<Bars*>(tail + 4 * kCandBuf * sizeof(uint2));
+    Bars* bars = reinterpret_cast<Bars*>(tail + kEpilogueWarps * kCandBuf * sizeof(uint2));
+    // the cluster's blocks take adjacent panels and the same column tiles
+    const int rank = kCluster > 1 ? (int)(blockIdx.x % kCluster) : 0;
+    const int first = (int)(blockIdx.x / kCluster), stride = (int)(gridDim.x / kCluster);
+    constexpr uint16_t kAll = (uint16_t)((1u << kCluster) - 1u);
     if (*reinterpret_cast<volatile uint32_t*>(&a.ctl->overflow)) return;   // an earlier round gave up
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < a.stages; ++s) { bar_init(&bars->full[s], 1); bar_init(&bars->empty[s], 1); }
+        for (int s = 0; s < 2 * a.depth; ++s) { bar_init(&bars->full[s], 1); bar_init(&bars->empty[s], kCluster); }
         bar_init(&bars->a_full, 1);
-        bar_init(&bars->a_empty, 1);
-        for (int b = 0; b < 2; ++b) { bar_init(&bars->acc_full[b], 1); bar_init(&bars->acc_empty[b], 4); }
-        bar_init(&bars->drain, 1);
+        bar_init(&bars->a_empty, 2);
+        for (int b = 0; b < 2; ++b) { bar_init(&bars->acc_full[b], 1); bar_init(&bars->acc_empty[b], kEpilogueWarps); }
+        bar_init(&bars->drain, 2);
+        for (int w = 0; w < kEpilogueWarps; ++w) bars->held[w] = 0;
         bars->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -583,7 +676,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = bars->tmem;
     const uint32_t scales = tmem + 2 * kCols;
-    if (warp >= 2) {
+    if (warp >= 3 && warp < 7) {
         // block scales: 2^0 everywhere (ue8m0 127)
         const uint32_t mine = scales + ((uint32_t)(32 * (warp & 3)) << 16);
         tmem_fill32(mine, 0x7F7F7F7Fu);
@@ -592,165 +685,167 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (kCluster > 1) cluster_sync();   // every block's barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t step = 0, item = 0, a_loads = 0;
+            // two rings of stages, for the even and the odd tiles: each ring
+            // has one consumer, which meets every phase of its barriers
+            uint32_t stage[2] = {0, 0}, phase[2] = {1, 1}, steps[2] = {0, 0};
+            uint32_t item = 0, a_loads = 0, tile = 0;
+            const uint32_t depth = (uint32_t)a.depth;
             bool ok = true;
-            for (int it = blockIdx.x; it < a.nitems && ok; it += gridDim.x, ++item) {
+            for (int sg = first; sg < a.nsegs && ok; sg += stride)
+            for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
                 const int4 q = __ldg(a.items + it);
+                const int row0 = kRows * (kCluster * q.x + rank);
                 if (kResident) {
-                    if (item > 0 && !bar_wait(&bars->a_empty, (item - 1) & 1, bars, a.ctl)) break;
+                    if (!bar_wait(&bars->a_empty, (item & 1) ^ 1, bars, a.ctl)) { ok = false; break; }
                     bar_expect(&bars->a_full, (uint32_t)bytes_a);
                     ++a_loads;
                     for (int k = 0; k < a.chunks; ++k)
-                        tma_load(&map_rows, smem0 + k * kChunkA, 128 * k, kRows * q.x, &bars->a_full);
+                        tma_load(&map_rows, smem0 + k * kChunkA, 128 * k, row0, &bars->a_full);
                 }
-                for (int t = q.y; t < q.z && ok; ++t) {
-                    for (int k = 0; k < a.chunks; ++k, ++step) {
-                        const uint32_t s = step % a.stages, use = step / a.stages;
-                        if (use > 0 && !bar_wait(&bars->empty[s], (use - 1) & 1, bars, a.ctl)) { ok = false; break; }
-                        bar_expect(&bars->full[s], kStage);
-                        const uint32_t dst = ring + s * kStage;
-                        if (!kResident) tma_load(&map_rows, dst + kChunkB, 128 * k, kRows * q.x, &bars->full[s]);
-                        tma_load(&map_cols, dst, 128 * k, kCols * t, &bars->full[s]);
+                for (int t = q.y; t < q.z && ok; ++t, ++tile) {
+                    const uint32_t g = tile & 1u;
+                    uint32_t st = stage[g], ph = phase[g];
+                    for (int k = 0; k < a.chunks; ++k) {
+                        const uint32_t slot = g * depth + st;
+                        if (!bar_wait(&bars->empty[slot], ph, bars, a.ctl)) { ok = false; break; }
+                        bar_expect(&bars->full[slot], kStage);
+                        ++steps[g];
+                        const uint32_t dst = ring + slot * kStage;
+                        if (!kResident) tma_load(&map_rows, dst + kChunkB, 128 * k, row0, &bars->full[slot]);
+                        if (kCluster == 1) {
+                            tma_load(&map_cols, dst, 128 * k, kCols * t, &bars->full[slot]);
+                        } else {
+                            // this block's share of the columns, to all
+                            constexpr int kPart = kCols / kCluster;
+                            tma_load_all(&map_cols, dst + rank * kPart * 128, 128 * k, kCols * t + rank * kPart,
+                                         &bars->full[slot], kAll);
+                        }
+                        if (++st == depth) { st = 0; ph ^= 1; }
                     }
+                    stage[g] = st;
+                    phase[g] = ph;
                 }
             }
             if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
                 // the block gives up: let the copies in flight land first
-                const unsigned long long t0 = now_ns();
-                for (int s = 0; s < a.stages; ++s) {
-                    const uint32_t uses = step / a.stages + (s < (int)(step % a.stages) ? 1 : 0);
-                    while (uses > 0 && !bar_try(&bars->full[s], (uses - 1) & 1) && now_ns() - t0 < kWaitNs) {}
-                }
-                while (a_loads > 0 && !bar_try(&bars->a_full, (a_loads - 1) & 1) && now_ns() - t0 < kWaitNs) {}
+                const long long t0 = clock64();
+                for (uint32_t g = 0; g < 2; ++g)
+                    for (uint32_t s = 0; s < depth; ++s) {
+                        const uint32_t uses = steps[g] / depth + (s < steps[g] % depth ? 1u : 0u);
+                        while (uses > 0 && !bar_try(&bars->full[g * depth + s], (uses - 1) & 1) &&
+                               clock64() - t0 < kWaitCycles) {}
+                    }
+                while (a_loads > 0 && !bar_try(&bars->a_full, (a_loads - 1) & 1) && clock64() - t0 < kWaitCycles) {}
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t step = 0, item = 0, tile = 0;
-            bool ok = true;
-            for (int it = blockIdx.x; it < a.nitems && ok; it += gridDim.x, ++item) {
-                const int4 q = __ldg(a.items + it);
-                if (kResident && !bar_wait(&bars->a_full, item & 1, bars, a.ctl)) break;
-                for (int t = q.y; t < q.z && ok; ++t, ++tile) {
-                    const uint32_t b = tile & 1, use = tile >> 1;
-                    if (use > 0 && !bar_wait(&bars->acc_empty[b], (use - 1) & 1, bars, a.ctl)) { ok = false; break; }
+    } else if (warp <= 2) {
+        // Two warps issue, one for each accumulator: an MMA costs its issuer
+        // about 70 cycles and a chunk's barrier and commit as much again,
+        // more than the 112 cycles it takes the tensor cores.  The whole warp
+        // runs the loop, so that its operands stay in uniform registers; one
+        // elected thread issues.
+        const uint32_t mine = (uint32_t)warp - 1u;
+        const uint32_t depth = (uint32_t)a.depth, slot0 = mine * depth;
+        uint32_t stage = 0, phase = 0, item = 0, tile = 0, bphase = 1;
+        bool ok = true;
+        const uint64_t desc_a = operand_desc(smem0), desc_b = operand_desc(ring + slot0 * kStage);
+        const uint32_t acc = tmem + mine * kCols;
+        for (int sg = first; sg < a.nsegs && ok; sg += stride)
+        for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
+            const int4 q = __ldg(a.items + it);
+            if (kResident && !bar_wait(&bars->a_full, item & 1, bars, a.ctl)) { ok = false; break; }
+            for (int t = q.y; t < q.z && ok; ++t, ++tile) {
+                if ((tile & 1u) != mine) continue;
+                if (!bar_wait(&bars->acc_empty[mine], bphase, bars, a.ctl)) { ok = false; break; }
+                bphase ^= 1;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int k = 0; k < a.chunks; ++k) {
+                    if (!bar_wait(&bars->full[slot0 + stage], phase, bars, a.ctl)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int k = 0; k < a.chunks; ++k, ++step) {
-                        const uint32_t s = step % a.stages, suse = step / a.stages;
-                        if (!bar_wait(&bars->full[s], suse & 1, bars, a.ctl)) { ok = false; break; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t bs = ring + s * kStage;
-                        const uint64_t da = operand_desc(kResident ? smem0 + k * kChunkA : bs + kChunkB);
-                        const uint64_t db = operand_desc(bs);
+                    const uint64_t db = desc_b + stage * (kStage >> 4);
+                    const uint64_t da = kResident ? desc_a + k * (kChunkA >> 4) : db + (kChunkB >> 4);
+                    if (elect_one()) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)   // 64 dimensions (32 bytes) each
-                            mma_mxf4(tmem + b * kCols, da + 2 * i, db + 2 * i, scales, scales + 32, k + i > 0);
-                        mma_commit(&bars->empty[s]);
+                            mma_mxf4(acc, da + 2 * i, db + 2 * i, scales, scales + 32, k + i > 0);
+                        if (kCluster == 1) mma_commit(&bars->empty[slot0 + stage]);
+                        else mma_commit_all(&bars->empty[slot0 + stage], kAll);
+                        if (k == a.chunks - 1) mma_commit(&bars->acc_full[mine]);
                     }
-                    if (ok) mma_commit(&bars->acc_full[b]);
+                    __syncwarp();
+                    if (++stage == depth) { stage = 0; phase ^= 1; }
                 }
-                if (ok && kResident) mma_commit(&bars->a_empty);
             }
-            if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
-                mma_commit(&bars->drain);
-                const unsigned long long t0 = now_ns();
-                while (!bar_try(&bars->drain, 0) && now_ns() - t0 < kWaitNs) {}
-            }
+            if (ok && kResident && elect_one()) mma_commit(&bars->a_empty);
+            __syncwarp();
+        }
+        if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
+            if (elect_one()) mma_commit(&bars->drain);
+            __syncwarp();
+            const long long t0 = clock64();
+            while (!bar_try(&bars->drain, 0) && clock64() - t0 < kWaitCycles) {}
         }
         __syncwarp();
     } else {
         const int part = warp & 3;                     // TMEM lanes 32 part .. 32 part + 31
-        uint2* mine = cbuf + (warp - 2) * kCandBuf;
-        int held = 0;
+        const int lead = (warp - 3) >> 2;              // its first 32-column step
+        uint2* mine = cbuf + (warp - 3) * kCandBuf;
+        uint32_t* held = &bars->held[warp - 3];
         uint32_t tile = 0;
         bool ok = true;
-        for (int it = blockIdx.x; it < a.nitems && ok; it += gridDim.x) {
+        for (int sg = first; sg < a.nsegs && ok; sg += stride)
+        for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it) {
             const int4 q = __ldg(a.items + it);
-            const int row = kRows * q.x + 32 * part + lane;
+            const int row = kRows * (kCluster * q.x + rank) + 32 * part + lane;
             const float rneed = row < a.n ? __ldg(a.need + row) : 1e9f;
             // half a count of slack: S is a multiple of 1/4
             const float rx = row < a.n ? (float)__ldg(a.excess + row) + 0.5f : 0.0f;
             for (int t = q.y; t < q.z; ++t, ++tile) {
                 const uint32_t b = tile & 1, use = tile >> 1;
+                const int c0 = kCols * t + 32 * lead;      // this warp's columns: 32 of every 32 kEpiPer
+                float need[kEpiSteps];
+#pragma unroll
+                for (int k = 0; k < kEpiSteps; ++k) {
+                    const int c = c0 + 32 * kEpiPer * k;
+                    need[k] = c < a.n && row < a.n ? fminf(rneed, __ldg(a.cmin + (c >> 5))) - rx : 1e9f;
+                }
                 if (!bar_wait(&bars->acc_full[b], use & 1, bars, a.ctl)) { ok = false; break; }
                 __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + b * kCols + ((uint32_t)(32 * part) << 16);
-#pragma unroll 1
-                for (int c = 0; c < kCols / 32; ++c) {
-                    const int c0 = kCols * t + 32 * c;
-                    float v[32];
-                    TMEM_LD32(v, acc + 32 * c);
-                    const float cm = c0 < a.n ? __ldg(a.cmin + (c0 >> 5)) : 1e9f;
-                    const float thr = row < a.n ? fminf(rneed, cm) - rx : 1e9f;
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    float mx[4];
+                const uint32_t acc = tmem + b * kCols + 32 * lead + ((uint32_t)(32 * part) << 16);
+                // one block of 32 columns on its way while the other is compared
+                float v[2][32];
+                TMEM_LD32(v[0], acc);
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        mx[g] = v[8 * g];
-#pragma unroll
-                        for (int e = 1; e < 8; ++e) mx[g] = fmaxf(mx[g], v[8 * g + e]);
-                    }
-                    const bool hit = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) >= thr;
-                    if (__any_sync(0xffffffffu, hit)) {
-                        uint32_t mask = 0;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) mask |= v[e] >= thr ? 1u << e : 0u;
-                        if (c0 + 32 > a.n) mask &= c0 < a.n ? (1u << (a.n - c0)) - 1u : 0u;
-                        const int d = row - c0;        // only columns beyond the row
-                        if (d >= 0) mask &= d >= 31 ? 0u : ~0u << (d + 1);
-                        const int mycount = __popc(mask);
-                        int x = mycount;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const int y = __shfl_up_sync(0xffffffffu, x, o);
-                            if (lane >= o) x += y;
+                for (int k = 0; k < kEpiSteps; ++k) {
+                    if (kEpiPer * k + lead < kCols / 32) {
+                        TMEM_WAIT32(v[k & 1]);
+                        if (kEpiPer * (k + 1) + lead < kCols / 32) {
+                            TMEM_LD32(v[(k + 1) & 1], acc + 32 * kEpiPer * (k + 1));
+                        } else {
+                            // the accumulator is free before the last compare
+                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(&bars->acc_empty[b]);
                         }
-                        const int total = __shfl_sync(0xffffffffu, x, 31);
-                        if (total > 0) {
-                            if (held + total > kCandBuf) {
-                                __syncwarp();
-                                cand_flush(a, mine, held, lane);
-                                __syncwarp();
-                                held = 0;
-                            }
-                            int at = held + x - mycount;
-                            if (total <= kCandBuf) {
-                                while (mask) {
-                                    const int e = __ffs(mask) - 1;
-                                    mask &= mask - 1;
-                                    mine[at++] = make_uint2((uint32_t)row, (uint32_t)(c0 + e));
-                                }
-                                held += total;
-                            } else {
-                                unsigned long long base = 0;
-                                if (lane == 0) base = atomicAdd(&a.ctl->cand[a.round], (unsigned long long)total);
-                                base = __shfl_sync(0xffffffffu, base, 0) + (unsigned)(x - mycount);
-                                while (mask) {
-                                    const int e = __ffs(mask) - 1;
-                                    mask &= mask - 1;
-                                    cand_put(a, base++, (uint32_t)row, (uint32_t)(c0 + e));
-                                }
-                            }
-                        }
+                        take_candidates(a, v[k & 1], need[k], row, c0 + 32 * kEpiPer * k, mine, held, lane);
                     }
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) bar_arrive(&bars->acc_empty[b]);
             }
         }
         __syncwarp();
-        cand_flush(a, mine, held, lane);
+        cand_flush(a, mine, (int)min(*reinterpret_cast<volatile uint32_t*>(held), (uint32_t)kCandBuf), lane);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (kCluster > 1) cluster_sync();   // no block leaves while another may still write to it
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
@@ -758,7 +853,8 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
 // ---- the exact count --------------------------------------------------------
 
 struct VerifyArgs {
-    const uint64_t* cand;
+    const uint2* cand;
+    uint32_t* candidx;        // index of a candidate among its row's
     uint2* sorted;            // (row, column), the candidates of a row together
     uint32_t* rowcnt;
     uint32_t* rowoff;
@@ -790,6 +886,14 @@ __device__ __forceinline__ bool round_fits(const VerifyArgs& a, unsigned long lo
     return false;
 }
 
+// Candidates per row, and each one's index among its row's.
+__global__ void __launch_bounds__(256) filter_count_kernel(const VerifyArgs a) {
+    const unsigned long long found = a.ctl->cand[a.round];
+    if (!round_fits(a, found)) return;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < found; i += gridDim.x * 256ull)
+        a.candidx[i] = atomicAdd(a.rowcnt + a.cand[i].x, 1u);
+}
+
 // A stretch of the sorted list for each row with candidates (rows in any
 // order: one atomic per warp); clears the counts for the next round.
 __global__ void __launch_bounds__(256) filter_rows_kernel(const VerifyArgs a) {
@@ -816,9 +920,8 @@ __global__ void __launch_bounds__(256) filter_scatter_kernel(const VerifyArgs a)
     const unsigned long long found = a.ctl->cand[a.round];
     if (!round_fits(a, found)) return;
     for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < found; i += gridDim.x * 256ull) {
-        const uint64_t v = a.cand[i];
-        const uint32_t row = (uint32_t)(v >> 40);
-        a.sorted[a.rowoff[row] + (uint32_t)(v & 0xFFFFFu)] = make_uint2(row, (uint32_t)(v >> 20) & 0xFFFFFu);
+        const uint2 p = a.cand[i];
+        a.sorted[a.rowoff[p.x] + a.candidx[i]] = p;
     }
 }
 
@@ -1036,7 +1139,7 @@ size_t kmer_filter_bytes(const int32_t* len, int n, int k) {
     }
     const int64_t read = (max_len / 16 + 5) * 4 + dims_for(tuples, n, k, kMostCut) / 2 + (most + 8) * 2 + 64;
     const int64_t pairs = (int64_t)n * (n + 512) / 2;
-    return (size_t)(n * read + tuples * 4 + candidate_room(pairs) * 16 + pairs / (kRows * kCols) * 16 + (1 << 20));
+    return (size_t)(n * read + tuples * 4 + candidate_room(pairs) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
 }
 
 // Rule: K >= 5 (K = 4 has 256 bins at most, and the bound leaves a third to
@@ -1181,49 +1284,88 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     }
     const int plo = k == 8 ? 0 : olo / kRows, phi = k == 8 ? panels : (ohi + kRows - 1) / kRows;
     int64_t work = 0;
-    auto first_tile = [&](int p) { return kRows * p / kCols; };
-    auto end_tile = [&](int p) { return pend.empty() ? tiles : (pend[p] + kCols - 1) / kCols; };
-    for (int p = plo; p < phi; ++p) work += end_tile(p) - first_tile(p);
-    // rounds of at most 2^33 pairs, items of at most 64 tiles and at least
-    // four items per SM where there are that many tiles
-    const int64_t pairs = work * kRows * kCols;
+    // groups of kCluster panels: from the first one's rows to the last one's end
+    const int glo = plo / kCluster, ghi = (phi + kCluster - 1) / kCluster;
+    auto first_tile = [&](int g) { return kRows * kCluster * g / kCols; };
+    auto end_tile = [&](int g) {
+        return pend.empty() ? tiles : (pend[std::min(panels, kCluster * (g + 1)) - 1] + kCols - 1) / kCols;
+    };
+    for (int g = glo; g < ghi; ++g) work += end_tile(g) - first_tile(g);
+    // rounds of at most 2^33 pairs; segments: four per cluster and round, at
+    // least one tile each
+    const int64_t pairs = work * kCluster * kRows * kCols;
     const int rounds = (int)std::min<int64_t>(kMaxRounds, std::max<int64_t>(1, (pairs + (1ll << 33) - 1) >> 33));
-    const int run = (int)std::max<int64_t>(1, std::min<int64_t>(64, work / (4ll * ctx->sm_count * rounds)));
+    const int64_t nclusters = ctx->sm_count / kCluster;
+    const int64_t nsegs = std::max<int64_t>(1, std::min<int64_t>(work, 4 * nclusters * rounds));
     std::vector<int4>& items = j.h_items;
+    std::vector<int>& segs = j.h_segs;
     items.clear();
-    for (int p = plo; p < phi; ++p)
-        for (int a = first_tile(p), e = end_tile(p); a < e; a += run) items.push_back(make_int4(p, a, std::min(e, a + run), 0));
+    segs.clear();
+    int64_t done = 0;
+    for (int g = glo; g < ghi; ++g) {
+        for (int a = first_tile(g), e = end_tile(g); a < e;) {
+            const int64_t seg = (int64_t)segs.size();
+            if (done == work * seg / nsegs) {
+                segs.push_back((int)items.size());
+                continue;
+            }
+            const int64_t left = work * seg / nsegs - done;   // tiles to the end of the open segment
+            const int c = (int)std::min<int64_t>(e - a, left);
+            items.push_back(make_int4(g, a, a + c, 0));
+            a += c;
+            done += c;
+        }
+    }
+    segs.push_back((int)items.size());
     if (items.empty()) return CRISPY_OK;
-    CRISPY_TRY(ensure(ctx, j.f_items, items.size() * sizeof(int4)));
-    CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+    const size_t item_bytes = items.size() * sizeof(int4);
+    CRISPY_TRY(ensure(ctx, j.f_items, item_bytes + segs.size() * sizeof(int)));
+    CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.ptr, items.data(), item_bytes, cudaMemcpyHostToDevice, s));
+    CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.as<char>() + item_bytes, segs.data(), segs.size() * sizeof(int),
+                                   cudaMemcpyHostToDevice, s));
     const int64_t ccap = candidate_room((pairs + rounds - 1) / rounds);
-    CRISPY_TRY(ensure(ctx, j.f_cand, (size_t)ccap * sizeof(uint64_t)));
+    CRISPY_TRY(ensure(ctx, j.f_cand, (size_t)ccap * sizeof(uint2)));
+    CRISPY_TRY(ensure(ctx, j.f_candidx, (size_t)ccap * 4));
     CRISPY_TRY(ensure(ctx, j.f_sorted, (size_t)ccap * sizeof(uint2)));
     CRISPY_TRY(ensure(ctx, j.f_rows, (size_t)n * 8));
     CRISPY_CK(ctx, cudaMemsetAsync(j.f_rows.ptr, 0, (size_t)n * 4, s));
 
     const int chunks = j.f_dims / 256;
     const bool resident = chunks <= kResidentChunks;
-    const size_t fixed = 1024 + 4 * kCandBuf * sizeof(uint2) + sizeof(Bars);
+    const size_t fixed = 1024 + kEpilogueWarps * kCandBuf * sizeof(uint2) + sizeof(Bars);
     const size_t bytes_a = resident ? (size_t)chunks * kChunkA : 0;
     const size_t stage = resident ? kChunkB : kChunkA + kChunkB;
-    const int stages = (int)std::min<size_t>(kMaxStages, (kSmemLimit - fixed - bytes_a) / stage);
-    const size_t smem = fixed + bytes_a + stages * stage;
-    auto kern = resident ? kmer_filter_kernel<true> : kmer_filter_kernel<false>;
+    const int depth = (int)std::min<size_t>(kMaxDepth, (kSmemLimit - fixed - bytes_a) / (2 * stage));
+    const size_t smem = fixed + bytes_a + 2 * depth * stage;
+    auto kern = resident ? kmer_filter_kernel<true, kCluster> : kmer_filter_kernel<false, kCluster>;
     CRISPY_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CUtensorMap map_rows, map_cols;
     CRISPY_TRY(signature_map(ctx, &map_rows, j.f_sig.ptr, j.f_dims / 2, n, kRows));
-    CRISPY_TRY(signature_map(ctx, &map_cols, j.f_sig.ptr, j.f_dims / 2, n, kCols));
+    CRISPY_TRY(signature_map(ctx, &map_cols, j.f_sig.ptr, j.f_dims / 2, n, kCols / kCluster));
+    // clusters the device holds at once (an odd SM of a cluster of SMs stays idle)
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kCluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(kFilterThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.gridDim = dim3(ctx->sm_count / kCluster * kCluster);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1)
+        clusters = ctx->sm_count / kCluster;
 
     FilterArgs fa{};
     fa.chunks = chunks;
-    fa.stages = stages;
+    fa.depth = depth;
     fa.n = n;
     fa.need = j.f_need.as<float>();
     fa.cmin = j.f_cmin.as<float>();
     fa.excess = j.f_excess.as<uint16_t>();
-    fa.cand = j.f_cand.as<uint64_t>();
-    fa.rowcnt = j.f_rows.as<uint32_t>();
+    fa.cand = j.f_cand.as<uint2>();
     fa.cap = (unsigned long long)ccap;
     fa.ctl = ctl;
     VerifyArgs va{};
@@ -1231,8 +1373,9 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     va.cap = fa.cap;
     va.ctl = ctl;
     va.sorted = j.f_sorted.as<uint2>();
-    va.rowcnt = fa.rowcnt;
-    va.rowoff = fa.rowcnt + n;
+    va.candidx = j.f_candidx.as<uint32_t>();
+    va.rowcnt = j.f_rows.as<uint32_t>();
+    va.rowoff = va.rowcnt + n;
     va.distinct = j.f_distinct.as<uint16_t>();
     va.dstride = j.f_dstride;
     va.meta = j.f_meta.as<int4>();
@@ -1258,18 +1401,21 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, filter_verify_kernel, kVerifyWarps * 32, vsmem);
     per_sm = std::max(1, per_sm);
     ev_begin(ctx, ctx->ev_kmer, s);
-    const int64_t ni = (int64_t)items.size();
+    fa.items = j.f_items.as<int4>();
+    const int cgrid = std::min((n + 63) / 64, ctx->sm_count * 8);
     for (int r = 0; r < rounds; ++r) {
-        const int64_t i0 = ni * r / rounds, i1 = ni * (r + 1) / rounds;
+        const int64_t i0 = nsegs * r / rounds, i1 = nsegs * (r + 1) / rounds;
         if (i1 <= i0) continue;
-        fa.items = j.f_items.as<int4>() + i0;
-        fa.nitems = (int)(i1 - i0);
+        fa.segs = reinterpret_cast<const int*>(j.f_items.as<char>() + item_bytes) + i0;
+        fa.nsegs = (int)(i1 - i0);
         fa.round = va.round = r;
-        kern<<<(unsigned)std::min<int64_t>(ctx->sm_count, i1 - i0), kFilterThreads, smem, s>>>(map_rows, map_cols, fa);
+        cfg.gridDim = dim3((unsigned)(kCluster * std::min<int64_t>(clusters, i1 - i0)));
+        CRISPY_CK(ctx, cudaLaunchKernelEx(&cfg, kern, map_rows, map_cols, fa));
+        filter_count_kernel<<<cgrid, 256, 0, s>>>(va);
         filter_rows_kernel<<<(n + 255) / 256, 256, 0, s>>>(va);
-        filter_scatter_kernel<<<std::min((n + 255) / 256, ctx->sm_count * 8), 256, 0, s>>>(va);
+        filter_scatter_kernel<<<cgrid, 256, 0, s>>>(va);
         filter_verify_kernel<<<ctx->sm_count * per_sm, kVerifyWarps * 32, vsmem, s>>>(va);
-        count_launch(ctx, 4);
+        count_launch(ctx, 5);
     }
     ev_end(ctx, ctx->ev_kmer, s);
     ctx->stats.kmer_launches += rounds;

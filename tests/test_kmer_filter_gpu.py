@@ -88,3 +88,21 @@ def test_filter_gives_up(engine, monkeypatch):
     # one centroid: nearly every pair is a candidate, more than the buffer holds
     reads = _reads(1800, 950, cents=1)
     assert _check(engine, monkeypatch, reads, 6, 0.3) > 300000
+
+
+@pytest.mark.parametrize("n,length", [(12000, 120), (12000, 250), (12000, 400), (9000, 550), (9000, 1100)])
+def test_filter_many_tiles(engine, monkeypatch, n, length):
+    # several tiles per block, so that every ring and both accumulators wrap
+    # (1 to 4 chunks with resident rows, more streamed), against the tile
+    # kernels, twice
+    reads = _reads(n, 960 + length, root=length + 20, dist="uniform", a=length - 20, b=length, cents=n // 40)
+    buf, offs, lens = synth.pack_reads(reads)
+    got = []
+    for on in ("0", "1", "1"):
+        monkeypatch.setenv("CRISPY_KMER_FILTER", on)
+        engine.kmer_prepare(buf, offs, lens, 6)
+        got.append(engine.kmer_fetch(engine.kmer_run(0.15, cg.MODE_BATCHED, True), True))
+    assert len(got[0][0]) > n
+    for pairs, d in got[1:]:
+        assert np.array_equal(pairs, got[0][0])
+        assert np.array_equal(d.view(np.uint32), got[0][1].view(np.uint32))
