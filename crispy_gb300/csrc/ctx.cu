@@ -220,6 +220,13 @@ int graph_run(crispy_ctx* ctx, cudaStream_t s, const std::string& key,
         ctx->stats.graph_launches++;
         return CRISPY_OK;
     }
+    // the first use of a key runs as it stands: capturing and instantiating
+    // costs more than one replay saves, and many keys hold a count that never
+    // comes again
+    if (ctx->graph_seen.insert(key).second) {
+        if (ctx->graph_seen.size() > 256) ctx->graph_seen = {key};
+        return enqueue();
+    }
     if (ctx->graphs.size() >= 64) graph_clear(ctx);
     const int64_t before = ctx->stats.kernels_launched;
     CRISPY_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));

@@ -488,13 +488,23 @@ __global__ void gen_flag_kernel(const float* __restrict__ dist, int64_t n, float
     flags[i] = (d < thr || (double)fabsf(__fsub_rn(d, thr)) < 0.00001) ? 1 : 0;
 }
 
+// Sort key of a distance ML / AL: 0 or at least 1 / 4,095, so the patterns of
+// the others start above 2^-13's and take 27 bits.
+constexpr uint32_t kDistBase = 0x39000000u;   // 2^-13
+constexpr int kDistBits = 27;
+__device__ __forceinline__ uint32_t dist_key(float d) {
+    const uint32_t u = __float_as_uint(d);
+    return u > kDistBase ? u - kDistBase : 0u;
+}
+__device__ __forceinline__ float key_dist(uint32_t k) { return __uint_as_float(k ? k + kDistBase : 0u); }
+
 __global__ void gen_keys_kernel(const float* __restrict__ dist, const uint32_t* __restrict__ surv,
                                 int64_t base, int64_t count, uint32_t* __restrict__ keys,
                                 uint32_t* __restrict__ vals) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const uint32_t p = surv[base + i];
-    keys[i] = __float_as_uint(dist[p]);
+    keys[i] = dist_key(dist[p]);
     vals[i] = p;
 }
 
@@ -508,7 +518,7 @@ __global__ void gen_gather_kernel(const int2* __restrict__ pairs, const uint32_t
     if (i >= count) return;
     const int2 pr = pairs[vals[i]];
     out_pairs[i] = make_uint2((uint32_t)(pr.x - pair_base), (uint32_t)(pr.y - pair_base));
-    out_dists[i] = __uint_as_float(keys[i]);
+    out_dists[i] = key_dist(keys[i]);
 }
 
 // Windowed runs: append one load window's survivors (pair, distance) to the
@@ -527,7 +537,7 @@ __global__ void gen_poskeys_kernel(const float* __restrict__ dist, int64_t count
                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    keys[i] = __float_as_uint(dist[i]);
+    keys[i] = dist_key(dist[i]);
     vals[i] = (uint32_t)i;
 }
 
@@ -577,6 +587,7 @@ static_assert(2 * kNumBins < 32, "order-bins overflow the 18-bit sort key");
 // (it sizes that kernel's tag storage), [kStatWindows + 2w] widest band-slot
 // bin of load window w (kNumBins = wide), [kStatWindows + 2w + 1] 1 when
 // the window holds a pair beyond the 16-bit range.
+constexpr int kOrderBits = 18;   // the sort key: order-bin << 13 | 8191 - sweep end
 constexpr int kStatBins = 2, kStatWindows = 32;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
@@ -844,7 +855,7 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         if (sorted) {
             uint32_t* sk = nullptr;
             CRISPY_TRY(sort_u32_payload(ctx, s, g.ckeys.as<uint32_t>(), g.ckeys_alt.as<uint32_t>(),
-                                        g.cvals.as<uint32_t>(), g.cvals_alt.as<uint32_t>(), count, 18, &sk,
+                                        g.cvals.as<uint32_t>(), g.cvals_alt.as<uint32_t>(), count, kOrderBits, &sk,
                                         &d_order, g.scan));
         }
         CRISPY_CK(ctx, cudaGetLastError());
@@ -857,9 +868,7 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
             (uint64_t)(uintptr_t)g.ckeys_alt.ptr, (uint64_t)(uintptr_t)g.cvals.ptr,
             (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr});
         CRISPY_TRY(graph_run(ctx, s, key, classify));
-        // where the 3-pass (18-bit) sort leaves the payload: the alternate
-        // buffer, or the input when there is nothing to sort
-        d_order = count > 1 ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
+        d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
     } else {
         CRISPY_TRY(classify());
     }
@@ -1079,9 +1088,8 @@ int gen_finish(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t npa
                                                   g.keys.as<uint32_t>(), g.vals.as<uint32_t>());
             count_launch(ctx);
             uint32_t *sk = nullptr, *sv = nullptr;
-            // distances lie in [0, 1]: sorted on their 32-bit patterns
             CRISPY_TRY(sort_u32_payload(ctx, s, g.keys.as<uint32_t>(), g.keys_alt.as<uint32_t>(),
-                                        g.vals.as<uint32_t>(), g.vals_alt.as<uint32_t>(), c, 32, &sk,
+                                        g.vals.as<uint32_t>(), g.vals_alt.as<uint32_t>(), c, kDistBits, &sk,
                                         &sv, g.scan));
             gen_gather_kernel<<<blocks, 256, 0, s>>>(d_pairs, sk, sv, c, g.out_pairs.as<uint2>(),
                                                     g.out_dists.as<float>(), pair_base);
@@ -1326,7 +1334,7 @@ int gen_run_windowed(crispy_ctx* ctx, cudaStream_t s, const int2* host_pairs, in
         uint32_t *sk = nullptr, *sv = nullptr;
         CRISPY_TRY(ensure(ctx, g.scan, sort_tmp_bytes(c)));
         CRISPY_TRY(sort_u32_payload(ctx, s, g.keys.as<uint32_t>(), g.keys_alt.as<uint32_t>(), g.vals.as<uint32_t>(),
-                                    g.vals_alt.as<uint32_t>(), c, 32, &sk, &sv, g.scan));
+                                    g.vals_alt.as<uint32_t>(), c, kDistBits, &sk, &sv, g.scan));
         gen_gather_kernel<<<blocks, 256, 0, s>>>(g.acc_pairs.as<int2>(), sk, sv, c, g.out_pairs.as<uint2>(),
                                                 g.out_dists.as<float>());
         count_launch(ctx);

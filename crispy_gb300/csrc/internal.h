@@ -10,6 +10,7 @@
 #include <new>
 #include <functional>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -166,6 +167,7 @@ struct crispy_ctx {
     crispy::PreJob pre;
     crispy::StreamEvents ev_kmer, ev_gen;
     std::map<std::string, crispy::GraphEntry> graphs;   // captured launch sequences
+    std::set<std::string> graph_seen;                    // keys that ran once, uncaptured
     bool use_graphs = true;
     // the batched k-mer run may tune its split per read set (off for the
     // server's contexts: every job is a new read set, and tuning one costs
@@ -200,8 +202,9 @@ double ev_sum_ms(StreamEvents& ev);
 void count_launch(crispy_ctx* ctx, int n = 1);
 
 // Run a launch sequence through a CUDA graph: the first call with a key
-// captures `enqueue` (which must only enqueue work on s: no host syncs, no
-// allocation) and instantiates it; later calls with the same key replay it.
+// enqueues it as it stands, the second captures `enqueue` (which must only
+// enqueue work on s: no host syncs, no allocation) and instantiates it; later
+// calls with the same key replay it.
 // The key must name every size and device address the sequence bakes in.
 int graph_run(crispy_ctx* ctx, cudaStream_t s, const std::string& key,
               const std::function<int()>& enqueue);
@@ -262,6 +265,8 @@ int gen_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, const st
 
 // radix sort / scan helpers (sort.cu)
 size_t sort_tmp_bytes(int64_t n);   // scratch a sort of n items needs
+// whether a sort leaves its result in the alternate buffers
+bool sort_lands_in_alt(int64_t n, int key_bits);
 int sort_u64_payload(crispy_ctx* ctx, cudaStream_t s, uint64_t* keys, uint64_t* keys_alt,
                      uint32_t* vals, uint32_t* vals_alt, int64_t n, int key_bits,
                      bool with_vals, uint64_t** sorted_keys, uint32_t** sorted_vals,

@@ -780,13 +780,14 @@ struct TileArgs {
     // of 128 positions; 128-row kernel, batched form): per item its job and
     // its end column group; per job (base, n, A, stage_dim) and its
     // threshold tables at mmin / smin + tbl[job]; survivors carry the job
-    // in key bits 44 and up and count per job in job_counter.
+    // in the key bits from tag_shift up and count per job in job_counter.
     const int* item_job;
     const int* item_cend;
     const int* item_cstart;   // first column group per item (nullptr: the row group's own)
     const int4* cjob;
     const int* ctbl;
     unsigned long long* job_counter;
+    int tag_shift;
 };
 
 // Parameters of the job a survivor belongs to (the whole run, or one job of
@@ -969,7 +970,7 @@ __device__ __forceinline__ void finish_half(const TileArgs& a, const EmitJob& ej
             mn = min(rowT[b], tc);
             pass = m >= (int)ej.mmin[mn];
         }
-        emit(a.counter, a.keys, a.vals, a.cap, ej.n, ej.A, ej.sd, a.perm, a.olo, a.ohi, pass, r, c, m, mn,
+        emit(a.counter, a.keys, a.vals, a.cap, ej.A, ej.sd, a.perm, a.olo, a.ohi, pass, r, c, m, mn,
              ej.base, ej.tag, ej.jcount);
     }
 }
@@ -1092,7 +1093,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) kmer_tile_kernel(TileArgs a) 
             ej.mmin = a.mmin + a.ctbl[jb];
             ej.smin = a.smin + a.ctbl[jb];
             ej.base = cj.x; ej.n = cj.y; ej.A = cj.z; ej.sd = cj.w;
-            ej.tag = (uint64_t)jb << 44;
+            ej.tag = (uint64_t)jb << a.tag_shift;
             ej.jcount = a.job_counter + jb;
         }
         __syncthreads();   // every thread has read s_item
@@ -1519,7 +1520,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) kmer_tile128_kernel(TileArgs 
             ej.mmin = a.mmin + a.ctbl[jb];
             ej.smin = a.smin + a.ctbl[jb];
             ej.base = cj.x; ej.n = cj.y; ej.A = cj.z; ej.sd = cj.w;
-            ej.tag = (uint64_t)jb << 44;
+            ej.tag = (uint64_t)jb << a.tag_shift;
             ej.jcount = a.job_counter + jb;
         }
         __syncthreads();   // every thread has read s_item
@@ -1858,7 +1859,7 @@ __device__ __forceinline__ void emit8(const TileArgs& a, const Rows8& rs, const 
             mn = min(rs.rowT[bit], tc);
             pass = m >= (int)a.mmin[mn];
         }
-        emit(a.counter, a.keys, a.vals, a.cap, a.n, a.A, a.stage_dim, a.perm, a.olo, a.ohi, pass, r, c, m, mn);
+        emit(a.counter, a.keys, a.vals, a.cap, a.A, a.stage_dim, a.perm, a.olo, a.ohi, pass, r, c, m, mn);
     }
 }
 
@@ -2290,7 +2291,7 @@ __global__ void __launch_bounds__(256) kmer_dense_kernel(DenseArgs a) {
                 mn = min(Tr, Tc);
                 pass = m >= (int)a.mmin[mn];
             }
-            emit(a.counter, a.keys, a.vals, a.cap, a.n, a.A, a.stage_dim, a.perm, a.olo, a.ohi, pass, r, c, m, mn);
+            emit(a.counter, a.keys, a.vals, a.cap, a.A, a.stage_dim, a.perm, a.olo, a.ohi, pass, r, c, m, mn);
         }
         __syncthreads();
         for (int p = threadIdx.x; p < Tr; p += blockDim.x) hist[kmer_at(s, p, a.K) >> 1] = 0;
@@ -2299,28 +2300,26 @@ __global__ void __launch_bounds__(256) kmer_dense_kernel(DenseArgs a) {
 }
 
 __global__ void kmer_decode_kernel(const uint64_t* __restrict__ keys,
-                                   const uint32_t* __restrict__ vals, int64_t count, int n,
+                                   const uint32_t* __restrict__ vals, int64_t count, int A, int sd,
                                    int2* __restrict__ pairs, float* __restrict__ dists) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    const uint64_t k = keys[i];
-    const uint64_t rc = k % ((uint64_t)n * (uint64_t)n);
-    pairs[i] = make_int2((int)(rc / (uint64_t)n), (int)(rc % (uint64_t)n));
+    pairs[i] = stage_pair(keys[i], A, sd);
     if (dists) dists[i] = __uint_as_float(vals[i]);
 }
 
-// Cohort survivors after the sort: job in key bits 44 and up, then the
-// job's own stage key; pairs come out at cohort positions (base added).
+// Cohort survivors after the sort: job in the key bits from tag_shift up,
+// then the job's own stage key; pairs come out at cohort positions (base
+// added).
 __global__ void kmer_decode_cohort_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-                                          int64_t count, const int4* __restrict__ cjob,
+                                          int64_t count, const int4* __restrict__ cjob, int tag_shift,
                                           int2* __restrict__ pairs, float* __restrict__ dists) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const uint64_t k = keys[i];
-    const int4 cj = cjob[(int)(k >> 44)];
-    const uint64_t n = (uint64_t)cj.y;
-    const uint64_t rc = (k & ((1ull << 44) - 1)) % (n * n);
-    pairs[i] = make_int2(cj.x + (int)(rc / n), cj.x + (int)(rc % n));
+    const int4 cj = cjob[(int)(k >> tag_shift)];
+    const int2 p = stage_pair(k & ((1ull << tag_shift) - 1), cj.z, cj.w);
+    pairs[i] = make_int2(cj.x + p.x, cj.x + p.y);
     if (dists) dists[i] = __uint_as_float(vals[i]);
 }
 
@@ -2848,7 +2847,6 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     j.f_pairs = j.f_found = 0;
     if (filter) CRISPY_TRY(kmer_filter_build(ctx, thr));
     const int sd = (n + A - 1) / A;
-    const int64_t nstages = (int64_t)sd * (sd + 1) / 2;
 
     std::vector<uint16_t> mmin, smin;
     build_mmin(thr, j.max_t, mmin, smin);
@@ -3191,7 +3189,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         return CRISPY_OK;
     };
     // stable order: (stage, row, col)
-    const int key_bits = bits_for((uint64_t)nstages * (uint64_t)n * (uint64_t)n);
+    const int key_bits = stage_key_bits(A, sd);
     auto sort_decode = [&]() -> int {
         uint64_t* sk = nullptr;
         uint32_t* sv = nullptr;
@@ -3200,7 +3198,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
                                     dists != 0, &sk, &sv, j.sort_tmp));
         if (j.nsurv > 0) {
             kmer_decode_kernel<<<(unsigned)((j.nsurv + 255) / 256), 256, 0, s>>>(
-                sk, sv, j.nsurv, n, j.pairs.as<int2>(), dists ? j.dists.as<float>() : nullptr);
+                sk, sv, j.nsurv, A, sd, j.pairs.as<int2>(), dists ? j.dists.as<float>() : nullptr);
             count_launch(ctx);
             CRISPY_CK(ctx, cudaGetLastError());
         }
@@ -3500,9 +3498,8 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
         tbl[c] = (int)mmin_all.size();
         mmin_all.insert(mmin_all.end(), mm.begin(), mm.end());
         smin_all.insert(smin_all.end(), sm.begin(), sm.end());
-        key_hi = std::max(key_hi, bits_for((uint64_t)sd * (sd + 1) / 2 * (uint64_t)q.n * (uint64_t)q.n));
+        key_hi = std::max(key_hi, stage_key_bits(A, sd));
     }
-    if (key_hi > 44) return fail(ctx, CRISPY_E_UNSUPPORTED, "cohort: stage keys of %d bits", key_hi);
     // row groups of each job, each over its own job's column groups; rows of
     // 32-read groups with too many high-level entries would need the dense
     // kernel, which the cohort form does not run
@@ -3589,6 +3586,7 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
     ta.cjob = reinterpret_cast<const int4*>(d + off_cj);
     ta.ctbl = reinterpret_cast<const int*>(d + off_tbl);
     ta.job_counter = reinterpret_cast<unsigned long long*>(d + off_cnt);
+    ta.tag_shift = key_hi;
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile, kTileThreads, tsmem);
     const int grid = (int)std::min<int64_t>((int64_t)std::max(1, per_sm) * ctx->sm_count, (int64_t)ni);
@@ -3618,11 +3616,11 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
     uint64_t* sk = nullptr;
     uint32_t* sv = nullptr;
     CRISPY_TRY(sort_u64_payload(ctx, s, j.keys.as<uint64_t>(), j.keys_alt.as<uint64_t>(), j.vals.as<uint32_t>(),
-                                j.vals_alt.as<uint32_t>(), j.nsurv, 44 + bits_for((uint64_t)nj), true, &sk, &sv,
+                                j.vals_alt.as<uint32_t>(), j.nsurv, key_hi + bits_for((uint64_t)nj), true, &sk, &sv,
                                 j.sort_tmp));
     if (j.nsurv > 0) {
         kmer_decode_cohort_kernel<<<(unsigned)((j.nsurv + 255) / 256), 256, 0, s>>>(
-            sk, sv, j.nsurv, ta.cjob, j.pairs.as<int2>(), j.dists.as<float>());
+            sk, sv, j.nsurv, ta.cjob, key_hi, j.pairs.as<int2>(), j.dists.as<float>());
         count_launch(ctx);
         CRISPY_CK(ctx, cudaGetLastError());
     }

@@ -9,14 +9,31 @@
 namespace crispy {
 namespace {
 
-__device__ __forceinline__ uint64_t stage_key(int r, int c, int n, int A, int sd) {
-    // kmerCUDA.cu:79-111 + Trag_reverse_eq (kmerMain.cpp:205-216): stages
-    // enumerate the upper triangle of the stageDim grid row-major; inside a
-    // stage the host scan is row-major (kmerMain.cpp:175-195).
-    const int64_t sx = r / A, sy = c / A;
-    const int64_t s = sx * sd - sx * (sx - 1) / 2 + (sy - sx);
-    return ((uint64_t)s * (uint64_t)n + (uint64_t)r) * (uint64_t)n + (uint64_t)c;
+// Bits of 0 .. v - 1.
+__host__ __device__ __forceinline__ int index_bits(int v) {
+    int b = 0;
+    while (b < 31 && (1 << b) < v) ++b;
+    return b;
 }
+
+// kmerCUDA.cu:79-111 + Trag_reverse_eq (kmerMain.cpp:205-216): stages
+// enumerate the upper triangle of the stageDim grid row-major; inside a stage
+// the host scan is row-major (kmerMain.cpp:175-195).  The key holds stage row,
+// stage column, row and column inside the stage, from the top, each in as
+// many bits as it needs: 36 bits at 100,000 reads, 42 at the most.
+__device__ __forceinline__ uint64_t stage_key(int r, int c, int A, int sd) {
+    const int ab = 32 - __clz(A - 1), sb = sd > 1 ? 32 - __clz(sd - 1) : 0;
+    const int sx = r / A, sy = c / A;
+    return ((((uint64_t)sx << sb) | (uint64_t)sy) << (2 * ab)) | ((uint64_t)(r - sx * A) << ab) |
+           (uint64_t)(c - sy * A);
+}
+__device__ __forceinline__ int2 stage_pair(uint64_t key, int A, int sd) {
+    const int ab = 32 - __clz(A - 1), sb = sd > 1 ? 32 - __clz(sd - 1) : 0;
+    const uint32_t am = (1u << ab) - 1u, sm = (1u << sb) - 1u;
+    return make_int2((int)(key >> (2 * ab + sb)) * A + (int)((uint32_t)(key >> ab) & am),
+                     (int)((uint32_t)(key >> (2 * ab)) & sm) * A + (int)((uint32_t)key & am));
+}
+inline int stage_key_bits(int A, int sd) { return 2 * index_bits(A) + 2 * index_bits(sd); }
 
 // Survivor emission with one atomic per warp.  All 32 lanes call it.
 // (r, c) are positions in the job's read order; with a read order (perm !=
@@ -24,7 +41,7 @@ __device__ __forceinline__ uint64_t stage_key(int r, int c, int n, int A, int sd
 // reordered so that the lower ID comes first, and only pairs whose lower ID
 // lies in [olo, ohi) are kept (the stage rows of one pass).
 __device__ __forceinline__ void emit(unsigned long long* counter, uint64_t* keys, uint32_t* vals,
-                                     int64_t cap, int n, int A, int sd, const int32_t* perm,
+                                     int64_t cap, int A, int sd, const int32_t* perm,
                                      int olo, int ohi, bool pass, int r, int c, int m, int mn,
                                      int base_pos = 0, uint64_t tag = 0, unsigned long long* jcount = nullptr) {
     if (perm != nullptr && pass) {
@@ -46,7 +63,7 @@ __device__ __forceinline__ void emit(unsigned long long* counter, uint64_t* keys
     if (pass) {
         const unsigned long long idx = base + __popc(pm & ((1u << lane) - 1u));
         if (idx < (unsigned long long)cap) {
-            keys[idx] = tag | stage_key(r - base_pos, c - base_pos, n, A, sd);
+            keys[idx] = tag | stage_key(r - base_pos, c - base_pos, A, sd);
             // kmerKernel.cu:47: 1.0f - (float)matches / min(T1, T2), IEEE
             const float d = __fsub_rn(1.0f, __fdiv_rn((float)m, (float)mn));
             vals[idx] = __float_as_uint(d);

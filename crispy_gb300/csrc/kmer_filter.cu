@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kVerifyWarps * 32) filter_verify_kernel(const 
             pass = lim != 0xFFFFu && (uint32_t)my_m >= lim;
             if (a.perm == nullptr) pass = pass && (int)rc.x >= a.olo && (int)rc.x < a.ohi;
         }
-        emit(a.counter, a.keys, a.vals, a.out_cap, a.n, a.A, a.sd, a.perm, a.olo, a.ohi, pass, (int)rc.x,
+        emit(a.counter, a.keys, a.vals, a.out_cap, a.A, a.sd, a.perm, a.olo, a.ohi, pass, (int)rc.x,
              (int)rc.y, my_m, my_mn);
     }
 }
