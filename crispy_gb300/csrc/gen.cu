@@ -569,11 +569,92 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 // Pairs are binned by band slots; bin 0 is the wide-band kernel.  Bins are
 // fine where bands are common (kBand 31-79 at band 10 on 300-800 nt reads)
 // so that few slots of a pair sit outside its band.
-constexpr int kBinSlots[] = {0, 8, 16, 32, 40, 48, 56, 64, 80, 96, 128, 192, 256};
+constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256};
 constexpr int kNumBins = sizeof(kBinSlots) / sizeof(kBinSlots[0]);
-__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 32, 40, 48, 56, 64, 80, 96, 128, 192, 256};
+__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256};
 // the sort key holds the order-bin (up to 2 * kNumBins) in 5 bits
 static_assert(2 * kNumBins < 32, "order-bins overflow the 18-bit sort key");
+
+// Which diagonals to sweep a pair over.  The narrow sweep -lo .. hi is the
+// whole band's result if its score is above 5 x the diagonal moves of any path
+// outside it (gen16.cu), that is if lo and hi exceed, by more than the length
+// difference on the longer read's side, a fifth of what the score falls short
+// of 5 x the shorter read.  0.4 of the shorter read's 8-mers that the longer
+// one lacks, and 3, is that in 99.8 % of the pairs (reads of 250, 400 and
+// 1,400 nt; a mismatch takes 9 from the score and about 8 8-mers), and leaves
+// 0.76 (99,999 reads of 300-500 nt, band 10), 0.74 (20,000 of 250 nt), 0.46
+// (band 5) and 0.28 (band 2) of the band's slots; at 0.35 it is 98 %, whose
+// second sweep costs more than the slots saved.  One warp
+// per pair: the longer read's 8-mers in a hashed bitmap, the shorter's looked
+// up in it.
+constexpr int kBandWarps = 8;
+constexpr int kBandBits = 14;
+__global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32_t* __restrict__ packed,
+                                                                    const int64_t* __restrict__ woff,
+                                                                    const int32_t* __restrict__ len,
+                                                                    const int2* __restrict__ pairs, int64_t count,
+                                                                    int band, uint32_t* __restrict__ bands) {
+    __shared__ __align__(16) uint32_t bitmap[kBandWarps][1 << (kBandBits - 5)];
+    const int lane = threadIdx.x & 31;
+    uint32_t* bm = bitmap[threadIdx.x >> 5];
+    const int64_t nw = (int64_t)gridDim.x * kBandWarps;
+    for (int64_t p = (int64_t)blockIdx.x * kBandWarps + (threadIdx.x >> 5); p < count; p += nw) {
+        const int2 pr = pairs[p];
+        const int l1 = len[pr.x], l2 = len[pr.y];
+        const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
+        const int gap = abs(l1 - l2);
+        int lo = kb, hi = kb;
+        // bands of up to 16 slots have nothing to save, nor have those that
+        // the smallest estimate fills
+        if (l1 + l2 <= kGen16MaxSum && kb >= 16 && gap + 6 < 2 * kb) {
+            const int rs = l1 <= l2 ? pr.x : pr.y, rl = l1 <= l2 ? pr.y : pr.x;
+            const int ts = min(l1, l2) - 7, tl = max(l1, l2) - 7;
+            for (int q = lane; q < 1 << (kBandBits - 7); q += 32)
+                reinterpret_cast<uint4*>(bm)[q] = make_uint4(0u, 0u, 0u, 0u);
+            __syncwarp();
+            const uint32_t* wl = packed + woff[rl];
+            for (int t = lane; t < tl; t += 32) {
+                const uint32_t v = __funnelshift_l(wl[(t >> 4) + 1], wl[t >> 4], 2 * (t & 15)) >> 16;
+                const uint32_t h = (v * 0x9E3779B1u) >> (32 - kBandBits);
+                atomicOr(&bm[h >> 5], 1u << (h & 31u));
+            }
+            __syncwarp();
+            const uint32_t* ws = packed + woff[rs];
+            int miss = 0;
+            for (int t = lane; t < ts; t += 32) {
+                const uint32_t v = __funnelshift_l(ws[(t >> 4) + 1], ws[t >> 4], 2 * (t & 15)) >> 16;
+                const uint32_t h = (v * 0x9E3779B1u) >> (32 - kBandBits);
+                miss += !((bm[h >> 5] >> (h & 31u)) & 1u);
+            }
+            miss = __reduce_add_sync(0xffffffffu, miss);
+            const int e = miss * 13 / 32 + 3;
+            lo = min(kb, e + max(0, l1 - l2));
+            hi = min(kb, e + max(0, l2 - l1));
+        }
+        if (lane == 0) bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+        __syncwarp();
+    }
+}
+
+// The same estimate from kmerDist's own count: of the shorter read's T K-mers
+// T * distance find no partner, so 8 / K times that stands for the 8-mers.
+__global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, const int2* __restrict__ pairs,
+                                           const float* __restrict__ kdist, int K, int64_t count, int band,
+                                           uint32_t* __restrict__ bands) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= count) return;
+    const int2 pr = pairs[p];
+    const int l1 = len[pr.x], l2 = len[pr.y];
+    const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
+    int lo = kb, hi = kb;
+    if (l1 + l2 <= kGen16MaxSum && kb >= 16) {
+        const float miss = kdist[p] * (float)(min(l1, l2) - K + 1);
+        const int e = (int)fminf(miss * 3.25f / (float)K, 4096.0f) + 3;
+        lo = min(kb, e + max(0, l1 - l2));
+        hi = min(kb, e + max(0, l2 - l1));
+    }
+    bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+}
 
 // Per-pair classification for the launch plan, on the device.  Order-bin
 // ob: band-slot bin b (1..12) for a pair the 16-bit kernel takes (L1 + L2
@@ -588,16 +669,20 @@ static_assert(2 * kNumBins < 32, "order-bins overflow the 18-bit sort key");
 // bin of load window w (kNumBins = wide), [kStatWindows + 2w + 1] 1 when
 // the window holds a pair beyond the 16-bit range.
 constexpr int kOrderBits = 18;   // the sort key: order-bin << 13 | 8191 - sweep end
-constexpr int kStatBins = 2, kStatWindows = 32;
+constexpr int kStatBins = 2, kStatWindows = 40;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
+// bands: the diagonals each pair is swept over (nullptr: all of its band);
+// list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
                                     const int32_t* __restrict__ len, int band, int nbins,
+                                    const uint32_t* __restrict__ bands, const uint32_t* __restrict__ list,
                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                     unsigned long long* __restrict__ stats) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const bool ok = p < count;
+    const bool ok = at < count;
+    const int64_t p = ok && list ? (int64_t)list[at] : at;
     unsigned long long cells = 0;
     int kb = 0, ob = -1, wb = -1, lng = 0;
     int sum_reg = 0;   // L1 + L2 of a pair for the register kernels' 16-bit form
@@ -605,21 +690,26 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         const int2 pr = pairs[p];
         const int l1 = len[pr.x], l2 = len[pr.y];
         kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
+        int lo = kb, hi = kb;
+        if (bands) {
+            lo = (int)(bands[p] & 0xFFFFu);
+            hi = (int)(bands[p] >> 16);
+        }
         int bin = 0;
         for (int b = 1; b < nbins; ++b)
-            if (c_bin_slots[b] >= kb + 1) { bin = b; break; }
+            if (c_bin_slots[b] >= (lo + hi) / 2 + 1) { bin = b; break; }
         lng = l1 + l2 > kGen16MaxSum ? 1 : 0;
         if (bin != 0 && !lng) sum_reg = l1 + l2;
         wb = bin == 0 ? nbins : bin;
         ob = bin == 0 ? 2 * nbins : bin + lng * nbins;   // wide pairs sort last
         if (keys) {
             int se = 0;
-            if (max(1, l2 - kb) <= min(l1, l2 + kb)) se = l2 + min(l1, l2 + kb);
-            if (max(1, l1 - kb) <= min(l2, l1 + kb)) se = max(se, l1 + min(l2, l1 + kb));
-            keys[p] = ((uint32_t)ob << 13) | (uint32_t)(8191 - min(se + (kb & 1), 8191));
-            vals[p] = (uint32_t)p;
+            if (max(1, l2 - hi) <= min(l1, l2 + lo)) se = l2 + min(l1, l2 + lo);
+            if (max(1, l1 - lo) <= min(l2, l1 + hi)) se = max(se, l1 + min(l2, l1 + hi));
+            keys[at] = ((uint32_t)ob << 13) | (uint32_t)(8191 - min(se + (lo & 1), 8191));
+            vals[at] = (uint32_t)p;
         }
-        cells = (unsigned long long)band_cells_of(l1, l2, band);
+        if (!list) cells = (unsigned long long)band_cells_of(l1, l2, band);
     }
     // one atomic per warp and counter: the counters are few and shared by
     // every pair, so per-pair atomics would serialise
@@ -633,7 +723,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     }
     const unsigned same_bin = __match_any_sync(0xffffffffu, ob);
     if (ok && lane == __ffs(same_bin) - 1) atomicAdd(&stats[kStatBins + ob], (unsigned long long)__popc(same_bin));
-    const int64_t win = ok ? p / CRISPY_GEN_WINDOW : -1;
+    const int64_t win = ok ? at / CRISPY_GEN_WINDOW : -1;
     const unsigned same_win = __match_any_sync(0xffffffffu, (unsigned long long)win);
     const int wbw = __reduce_max_sync(same_win, wb);   // max over the lanes of this window
     const int lw = __reduce_max_sync(same_win, lng);
@@ -643,7 +733,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     }
 }
 // untuned 32-bit shape per bin (the plain form always uses it)
-constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13};
+constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13};
 static_assert(kStatMaxSum16 < kStatWindows, "per-bin counters overlap the window slots");
 
 using WarpFn = void (*)(GenArgs);
@@ -707,11 +797,29 @@ int shape_slots(int shape) {
     return kShapes[shape].g * kShapes[shape].c;
 }
 // untuned 16-bit shape per bin (index into gen16's shapes), -1 = none
-constexpr int kDefault16[kNumBins] = {-1, 0, 1, 2, 4, 5, 7, 8, 9, 10, 11, 12, 13};
+constexpr int kDefault16[kNumBins] = {-1, 0, 1, 14, 2, 4, 5, 7, 8, 9, 10, 11, 12, 15, 13};
 int default_shape(int order_bin) {
     if (order_bin >= 1 && order_bin < kNumBins && kDefault16[order_bin] >= 0)
         return kNumShapes + kDefault16[order_bin];
     return kDefaultShape[order_bin > kNumBins ? order_bin - kNumBins : order_bin];
+}
+
+// Few pairs: the 16-bit shape with the most lanes per pair that still puts
+// every pair on the chip at once.  A step then costs its chain of dependent
+// instructions, and the fewer registers a lane holds the shorter that is
+// (about 70 cycles at 1 register, 150 at 7): 200 pairs of 250 nt 60 -> 33 us.
+// -1: enough pairs for the bin's own shape.
+int latency_shape(int order_bin, int64_t n_items, int sms) {
+    if (order_bin < 1 || order_bin >= kNumBins) return -1;
+    const int need = kBinSlots[order_bin];
+    int best = -1;
+    for (int i = 0; i < gen16_num_shapes(); ++i) {
+        const Shape16 h = gen16_shape(i);
+        if (2 * h.g * h.r < need || h.r > 2) continue;
+        if (n_items * h.g > 32ll * 12 * sms) continue;   // at most 12 warps per SM
+        if (best < 0 || h.r < gen16_shape(best).r || (h.r == gen16_shape(best).r && h.g < gen16_shape(best).g)) best = i;
+    }
+    return best < 0 ? -1 : kNumShapes + best;
 }
 
 // CRISPY_GEN_SHAPE=<index> makes the batched form run every bin the shape
@@ -749,7 +857,8 @@ __global__ void gather_stride_kernel(const uint32_t* __restrict__ src, int64_t n
 int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs& a,
                const uint32_t* d_order, int64_t n_items, DevBuf& sample_buf, DevBuf& queue_buf,
                DevBuf& dirs_buf, int* out) {
-    const int dflt = default_shape(bin);
+    const int few = latency_shape(bin, n_items, ctx->sm_count);
+    const int dflt = few >= 0 ? few : default_shape(bin);
     *out = dflt;
     if (!autotune_enabled() || n_items < 4096) return CRISPY_OK;
     const TuneKey key{band, bin, 0, ctx->sm_count};
@@ -793,6 +902,7 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
             t.count = want;
             t.dirs = dirs_buf.as<uint32_t>();
             t.dirs_words = dir_words;
+            t.retry = nullptr;   // a timing run proves nothing
             t.queue = queue_buf.as<unsigned int>() + (qslot++ % 64);
             CRISPY_CK(ctx, cudaMemsetAsync(t.queue, 0, 4, s));
             cudaEventRecord(e0, s);
@@ -822,21 +932,45 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
 
 }  // namespace
 
-// Launch plan for `count` pairs, computed on the device (no host pass over
-// the pairs): PLAIN = the thread-per-pair kernel per 589,824-pair load
-// window (as the reference launches per window, genCUDA.cu:156-209);
-// STAGED = the warp kernel per window, in the untuned shape the window's
-// widest pair needs; BATCHED = pairs sorted by band-slot bin and, inside a
-// bin, longest first, one persistent launch per bin on a device work
-// counter in the autotuned shape.
-int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count,
-                      int band, int mode, float* d_dist, int32_t* d_score, int32_t* d_ml,
-                      int32_t* d_al) {
+namespace {
+
+int launch_wide(crispy_ctx* ctx, const GenArgs& ga, int kbmax, const uint32_t* order, int64_t n_items,
+                cudaStream_t ls, bool timed) {
     GenJob& g = ctx->gen;
-    if (count <= 0) return CRISPY_OK;
+    const int rs = 2 * kbmax + 3;
+    const int threads = 128;
+    const int64_t want_threads = std::min<int64_t>(n_items, (int64_t)ctx->sm_count * 4 * threads);
+    const int blocks = (int)((want_threads + threads - 1) / threads);
+    CRISPY_TRY(ensure(ctx, g.buckets, (size_t)blocks * threads * rs * 6 * sizeof(int)));
+    WideArgs w{};
+    w.g = ga; w.g.order = order; w.g.count = n_items;
+    w.scratch = g.buckets.as<int>(); w.row_stride = rs;
+    if (timed) ev_begin(ctx, ctx->ev_gen, ls);
+    gen_wide_kernel<<<blocks, threads, 0, ls>>>(w);
+    if (timed) ev_end(ctx, ctx->ev_gen, ls);
+    count_launch(ctx);
+    ctx->stats.gen_launches++;
+    return CRISPY_OK;
+}
+
+// Whether a batched run sweeps narrow bands first: from about 1e9 band cells
+// (0.4 ms) on, where the saved slots outweigh the estimate, its read-back and
+// the second sweep's latency (about 100 us together; 7,000 pairs of 250 nt at
+// band 10 lost 180 us of 460).  CRISPY_GEN_NARROW=0 / 1 forces it off / on.
+bool narrow_pays(const GenJob& g, int64_t count, int band) {
+    if (const char* e = std::getenv("CRISPY_GEN_NARROW")) return e[0] != '0';
+    const double half = band >= 2 ? (double)g.max_len / band : (double)g.max_len;
+    return (double)count * half * g.max_len >= 5e8;
+}
+
+// Classification of `count` pairs (all, or those of `list`): statistics to
+// the host and, for the batched form, the launch order.
+int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count, int band, bool sorted,
+                 const uint32_t* bands, const uint32_t* list, std::vector<unsigned long long>& st,
+                 uint32_t** d_order) {
+    GenJob& g = ctx->gen;
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
     const int nstats = kStatWindows + 2 * (int)nwin;
-    const bool sorted = mode == CRISPY_MODE_BATCHED;
     CRISPY_TRY(ensure(ctx, g.cstats, (size_t)nstats * 8));
     if (sorted) {
         CRISPY_TRY(ensure(ctx, g.ckeys, (size_t)count * 4));
@@ -845,18 +979,17 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         CRISPY_TRY(ensure(ctx, g.cvals_alt, (size_t)count * 4));
     }
     unsigned long long* d_stats = g.cstats.as<unsigned long long>();
-    uint32_t* d_order = nullptr;
     auto classify = [&]() -> int {
         CRISPY_CK(ctx, cudaMemsetAsync(d_stats, 0, (size_t)nstats * 8, s));
         gen_classify_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-            d_pairs, count, g.len.as<int32_t>(), band, kNumBins,
+            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, bands, list,
             sorted ? g.ckeys.as<uint32_t>() : nullptr, sorted ? g.cvals.as<uint32_t>() : nullptr, d_stats);
         count_launch(ctx);
         if (sorted) {
-            uint32_t* sk = nullptr;
+            uint32_t *sk = nullptr, *sv = nullptr;
             CRISPY_TRY(sort_u32_payload(ctx, s, g.ckeys.as<uint32_t>(), g.ckeys_alt.as<uint32_t>(),
                                         g.cvals.as<uint32_t>(), g.cvals_alt.as<uint32_t>(), count, kOrderBits, &sk,
-                                        &d_order, g.scan));
+                                        &sv, g.scan));
         }
         CRISPY_CK(ctx, cudaGetLastError());
         return CRISPY_OK;
@@ -866,18 +999,22 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         const std::string key = "gclass," + key_of({(uint64_t)count, (uint64_t)band, (uint64_t)(uintptr_t)d_pairs,
             (uint64_t)(uintptr_t)g.len.ptr, (uint64_t)(uintptr_t)d_stats, (uint64_t)(uintptr_t)g.ckeys.ptr,
             (uint64_t)(uintptr_t)g.ckeys_alt.ptr, (uint64_t)(uintptr_t)g.cvals.ptr,
-            (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr});
+            (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr, (uint64_t)(uintptr_t)bands,
+            (uint64_t)(uintptr_t)list});
         CRISPY_TRY(graph_run(ctx, s, key, classify));
-        d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
+        *d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
     } else {
         CRISPY_TRY(classify());
     }
-    std::vector<unsigned long long> st(nstats);
+    st.resize(nstats);
     CRISPY_CK(ctx, cudaMemcpyAsync(st.data(), d_stats, (size_t)nstats * 8, cudaMemcpyDeviceToHost, s));
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
-    const int kbmax = (int)st[1];
-    ctx->stats.gen_cells += (int64_t)st[0];
-    ctx->stats.gen_pairs += count;
+    return CRISPY_OK;
+}
+
+GenArgs gen_base_args(crispy_ctx* ctx, const int2* d_pairs, int band, const std::vector<unsigned long long>& st,
+                      float* d_dist, int32_t* d_score, int32_t* d_ml, int32_t* d_al) {
+    GenJob& g = ctx->gen;
     GenArgs base{};
     for (int& o : base.one) o = 1;
     base.packed = g.packed.as<uint32_t>();
@@ -887,66 +1024,20 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
     base.band = band;
     base.dist = d_dist; base.score = d_score; base.ml = d_ml; base.al = d_al;
     base.dir_blocks = gen16_dir_blocks((int)st[kStatMaxSum16]);
-    auto launch_wide = [&](const GenArgs& ga, const uint32_t* order, int64_t n_items, cudaStream_t ls,
-                           bool timed) -> int {
-        const int rs = 2 * kbmax + 3;
-        const int threads = 128;
-        const int64_t want_threads = std::min<int64_t>(n_items, (int64_t)ctx->sm_count * 4 * threads);
-        const int blocks = (int)((want_threads + threads - 1) / threads);
-        CRISPY_TRY(ensure(ctx, g.buckets, (size_t)blocks * threads * rs * 6 * sizeof(int)));
-        WideArgs w{};
-        w.g = ga; w.g.order = order; w.g.count = n_items;
-        w.scratch = g.buckets.as<int>(); w.row_stride = rs;
-        if (timed) ev_begin(ctx, ctx->ev_gen, ls);
-        gen_wide_kernel<<<blocks, threads, 0, ls>>>(w);
-        if (timed) ev_end(ctx, ctx->ev_gen, ls);
-        count_launch(ctx);
-        ctx->stats.gen_launches++;
-        return CRISPY_OK;
-    };
-    if (mode == CRISPY_MODE_PLAIN || mode == CRISPY_MODE_STAGED) {
-        // tag storage for the windows the 16-bit kernel takes (one at a time)
-        int64_t dir_words = 0;
-        for (int64_t w = 0; mode == CRISPY_MODE_STAGED && w < nwin; ++w) {
-            const int wb = (int)st[kStatWindows + 2 * w];
-            const int sh = wb >= kNumBins ? -1 : default_shape(st[kStatWindows + 2 * w + 1] ? wb + kNumBins : wb);
-            if (sh >= 0 && is16(sh))
-                dir_words = std::max(dir_words, gen16_dir_words(ctx, sh - kNumShapes,
-                                                                std::min<int64_t>(CRISPY_GEN_WINDOW, count - w * CRISPY_GEN_WINDOW),
-                                                                base.dir_blocks));
-        }
-        if (dir_words) {
-            CRISPY_TRY(ensure(ctx, g.dirs, (size_t)dir_words * 4));
-            base.dirs = g.dirs.as<uint32_t>();
-            base.dirs_words = dir_words;
-        }
-        for (int64_t w = 0; w < nwin; ++w) {
-            const int64_t w0 = w * CRISPY_GEN_WINDOW;
-            const int64_t n_items = std::min<int64_t>(CRISPY_GEN_WINDOW, count - w0);
-            GenArgs a = base;
-            a.pairs = d_pairs + w0;
-            a.count = n_items;
-            a.dist = d_dist + w0;
-            a.score = d_score ? d_score + w0 : nullptr;
-            a.ml = d_ml ? d_ml + w0 : nullptr;
-            a.al = d_al ? d_al + w0 : nullptr;
-            const int wb = (int)st[kStatWindows + 2 * w];   // widest band-slot bin (kNumBins = wide)
-            const bool lng = st[kStatWindows + 2 * w + 1] != 0;
-            if (mode == CRISPY_MODE_PLAIN || wb >= kNumBins) {
-                CRISPY_TRY(launch_wide(a, nullptr, n_items, s, true));
-            } else {
-                CRISPY_TRY(launch_shape(ctx, s, default_shape(lng ? wb + kNumBins : wb), a, true));
-                ctx->stats.gen_launches++;
-            }
-        }
-        CRISPY_CK(ctx, cudaGetLastError());
-        return CRISPY_OK;
-    }
-    // BATCHED: bins in ascending width, wide last.  Every bin's shape is
-    // picked first (the autotuner times its samples alone on s); then the
-    // bins' persistent launches alternate between two side streams, so that
-    // a bin's tail (its last, shortest pairs on a few SMs) overlaps the next
-    // bin's start.  One event pair on s brackets them all.
+    return base;
+}
+
+constexpr int64_t kSmallBin = 4096;   // pairs
+
+// BATCHED: bins in ascending width, wide last.  Every bin's shape is picked
+// first (the autotuner times its samples alone on s); then the bins'
+// persistent launches alternate between two side streams, so that a bin's
+// tail (its last, shortest pairs on a few SMs) overlaps the next bin's start.
+// One event pair on s brackets them all.
+int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band, const uint32_t* d_order,
+                 const std::vector<unsigned long long>& st) {
+    GenJob& g = ctx->gen;
+    const int kbmax = (int)st[1];
     struct BinRun {
         int ob;
         int64_t at, n;
@@ -959,18 +1050,30 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         if (n_items == 0) continue;
         BinRun r{ob, at, n_items, -1};
         at += n_items;
-        if (ob != kWideOrderBin) {
-            GenArgs a = base;
-            a.order = d_order + r.at;
-            a.count = n_items;
-            CRISPY_TRY(pick_shape(ctx, s, band, ob, a, a.order, n_items, g.tune_sample, g.tune_queue, g.dirs,
-                                  &r.shape));
-            const int forced = forced_shape();
-            if (forced >= 0 && shape_slots(forced) >= kBinSlots[ob < kNumBins ? ob : ob - kNumBins] &&
-                !(is16(forced) && ob >= kNumBins))
-                r.shape = forced;
+        // a bin too small to fill the chip joins the next one of the same
+        // kernel, up to twice its slots: two short launches side by side cost
+        // more than one (1,300 and 5,200 pairs of 250 nt: 330 -> 230 us a run)
+        if (!runs.empty() && runs.back().n < kSmallBin && ob != kWideOrderBin &&
+            (runs.back().ob < kNumBins) == (ob < kNumBins)) {
+            const int a = runs.back().ob, base_bin = ob < kNumBins ? 0 : kNumBins;
+            if (kBinSlots[ob - base_bin] <= 2 * kBinSlots[a - base_bin]) {
+                r.at = runs.back().at;
+                r.n += runs.back().n;
+                runs.pop_back();
+            }
         }
         runs.push_back(r);
+    }
+    for (BinRun& r : runs) {
+        if (r.ob == kWideOrderBin) continue;
+        GenArgs a = base;
+        a.order = d_order + r.at;
+        a.count = r.n;
+        CRISPY_TRY(pick_shape(ctx, s, band, r.ob, a, a.order, r.n, g.tune_sample, g.tune_queue, g.dirs, &r.shape));
+        const int forced = forced_shape();
+        if (forced >= 0 && shape_slots(forced) >= kBinSlots[r.ob < kNumBins ? r.ob : r.ob - kNumBins] &&
+            !(is16(forced) && r.ob >= kNumBins))
+            r.shape = forced;
     }
     CRISPY_TRY(ensure(ctx, g.queue, 64 * 4));
     CRISPY_CK(ctx, cudaMemsetAsync(g.queue.ptr, 0, 64 * 4, s));   // one counter per order-bin (< 64)
@@ -990,7 +1093,7 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         const BinRun& r = runs[i];
         cudaStream_t ls = fork ? ctx->side[i & 1] : s;
         if (r.ob == kWideOrderBin) {
-            CRISPY_TRY(launch_wide(base, d_order + r.at, r.n, ls, false));
+            CRISPY_TRY(launch_wide(ctx, base, kbmax, d_order + r.at, r.n, ls, false));
             continue;
         }
         GenArgs a = base;
@@ -1011,6 +1114,105 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         }
     }
     ev_end(ctx, ctx->ev_gen, s);
+    CRISPY_CK(ctx, cudaGetLastError());
+    return CRISPY_OK;
+}
+
+}  // namespace
+
+// Launch plan for `count` pairs, computed on the device (no host pass over
+// the pairs): PLAIN = the thread-per-pair kernel per 589,824-pair load
+// window (as the reference launches per window, genCUDA.cu:156-209);
+// STAGED = the warp kernel per window, in the untuned shape the window's
+// widest pair needs; BATCHED = pairs sorted by band-slot bin and, inside a
+// bin, longest first, one persistent launch per bin on a device work
+// counter in the autotuned shape; large runs sweep each pair over the
+// diagonals it is likely to need first and the few pairs whose score does not
+// prove the result over the whole band after that.
+// kdist (may be nullptr): the pairs' K-mer distances at K = kdist_k.
+int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count,
+                      int band, int mode, float* d_dist, int32_t* d_score, int32_t* d_ml,
+                      int32_t* d_al, const float* kdist = nullptr, int kdist_k = 0) {
+    GenJob& g = ctx->gen;
+    if (count <= 0) return CRISPY_OK;
+    std::vector<unsigned long long> st;
+    uint32_t* d_order = nullptr;
+    if (mode == CRISPY_MODE_BATCHED) {
+        // (a forced shape sweeps whole bands, up to the shape's full width)
+        const bool narrow = forced_shape() < 0 && narrow_pays(g, count, band);
+        uint32_t *bands = nullptr, *retry = nullptr;
+        if (narrow) {
+            CRISPY_TRY(ensure(ctx, g.bands, (size_t)count * 4));
+            CRISPY_TRY(ensure(ctx, g.retry, (size_t)(count + 1) * 4));
+            bands = g.bands.as<uint32_t>();
+            retry = g.retry.as<uint32_t>();
+            CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));
+            if (kdist && kdist_k >= 5) {
+                gen_bands_from_kmer_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
+                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, count, band, bands);
+            } else {
+                const int blocks = (int)std::min<int64_t>((count + kBandWarps - 1) / kBandWarps, 8ll * ctx->sm_count);
+                gen_bands_kernel<<<blocks, kBandWarps * 32, 0, s>>>(g.packed.as<uint32_t>(), g.woff.as<int64_t>(),
+                                                                   g.len.as<int32_t>(), d_pairs, count, band, bands);
+            }
+            count_launch(ctx);
+        }
+        CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, true, bands, nullptr, st, &d_order));
+        ctx->stats.gen_cells += (int64_t)st[0];
+        ctx->stats.gen_pairs += count;
+        GenArgs base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
+        base.bands = bands;
+        base.retry = retry;
+        CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));
+        if (!narrow) return CRISPY_OK;
+        uint32_t left = 0;
+        CRISPY_CK(ctx, cudaMemcpyAsync(&left, retry, 4, cudaMemcpyDeviceToHost, s));
+        CRISPY_CK(ctx, cudaStreamSynchronize(s));
+        if (left == 0) return CRISPY_OK;
+        CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, nullptr, retry + 1, st, &d_order));
+        return gen_run_bins(ctx, s, gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al), band,
+                            d_order, st);
+    }
+    CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, nullptr, nullptr, st, &d_order));
+    const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
+    const int kbmax = (int)st[1];
+    ctx->stats.gen_cells += (int64_t)st[0];
+    ctx->stats.gen_pairs += count;
+    GenArgs base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
+    // tag storage for the windows the 16-bit kernel takes (one at a time)
+    int64_t dir_words = 0;
+    for (int64_t w = 0; mode == CRISPY_MODE_STAGED && w < nwin; ++w) {
+        const int wb = (int)st[kStatWindows + 2 * w];
+        const int sh = wb >= kNumBins ? -1 : default_shape(st[kStatWindows + 2 * w + 1] ? wb + kNumBins : wb);
+        if (sh >= 0 && is16(sh))
+            dir_words = std::max(dir_words, gen16_dir_words(ctx, sh - kNumShapes,
+                                                            std::min<int64_t>(CRISPY_GEN_WINDOW, count - w * CRISPY_GEN_WINDOW),
+                                                            base.dir_blocks));
+    }
+    if (dir_words) {
+        CRISPY_TRY(ensure(ctx, g.dirs, (size_t)dir_words * 4));
+        base.dirs = g.dirs.as<uint32_t>();
+        base.dirs_words = dir_words;
+    }
+    for (int64_t w = 0; w < nwin; ++w) {
+        const int64_t w0 = w * CRISPY_GEN_WINDOW;
+        const int64_t n_items = std::min<int64_t>(CRISPY_GEN_WINDOW, count - w0);
+        GenArgs a = base;
+        a.pairs = d_pairs + w0;
+        a.count = n_items;
+        a.dist = d_dist + w0;
+        a.score = d_score ? d_score + w0 : nullptr;
+        a.ml = d_ml ? d_ml + w0 : nullptr;
+        a.al = d_al ? d_al + w0 : nullptr;
+        const int wb = (int)st[kStatWindows + 2 * w];   // widest band-slot bin (kNumBins = wide)
+        const bool lng = st[kStatWindows + 2 * w + 1] != 0;
+        if (mode == CRISPY_MODE_PLAIN || wb >= kNumBins) {
+            CRISPY_TRY(launch_wide(ctx, a, kbmax, nullptr, n_items, s, true));
+        } else {
+            CRISPY_TRY(launch_shape(ctx, s, default_shape(lng ? wb + kNumBins : wb), a, true));
+            ctx->stats.gen_launches++;
+        }
+    }
     CRISPY_CK(ctx, cudaGetLastError());
     return CRISPY_OK;
 }
@@ -1486,7 +1688,7 @@ int crispy_gen_run_from_kmer(crispy_ctx* ctx, int band, float thr, int mode, cri
     } else if (npairs > 0) {
         CRISPY_TRY(ensure(ctx, g.dist, (size_t)npairs * 4));
         CRISPY_TRY(gen_dispatch_impl(ctx, s, k.pairs.as<int2>(), npairs, band, mode, g.dist.as<float>(),
-                                     nullptr, nullptr, nullptr));
+                                     nullptr, nullptr, nullptr, k.dists_kept ? k.dists.as<float>() : nullptr, k.k));
         CRISPY_TRY(gen_finish(ctx, s, k.pairs.as<int2>(), npairs, thr, sink, user, &ns,
                               mode == CRISPY_MODE_BATCHED));
     }
@@ -1532,7 +1734,8 @@ int gen_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, const st
     if (total > 0) {
         CRISPY_TRY(ensure(ctx, g.dist, (size_t)total * 4));
         CRISPY_TRY(gen_dispatch_impl(ctx, s, k.pairs.as<int2>(), total, band, CRISPY_MODE_BATCHED,
-                                     g.dist.as<float>(), nullptr, nullptr, nullptr));
+                                     g.dist.as<float>(), nullptr, nullptr, nullptr,
+                                     k.dists_kept ? k.dists.as<float>() : nullptr, k.k));
     }
     int64_t off = 0;
     for (size_t c = 0; c < jobs.size(); ++c) {

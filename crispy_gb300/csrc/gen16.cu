@@ -42,13 +42,29 @@
 // (genCPU.cpp:426-440: a diagonal adds 1 - hit to ML, a gap 1; AL counts
 // every move from the boundary cell's own AL = i0 + j0).
 //
+// Narrow sweeps.  A pair may be swept over diagonals -lo .. hi of its band
+// alone.  Let N be the most diagonal moves of any lattice path that touches a
+// diagonal of the band left out: min(L2, L1 - lo - 1) on the low side,
+// min(L1, L2 - hi - 1) on the high side.  A gap never gains and a diagonal
+// gains at most 5, so whatever reaches a cell by way of the outside has a
+// value of at most 5 x its diagonal moves.  If the narrow sweep's score is
+// above 5 N, its result is the whole band's: call a cell tainted if its value,
+// choice or chosen predecessor's taint differs between the two sweeps; by
+// induction along the anti-diagonals both its values are at most 5 x the
+// diagonal moves of some prefix by way of the outside (the larger of the two
+// maxima comes from the outside or from a tainted cell, and bounds the other).
+// No such value can reach the score: the score's cell and every cell of its
+// path are untainted, ties included, and every tainted cell of the last row
+// or column lies below it.  Pairs whose score does not prove this are listed
+// and swept again over the whole band.
+//
 // Layout.  G lanes per pair, R registers per lane: register r of lane l
 // holds slot l*R + r in its low half and slot G*R + l*R + r in its high
-// half.  Slot q hosts diagonal 2q - kBand + P at step parity P; its up /
+// half.  Slot q hosts diagonal 2q - lo + P at step parity P; its up /
 // left neighbours are slots q + 1 / q - 1 of the previous step, i.e.
 // registers r + 1 / r - 1 of the same lane, so only the lane's edge
 // register crosses lanes (one shuffle of keys per step).
-// Tags: step tau = s + (kBand & 1) (odd bands run one step late) lies in
+// Tags: step tau = s + (lo & 1) (odd starts run one step late) lies in
 // block b = tau / 16 at parity P = tau % 2; register r of lane l keeps the
 // block's tags of parity P in word ((2b + P) * G + l) * R + r of the pair's
 // region, the step's tag at bits 2 (7 - (tau % 16) / 2) of the half, so a
@@ -136,7 +152,8 @@ struct St {
 };
 
 struct Pair16 {
-    int kb, l1, l2, shift;   // shift = kb & 1: odd bands run one step late
+    int lo, hi;              // the diagonals swept: -lo .. hi
+    int l1, l2, shift;       // shift = lo & 1: odd starts run one step late
     // steps at which this lane may hold a last-row / last-column cell: four
     // windows of 2R steps (last row, then last column; low and high slots)
     int tw[4];
@@ -159,7 +176,7 @@ __device__ __forceinline__ void window32(const uint32_t* sm, int pos, uint32_t& 
 // Mismatch flags of 32 steps.  Parity-0 cells k = 0..15 of slot q compare
 // read1[j0 - 1 + k] with read2[i0 - 1 + k], parity-1 cells read1[j0 - 1 + k]
 // with read2[i0 + k], (i0, j0) = ((s0 + d0) / 2, (s0 - d0) / 2) the slot's
-// parity-0 cell at the set-up, d0 = 2q - kb.  The lane's R slots of a half
+// parity-0 cell at the set-up, d0 = 2q - lo.  The lane's R slots of a half
 // are consecutive, q = qb + r: read1 windows start at J - r, read2 windows
 // at I + r, all inside one 32-symbol window per read.  A flag sits at bit k
 // of its half (a mismatch: either plane differs).  A finished pair's caps
@@ -171,7 +188,7 @@ __device__ __forceinline__ void block_setup(St<R>& st, const uint32_t* sm1, cons
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int qb = (h * G + gl) * R;
-        const int d0 = 2 * qb - pc.kb;
+        const int d0 = 2 * qb - pc.lo;
         const int I = ((s0 + d0) >> 1) - 1, J = ((s0 - d0) >> 1) - 1;   // s0 + d0 is even
         uint32_t a0, a1, b0, b1;
         window32(sm1, J - (R - 1), a0, a1);   // read1 from J - (R-1): slot r at offset R-1-r
@@ -219,8 +236,8 @@ template <int G, int R, int P>
 __device__ __forceinline__ void boundary_slot(int d, const Pair16& pc, int gl, int* r, int* h) {
     *r = -1;
     *h = 0;
-    if (pc.l1 <= 0 || d < -pc.kb || d > pc.kb) return;   // no pair, or outside the band
-    const int q = (d + pc.kb - P) >> 1;
+    if (pc.l1 <= 0 || d < -pc.lo || d > pc.hi) return;   // no pair, or outside the band
+    const int q = (d + pc.lo - P) >> 1;
     const int rl = q - gl * R, rh = q - (G + gl) * R;
     if ((unsigned)rl < (unsigned)R) { *r = rl; *h = 0; }
     else if ((unsigned)rh < (unsigned)R) { *r = rh; *h = 1; }
@@ -263,11 +280,11 @@ template <int G, int R, int P>
 __device__ __forceinline__ void track16(const St<R>& st, int gl, int s, const Pair16& pc, Best16& col,
                                         Best16& row) {
     const int dr = 2 * pc.l2 - s, jr = s - pc.l2;
-    const int qr = (dr + pc.kb - P) >> 1;
+    const int qr = (dr + pc.lo - P) >> 1;
     const int dc = s - 2 * pc.l1, ic = s - pc.l1;
-    const int qc = (dc + pc.kb - P) >> 1;
-    const bool hr = jr >= 1 && jr <= pc.l1 && dr >= -pc.kb && dr <= pc.kb && mine(qr, gl, G, R);
-    const bool hc = ic >= 1 && ic <= pc.l2 && dc >= -pc.kb && dc <= pc.kb && mine(qc, gl, G, R);
+    const int qc = (dc + pc.lo - P) >> 1;
+    const bool hr = jr >= 1 && jr <= pc.l1 && dr >= -pc.lo && dr <= pc.hi && mine(qr, gl, G, R);
+    const bool hc = ic >= 1 && ic <= pc.l2 && dc >= -pc.lo && dc <= pc.hi && mine(qc, gl, G, R);
     if (hr) {
         const uint32_t key = take<G, R, P>(st, qr, gl);
         const int m = ((int)key - 31 - 4 * s - kBase) >> 2;
@@ -458,7 +475,7 @@ __device__ __forceinline__ void walk16(const uint32_t* region, uint32_t* stage, 
             const int blk = tau >> 4;
             if (blk < lo) break;   // the next window
             const int par = tau & 1;
-            const int q = (i - j + pc.kb - par) >> 1;
+            const int q = (i - j + pc.lo - par) >> 1;
             const int hi = q >= kGR ? 1 : 0;
             const int qq = min(max(q - hi * kGR, 0), kGR - 1);   // in range for every in-band cell
             // the half's tags of this parity at steps tau, tau - 2, ... from bit 0 up
@@ -523,25 +540,30 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
         const int64_t item = base + sub;
         const bool valid = item < a.count;
         int64_t p = -1;
-        Pair16 pc{0, 0, 0, 0, {INT_MIN / 2, INT_MIN / 2, INT_MIN / 2, INT_MIN / 2}};
+        Pair16 pc{0, 0, 0, 0, 0, {INT_MIN / 2, INT_MIN / 2, INT_MIN / 2, INT_MIN / 2}};
         int2 pr = make_int2(0, 0);
         if (valid) {
             p = a.order ? (int64_t)a.order[item] : item;
             pr = a.pairs[p];
             pc.l1 = a.len[pr.x];
             pc.l2 = a.len[pr.y];
-            pc.kb = kband16(pc.l1, pc.l2, a.band);
+            pc.lo = pc.hi = kband16(pc.l1, pc.l2, a.band);
+            if (a.bands) {
+                const uint32_t b = a.bands[p];
+                pc.lo = (int)(b & 0xFFFFu);
+                pc.hi = (int)(b >> 16);
+            }
         }
-        pc.shift = pc.kb & 1;
+        pc.shift = pc.lo & 1;
         if (valid) {
-            // last row i = l2: slot (2 l2 - s + kb - P) / 2 falls in [qa, qa + R) for
-            // s in [2 l2 + kb - 2 qa - 2R + 1, 2 l2 + kb - 2 qa]; last column j = l1:
-            // slot (s - 2 l1 + kb - P) / 2 for s in [2 l1 - kb + 2 qa, 2 l1 - kb + 2 qa + 2R - 1]
+            // last row i = l2: slot (2 l2 - s + lo - P) / 2 falls in [qa, qa + R) for
+            // s in [2 l2 + lo - 2 qa - 2R + 1, 2 l2 + lo - 2 qa]; last column j = l1:
+            // slot (s - 2 l1 + lo - P) / 2 for s in [2 l1 - lo + 2 qa, 2 l1 - lo + 2 qa + 2R - 1]
             const int qlo = gl * R, qhi = (G + gl) * R;
-            pc.tw[0] = 2 * pc.l2 + pc.kb - 2 * qlo - 2 * R + 1;
-            pc.tw[1] = 2 * pc.l2 + pc.kb - 2 * qhi - 2 * R + 1;
-            pc.tw[2] = 2 * pc.l1 - pc.kb + 2 * qlo;
-            pc.tw[3] = 2 * pc.l1 - pc.kb + 2 * qhi;
+            pc.tw[0] = 2 * pc.l2 + pc.lo - 2 * qlo - 2 * R + 1;
+            pc.tw[1] = 2 * pc.l2 + pc.lo - 2 * qhi - 2 * R + 1;
+            pc.tw[2] = 2 * pc.l1 - pc.lo + 2 * qlo;
+            pc.tw[3] = 2 * pc.l1 - pc.lo + 2 * qhi;
         }
         const int nw1 = (pc.l1 + 15) >> 4, nw2 = (pc.l2 + 15) >> 4;
         const uint32_t* g1 = a.packed + (valid ? a.woff[pr.x] : 0);
@@ -565,23 +587,23 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
         // the sweep ends at the last in-band cell of the last row or column
         int s_end = -1;
         if (valid) {
-            if (max(1, pc.l2 - pc.kb) <= min(pc.l1, pc.l2 + pc.kb)) s_end = pc.l2 + min(pc.l1, pc.l2 + pc.kb);
-            if (max(1, pc.l1 - pc.kb) <= min(pc.l2, pc.l1 + pc.kb))
-                s_end = max(s_end, pc.l1 + min(pc.l2, pc.l1 + pc.kb));
+            if (max(1, pc.l2 - pc.hi) <= min(pc.l1, pc.l2 + pc.lo)) s_end = pc.l2 + min(pc.l1, pc.l2 + pc.lo);
+            if (max(1, pc.l1 - pc.lo) <= min(pc.l2, pc.l1 + pc.hi))
+                s_end = max(s_end, pc.l1 + min(pc.l2, pc.l1 + pc.hi));
         }
         const int t_end = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(0, s_end + pc.shift));
         // the region holds dir_blocks blocks (sized on the host for the
         // launch's longest pair); a sweep that would not fit stores nothing
         // and reports ML = AL = -1
         const bool fits = (t_end >> 4) < a.dir_blocks;
-        const int clean_hi = 2 * min(pc.l1, pc.l2) - pc.kb - 1;
+        const int clean_hi = min(2 * pc.l2 - pc.hi, 2 * pc.l1 - pc.lo) - 1;
         constexpr int kBlock = kSteps;
         for (int t0 = 0; t0 <= t_end; t0 += kBlock) {
             const int s0 = t0 - pc.shift;
             const bool finished = s0 > s_end;
             if ((t0 & (kSetupSteps - 1)) == 0) block_setup<G, R>(st, sm1, sm2, gl, s0, pc, finished);
             uint32_t* dst = fits && !finished ? region + ((int64_t)(t0 >> 4) * 2 * G + gl) * R : nullptr;
-            const bool started = s0 > pc.kb;   // every boundary cell is behind (s = |d| <= kb)
+            const bool started = s0 > max(pc.lo, pc.hi);   // every boundary cell is behind (s = |d|)
             const bool clean = finished || (started && s0 + kBlock - 1 < clean_hi);
             if (__all_sync(0xffffffffu, clean))
                 block16<G, R, kClean>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
@@ -613,6 +635,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
             if (a.score) a.score[p] = b.m;
             if (a.ml) a.ml[p] = mlv;
             if (a.al) a.al[p] = alv;
+            if (a.retry) {
+                // most diagonal moves of any path that leaves the diagonals
+                // swept for another of the band
+                const int kb = kband16(pc.l1, pc.l2, a.band);
+                int most = INT_MIN / 8;
+                if (pc.lo < kb) most = min(pc.l1 - pc.lo - 1, pc.l2);
+                if (pc.hi < kb) most = max(most, min(pc.l2 - pc.hi - 1, pc.l1));
+                if (b.at < 0 || b.m <= 5 * most) a.retry[1 + atomicAdd(a.retry, 1u)] = (uint32_t)p;
+            }
         }
         __syncwarp();
         if (!a.queue) base += stride;
@@ -620,7 +651,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
 }
 
 constexpr Shape16 kShapes16[] = {{4, 1}, {4, 2}, {4, 4}, {8, 2}, {4, 5}, {4, 6}, {8, 3},
-                                 {4, 7}, {8, 4}, {8, 5}, {8, 6}, {16, 4}, {16, 6}, {32, 4}};
+                                 {4, 7}, {8, 4}, {8, 5}, {8, 6}, {16, 4}, {16, 6}, {32, 4},
+                                 {4, 3}, {16, 7}, {16, 1}, {16, 2}, {32, 1}, {32, 2}};
 constexpr int kNumShapes16 = sizeof(kShapes16) / sizeof(kShapes16[0]);
 constexpr bool shapes_within_max_r() {
     for (const Shape16& h : kShapes16)
@@ -645,7 +677,13 @@ Fn16 fn16(int i) {
         case 10: return gen16_kernel<8, 6>;
         case 11: return gen16_kernel<16, 4>;
         case 12: return gen16_kernel<16, 6>;
-        default: return gen16_kernel<32, 4>;
+        case 13: return gen16_kernel<32, 4>;
+        case 14: return gen16_kernel<4, 3>;
+        case 15: return gen16_kernel<16, 7>;
+        case 16: return gen16_kernel<16, 1>;
+        case 17: return gen16_kernel<16, 2>;
+        case 18: return gen16_kernel<32, 1>;
+        default: return gen16_kernel<32, 2>;
     }
 }
 

@@ -29,6 +29,11 @@ struct GenArgs {
     uint32_t* dirs;
     int64_t dirs_words;
     int dir_blocks;
+    // 16-bit kernel only: the diagonals each pair is swept over, -lo .. hi as
+    // lo | hi << 16 by pair index (nullptr: the whole band), and the pairs
+    // whose result that does not prove ([0] their count, then pair indices)
+    const uint32_t* bands;
+    uint32_t* retry;
     // All 1.  Adds written as multiply-adds by these run on the FMA pipe;
     // distinct multipliers keep the compiler from factoring a common
     // product back into ALU adds.
@@ -41,7 +46,8 @@ struct GenArgs {
 constexpr int kGen16MaxSum = 3600;
 
 // Shapes of the 16-bit kernel: G lanes per pair, R registers per lane, so
-// a pair with kBand + 1 <= 2 * G * R band slots fits.
+// a pair swept over diagonals -lo .. hi with (lo + hi) / 2 + 1 <= 2 * G * R
+// band slots fits.
 struct Shape16 {
     int g, r;
 };

@@ -89,6 +89,7 @@ struct KmerJob {
     // pinned host memory when they outgrow the device share
     int64_t nsurv = 0;
     bool have_dists = false;
+    bool dists_kept = false;   // dists holds them on the device, asked for or not
     bool spilled = false;
     HostBuf h_spill_pairs, h_spill_dists;
     DevBuf keys, keys_alt, vals, vals_alt, pairs, dists, counter, mmin, smin, work;
@@ -122,6 +123,7 @@ struct GenJob {
     DevBuf pairs, dist, score, ml, al, flags, scan, blocksum, surv_idx, keys, keys_alt,
         vals, vals_alt, out_pairs, out_dists, order, buckets, queue, err, tune_sample, tune_queue,
         cstats, ckeys, ckeys_alt, cvals, cvals_alt, acc_pairs, acc_dists;
+    DevBuf bands, retry;   // diagonals swept per pair; pairs to sweep again
     DevBuf dirs;   // the 16-bit DP's cell tags (two halves: one per concurrent bin launch)
     HostBuf h_pairs, h_dists;
 };

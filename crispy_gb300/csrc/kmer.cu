@@ -3190,15 +3190,18 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     };
     // stable order: (stage, row, col)
     const int key_bits = stage_key_bits(A, sd);
+    // (the batched form keeps the distances on the device in any case: they
+    // tell genDist which diagonals a pair is likely to need)
+    const bool keep_dists = dists != 0 || mode == CRISPY_MODE_BATCHED;
     auto sort_decode = [&]() -> int {
         uint64_t* sk = nullptr;
         uint32_t* sv = nullptr;
         CRISPY_TRY(sort_u64_payload(ctx, s, j.keys.as<uint64_t>(), j.keys_alt.as<uint64_t>(),
                                     j.vals.as<uint32_t>(), j.vals_alt.as<uint32_t>(), j.nsurv, key_bits,
-                                    dists != 0, &sk, &sv, j.sort_tmp));
+                                    keep_dists, &sk, &sv, j.sort_tmp));
         if (j.nsurv > 0) {
             kmer_decode_kernel<<<(unsigned)((j.nsurv + 255) / 256), 256, 0, s>>>(
-                sk, sv, j.nsurv, A, sd, j.pairs.as<int2>(), dists ? j.dists.as<float>() : nullptr);
+                sk, sv, j.nsurv, A, sd, j.pairs.as<int2>(), keep_dists ? j.dists.as<float>() : nullptr);
             count_launch(ctx);
             CRISPY_CK(ctx, cudaGetLastError());
         }
@@ -3210,7 +3213,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         CRISPY_TRY(ensure(ctx, j.dists, (size_t)std::max<int64_t>(j.nsurv, 1) * 4));
         CRISPY_TRY(ensure(ctx, j.sort_tmp, sort_tmp_bytes(j.nsurv)));
         if (mode == CRISPY_MODE_BATCHED && j.nsurv > 0) {
-            const std::string key = "ksort," + key_of({(uint64_t)j.nsurv, (uint64_t)key_bits, (uint64_t)dists,
+            const std::string key = "ksort," + key_of({(uint64_t)j.nsurv, (uint64_t)key_bits,
                 (uint64_t)n, (uint64_t)(uintptr_t)j.keys.ptr, (uint64_t)(uintptr_t)j.keys_alt.ptr,
                 (uint64_t)(uintptr_t)j.vals.ptr, (uint64_t)(uintptr_t)j.vals_alt.ptr,
                 (uint64_t)(uintptr_t)j.sort_tmp.ptr, (uint64_t)(uintptr_t)j.pairs.ptr, (uint64_t)(uintptr_t)j.dists.ptr});
@@ -3285,6 +3288,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         ctx->stats.kmer_spilled = 1;
     }
     j.have_dists = dists != 0;
+    j.dists_kept = keep_dists && !j.spilled;
     CRISPY_CK(ctx, cudaEventRecord(ctx->t_end, s));
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
     float tot = 0;
@@ -3625,7 +3629,7 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
         CRISPY_CK(ctx, cudaGetLastError());
     }
     j.spilled = false;
-    j.have_dists = true;
+    j.have_dists = j.dists_kept = true;
     counts.assign(jc.begin(), jc.end());
     CRISPY_CK(ctx, cudaEventRecord(ctx->t_end, s));
     CRISPY_CK(ctx, cudaStreamSynchronize(s));

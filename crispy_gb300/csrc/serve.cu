@@ -86,7 +86,7 @@ size_t estimate_base_bytes(const Job& j) {
     const size_t groups = (size_t)(j.n + 31) / 32;
     const size_t entries = (size_t)(2 * t + 32LL * (16 + 40) * groups) * 4 + (size_t)j.n * 136;
     const size_t survivors = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * 24;
-    const size_t gen = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * 48 + reads;
+    const size_t gen = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * 56 + reads;
     // the candidate filter's buffers, beside the entries a run that gives it
     // up needs as well
     const size_t filter = crispy::kmer_filter_bytes(j.len.data(), j.n, j.k);

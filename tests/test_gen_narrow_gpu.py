@@ -1,0 +1,113 @@
+"""Narrow sweeps of large batched genDist runs against the oracle.
+
+Large runs (CRISPY_GEN_NARROW=1: every run) sweep each pair over the diagonals
+it is likely to need and prove the result by its score, or sweep the whole
+band again.
+Score, ML, AL and distance must be the whole band's for similar reads (nearly
+all proved), for unrelated ones (nearly all swept again), for reads whose
+repeats make far diagonals score as well as the main one, at odd and even
+lengths and length differences on either side, and for bands from 10 to the
+unbanded alignment.
+"""
+import numpy as np
+import pytest
+
+import crispy_gb300 as cg
+import oracle
+from crispy_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def narrow(monkeypatch):
+    monkeypatch.setenv("CRISPY_GEN_NARROW", "1")
+
+
+def _check(engine, reads, pairs, bands):
+    buf, offs, lens = synth.pack_reads(reads)
+    engine.gen_prepare(buf, offs, lens)
+    for band in bands:
+        got = engine.gen_align(pairs, band, cg.MODE_BATCHED)
+        want = oracle.gen_all(buf, offs, lens, pairs, band)
+        for g, w in zip(got[1:], want[1:]):
+            bad = np.nonzero(g != w)[0]
+            assert len(bad) == 0, (band, pairs[bad[:4]].tolist(), g[bad[:4]], w[bad[:4]])
+        assert np.array_equal(got[0].view(np.uint32), want[0].view(np.uint32))
+
+
+def _random_pairs(n, m, seed):
+    return np.random.default_rng(seed).integers(0, n, (m, 2)).astype(np.int32)
+
+
+@pytest.mark.parametrize("spec", [
+    (120, 2, 260, "normal", 250, 30),        # one of two OTUs: similar pairs
+    (120, 60, 260, "uniform", 100, 260),     # mostly unrelated
+    (120, 3, 420, "uniform", 200, 400),      # length differences beyond the band
+    (120, 4, 90, "uniform", 1, 90),          # short
+])
+def test_narrow_read_sets(engine, spec):
+    n, cents, root, dist, a, b = spec
+    reads = synth.make_read_set(synth.ReadSetSpec(n, cents, root, dist, a, b, 6, 800 + cents))
+    _check(engine, reads, _random_pairs(len(reads), 4300, cents), (10, 5, 3, 2, 1))
+
+
+def test_narrow_repeats(engine):
+    # tandem repeats of 1 to 24 bases: shifting by a period costs only the
+    # overhang, so scores off the main diagonal come close to it
+    rng = np.random.default_rng(31)
+    reads = []
+    for i in range(160):
+        unit = rng.choice(np.frombuffer(b"ACGT", np.uint8), 1 + i % 24)
+        s = np.resize(unit, int(rng.integers(120, 300)))
+        for p in rng.integers(0, len(s), int(rng.integers(0, 6))):
+            s[p] = b"ACGT"[rng.integers(0, 4)]
+        reads.append(s.astype(np.uint8).tobytes())
+    same = np.array([[i, (i + 24 * k) % 160] for i in range(160) for k in range(1, 6)], np.int32)
+    pairs = np.concatenate([same, _random_pairs(160, 4100 - len(same) + 200, 32)])
+    _check(engine, reads, pairs, (10, 4, 2, 1))
+
+
+def test_narrow_planted_shifts(engine):
+    # copies with a stretch removed near one end: the path leaves the main
+    # diagonal by the stretch's length, within or beyond the estimate
+    rng = np.random.default_rng(33)
+    base = [rng.choice(np.frombuffer(b"ACGT", np.uint8), 300).tobytes() for _ in range(20)]
+    reads = list(base)
+    for k, s in enumerate(base):
+        for cut in (1, 2, 3, 5, 8, 13, 21, 34):
+            at = int(rng.integers(5, 250))
+            reads.append(s[:at] + s[at + cut:])
+            reads.append(s[cut:] + rng.choice(np.frombuffer(b"ACGT", np.uint8), cut).tobytes())
+    n = len(reads)
+    own = np.array([[k, 20 + 16 * k + c] for k in range(20) for c in range(16)], np.int32)
+    pairs = np.concatenate([own, own[:, ::-1], _random_pairs(n, 4200, 34)])
+    _check(engine, reads, pairs, (10, 5, 2))
+
+
+@pytest.mark.parametrize("k,thr", [(5, 0.3), (6, 0.45), (7, 0.5), (8, 0.5)])
+def test_narrow_from_kmer(engine, k, thr):
+    # the estimate from kmerDist's distances, close pairs and loose ones
+    reads = synth.make_read_set(synth.ReadSetSpec(500, 6, 320, "uniform", 150, 300, k, 840 + k))
+    buf, offs, lens = synth.pack_reads(reads)
+    engine.kmer_prepare(buf, offs, lens, k)
+    cnt = engine.kmer_run(thr, cg.MODE_BATCHED, False)
+    pairs, _ = engine.kmer_fetch(cnt, False)
+    assert cnt > 2000
+    engine.gen_prepare_from_kmer()
+    for band in (10, 5, 2):
+        d, _, _, _ = oracle.gen_all(buf, offs, lens, pairs, band)
+        want = oracle.gen_chunks(pairs, d, 0.2)
+        got = engine.gen_run_from_kmer(band, 0.2, cg.MODE_BATCHED)
+        assert len(got) == len(want)
+        for (ci, p, x), (wi, wp, wx) in zip(got, want):
+            assert ci == wi and np.array_equal(p, wp)
+            assert np.array_equal(x.view(np.uint32), wx.view(np.uint32))
+
+
+@pytest.mark.parametrize("count", [1, 7, 200, 1300, 1900, 2600, 3700])
+def test_few_pairs_shapes(engine, monkeypatch, count):
+    # runs of few pairs take the shapes with 16 and 32 lanes per pair
+    monkeypatch.setenv("CRISPY_GEN_NARROW", "0")
+    reads = synth.make_read_set(synth.ReadSetSpec(90, 5, 330, "uniform", 1, 330, 6, 850))
+    _check(engine, reads, _random_pairs(len(reads), count, count), (10, 5, 3, 2))
