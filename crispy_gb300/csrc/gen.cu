@@ -763,13 +763,13 @@ WarpFn shape_fn(int shape) {
 // Autotuner: for each bin of a batched run, every shape that covers the bin
 // without wasting more than half its slots is timed (CUDA events) on a
 // strided sample of the bin's pairs; the fastest is cached per (band, bin,
-// length bucket, SM count) for the life of the process.  Any shape gives the
+// narrow or whole sweeps, SM count) for the life of the process.  Any shape gives the
 // same bits, so tuning only picks speed.
 // ---------------------------------------------------------------------------
 struct TuneKey {
-    int band, bin, len_bucket, sms;   // bin = order-bin (above kNumBins: pairs beyond the 16-bit range)
+    int band, bin, narrow, sms;   // bin = order-bin (above kNumBins: pairs beyond the 16-bit range)
     bool operator<(const TuneKey& o) const {
-        return std::tie(band, bin, len_bucket, sms) < std::tie(o.band, o.bin, o.len_bucket, o.sms);
+        return std::tie(band, bin, narrow, sms) < std::tie(o.band, o.bin, o.narrow, o.sms);
     }
 };
 struct TuneEntry {
@@ -861,7 +861,9 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
     const int dflt = few >= 0 ? few : default_shape(bin);
     *out = dflt;
     if (!autotune_enabled() || n_items < 4096) return CRISPY_OK;
-    const TuneKey key{band, bin, 0, ctx->sm_count};
+    // narrow sweeps are tuned apart: only the 16-bit kernel knows them
+    const bool narrow = a.bands != nullptr;
+    const TuneKey key{band, bin, narrow ? 1 : 0, ctx->sm_count};
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tuned.find(key);
@@ -880,7 +882,7 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
     const int need = kBinSlots[bin < kNumBins ? bin : bin - kNumBins];
     auto candidate = [&](int sh) {
         const int slots = shape_slots(sh);
-        return slots >= need && slots <= 2 * need && !(is16(sh) && bin >= kNumBins);
+        return slots >= need && slots <= 2 * need && !(is16(sh) && bin >= kNumBins) && (is16(sh) || !narrow || bin >= kNumBins);
     };
     int64_t dir_words = 0;   // tag storage of the 16-bit candidates
     for (int sh = 0; sh < num_shapes_all(); ++sh)

@@ -111,3 +111,16 @@ def test_few_pairs_shapes(engine, monkeypatch, count):
     monkeypatch.setenv("CRISPY_GEN_NARROW", "0")
     reads = synth.make_read_set(synth.ReadSetSpec(90, 5, 330, "uniform", 1, 330, 6, 850))
     _check(engine, reads, _random_pairs(len(reads), count, count), (10, 5, 3, 2))
+
+
+def test_narrow_after_whole_bands_were_tuned(engine, monkeypatch):
+    # the shape tuned for a bin of whole bands may be the 32-bit kernel's,
+    # which sweeps nothing else; narrow sweeps have their own choice.  Short
+    # reads fill the small bins that longer reads' narrow sweeps fall into.
+    rng = np.random.default_rng(41)
+    short = [rng.choice(np.frombuffer(b"ACGT", np.uint8), int(rng.integers(30, 300))).tobytes() for _ in range(200)]
+    monkeypatch.setenv("CRISPY_GEN_NARROW", "0")
+    _check(engine, short, _random_pairs(200, 30000, 42), (10, 5))
+    monkeypatch.setenv("CRISPY_GEN_NARROW", "1")
+    reads = synth.make_read_set(synth.ReadSetSpec(150, 2, 330, "uniform", 290, 320, 6, 860))
+    _check(engine, reads, _random_pairs(len(reads), 20000, 43), (10, 5))
