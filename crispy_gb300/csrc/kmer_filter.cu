@@ -251,16 +251,21 @@ constexpr uint32_t kSlotEmpty = 0xFFFFFFFFu;
 // One warp per position.  Occurrence ranks come from a counter table in
 // shared memory: direct (two 16-bit counters per word) up to K = 6, an
 // open-addressing table (K-mer << 16 | count, load at most 1/2) above.
-// Repeats take the next free words of one array, whose size bounds them all.
+// Repeats take the next free words of one array, whose size bounds them all;
+// up to kStaged of a read's are collected on the way (a second pass over the
+// read's distinct K-mers for them cost as much as the first).
+constexpr int kStaged = 96;
 template <bool kDirect>
 __global__ void __launch_bounds__(kListWarps * 32) filter_lists_kernel(
     const uint32_t* __restrict__ packed, int stride, const int32_t* __restrict__ tcount,
     const int32_t* __restrict__ perm, int n, int K, int words, int hshift, uint16_t* __restrict__ distinct,
     int dstride, int4* __restrict__ meta, uint32_t* __restrict__ repeats, uint32_t* cursor) {
     extern __shared__ __align__(16) uint32_t tables[];
+    __shared__ uint32_t staged_all[kListWarps][kStaged];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* staged = staged_all[threadIdx.x >> 5];
     uint32_t* tbl = tables + (threadIdx.x >> 5) * words;
     const uint32_t blank = kDirect ? 0u : kSlotEmpty;
     const int nw = gridDim.x * kListWarps;
@@ -298,18 +303,26 @@ __global__ void __launch_bounds__(kListWarps * 32) filter_lists_kernel(
             if (rank == 0u) dst[nd + __popc(one & lt)] = (uint16_t)v;
             if (p0 == 0) first = __shfl_sync(full, v, __ffs(one) - 1);
             nd += __popc(one);
-            nr += __popc(__ballot_sync(full, p < T && rank != 0u));
+            const bool again = p < T && rank != 0u;
+            const unsigned rep = __ballot_sync(full, again);
+            if (again) {
+                const int k = nr + __popc(rep & lt);
+                if (k < kStaged) staged[k] = (rank << 16) | v;
+            }
+            nr += __popc(rep);
         }
         const int pad = (8 - (nd & 7)) & 7;
         if (lane < pad) dst[nd + lane] = (uint16_t)first;
         uint32_t at = 0;
         if (nr > 0) {
-            // the repeats: every distinct K-mer's counter says how many
             if (lane == 0) at = atomicAdd(cursor, (uint32_t)nr);
             at = __shfl_sync(full, at, 0);
             __syncwarp();
             uint32_t done = at;
-            for (int p0 = 0; p0 < nd; p0 += 32) {
+            if (nr <= kStaged)
+                for (int q = lane; q < nr; q += 32) repeats[at + q] = staged[q];
+            // more: every distinct K-mer's counter says how many it has
+            for (int p0 = 0; p0 < nd && nr > kStaged; p0 += 32) {
                 const int p = p0 + lane;
                 uint32_t v = 0, c = 0;
                 if (p < nd) {
@@ -930,77 +943,106 @@ constexpr int kVerifyWarps = 8;
 // Slots of the table of a row's repeats: a read of 400 nt has about 20 at
 // K = 6, one of 1,400 about 220.  Rows with more than half as many repeats
 // (long runs of few bases) search the row's list instead.
-int rep_slots_for(int max_t) { return max_t <= 512 ? 256 : 1024; }
+int rep_slots_for(int max_t) { return max_t <= 512 ? 256 : max_t <= 1536 ? 512 : 1024; }
 
 // A warp takes up to 32 consecutive candidates of the sorted list.  Per row
-// (about 4 to 30 candidates each) it sets the row's distinct K-mers in a
-// bitmap in shared memory and its repeats in a small table; per candidate it
-// streams the column's lists, eight K-mers to a 128-bit load, and tests each
-// K-mer with one shared load.  The bitmap is cleared through the row's list,
-// so its size (8 KB at K = 8) costs nothing per row.
-__global__ void __launch_bounds__(kVerifyWarps * 32) filter_verify_kernel(const VerifyArgs a) {
+// (about 4 to 30 candidates each) it marks the row's distinct K-mers in a map
+// in shared memory -- a byte each for short reads up to K = 6 (4 KB a warp; a
+// look-up is one load and one add), a bit each otherwise -- and puts its repeats in a small
+// table; per candidate it streams the column's lists, eight K-mers to a
+// 128-bit load, and looks each K-mer up.  The first words of the next
+// candidate are on their way while one is counted.  The map is cleared
+// through the row's list, so its size costs nothing per row.
+//
+// Bound: the look-ups' shared-memory wavefronts (about 3 per 32 random
+// addresses) and issue slots.
+template <bool kBytes, bool kK8>
+__global__ void __launch_bounds__(kVerifyWarps * 32, kK8 ? 3 : 5) filter_verify_kernel(const VerifyArgs a) {
     extern __shared__ __align__(16) uint32_t vsmem[];
     const unsigned full = 0xffffffffu;
     const unsigned long long found = a.ctl->cand[a.round];
     if (!round_fits(a, found)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bwords = 1 << (2 * a.K - 5);
+    const int mwords = kBytes ? 1 << (2 * a.K - 2) : 1 << (2 * a.K - 5);
     const uint32_t rmask = (uint32_t)a.rep_slots - 1u;
     const int rshift = __clz(a.rep_slots) + 1;      // 32 - log2(slots)
     const int rep_most = a.rep_slots / 2;
-    uint32_t* bm = vsmem + warp * (bwords + a.rep_slots);
-    uint32_t* rt = bm + bwords;
-    for (int q = lane; q < bwords; q += 32) bm[q] = 0;
+    uint32_t* map = vsmem + warp * (mwords + a.rep_slots);
+    uint8_t* mapb = reinterpret_cast<uint8_t*>(map);
+    uint32_t* rt = map + mwords;
+    for (int q = lane; q < mwords; q += 32) map[q] = 0;
     for (int q = lane; q < a.rep_slots; q += 32) rt[q] = kSlotEmpty;
     __syncwarp();
+    // the marks of a row's list set or taken back
+    auto mark = [&](const uint4* list, int nd, bool on) {
+        for (int q = lane; q < (nd + 7) / 8; q += 32) {
+            const uint4 e = list[q];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t w = k == 0 ? e.x : k == 1 ? e.y : k == 2 ? e.z : e.w;
+                if (kBytes) {
+                    mapb[w & 0xFFFFu] = on;
+                    mapb[w >> 16] = on;
+                } else if (on) {
+                    atomicOr(&map[(w & 0xFFFFu) >> 5], 1u << (w & 31u));
+                    atomicOr(&map[w >> 21], 1u << ((w >> 16) & 31u));
+                } else {
+                    map[(w & 0xFFFFu) >> 5] = 0;
+                    map[w >> 21] = 0;
+                }
+            }
+        }
+    };
     const int64_t total = (int64_t)found;
     const int64_t nw = (int64_t)gridDim.x * kVerifyWarps;
     const int batch = (int)min((int64_t)32, (total + nw - 1) / nw);
     int cur = -1;
     int4 mr = make_int4(0, 0, 0, 0);
-    const uint4* lr = nullptr;
     for (int64_t b0 = ((int64_t)blockIdx.x * kVerifyWarps + warp) * batch; b0 < total; b0 += nw * batch) {
         const int cnt = (int)min((int64_t)batch, total - b0);
         uint2 rc = make_uint2(0u, 0u);
-        int4 mine = make_int4(0, 0, 0, 0);
+        uint32_t sizes = 0, first_rep = 0;     // distinct K-mers | repeats << 16; first repeat
+        uint32_t lim = 0xFFFFu;                // smallest count that passes
         bool same = true, live = false;
         if (lane < cnt) {
             rc = a.sorted[b0 + lane];
-            mine = a.meta[rc.y];
-            live = true;
-            if (a.hkey != nullptr) {
-                // K = 8: reads of different H keys share no L half, and can
-                // pass only with an H-heavy read among them
+            const int4 m = a.meta[rc.y];
+            sizes = (uint32_t)m.x | (uint32_t)m.y << 16;
+            first_rep = (uint32_t)m.z;
+            lim = a.mmin[min(m.w, a.meta[rc.x].w)];
+            live = lim != 0xFFFFu;
+            if (kK8) {
+                // reads of different H keys share no L half, and can pass
+                // only with an H-heavy read among them
                 same = a.hkey[rc.x] == a.hkey[rc.y];
-                live = same || (a.heavy[rc.x] | a.heavy[rc.y]) != 0;
+                live = live && (same || (a.heavy[rc.x] | a.heavy[rc.y]) != 0);
             }
         }
         int my_m = 0, my_mn = 0;
-        for (unsigned todo = __ballot_sync(full, live); todo; todo &= todo - 1) {
-            const int i = __ffs(todo) - 1;
-            const int r = (int)__shfl_sync(full, rc.x, i), c = (int)__shfl_sync(full, rc.y, i);
+        unsigned todo = __ballot_sync(full, live);
+        int i = todo ? __ffs(todo) - 1 : 0;
+        uint32_t c = __shfl_sync(full, rc.y, i), sz = __shfl_sync(full, sizes, i);
+        uint4 head = make_uint4(0u, 0u, 0u, 0u);
+        if (kBytes && todo && 8 * lane < (int)(sz & 0xFFFFu))
+            head = reinterpret_cast<const uint4*>(a.distinct + (int64_t)c * a.dstride)[lane];
+        while (todo) {
+            todo &= todo - 1;
+            // the next candidate
+            const int i2 = todo ? __ffs(todo) - 1 : i;
+            const uint32_t c2 = __shfl_sync(full, rc.y, i2), sz2 = __shfl_sync(full, sizes, i2);
+            uint4 head2 = head;
+            if (kBytes && todo && 8 * lane < (int)(sz2 & 0xFFFFu))
+                head2 = reinterpret_cast<const uint4*>(a.distinct + (int64_t)c2 * a.dstride)[lane];
+            const int r = (int)__shfl_sync(full, rc.x, i);
             if (r != cur) {
-                if (cur >= 0) {     // take the last row's marks back
-                    for (int q = lane; q < (mr.x + 7) / 8; q += 32) {
-                        const uint4 e = lr[q];
-                        for (uint32_t w : {e.x, e.y, e.z, e.w}) {
-                            bm[(w & 0xFFFFu) >> 5] = 0;
-                            bm[w >> 21] = 0;
-                        }
-                    }
+                if (cur >= 0) {
+                    mark(reinterpret_cast<const uint4*>(a.distinct + (int64_t)cur * a.dstride), mr.x, false);
                     if (mr.y > 0) for (int q = lane; q < a.rep_slots; q += 32) rt[q] = kSlotEmpty;
                     __syncwarp();
                 }
                 cur = r;
                 mr = a.meta[r];
-                lr = reinterpret_cast<const uint4*>(a.distinct + (int64_t)r * a.dstride);
-                for (int q = lane; q < (mr.x + 7) / 8; q += 32) {
-                    const uint4 e = lr[q];
-                    for (uint32_t w : {e.x, e.y, e.z, e.w}) {
-                        atomicOr(&bm[(w & 0xFFFFu) >> 5], 1u << (w & 31u));
-                        atomicOr(&bm[w >> 21], 1u << ((w >> 16) & 31u));
-                    }
-                }
+                mark(reinterpret_cast<const uint4*>(a.distinct + (int64_t)r * a.dstride), mr.x, true);
                 if (mr.y <= rep_most) {
                     for (int q = lane; q < mr.y; q += 32) {
                         const uint32_t e = a.repeats[mr.z + q];
@@ -1010,21 +1052,26 @@ __global__ void __launch_bounds__(kVerifyWarps * 32) filter_verify_kernel(const 
                 }
                 __syncwarp();
             }
-            const int nd = __shfl_sync(full, mine.x, i), nr = __shfl_sync(full, mine.y, i);
-            const int rep = __shfl_sync(full, mine.z, i), tc = __shfl_sync(full, mine.w, i);
+            const int nd = (int)(sz & 0xFFFFu), nr = (int)(sz >> 16);
             // K = 8, different keys: only the K-mers >= 0x8000 (H) count
-            const bool both = __shfl_sync(full, (int)same, i) != 0;
-            const uint4* lc = reinterpret_cast<const uint4*>(a.distinct + (int64_t)c * a.dstride);
+            const bool both = !kK8 || __shfl_sync(full, (int)same, i) != 0;
             const int nq = (nd + 7) / 8;
-            int m = 0;
+            uint32_t m = 0;
             for (int q = lane; q < nq; q += 32) {
-                const uint4 e = lc[q];
+                const uint4 e = kBytes && q == lane ? head
+                                                    : reinterpret_cast<const uint4*>(a.distinct + (int64_t)c * a.dstride)[q];
                 uint32_t hits = 0, first = 0;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint32_t w = k == 0 ? e.x : k == 1 ? e.y : k == 2 ? e.z : e.w;
-                    uint32_t lo = (bm[(w & 0xFFFFu) >> 5] >> (w & 31u)) & 1u;
-                    uint32_t hi = (bm[w >> 21] >> ((w >> 16) & 31u)) & 1u;
+                    uint32_t lo, hi;
+                    if (kBytes) {
+                        lo = mapb[w & 0xFFFFu];
+                        hi = mapb[w >> 16];
+                    } else {
+                        lo = (map[(w & 0xFFFFu) >> 5] >> (w & 31u)) & 1u;
+                        hi = (map[w >> 21] >> ((w >> 16) & 31u)) & 1u;
+                    }
                     if (!both) {
                         lo &= w >> 15;
                         hi &= w >> 31;
@@ -1032,33 +1079,42 @@ __global__ void __launch_bounds__(kVerifyWarps * 32) filter_verify_kernel(const 
                     if (k == 0) first = lo;
                     hits += lo + hi;
                 }
-                m += (int)hits;
+                m += hits;
                 // the padding: copies of the list's first K-mer
-                if (q == 0) m -= (int)first * (8 * nq - nd);
+                if (q == 0) m -= first * (uint32_t)(8 * nq - nd);
             }
-            for (int q = lane; q < nr; q += 32) {
-                const uint32_t e = a.repeats[rep + q];
-                if (!both && !(e & 0x8000u)) continue;
-                if (mr.y <= rep_most) {
-                    uint32_t h = (e * 0x9E3779B1u) >> rshift;
-                    uint32_t v;
-                    while ((v = rt[h]) != kSlotEmpty && v != e) h = (h + 1u) & rmask;
-                    m += v == e;
-                } else {
-                    for (int k = 0; k < mr.y; ++k)
-                        if (a.repeats[mr.z + k] == e) { ++m; break; }
-                }
-            }
+            // the repeats only where they can still lift the count over the cut
             m = __reduce_add_sync(full, m);
-            if (lane == i) {
-                my_m = m;
-                my_mn = min(mr.w, tc);
+            if (nr > 0 && m + (uint32_t)min(nr, mr.y) >= __shfl_sync(full, lim, i)) {
+                const uint32_t rep = __shfl_sync(full, first_rep, i);
+                uint32_t more = 0;
+                for (int q = lane; q < nr; q += 32) {
+                    const uint32_t e = a.repeats[rep + q];
+                    if (!both && !(e & 0x8000u)) continue;
+                    if (mr.y <= rep_most) {
+                        uint32_t h = (e * 0x9E3779B1u) >> rshift;
+                        uint32_t v;
+                        while ((v = rt[h]) != kSlotEmpty && v != e) h = (h + 1u) & rmask;
+                        more += v == e;
+                    } else {
+                        for (int k = 0; k < mr.y; ++k)
+                            if (a.repeats[mr.z + k] == e) { ++more; break; }
+                    }
+                }
+                m += __reduce_add_sync(full, more);
             }
+            if (lane == i) {
+                my_m = (int)m;
+                my_mn = min(mr.w, nd + nr);
+            }
+            i = i2;
+            c = c2;
+            sz = sz2;
+            head = head2;
         }
         bool pass = false;
         if (live) {
-            const uint32_t lim = a.mmin[my_mn];
-            pass = lim != 0xFFFFu && (uint32_t)my_m >= lim;
+            pass = (uint32_t)my_m >= lim;
             if (a.perm == nullptr) pass = pass && (int)rc.x >= a.olo && (int)rc.x < a.ohi;
         }
         emit(a.counter, a.keys, a.vals, a.out_cap, a.A, a.sd, a.perm, a.olo, a.ohi, pass, (int)rc.x,
@@ -1127,7 +1183,8 @@ int dims_for(int64_t tuples, int n, int k, float thr) {
 }
 }  // namespace
 
-// Device bytes the filter's buffers take for reads of these lengths.
+// Device bytes the filter's buffers take for reads of these lengths (and
+// genDist's copy of the packed reads).
 size_t kmer_filter_bytes(const int32_t* len, int n, int k) {
     if (k < 5 || n <= 0) return 0;
     int64_t tuples = 0, most = 0, max_len = 0;
@@ -1137,7 +1194,7 @@ size_t kmer_filter_bytes(const int32_t* len, int n, int k) {
         most = std::max(most, t);
         max_len = std::max<int64_t>(max_len, len[r]);
     }
-    const int64_t read = (max_len / 16 + 5) * 4 + dims_for(tuples, n, k, kMostCut) / 2 + (most + 8) * 2 + 64;
+    const int64_t read = 2 * (max_len / 16 + 5) * 4 + dims_for(tuples, n, k, kMostCut) / 2 + (most + 8) * 2 + 64;
     const int64_t pairs = (int64_t)n * (n + 512) / 2;
     return (size_t)(n * read + tuples * 4 + candidate_room(pairs) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
 }
@@ -1395,10 +1452,15 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     va.keys = j.keys.as<uint64_t>();
     va.vals = j.vals.as<uint32_t>();
     va.out_cap = cap;
-    const size_t vsmem = (size_t)kVerifyWarps * ((1 << (2 * k - 5)) + va.rep_slots) * 4;
-    CRISPY_CK(ctx, cudaFuncSetAttribute(filter_verify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vsmem));
+    // byte marks where they leave room for five blocks per SM
+    const bool bytes = k <= 6 && va.rep_slots == 256;
+    const int map_words = bytes ? 1 << (2 * k - 2) : 1 << (2 * k - 5);
+    const size_t vsmem = (size_t)kVerifyWarps * (map_words + va.rep_slots) * 4;
+    auto verify = bytes ? filter_verify_kernel<true, false>
+                        : k < 8 ? filter_verify_kernel<false, false> : filter_verify_kernel<false, true>;
+    CRISPY_CK(ctx, cudaFuncSetAttribute(verify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vsmem));
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, filter_verify_kernel, kVerifyWarps * 32, vsmem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, verify, kVerifyWarps * 32, vsmem);
     per_sm = std::max(1, per_sm);
     ev_begin(ctx, ctx->ev_kmer, s);
     fa.items = j.f_items.as<int4>();
@@ -1414,7 +1476,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
         filter_count_kernel<<<cgrid, 256, 0, s>>>(va);
         filter_rows_kernel<<<(n + 255) / 256, 256, 0, s>>>(va);
         filter_scatter_kernel<<<cgrid, 256, 0, s>>>(va);
-        filter_verify_kernel<<<ctx->sm_count * per_sm, kVerifyWarps * 32, vsmem, s>>>(va);
+        verify<<<ctx->sm_count * per_sm, kVerifyWarps * 32, vsmem, s>>>(va);
         count_launch(ctx, 5);
     }
     ev_end(ctx, ctx->ev_kmer, s);
