@@ -478,6 +478,14 @@ __global__ void gen_pack_kernel(const uint8_t* __restrict__ seq, const int64_t* 
     }
 }
 
+// Lengths and word offsets of reads packed a fixed stride each.
+__global__ void gen_stride_kernel(const int32_t* __restrict__ tuples, int n, int K, int stride,
+                                  int32_t* __restrict__ len, int64_t* __restrict__ woff) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) len[i] = tuples[i] + K - 1;
+    if (i <= n) woff[i] = (int64_t)i * stride;
+}
+
 // genCUDA.cu:219: keep iff dist < thr or |dist - thr| < 1e-5 (float
 // subtraction, double comparison).
 __global__ void gen_flag_kernel(const float* __restrict__ dist, int64_t n, float thr,
@@ -1381,6 +1389,25 @@ int crispy_gen_prepare_from_kmer(crispy_ctx* ctx) {
     g.ready = false;
     const int n = j.n;
     g.n = n;
+    if (j.f_ready) {
+        // the k-mer run left the reads packed, a fixed stride each: a copy,
+        // and lengths and offsets written on the device
+        if (j.min_len <= 0) return fail(ctx, CRISPY_E_INPUT, "a read is empty");
+        g.max_len = j.max_len;
+        cudaStream_t s = ctx->stream;
+        const size_t words = (size_t)n * j.f_stride;
+        CRISPY_TRY(ensure(ctx, g.len, (size_t)n * 4));
+        CRISPY_TRY(ensure(ctx, g.woff, (size_t)(n + 1) * 8));
+        CRISPY_TRY(ensure(ctx, g.packed, (words + 4) * 4));
+        CRISPY_CK(ctx, cudaMemcpyAsync(g.packed.ptr, j.f_packed.ptr, words * 4, cudaMemcpyDeviceToDevice, s));
+        gen_stride_kernel<<<(n + 256) / 256, 256, 0, s>>>(j.t0.as<int32_t>(), n, j.k, j.f_stride,
+                                                          g.len.as<int32_t>(), g.woff.as<int64_t>());
+        count_launch(ctx);
+        CRISPY_CK(ctx, cudaGetLastError());
+        CRISPY_CK(ctx, cudaStreamSynchronize(s));   // the caller may change the stream next
+        g.ready = true;
+        return CRISPY_OK;
+    }
     g.h_len.resize(n);
     g.h_woff.resize(n + 1);
     int64_t words = 0;

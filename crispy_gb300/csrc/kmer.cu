@@ -2555,6 +2555,7 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
     j.k = k;
     j.h_t.resize(n);
     j.max_len = 0;
+    j.min_len = CRISPY_MAX_READ_LEN;
     j.max_t = 0;
     for (int r = 0; r < n; ++r) {
         if (lengths[r] > CRISPY_MAX_READ_LEN)
@@ -2563,6 +2564,7 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
             return fail(ctx, CRISPY_E_INPUT, "read %d length %d shorter than K-1", r, lengths[r]);
         j.h_t[r] = lengths[r] - k + 1;
         j.max_len = std::max(j.max_len, (int)lengths[r]);
+        j.min_len = std::min(j.min_len, (int)lengths[r]);
         j.max_t = std::max(j.max_t, j.h_t[r]);
     }
     j.ngroups = (n + 31) / 32;
