@@ -601,7 +601,8 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
                                                                     const int64_t* __restrict__ woff,
                                                                     const int32_t* __restrict__ len,
                                                                     const int2* __restrict__ pairs, int64_t count,
-                                                                    int band, uint32_t* __restrict__ bands) {
+                                                                    int band, int max_sum,
+                                                                    uint32_t* __restrict__ bands) {
     __shared__ __align__(16) uint32_t bitmap[kBandWarps][1 << (kBandBits - 5)];
     const int lane = threadIdx.x & 31;
     uint32_t* bm = bitmap[threadIdx.x >> 5];
@@ -614,7 +615,7 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
         int lo = kb, hi = kb;
         // bands of up to 16 slots have nothing to save, nor have those that
         // the smallest estimate fills
-        if (l1 + l2 <= kGen16MaxSum && kb >= 16 && gap + 6 < 2 * kb) {
+        if (l1 + l2 <= max_sum && kb >= 16 && gap + 6 < 2 * kb) {
             const int rs = l1 <= l2 ? pr.x : pr.y, rl = l1 <= l2 ? pr.y : pr.x;
             const int ts = min(l1, l2) - 7, tl = max(l1, l2) - 7;
             for (int q = lane; q < 1 << (kBandBits - 7); q += 32)
@@ -648,14 +649,14 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
 // T * distance find no partner, so 8 / K times that stands for the 8-mers.
 __global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, const int2* __restrict__ pairs,
                                            const float* __restrict__ kdist, int K, int64_t count, int band,
-                                           uint32_t* __restrict__ bands) {
+                                           int max_sum, uint32_t* __restrict__ bands) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= count) return;
     const int2 pr = pairs[p];
     const int l1 = len[pr.x], l2 = len[pr.y];
     const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
     int lo = kb, hi = kb;
-    if (l1 + l2 <= kGen16MaxSum && kb >= 16) {
+    if (l1 + l2 <= max_sum && kb >= 16) {
         const float miss = kdist[p] * (float)(min(l1, l2) - K + 1);
         const int e = (int)fminf(miss * 3.25f / (float)K, 4096.0f) + 3;
         lo = min(kb, e + max(0, l1 - l2));
@@ -683,7 +684,7 @@ constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
 // bands: the diagonals each pair is swept over (nullptr: all of its band);
 // list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
-                                    const int32_t* __restrict__ len, int band, int nbins,
+                                    const int32_t* __restrict__ len, int band, int nbins, int max_sum,
                                     const uint32_t* __restrict__ bands, const uint32_t* __restrict__ list,
                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                     unsigned long long* __restrict__ stats) {
@@ -707,7 +708,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         for (int b = 1; b < nbins; ++b)
             if (c_bin_slots[b] >= (lo + hi) / 2 + 1) { bin = b; break; }
         lng = l1 + l2 > kGen16MaxSum ? 1 : 0;
-        if (bin != 0 && !lng) sum_reg = l1 + l2;
+        if (bin != 0 && l1 + l2 <= max_sum) sum_reg = l1 + l2;
         wb = bin == 0 ? nbins : bin;
         ob = bin == 0 ? 2 * nbins : bin + lng * nbins;   // wide pairs sort last
         if (keys) {
@@ -963,6 +964,12 @@ int launch_wide(crispy_ctx* ctx, const GenArgs& ga, int kbmax, const uint32_t* o
     return CRISPY_OK;
 }
 
+// CRISPY_GEN_EXT=0 keeps pairs beyond the 16-bit range on the 32-bit kernel.
+bool gen16_ext_on() {
+    const char* e = std::getenv("CRISPY_GEN_EXT");
+    return !(e && e[0] == '0');
+}
+
 // Whether a batched run sweeps narrow bands first: from about 1e9 band cells
 // (0.4 ms) on, where the saved slots outweigh the estimate, its read-back and
 // the second sweep's latency (about 100 us together; 7,000 pairs of 250 nt at
@@ -976,7 +983,7 @@ bool narrow_pays(const GenJob& g, int64_t count, int band) {
 // Classification of `count` pairs (all, or those of `list`): statistics to
 // the host and, for the batched form, the launch order.
 int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count, int band, bool sorted,
-                 const uint32_t* bands, const uint32_t* list, std::vector<unsigned long long>& st,
+                 int max_sum, const uint32_t* bands, const uint32_t* list, std::vector<unsigned long long>& st,
                  uint32_t** d_order) {
     GenJob& g = ctx->gen;
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
@@ -992,7 +999,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
     auto classify = [&]() -> int {
         CRISPY_CK(ctx, cudaMemsetAsync(d_stats, 0, (size_t)nstats * 8, s));
         gen_classify_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, bands, list,
+            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, max_sum, bands, list,
             sorted ? g.ckeys.as<uint32_t>() : nullptr, sorted ? g.cvals.as<uint32_t>() : nullptr, d_stats);
         count_launch(ctx);
         if (sorted) {
@@ -1010,7 +1017,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
             (uint64_t)(uintptr_t)g.len.ptr, (uint64_t)(uintptr_t)d_stats, (uint64_t)(uintptr_t)g.ckeys.ptr,
             (uint64_t)(uintptr_t)g.ckeys_alt.ptr, (uint64_t)(uintptr_t)g.cvals.ptr,
             (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr, (uint64_t)(uintptr_t)bands,
-            (uint64_t)(uintptr_t)list});
+            (uint64_t)(uintptr_t)list, (uint64_t)max_sum});
         CRISPY_TRY(graph_run(ctx, s, key, classify));
         *d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
     } else {
@@ -1076,7 +1083,12 @@ int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band,
     }
     for (BinRun& r : runs) {
         if (r.ob == kWideOrderBin) continue;
+        if (base.ext && r.ob > kNumBins) {
+            r.shape = kNumShapes + gen16_ext_shape(kBinSlots[r.ob - kNumBins]);
+            continue;
+        }
         GenArgs a = base;
+        a.ext = 0;
         a.order = d_order + r.at;
         a.count = r.n;
         CRISPY_TRY(pick_shape(ctx, s, band, r.ob, a, a.order, r.n, g.tune_sample, g.tune_queue, g.dirs, &r.shape));
@@ -1092,7 +1104,8 @@ int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band,
     int64_t dir_words = 0;
     for (const BinRun& r : runs)
         if (r.shape >= 0 && is16(r.shape))
-            dir_words = std::max(dir_words, gen16_dir_words(ctx, r.shape - kNumShapes, r.n, base.dir_blocks));
+            dir_words = std::max(dir_words, gen16_dir_words(ctx, r.shape - kNumShapes, r.n, base.dir_blocks,
+                                                            base.ext && r.ob > kNumBins));
     if (dir_words) CRISPY_TRY(ensure(ctx, g.dirs, (size_t)dir_words * 4 * (fork ? 2 : 1)));
     ev_begin(ctx, ctx->ev_gen, s);
     if (fork) {
@@ -1110,6 +1123,7 @@ int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band,
         a.order = d_order + r.at;
         a.count = r.n;
         a.queue = g.queue.as<unsigned int>() + r.ob;
+        a.ext = base.ext && r.ob > kNumBins;
         if (dir_words) {
             a.dirs = g.dirs.as<uint32_t>() + (fork ? (int64_t)(i & 1) * dir_words : 0);
             a.dirs_words = dir_words;
@@ -1150,40 +1164,46 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
     if (mode == CRISPY_MODE_BATCHED) {
         // (a forced shape sweeps whole bands, up to the shape's full width)
         const bool narrow = forced_shape() < 0 && narrow_pays(g, count, band);
+        // pairs beyond the 16-bit range: its extended form first
+        const bool ext = forced_shape() < 0 && 2 * g.max_len > kGen16MaxSum && gen16_ext_on();
+        const int max_sum = ext ? kGen16ExtSum : kGen16MaxSum;
         uint32_t *bands = nullptr, *retry = nullptr;
-        if (narrow) {
-            CRISPY_TRY(ensure(ctx, g.bands, (size_t)count * 4));
+        if (narrow || ext) {
             CRISPY_TRY(ensure(ctx, g.retry, (size_t)(count + 1) * 4));
-            bands = g.bands.as<uint32_t>();
             retry = g.retry.as<uint32_t>();
             CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));
+        }
+        if (narrow) {
+            CRISPY_TRY(ensure(ctx, g.bands, (size_t)count * 4));
+            bands = g.bands.as<uint32_t>();
             if (kdist && kdist_k >= 5) {
                 gen_bands_from_kmer_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, count, band, bands);
+                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, count, band, max_sum, bands);
             } else {
                 const int blocks = (int)std::min<int64_t>((count + kBandWarps - 1) / kBandWarps, 8ll * ctx->sm_count);
                 gen_bands_kernel<<<blocks, kBandWarps * 32, 0, s>>>(g.packed.as<uint32_t>(), g.woff.as<int64_t>(),
-                                                                   g.len.as<int32_t>(), d_pairs, count, band, bands);
+                                                                   g.len.as<int32_t>(), d_pairs, count, band, max_sum, bands);
             }
             count_launch(ctx);
         }
-        CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, true, bands, nullptr, st, &d_order));
+        CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, true, max_sum, bands, nullptr, st, &d_order));
         ctx->stats.gen_cells += (int64_t)st[0];
         ctx->stats.gen_pairs += count;
         GenArgs base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
         base.bands = bands;
         base.retry = retry;
+        base.ext = ext;
         CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));
-        if (!narrow) return CRISPY_OK;
+        if (!retry) return CRISPY_OK;
         uint32_t left = 0;
         CRISPY_CK(ctx, cudaMemcpyAsync(&left, retry, 4, cudaMemcpyDeviceToHost, s));
         CRISPY_CK(ctx, cudaStreamSynchronize(s));
         if (left == 0) return CRISPY_OK;
-        CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, nullptr, retry + 1, st, &d_order));
+        CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, kGen16MaxSum, nullptr, retry + 1, st, &d_order));
         return gen_run_bins(ctx, s, gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al), band,
                             d_order, st);
     }
-    CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, nullptr, nullptr, st, &d_order));
+    CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, kGen16MaxSum, nullptr, nullptr, st, &d_order));
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
     const int kbmax = (int)st[1];
     ctx->stats.gen_cells += (int64_t)st[0];

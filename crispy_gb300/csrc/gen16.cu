@@ -1,6 +1,7 @@
 // gen16.cu -- genDist's banded Needleman-Wunsch with two cells per 32-bit
 // register: the DP the batched and staged runs take for every pair with
-// L1 + L2 <= kGen16MaxSum (3600) that fits a register band.
+// L1 + L2 <= kGen16MaxSum (3600) that fits a register band, and batched runs
+// for longer ones too (with a floor under the keys, kBaseExt below).
 //
 // Reference semantics are those of gen.cu (genCPU.cpp:290-466 restated by
 // genKernel.cu:372-780): rows i over read2 = pair[1], columns j over read1 =
@@ -115,6 +116,22 @@ constexpr uint32_t kOut2 = kOut * kLo;
 constexpr int kRefNegInf = -1000000;    // genCPU.cpp:350 initial last-row/column maximum
 static_assert(18 * (kGen16MaxSum + kSlack) + 131 < 65536, "16-bit keys would wrap");
 static_assert(kBase % 4 == 0, "the score is read back as (K - 4s - kBase) / 4");
+// Pairs of up to kGen16ExtSum: the base that keeps the largest key in range,
+// and a floor under the keys of in-band cells, above every candidate of a
+// closed cell.  A cell is raised to the floor at step s only where its value
+// is below (kFloor - kBaseExt) / 4 - s, which values of at least -2 s reach
+// from s = kFloorFrom on.  A raised cell's path can still gain 5 per diagonal
+// move, (L1 + L2 - s) / 2 of them at the most, so (by the argument for narrow
+// sweeps) a score above floor_bound() is the true one.
+constexpr int kBaseExt = 65535 - 131 - 14 * (kGen16ExtSum + kSlack);
+constexpr uint32_t kFloor = 128u;
+constexpr int kFloorFrom = (kBaseExt - (int)kFloor) / 4;
+static_assert(kBaseExt % 4 == 0 && kBaseExt > (int)kFloor, "extended keys");
+__device__ __forceinline__ int floor_bound(int l1, int l2) {
+    return -2 * kFloorFrom + (5 * max(0, l1 + l2 - kFloorFrom) + 1) / 2;
+}
+template <bool kExt>
+constexpr int key_base() { return kExt ? kBaseExt : kBase; }
 
 constexpr int kClean = 0, kTrack = 1, kStart = 2;
 
@@ -244,8 +261,9 @@ __device__ __forceinline__ void boundary_slot(int d, const Pair16& pc, int gl, i
 }
 
 // Sets one half to a boundary cell at step s (M = 0) and opens its cap.
+template <bool kExt>
 __device__ __forceinline__ void boundary_set(uint32_t& K, uint32_t& CP, int h, int s, uint32_t tag) {
-    const uint32_t key = tag + (uint32_t)(4 * s + kBase);
+    const uint32_t key = tag + (uint32_t)(4 * s + key_base<kExt>());
     if (h == 0) {
         K = (K & 0xFFFF0000u) | key;
         CP |= 0x0000FFFFu;
@@ -276,7 +294,7 @@ __device__ __forceinline__ bool mine(int q, int gl, int G, int R) {
 // Last row (i = l2, tracked as `col`, ordered by j) and last column (j = l1,
 // `row`, ordered by i): each holds at most one cell per step; the lane that
 // holds it keeps the last maximum (>=), genCPU.cpp:442-464.
-template <int G, int R, int P>
+template <int G, int R, int P, bool kExt>
 __device__ __forceinline__ void track16(const St<R>& st, int gl, int s, const Pair16& pc, Best16& col,
                                         Best16& row) {
     const int dr = 2 * pc.l2 - s, jr = s - pc.l2;
@@ -287,12 +305,12 @@ __device__ __forceinline__ void track16(const St<R>& st, int gl, int s, const Pa
     const bool hc = ic >= 1 && ic <= pc.l2 && dc >= -pc.lo && dc <= pc.hi && mine(qc, gl, G, R);
     if (hr) {
         const uint32_t key = take<G, R, P>(st, qr, gl);
-        const int m = ((int)key - 31 - 4 * s - kBase) >> 2;
+        const int m = ((int)key - 31 - 4 * s - key_base<kExt>()) >> 2;
         if (m >= col.m) { col.m = m; col.at = jr; }
     }
     if (hc) {
         const uint32_t key = take<G, R, P>(st, qc, gl);
-        const int m = ((int)key - 31 - 4 * s - kBase) >> 2;
+        const int m = ((int)key - 31 - 4 * s - key_base<kExt>()) >> 2;
         if (m >= row.m) { row.m = m; row.at = ic; }
     }
 }
@@ -301,7 +319,7 @@ __device__ __forceinline__ void track16(const St<R>& st, int gl, int s, const Pa
 // are the lane's byte selectors for the edge register's neighbour: identity,
 // or (lane 0 at parity 0) its low half moved up over an empty slot, or (the
 // last lane at parity 1) its high half moved down under an empty slot.
-template <int G, int R, int P, int kMode>
+template <int G, int R, int P, int kMode, bool kExt>
 __device__ __forceinline__ void step16(St<R>& st, int gl, int s, const Pair16& pc, const Mul& mu,
                                        uint32_t sel0, uint32_t sel1, Best16& col, Best16& row) {
     uint32_t nK;
@@ -336,11 +354,12 @@ __device__ __forceinline__ void step16(St<R>& st, int gl, int s, const Pair16& p
         st.MW[P][r] >>= 1;
         const uint32_t kd = mm * mu.n36 + st.K[P][r];
         uint32_t K = __vimax3_u16x2(kd, upK, lfK);
+        if (kExt) K = __vmaxu2(K, kFloor * kLo);
         K = __vminu2(K, st.CP[P][r]);
         if (kMode == kStart && (r == ra || r == rb)) {
             // a boundary cell: its own key, not the recurrence's
-            if (r == ra) boundary_set(K, st.CP[P][r], ha, s, 0u);
-            if (r == rb) boundary_set(K, st.CP[P][r], hb, s, 1u);
+            if (r == ra) boundary_set<kExt>(K, st.CP[P][r], ha, s, 0u);
+            if (r == rb) boundary_set<kExt>(K, st.CP[P][r], hb, s, 1u);
         }
         const uint32_t t = K & (3u * kLo), x2 = K & (2u * kLo);
         st.U[r] = x2 * mu.n14 + (t * mu.n5 + (K * mu.one + mu.c5));
@@ -351,20 +370,20 @@ __device__ __forceinline__ void step16(St<R>& st, int gl, int s, const Pair16& p
     if (kMode != kClean) {
         const bool near = (unsigned)(s - pc.tw[0]) < 2u * R || (unsigned)(s - pc.tw[1]) < 2u * R ||
                           (unsigned)(s - pc.tw[2]) < 2u * R || (unsigned)(s - pc.tw[3]) < 2u * R;
-        if (near) track16<G, R, P>(st, gl, s, pc, col, row);
+        if (near) track16<G, R, P, kExt>(st, gl, s, pc, col, row);
     }
 }
 
 // A block of 16 steps, after which the lane's tag words go to `dst`
 // (parity P at dst + P * G * R; nullptr: not stored).
-template <int G, int R, int kMode>
+template <int G, int R, int kMode, bool kExt>
 __device__ __forceinline__ void block16(St<R>& st, int gl, int s0, const Pair16& pc, const Mul& mu,
                                         uint32_t sel0, uint32_t sel1, Best16& col, Best16& row,
                                         uint32_t* dst) {
 #pragma unroll 1
     for (int t = 0; t < kSteps; t += 2) {
-        step16<G, R, 0, kMode>(st, gl, s0 + t, pc, mu, sel0, sel1, col, row);
-        step16<G, R, 1, kMode>(st, gl, s0 + t + 1, pc, mu, sel0, sel1, col, row);
+        step16<G, R, 0, kMode, kExt>(st, gl, s0 + t, pc, mu, sel0, sel1, col, row);
+        step16<G, R, 1, kMode, kExt>(st, gl, s0 + t + 1, pc, mu, sel0, sel1, col, row);
     }
     if (dst) {
 #pragma unroll
@@ -511,7 +530,7 @@ __device__ __forceinline__ void walk16(const uint32_t* region, uint32_t* stage, 
     *gp = g;
 }
 
-template <int G, int R>
+template <int G, int R, bool kExt = false>
 __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenArgs a) {
     constexpr int kPerWarp = 32 / G;
     static_assert(R <= 16, "a lane's slot windows must fit one 32-symbol window per read");
@@ -606,11 +625,11 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
             const bool started = s0 > max(pc.lo, pc.hi);   // every boundary cell is behind (s = |d|)
             const bool clean = finished || (started && s0 + kBlock - 1 < clean_hi);
             if (__all_sync(0xffffffffu, clean))
-                block16<G, R, kClean>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
+                block16<G, R, kClean, kExt>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
             else if (__all_sync(0xffffffffu, started || finished))
-                block16<G, R, kTrack>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
+                block16<G, R, kTrack, kExt>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
             else
-                block16<G, R, kStart>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
+                block16<G, R, kStart, kExt>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
         }
         col = group_best16<G>(col);
         row = group_best16<G>(row);
@@ -642,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
                 int most = INT_MIN / 8;
                 if (pc.lo < kb) most = min(pc.l1 - pc.lo - 1, pc.l2);
                 if (pc.hi < kb) most = max(most, min(pc.l2 - pc.hi - 1, pc.l1));
-                if (b.at < 0 || b.m <= 5 * most) a.retry[1 + atomicAdd(a.retry, 1u)] = (uint32_t)p;
+                if (b.at < 0 || b.m <= 5 * most || (kExt && b.m <= floor_bound(pc.l1, pc.l2))) a.retry[1 + atomicAdd(a.retry, 1u)] = (uint32_t)p;
             }
         }
         __syncwarp();
@@ -687,16 +706,37 @@ Fn16 fn16(int i) {
     }
 }
 
+// The shapes pairs beyond kGen16MaxSum run in.
+Fn16 fn16_ext(int i) {
+    switch (i) {
+        case 5: return gen16_kernel<4, 6, true>;
+        case 9: return gen16_kernel<8, 5, true>;
+        case 11: return gen16_kernel<16, 4, true>;
+        case 12: return gen16_kernel<16, 6, true>;
+        case 13: return gen16_kernel<32, 4, true>;
+        case 15: return gen16_kernel<16, 7, true>;
+        default: return nullptr;
+    }
+}
+
 }  // namespace
 
+int gen16_ext_shape(int slots) {
+    int best = -1;
+    for (int i = 0; i < kNumShapes16; ++i) {
+        const int has = 2 * kShapes16[i].g * kShapes16[i].r;
+        if (fn16_ext(i) && has >= slots && (best < 0 || has < 2 * kShapes16[best].g * kShapes16[best].r)) best = i;
+    }
+    return best;
+}
 int gen16_num_shapes() { return kNumShapes16; }
 Shape16 gen16_shape(int i) { return kShapes16[i]; }
 int gen16_pairs_per_block(int i) { return kWarps * (32 / kShapes16[i].g); }
 
 namespace {
-int gen16_grid(crispy_ctx* ctx, int shape, int64_t count) {
+int gen16_grid(crispy_ctx* ctx, int shape, int64_t count, bool ext) {
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn16(shape), kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ext ? fn16_ext(shape) : fn16(shape), kThreads, 0);
     const int64_t per_block = gen16_pairs_per_block(shape);
     return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::max(1, per_sm) * ctx->sm_count,
                                                        (count + per_block - 1) / per_block));
@@ -719,19 +759,21 @@ int64_t gen16_lane_regs_per_sm() {
     return v;
 }
 
-int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks) {
+int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks, bool ext) {
     const Shape16 h = kShapes16[shape];
     // one region per pair slot of the grid: blocks x threads / G pairs
-    return (int64_t)gen16_grid(ctx, shape, count) * kThreads / h.g * dir_blocks * 2 * h.g * h.r;
+    return (int64_t)gen16_grid(ctx, shape, count, ext) * kThreads / h.g * dir_blocks * 2 * h.g * h.r;
 }
 
 int gen16_launch(crispy_ctx* ctx, cudaStream_t s, int shape, const GenArgs& a, bool timed) {
-    const int blocks = gen16_grid(ctx, shape, a.count);
-    if (!a.dirs || a.dir_blocks < 1 || a.dirs_words < gen16_dir_words(ctx, shape, a.count, a.dir_blocks))
+    const bool ext = a.ext != 0;
+    if (ext && !fn16_ext(shape)) return fail(ctx, CRISPY_E_STATE, "gen16: shape %d has no extended form", shape);
+    const int blocks = gen16_grid(ctx, shape, a.count, ext);
+    if (!a.dirs || a.dir_blocks < 1 || a.dirs_words < gen16_dir_words(ctx, shape, a.count, a.dir_blocks, ext))
         return fail(ctx, CRISPY_E_STATE, "gen16: tag storage of %lld words for %lld pairs is too small",
                     (long long)a.dirs_words, (long long)a.count);
     if (timed) ev_begin(ctx, ctx->ev_gen, s);
-    fn16(shape)<<<blocks, kThreads, 0, s>>>(a);
+    (ext ? fn16_ext(shape) : fn16(shape))<<<blocks, kThreads, 0, s>>>(a);
     if (timed) ev_end(ctx, ctx->ev_gen, s);
     count_launch(ctx);
     return CRISPY_OK;

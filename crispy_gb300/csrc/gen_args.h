@@ -34,6 +34,7 @@ struct GenArgs {
     // whose result that does not prove ([0] their count, then pair indices)
     const uint32_t* bands;
     uint32_t* retry;
+    int ext;                 // pairs beyond kGen16MaxSum: the extended form of the shape
     // All 1.  Adds written as multiply-adds by these run on the FMA pipe;
     // distinct multipliers keep the compiler from factoring a common
     // product back into ALU adds.
@@ -44,6 +45,9 @@ struct GenArgs {
 // whose range covers pairs with L1 + L2 <= kGen16MaxSum; longer pairs take
 // the 32-bit kernels of gen.cu.
 constexpr int kGen16MaxSum = 3600;
+// The most L1 + L2 can be: batched runs take longer pairs through the
+// extended form first, whose results their scores prove.
+constexpr int kGen16ExtSum = 4096;
 
 // Shapes of the 16-bit kernel: G lanes per pair, R registers per lane, so
 // a pair swept over diagonals -lo .. hi with (lo + hi) / 2 + 1 <= 2 * G * R
@@ -60,7 +64,9 @@ constexpr int kGen16MaxR = 7;
 // 16-step blocks a pair's sweep runs at most, for pairs with L1 + L2 <= max_sum.
 inline int gen16_dir_blocks(int max_sum) { return (max_sum + 1) / 16 + 1; }
 // Words of choice storage a launch of shape i over `count` pairs needs.
-int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks);
+int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks, bool ext = false);
+// Narrowest shape with an extended form that covers the slots, -1: none.
+int gen16_ext_shape(int slots);
 // Largest resident threads x registers per lane of one SM over the shapes:
 // a launch holds at most this many tag words per SM and sub-block.
 int64_t gen16_lane_regs_per_sm();

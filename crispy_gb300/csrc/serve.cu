@@ -96,14 +96,14 @@ size_t estimate_base_bytes(const Job& j) {
 // Bytes of the 16-bit DP's cell tags a run over n reads of at most maxlen
 // symbols may ask for: two launches in flight, each holding one word per
 // resident lane, register and sub-block (two per 16-step block, for pairs
-// of L1 + L2 <= min(2 maxlen, kGen16MaxSum)), and never more lanes than
+// of L1 + L2 <= 2 maxlen), and never more lanes than
 // 32 per possible pair plus a block.  It depends on the run, not the job:
 // a cohort counts it once.
 size_t tag_bytes(int maxlen, int64_t n, int sms) {
     const int64_t pairs = n * (n - 1) / 2;
     const int64_t lane_regs = std::min<int64_t>((int64_t)sms * crispy::gen16_lane_regs_per_sm(),
                                                 (32 * pairs + 128) * crispy::kGen16MaxR);
-    const int64_t blocks = crispy::gen16_dir_blocks(std::min(2 * maxlen, crispy::kGen16MaxSum));
+    const int64_t blocks = crispy::gen16_dir_blocks(2 * maxlen);
     return (size_t)(2 * lane_regs * 2 * blocks * 4);
 }
 

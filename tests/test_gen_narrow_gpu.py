@@ -124,3 +124,19 @@ def test_narrow_after_whole_bands_were_tuned(engine, monkeypatch):
     monkeypatch.setenv("CRISPY_GEN_NARROW", "1")
     reads = synth.make_read_set(synth.ReadSetSpec(150, 2, 330, "uniform", 290, 320, 6, 860))
     _check(engine, reads, _random_pairs(len(reads), 20000, 43), (10, 5))
+
+
+@pytest.mark.parametrize("narrow_on", ["0", "1"])
+def test_long_reads_extended_keys(engine, monkeypatch, narrow_on):
+    # L1 + L2 around and beyond 3,600: similar pairs are proved by their
+    # score, unrelated ones and reads that share no symbol are swept again
+    monkeypatch.setenv("CRISPY_GEN_NARROW", narrow_on)
+    reads = synth.make_read_set(synth.ReadSetSpec(60, 3, 2100, "uniform", 1750, 2048, 6, 870))
+    rng = np.random.default_rng(45)
+    reads += [rng.choice(np.frombuffer(b"ACGT", np.uint8), int(L)).tobytes() for L in (1801, 2000, 2047, 2048)]
+    reads += [b"A" * 2048, b"C" * 2048, b"G" * 2001, b"A" * 1800, b"AC" * 1024, reads[0], reads[1][:1799] + b"T"]
+    n = len(reads)
+    fixed = [[n - 7, n - 6], [n - 7, n - 5], [n - 7, n - 7], [n - 3, n - 7], [n - 3, n - 6], [n - 2, 0], [n - 1, 1]]
+    pairs = np.concatenate([np.array(fixed, np.int32), _random_pairs(n, 240, 46)])
+    _check(engine, reads, pairs, (40, 20, 10))
+    _check(engine, reads, pairs[:60], (5,))
