@@ -516,6 +516,56 @@ __global__ void gen_keys_kernel(const float* __restrict__ dist, const uint32_t* 
     vals[i] = p;
 }
 
+// Cohort jobs: pair ranges [off[q], off[q + 1]), thresholds and read bases.
+struct CohortView {
+    const int64_t* off;
+    const float* thr;
+    const int32_t* base;
+    int njobs;
+};
+__device__ __forceinline__ int cohort_job_of(const CohortView& v, int64_t p) {
+    int lo = 0, hi = v.njobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (v.off[mid] <= p) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The cut of every pair by its own job's threshold, and each job's survivors.
+__global__ void gen_flag_cohort_kernel(const float* __restrict__ dist, int64_t n, const CohortView v,
+                                       uint8_t* __restrict__ flags, unsigned int* __restrict__ jobcnt) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int q = cohort_job_of(v, i);
+    const float d = dist[i], thr = v.thr[q];
+    const bool keep = d < thr || (double)fabsf(__fsub_rn(d, thr)) < 0.00001;
+    flags[i] = keep;
+    if (keep) atomicAdd(&jobcnt[q], 1u);
+}
+
+__global__ void gen_keys_cohort_kernel(const float* __restrict__ dist, const uint32_t* __restrict__ surv,
+                                       int64_t count, const CohortView v, uint64_t* __restrict__ keys,
+                                       uint32_t* __restrict__ vals) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const uint32_t p = surv[i];
+    keys[i] = ((uint64_t)cohort_job_of(v, p) << kDistBits) | dist_key(dist[p]);
+    vals[i] = p;
+}
+
+__global__ void gen_gather_cohort_kernel(const int2* __restrict__ pairs, const uint64_t* __restrict__ keys,
+                                         const uint32_t* __restrict__ vals, int64_t count, const CohortView v,
+                                         uint2* __restrict__ out_pairs, float* __restrict__ out_dists) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const uint64_t k = keys[i];
+    const int base = v.base[k >> kDistBits];
+    const int2 pr = pairs[vals[i]];
+    out_pairs[i] = make_uint2((uint32_t)(pr.x - base), (uint32_t)(pr.y - base));
+    out_dists[i] = key_dist((uint32_t)k & ((1u << kDistBits) - 1u));
+}
+
 // pair_base: the job's first position in a cohort's read set (0 otherwise),
 // so that output pairs hold the job's own read indices.
 __global__ void gen_gather_kernel(const int2* __restrict__ pairs, const uint32_t* __restrict__ keys,
@@ -1764,6 +1814,86 @@ namespace crispy {
 // persistent bin launches (the jobs share every launch); then each job's
 // slice is thresholded, chunked and sorted on its own, with its own
 // threshold, and its chunks (in its own read indices) go to its sink.
+namespace {
+
+// Threshold, sort and delivery of all of a cohort's jobs at once: one
+// compaction, one stable sort by (job, distance) and one read-back, where a
+// job by itself takes ten launches and two waits (27 jobs of 600 reads: about
+// 3 ms).  Each job has at most one load window of pairs, so one chunk.
+int gen_finish_cohort(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t total,
+                      const std::vector<CohortJob>& jobs, const std::vector<int64_t>& counts,
+                      std::vector<int64_t>& gen_counts) {
+    GenJob& g = ctx->gen;
+    const int nj = (int)jobs.size();
+    const size_t off_thr = (size_t)(nj + 1) * 8, off_base = off_thr + (size_t)nj * 4, off_cnt = off_base + (size_t)nj * 4;
+    std::vector<char> blob(off_cnt + (size_t)nj * 4, 0);
+    int64_t at = 0;
+    for (int q = 0; q < nj; ++q) {
+        reinterpret_cast<int64_t*>(blob.data())[q] = at;
+        reinterpret_cast<float*>(blob.data() + off_thr)[q] = jobs[q].thr;
+        reinterpret_cast<int32_t*>(blob.data() + off_base)[q] = jobs[q].base;
+        at += counts[q];
+    }
+    reinterpret_cast<int64_t*>(blob.data())[nj] = at;
+    CRISPY_TRY(ensure(ctx, g.cjobs, blob.size()));
+    CRISPY_CK(ctx, cudaMemcpyAsync(g.cjobs.ptr, blob.data(), blob.size(), cudaMemcpyHostToDevice, s));
+    char* d = g.cjobs.as<char>();
+    unsigned int* d_cnt = reinterpret_cast<unsigned int*>(d + off_cnt);
+    const CohortView v{reinterpret_cast<const int64_t*>(d), reinterpret_cast<const float*>(d + off_thr),
+                       reinterpret_cast<const int32_t*>(d + off_base), nj};
+    const int64_t ntiles = (total + kScanTile - 1) / kScanTile;
+    CRISPY_TRY(ensure(ctx, g.flags, (size_t)total));
+    CRISPY_TRY(ensure(ctx, g.surv_idx, (size_t)total * 4));
+    CRISPY_TRY(ensure(ctx, g.blocksum, (size_t)ntiles * 4));
+    const unsigned blocks = (unsigned)((total + 255) / 256);
+    gen_flag_cohort_kernel<<<blocks, 256, 0, s>>>(g.dist.as<float>(), total, v, g.flags.as<uint8_t>(), d_cnt);
+    count_launch(ctx);
+    CRISPY_TRY(compact_flags(ctx, s, g.flags.as<uint8_t>(), total, g.surv_idx.as<uint32_t>(),
+                             g.blocksum.as<uint32_t>(), g.scan, nullptr));
+    std::vector<unsigned int> cnt(nj);
+    CRISPY_CK(ctx, cudaMemcpyAsync(cnt.data(), d_cnt, (size_t)nj * 4, cudaMemcpyDeviceToHost, s));
+    CRISPY_CK(ctx, cudaStreamSynchronize(s));
+    int64_t kept = 0;
+    for (unsigned int c : cnt) kept += c;
+    if (kept == 0) return CRISPY_OK;
+    CRISPY_TRY(ensure(ctx, g.keys, (size_t)kept * 8));
+    CRISPY_TRY(ensure(ctx, g.keys_alt, (size_t)kept * 8));
+    CRISPY_TRY(ensure(ctx, g.vals, (size_t)kept * 4));
+    CRISPY_TRY(ensure(ctx, g.vals_alt, (size_t)kept * 4));
+    CRISPY_TRY(ensure(ctx, g.out_pairs, (size_t)kept * 8));
+    CRISPY_TRY(ensure(ctx, g.out_dists, (size_t)kept * 4));
+    CRISPY_TRY(ensure_host(ctx, g.h_pairs, (size_t)kept * 8));
+    CRISPY_TRY(ensure_host(ctx, g.h_dists, (size_t)kept * 4));
+    const unsigned kb = (unsigned)((kept + 255) / 256);
+    gen_keys_cohort_kernel<<<kb, 256, 0, s>>>(g.dist.as<float>(), g.surv_idx.as<uint32_t>(), kept, v,
+                                             g.keys.as<uint64_t>(), g.vals.as<uint32_t>());
+    int bits = kDistBits;
+    while ((1ll << (bits - kDistBits)) < nj) ++bits;
+    uint64_t* sk = nullptr;
+    uint32_t* sv = nullptr;
+    CRISPY_TRY(sort_u64_payload(ctx, s, g.keys.as<uint64_t>(), g.keys_alt.as<uint64_t>(), g.vals.as<uint32_t>(),
+                                g.vals_alt.as<uint32_t>(), kept, bits, true, &sk, &sv, g.scan));
+    gen_gather_cohort_kernel<<<kb, 256, 0, s>>>(d_pairs, sk, sv, kept, v, g.out_pairs.as<uint2>(),
+                                                g.out_dists.as<float>());
+    count_launch(ctx, 2);
+    CRISPY_CK(ctx, cudaGetLastError());
+    CRISPY_CK(ctx, cudaMemcpyAsync(g.h_pairs.ptr, g.out_pairs.ptr, (size_t)kept * 8, cudaMemcpyDeviceToHost, s));
+    CRISPY_CK(ctx, cudaMemcpyAsync(g.h_dists.ptr, g.out_dists.ptr, (size_t)kept * 4, cudaMemcpyDeviceToHost, s));
+    CRISPY_CK(ctx, cudaStreamSynchronize(s));
+    at = 0;
+    for (int q = 0; q < nj; ++q) {
+        if (cnt[q] == 0) continue;
+        if (jobs[q].sink && jobs[q].sink(jobs[q].user, 0, g.h_pairs.as<char>() + at * 8, g.h_dists.as<float>() + at,
+                                         cnt[q]) != 0)
+            return fail(ctx, CRISPY_E_IO, "sink aborted at chunk 0");
+        gen_counts[q] = cnt[q];
+        at += cnt[q];
+    }
+    return CRISPY_OK;
+}
+
+}  // namespace
+
 int gen_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, const std::vector<int64_t>& counts,
                    int band, std::vector<int64_t>& gen_counts) {
     GenJob& g = ctx->gen;
@@ -1785,6 +1915,13 @@ int gen_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, const st
         CRISPY_TRY(gen_dispatch_impl(ctx, s, k.pairs.as<int2>(), total, band, CRISPY_MODE_BATCHED,
                                      g.dist.as<float>(), nullptr, nullptr, nullptr,
                                      k.dists_kept ? k.dists.as<float>() : nullptr, k.k));
+    }
+    int64_t most = 0;
+    for (int64_t c : counts) most = std::max(most, c);
+    if (total > 0 && most <= CRISPY_GEN_WINDOW) {
+        CRISPY_TRY(gen_finish_cohort(ctx, s, k.pairs.as<int2>(), total, jobs, counts, gen_counts));
+        ctx->stats.gen_kernel_ms = ev_sum_ms(ctx->ev_gen);
+        return CRISPY_OK;
     }
     int64_t off = 0;
     for (size_t c = 0; c < jobs.size(); ++c) {
