@@ -321,7 +321,8 @@ int crispy_ctx_trim(crispy_ctx* ctx) {
     PreJob& pj = ctx->pre;
     for (DevBuf* b : {&pj.seq, &pj.off, &pj.len, &pj.freq, &pj.woff, &pj.pad, &pj.alive, &pj.idx,
                       &pj.idx_alt, &pj.flags, &pj.pos, &pj.tiles, &pj.out_idx, &pj.out_freq,
-                      &pj.counters, &pj.primer, &pj.tmp, &pj.stage_len, &pj.stage_off})
+                      &pj.counters, &pj.primer, &pj.tmp, &pj.stage_len, &pj.stage_off,
+                      &pj.keys, &pj.keys_alt, &pj.range})
         release(ctx, *b);
     pj.ready = false;
     k.ready = k.ent_ready = k.f_ready = false;

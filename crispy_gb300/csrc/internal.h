@@ -137,7 +137,7 @@ struct PreJob {
     int32_t n = 0;                 // records of the last call
     std::vector<int32_t> h_idx;    // kept record indices, _Clean order
     DevBuf seq, off, len, freq, woff, pad, alive, idx, idx_alt, flags, pos, tiles, out_idx,
-        out_freq, counters, primer, tmp, stage_len, stage_off;
+        out_freq, counters, primer, tmp, stage_len, stage_off, keys, keys_alt, range;
 };
 
 // An instantiated CUDA graph of one launch sequence and the number of

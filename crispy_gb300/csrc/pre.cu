@@ -13,9 +13,10 @@
 //      against each read's first 2 x primer-length bytes, one thread per
 //      read with its DP rows in shared memory;
 //   4. the surviving read indices are sorted by (length, bytes, record
-//      index): 2048-index tiles by a bitonic network in shared memory, then
+//      index): 1024-index tiles by a bitonic network in shared memory, then
 //      merge passes in which each index finds its place in the partner run
-//      by binary search.  The record index as last key makes every key
+//      by binary search, both on 128-bit keys (pre_key_kernel) that stand for
+//      the length and the first 28 bytes.  The record index as last key makes every key
 //      distinct, so the order equals the reference's stable sort;
 //   5. pre_last_kernel flags the last read of each run of equal sequences;
 //      compaction of those flags gives the kept reads and, from the gaps
@@ -37,7 +38,7 @@ namespace crispy {
 namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;   // tile padding: sorts after every read
-constexpr int kTile = 2048;               // indices per bitonic tile
+constexpr int kTile = 1024;               // indices per bitonic tile
 constexpr int kTileThreads = kTile / 2;
 constexpr int kMaxPrimer = 256;           // primer bases the shared-memory DP rows allow
 
@@ -54,12 +55,23 @@ __device__ __forceinline__ int cmp_bytes(const ReadSet& r, uint32_t a, uint32_t 
     const uint4* pa = r.pad + r.woff[a];
     const uint4* pb = r.pad + r.woff[b];
     const int nw = (L + 15) >> 4;
-    for (int w = 0; w < nw; ++w) {
-        const uint4 x = __ldg(pa + w), y = __ldg(pb + w);
-        if (x.x != y.x) return be32(x.x) < be32(y.x) ? -1 : 1;
-        if (x.y != y.y) return be32(x.y) < be32(y.y) ? -1 : 1;
-        if (x.z != y.z) return be32(x.z) < be32(y.z) ? -1 : 1;
-        if (x.w != y.w) return be32(x.w) < be32(y.w) ? -1 : 1;
+    // four words of each on their way at a time: duplicates compare to the end
+    for (int w0 = 0; w0 < nw; w0 += 4) {
+        uint4 xs[4], ys[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int w = min(w0 + q, nw - 1);
+            xs[q] = __ldg(pa + w);
+            ys[q] = __ldg(pb + w);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint4 x = xs[q], y = ys[q];
+            if (x.x != y.x) return be32(x.x) < be32(y.x) ? -1 : 1;
+            if (x.y != y.y) return be32(x.y) < be32(y.y) ? -1 : 1;
+            if (x.z != y.z) return be32(x.z) < be32(y.z) ? -1 : 1;
+            if (x.w != y.w) return be32(x.w) < be32(y.w) ? -1 : 1;
+        }
     }
     return 0;
 }
@@ -72,6 +84,58 @@ __device__ __forceinline__ bool read_less(const ReadSet& r, uint32_t a, uint32_t
     if (la != lb) return la < lb;
     const int c = cmp_bytes(r, a, b, la);
     return c ? c < 0 : a < b;
+}
+
+// Sort key of a read: its length (16 bits, saturated) and its first 28 bytes
+// as 4-bit classes that keep their order -- one class for each of NUL, A, C,
+// G, N and T, one for every range between them.  A byte of a range ends the
+// key (zeros follow; a length that does not fit leaves no class at all), so
+// two reads whose keys differ are in the order of their keys, and two whose
+// keys agree need the full comparison.
+struct ReadKey {
+    unsigned long long hi, lo;
+};
+__device__ __forceinline__ bool key_equal(const ReadKey& a, const ReadKey& b) { return a.hi == b.hi && a.lo == b.lo; }
+// kWhole: reads whose keys agree are compared; otherwise they keep the record
+// order, to be settled group by group afterwards.
+template <bool kWhole>
+__device__ __forceinline__ bool key_less(const ReadSet& r, const ReadKey& ka, uint32_t a, const ReadKey& kb, uint32_t b) {
+    if (ka.hi != kb.hi) return ka.hi < kb.hi;
+    if (ka.lo != kb.lo) return ka.lo < kb.lo;
+    return kWhole ? read_less(r, a, b) : a < b;
+}
+__device__ __forceinline__ uint32_t byte_class(uint32_t c) {
+    if (c == 0) return 0;
+    if (c < 'A') return 1;
+    if (c == 'A') return 2;
+    if (c < 'C') return 3;
+    if (c == 'C') return 4;
+    if (c < 'G') return 5;
+    if (c == 'G') return 6;
+    if (c < 'N') return 7;
+    if (c == 'N') return 8;
+    if (c < 'T') return 9;
+    return c == 'T' ? 10 : 11;
+}
+__global__ void pre_key_kernel(ReadSet r, const uint32_t* __restrict__ idx, int64_t m, ReadKey* __restrict__ keys) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t x = idx[i];
+    const int L = r.len[x];
+    const uint4* p = r.pad + r.woff[x];
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const uint4 w0 = L > 0 ? __ldg(p) : zero, w1 = L > 16 ? __ldg(p + 1) : zero;
+    const uint32_t words[7] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z};
+    unsigned long long hi = (unsigned long long)min(L, 0xFFFF) << 48, lo = 0;
+    bool open = L < 0xFFFF;
+#pragma unroll
+    for (int q = 0; q < 28; ++q) {
+        const uint32_t c = open ? byte_class((words[q / 4] >> (8 * (q % 4))) & 0xFFu) : 0u;
+        if (q < 12) hi |= (unsigned long long)c << (44 - 4 * q);
+        else lo |= (unsigned long long)c << (60 - 4 * (q - 12));
+        open = open && (c & 1u) == 0u;
+    }
+    keys[i] = ReadKey{hi, lo};
 }
 
 __global__ void pre_pad_kernel(const uint8_t* __restrict__ seq, const int64_t* __restrict__ off,
@@ -193,39 +257,60 @@ __global__ void pre_primer_kernel(ReadSet r, int n, const uint8_t* __restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) pre_tile_sort_kernel(uint32_t* idx, int64_t m, ReadSet r) {
+// Bitonic sort of one tile: keys and indices in shared memory.  With kWhole
+// the reads themselves are looked at where keys agree; a single such pair
+// makes its whole block wait for loads that depend on one another (85 us for
+// 60,000 reads, 152 with all reads compared at every step).
+template <bool kWhole>
+__global__ void __launch_bounds__(kTileThreads) pre_tile_sort_kernel(uint32_t* idx, ReadKey* keys, int64_t m,
+                                                                     ReadSet r) {
     __shared__ uint32_t s[kTile];
+    __shared__ ReadKey sk[kTile];
     const int64_t base = (int64_t)blockIdx.x * kTile;
-    for (int t = threadIdx.x; t < kTile; t += kTileThreads) s[t] = base + t < m ? idx[base + t] : kNone;
+    for (int t = threadIdx.x; t < kTile; t += kTileThreads) {
+        s[t] = base + t < m ? idx[base + t] : kNone;
+        sk[t] = base + t < m ? keys[base + t] : ReadKey{~0ull, ~0ull};
+    }
     __syncthreads();
     for (int k = 2; k <= kTile; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
             const int t = threadIdx.x;
             const int i = 2 * t - (t & (j - 1));   // bit j of i is clear; partner i + j
             const uint32_t a = s[i], b = s[i + j];
+            const ReadKey ka = sk[i], kb = sk[i + j];
             const bool up = (i & k) == 0;
-            if (up ? read_less(r, b, a) : read_less(r, a, b)) { s[i] = b; s[i + j] = a; }
+            if (up ? key_less<kWhole>(r, kb, b, ka, a) : key_less<kWhole>(r, ka, a, kb, b)) {
+                s[i] = b; s[i + j] = a;
+                sk[i] = kb; sk[i + j] = ka;
+            }
             __syncthreads();
         }
     }
     for (int t = threadIdx.x; t < kTile; t += kTileThreads)
-        if (base + t < m) idx[base + t] = s[t];
+        if (base + t < m) {
+            idx[base + t] = s[t];
+            keys[base + t] = sk[t];
+        }
 }
 
 // One merge pass over sorted runs of `width`: each index moves to its
 // position in the merged pair of runs, found by a binary search for the
-// number of smaller keys in the partner run.
-__global__ void pre_merge_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int64_t m,
+// number of smaller reads in the partner run (one load of a key per step
+// unless the reads have to be compared).
+template <bool kWhole>
+__global__ void pre_merge_kernel(const uint32_t* __restrict__ src, const ReadKey* __restrict__ skey,
+                                 uint32_t* __restrict__ dst, ReadKey* __restrict__ dkey, int64_t m,
                                  int64_t width, ReadSet r) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const int64_t run = i / width;
     const int64_t base = (run & ~1LL) * width;
     const uint32_t x = src[i];
+    const ReadKey kx = skey[i];
     int64_t lo, hi, p0, pos;
     if ((run & 1) == 0) {
         p0 = base + width;
-        if (p0 >= m) { dst[i] = x; return; }
+        if (p0 >= m) { dst[i] = x; dkey[i] = kx; return; }
         lo = p0; hi = min(base + 2 * width, m);
         pos = i - base;
     } else {
@@ -235,19 +320,71 @@ __global__ void pre_merge_kernel(const uint32_t* __restrict__ src, uint32_t* __r
     }
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
-        if (read_less(r, src[mid], x)) lo = mid + 1;
+        if (key_less<kWhole>(r, skey[mid], src[mid], kx, x)) lo = mid + 1;
         else hi = mid;
     }
-    dst[base + pos + (lo - p0)] = x;
+    const int64_t to = base + pos + (lo - p0);
+    dst[to] = x;
+    dkey[to] = kx;
+}
+
+// Groups of equal keys.  One warp per position finds its group's range; the
+// group's first position adds its comparisons to *work.
+constexpr unsigned kGroupMost = 4096;   // larger groups count as too much work
+__global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, uint2* __restrict__ range,
+                                 unsigned long long* __restrict__ work) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= m) return;
+    const ReadKey k = keys[p];
+    int64_t lo = p, hi = p + 1;
+    for (int run = 32; run == 32 && p - lo < kGroupMost;) {
+        const int64_t q = lo - 1 - lane;
+        const unsigned ne = ~__ballot_sync(full, q >= 0 && key_equal(keys[q], k));
+        run = ne ? __ffs(ne) - 1 : 32;
+        lo -= run;
+    }
+    for (int run = 32; run == 32 && hi - p <= kGroupMost;) {
+        const int64_t q = hi + lane;
+        const unsigned ne = ~__ballot_sync(full, q < m && key_equal(keys[q], k));
+        run = ne ? __ffs(ne) - 1 : 32;
+        hi += run;
+    }
+    if (lane == 0) {
+        range[p] = make_uint2((uint32_t)lo, (uint32_t)hi);
+        const unsigned long long g = (unsigned long long)(hi - lo);
+        if (g >= kGroupMost) atomicAdd(work, 1ull << 40);
+        else if (lo == p && g > 1) atomicAdd(work, g * g);
+    }
+}
+
+// Each read's place in its group: one warp counts the group's reads that come
+// before it.  Left undone (*work stays above the limit) where comparing within
+// the groups would cost more than the merges.
+__global__ void pre_rank_kernel(const uint32_t* __restrict__ src, const uint2* __restrict__ range, int64_t m, ReadSet r,
+                                const unsigned long long* __restrict__ work, unsigned long long limit,
+                                uint32_t* __restrict__ dst) {
+    if (*work > limit) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= m) return;
+    const uint32_t x = src[p];
+    const uint2 g = range[p];
+    unsigned before = 0;
+    if (g.y - g.x > 1)
+        for (uint32_t q = g.x + lane; q < g.y; q += 32) before += q != (uint32_t)p && read_less(r, src[q], x);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) dst[g.x + before] = x;
 }
 
 // flag[p] = 1 where sorted[p] is the last read of its run of equal sequences.
-__global__ void pre_last_kernel(const uint32_t* __restrict__ sorted, int64_t m, ReadSet r,
-                                uint8_t* __restrict__ flag) {
+__global__ void pre_last_kernel(const uint32_t* __restrict__ sorted, const ReadKey* __restrict__ keys, int64_t m,
+                                ReadSet r, uint8_t* __restrict__ flag) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= m) return;
     bool last = true;
-    if (p + 1 < m) {
+    if (p + 1 < m && key_equal(keys[p], keys[p + 1])) {
         const uint32_t a = sorted[p], b = sorted[p + 1];
         const int la = r.len[a];
         last = la != r.len[b] || cmp_bytes(r, a, b, la) != 0;
@@ -477,22 +614,63 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     // sort by (length, bytes, record index)
     uint32_t* a = j.idx.as<uint32_t>();
     uint32_t* b = j.idx_alt.as<uint32_t>();
-    if (m > 1) {
-        pre_tile_sort_kernel<<<(unsigned)((m + kTile - 1) / kTile), kTileThreads, 0, s>>>(a, m, rs);
+    CRISPY_TRY(ensure(ctx, j.keys, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
+    CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
+    CRISPY_TRY(ensure(ctx, j.range, (size_t)std::max<int64_t>(m, 1) * sizeof(uint2)));
+    unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
+    const unsigned long long limit = 32ull * (unsigned long long)m + 4096;
+    const unsigned blocks = (unsigned)((m + 255) / 256), wblocks = (unsigned)((m + 7) / 8);
+    ReadKey* ka = nullptr;
+    // keys first, reads of equal keys settled group by group; or, where the
+    // groups are large (many copies of a read), the reads compared throughout
+    auto sort_reads = [&](bool whole) {
+        a = j.idx.as<uint32_t>();
+        b = j.idx_alt.as<uint32_t>();
+        ka = j.keys.as<ReadKey>();
+        ReadKey* kb = j.keys_alt.as<ReadKey>();
+        pre_key_kernel<<<blocks, 256, 0, s>>>(rs, a, m, ka);
+        count_launch(ctx);
+        if (m < 2) return;
+        const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
+        if (whole) pre_tile_sort_kernel<true><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs);
+        else pre_tile_sort_kernel<false><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs);
         count_launch(ctx);
         for (int64_t w = kTile; w < m; w <<= 1) {
-            pre_merge_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(a, b, m, w, rs);
+            if (whole) pre_merge_kernel<true><<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs);
+            else pre_merge_kernel<false><<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs);
             count_launch(ctx);
             std::swap(a, b);
+            std::swap(ka, kb);
         }
+        if (whole) return;
+        pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, j.range.as<uint2>(), d_work);
+        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, limit, b);
+        count_launch(ctx, 2);
+        std::swap(a, b);
+    };
+    if (m > 0) {
+        sort_reads(false);
+        CRISPY_CK(ctx, cudaGetLastError());
     }
     int64_t kept = 0;
     if (m > 0) {
-        pre_last_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(a, m, rs, j.flags.as<uint8_t>());
-        count_launch(ctx);
-        CRISPY_CK(ctx, cudaGetLastError());
-        CRISPY_TRY(compact_flags(ctx, s, j.flags.as<uint8_t>(), m, j.pos.as<uint32_t>(), j.tiles.as<uint32_t>(),
-                                 j.tmp, &kept));
+        auto last_of_runs = [&]() -> int {
+            pre_last_kernel<<<blocks, 256, 0, s>>>(a, ka, m, rs, j.flags.as<uint8_t>());
+            count_launch(ctx);
+            CRISPY_CK(ctx, cudaGetLastError());
+            return compact_flags(ctx, s, j.flags.as<uint8_t>(), m, j.pos.as<uint32_t>(), j.tiles.as<uint32_t>(),
+                                 j.tmp, &kept);
+        };
+        unsigned long long work = 0;
+        CRISPY_CK(ctx, cudaMemcpyAsync(&work, d_work, 8, cudaMemcpyDeviceToHost, s));
+        CRISPY_TRY(last_of_runs());   // waits
+        if (work > limit) {
+            int64_t again = 0;
+            CRISPY_TRY(compact_flags(ctx, s, j.alive.as<uint8_t>(), n, j.idx.as<uint32_t>(), j.tiles.as<uint32_t>(),
+                                     j.tmp, &again));
+            sort_reads(true);
+            CRISPY_TRY(last_of_runs());
+        }
         pre_emit_kernel<<<(unsigned)((kept + 255) / 256), 256, 0, s>>>(a, j.pos.as<uint32_t>(), kept,
                                                                        j.out_idx.as<int32_t>(),
                                                                        j.out_freq.as<int32_t>());
