@@ -627,11 +627,12 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 // Pairs are binned by band slots; bin 0 is the wide-band kernel.  Bins are
 // fine where bands are common (kBand 31-79 at band 10 on 300-800 nt reads)
 // so that few slots of a pair sit outside its band.
-constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256};
+constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512};
+constexpr int kMaxSlots32 = 256;   // most slots of a 32-bit shape
 constexpr int kNumBins = sizeof(kBinSlots) / sizeof(kBinSlots[0]);
-__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256};
-// the sort key holds the order-bin (up to 2 * kNumBins) in 5 bits
-static_assert(2 * kNumBins < 32, "order-bins overflow the 18-bit sort key");
+__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512};
+// the sort key holds the order-bin (up to 2 * kNumBins) in 6 bits
+static_assert(2 * kNumBins < 64, "order-bins overflow the 18-bit sort key");
 
 // Which diagonals to sweep a pair over.  The narrow sweep -lo .. hi is the
 // whole band's result if its score is above 5 x the diagonal moves of any path
@@ -727,7 +728,7 @@ __global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, cons
 // (it sizes that kernel's tag storage), [kStatWindows + 2w] widest band-slot
 // bin of load window w (kNumBins = wide), [kStatWindows + 2w + 1] 1 when
 // the window holds a pair beyond the 16-bit range.
-constexpr int kOrderBits = 18;   // the sort key: order-bin << 13 | 8191 - sweep end
+constexpr int kOrderBits = 18;   // the sort key: order-bin << 12 | 4095 - sweep end / 2
 constexpr int kStatBins = 2, kStatWindows = 40;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
@@ -758,6 +759,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         for (int b = 1; b < nbins; ++b)
             if (c_bin_slots[b] >= (lo + hi) / 2 + 1) { bin = b; break; }
         lng = l1 + l2 > kGen16MaxSum ? 1 : 0;
+        if (l1 + l2 > max_sum && c_bin_slots[bin] > kMaxSlots32) bin = 0;   // the 32-bit kernel's widest shape
         if (bin != 0 && l1 + l2 <= max_sum) sum_reg = l1 + l2;
         wb = bin == 0 ? nbins : bin;
         ob = bin == 0 ? 2 * nbins : bin + lng * nbins;   // wide pairs sort last
@@ -765,7 +767,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
             int se = 0;
             if (max(1, l2 - hi) <= min(l1, l2 + lo)) se = l2 + min(l1, l2 + lo);
             if (max(1, l1 - lo) <= min(l2, l1 + hi)) se = max(se, l1 + min(l2, l1 + hi));
-            keys[at] = ((uint32_t)ob << 13) | (uint32_t)(8191 - min(se + (lo & 1), 8191));
+            keys[at] = ((uint32_t)ob << 12) | (uint32_t)(4095 - min((se + (lo & 1)) >> 1, 4095));
             vals[at] = (uint32_t)p;
         }
         if (!list) cells = (unsigned long long)band_cells_of(l1, l2, band);
@@ -792,7 +794,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     }
 }
 // untuned 32-bit shape per bin (the plain form always uses it)
-constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13};
+constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13, -1, -1};
 static_assert(kStatMaxSum16 < kStatWindows, "per-bin counters overlap the window slots");
 
 using WarpFn = void (*)(GenArgs);
@@ -856,7 +858,7 @@ int shape_slots(int shape) {
     return kShapes[shape].g * kShapes[shape].c;
 }
 // untuned 16-bit shape per bin (index into gen16's shapes), -1 = none
-constexpr int kDefault16[kNumBins] = {-1, 0, 1, 14, 2, 4, 5, 7, 8, 9, 10, 11, 12, 15, 13};
+constexpr int kDefault16[kNumBins] = {-1, 0, 1, 14, 2, 4, 5, 7, 8, 9, 10, 11, 12, 15, 13, 20, 21};
 int default_shape(int order_bin) {
     if (order_bin >= 1 && order_bin < kNumBins && kDefault16[order_bin] >= 0)
         return kNumShapes + kDefault16[order_bin];
@@ -1286,7 +1288,8 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         a.al = d_al ? d_al + w0 : nullptr;
         const int wb = (int)st[kStatWindows + 2 * w];   // widest band-slot bin (kNumBins = wide)
         const bool lng = st[kStatWindows + 2 * w + 1] != 0;
-        if (mode == CRISPY_MODE_PLAIN || wb >= kNumBins) {
+        // (a window with a pair beyond the 16-bit range runs in 32-bit shapes)
+        if (mode == CRISPY_MODE_PLAIN || wb >= kNumBins || (lng && kBinSlots[wb] > kMaxSlots32)) {
             CRISPY_TRY(launch_wide(ctx, a, kbmax, nullptr, n_items, s, true));
         } else {
             CRISPY_TRY(launch_shape(ctx, s, default_shape(lng ? wb + kNumBins : wb), a, true));

@@ -106,6 +106,9 @@ constexpr int kPlaneWords = kPlanePad + 64 + 2;
 constexpr int kSmWords = 2 * kPlaneWords;
 constexpr int kPairWords = 2 * kSmWords + 4;    // both reads of a pair, 4 words apart in banks
 static_assert(kPairWords % 32 == 4 && kSmWords % 4 == 0, "shared layout");
+// Shared words of a pair: its reads, later at least one 16-step block of tags.
+template <int G, int R>
+constexpr int pair_room() { return 2 * G * R + 4 > kPairWords ? (2 * G * R + 31) / 32 * 32 + 4 : kPairWords; }
 constexpr int kSteps = 16;           // steps per block: 8 cells per slot and parity
 constexpr int kSetupSteps = 32;      // steps per window set-up: 16 cells per slot and parity
 constexpr int kSlack = 32;           // steps a sweep may run past a pair's end
@@ -443,7 +446,7 @@ __device__ __forceinline__ void walk16(const uint32_t* region, uint32_t* stage, 
     constexpr int kBlockWords = 2 * kGR;   // a block: parity 0, parity 1
     constexpr int kBlock4 = kBlockWords / 4;
     constexpr bool kDouble = kSmWords / kBlockWords >= 1;   // two windows of at least a block
-    constexpr int kRoom = kDouble ? kSmWords / kBlockWords : (2 * kSmWords) / kBlockWords;
+    constexpr int kRoom = kDouble ? kSmWords / kBlockWords : (pair_room<G, R>() - 4) / kBlockWords;
     constexpr int kDepth = kRoom < 8 ? kRoom : 8;
     constexpr int kBuf4 = kSmWords / 4;   // uint4 per buffer (double-buffered)
     static_assert(kDepth >= 1 && kGR % 4 == 0, "tag staging");
@@ -536,7 +539,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
     static_assert(R <= 16, "a lane's slot windows must fit one 32-symbol window per read");
     // per pair: read1, read2; a stride of 4 words over 32 banks puts the
     // pairs of a warp, which read the same offsets, in different banks
-    __shared__ __align__(16) uint32_t smem[kWarps][kPerWarp][kPairWords];
+    __shared__ __align__(16) uint32_t smem[kWarps][kPerWarp][pair_room<G, R>()];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / G, gl = lane % G;
     uint32_t* sm1 = smem[warp][sub];
@@ -671,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
 
 constexpr Shape16 kShapes16[] = {{4, 1}, {4, 2}, {4, 4}, {8, 2}, {4, 5}, {4, 6}, {8, 3},
                                  {4, 7}, {8, 4}, {8, 5}, {8, 6}, {16, 4}, {16, 6}, {32, 4},
-                                 {4, 3}, {16, 7}, {16, 1}, {16, 2}, {32, 1}, {32, 2}};
+                                 {4, 3}, {16, 7}, {16, 1}, {16, 2}, {32, 1}, {32, 2}, {32, 6}, {32, 8}};
 constexpr int kNumShapes16 = sizeof(kShapes16) / sizeof(kShapes16[0]);
 constexpr bool shapes_within_max_r() {
     for (const Shape16& h : kShapes16)
@@ -702,7 +705,9 @@ Fn16 fn16(int i) {
         case 16: return gen16_kernel<16, 1>;
         case 17: return gen16_kernel<16, 2>;
         case 18: return gen16_kernel<32, 1>;
-        default: return gen16_kernel<32, 2>;
+        case 19: return gen16_kernel<32, 2>;
+        case 20: return gen16_kernel<32, 6>;
+        default: return gen16_kernel<32, 8>;
     }
 }
 
@@ -715,6 +720,8 @@ Fn16 fn16_ext(int i) {
         case 12: return gen16_kernel<16, 6, true>;
         case 13: return gen16_kernel<32, 4, true>;
         case 15: return gen16_kernel<16, 7, true>;
+        case 20: return gen16_kernel<32, 6, true>;
+        case 21: return gen16_kernel<32, 8, true>;
         default: return nullptr;
     }
 }

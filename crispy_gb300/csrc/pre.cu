@@ -618,7 +618,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
     CRISPY_TRY(ensure(ctx, j.range, (size_t)std::max<int64_t>(m, 1) * sizeof(uint2)));
     unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
-    const unsigned long long limit = 32ull * (unsigned long long)m + 4096;
+    const unsigned long long limit = 64ull * (unsigned long long)m + 4096;
     const unsigned blocks = (unsigned)((m + 255) / 256), wblocks = (unsigned)((m + 7) / 8);
     ReadKey* ka = nullptr;
     // keys first, reads of equal keys settled group by group; or, where the

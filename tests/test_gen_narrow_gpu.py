@@ -140,3 +140,18 @@ def test_long_reads_extended_keys(engine, monkeypatch, narrow_on):
     pairs = np.concatenate([np.array(fixed, np.int32), _random_pairs(n, 240, 46)])
     _check(engine, reads, pairs, (40, 20, 10))
     _check(engine, reads, pairs[:60], (5,))
+
+
+@pytest.mark.parametrize("narrow_on", ["0", "1"])
+def test_bands_beyond_256_slots(engine, monkeypatch, narrow_on):
+    # kBand 250 to 520: the 384- and 512-slot shapes, and the wide-band kernel
+    # beyond them; short runs, and one pair
+    monkeypatch.setenv("CRISPY_GEN_NARROW", narrow_on)
+    reads = synth.make_read_set(synth.ReadSetSpec(70, 3, 1650, "uniform", 1200, 1600, 6, 880))
+    pairs = _random_pairs(len(reads), 120, 47)
+    _check(engine, reads, pairs, (5, 4, 3))
+    _check(engine, reads, pairs[:1], (5,))
+    longr = synth.make_read_set(synth.ReadSetSpec(30, 2, 2100, "uniform", 1850, 2048, 6, 881))
+    _check(engine, longr, _random_pairs(len(longr), 60, 48), (6, 4))
+    short = synth.make_read_set(synth.ReadSetSpec(60, 3, 520, "uniform", 300, 500, 6, 882))
+    _check(engine, short, _random_pairs(len(short), 300, 49), (1,))
