@@ -257,13 +257,31 @@ __global__ void pre_primer_kernel(ReadSet r, int n, const uint8_t* __restrict__ 
     }
 }
 
+// Whether reads of equal keys are so many that comparing the reads throughout
+// costs less than settling them group by group: estimated from the equal
+// neighbours found inside the sorted tiles, of which `tiles` tiles taken
+// together hold about that many times more pairs.
+struct Ties {
+    const unsigned long long* neighbours;
+    unsigned long long tiles, limit;
+    __device__ bool many() const { return 2ull * *neighbours * tiles > limit; }
+};
+__global__ void pre_neighbour_kernel(const ReadKey* __restrict__ keys, int64_t m,
+                                     unsigned long long* __restrict__ neighbours) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool tie = p + 1 < m && (p + 1) % kTile != 0 && key_equal(keys[p], keys[p + 1]);
+    const int c = __popc(__ballot_sync(0xffffffffu, tie));
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(neighbours, (unsigned long long)c);
+}
+
 // Bitonic sort of one tile: keys and indices in shared memory.  With kWhole
 // the reads themselves are looked at where keys agree; a single such pair
 // makes its whole block wait for loads that depend on one another (85 us for
 // 60,000 reads, 152 with all reads compared at every step).
 template <bool kWhole>
 __global__ void __launch_bounds__(kTileThreads) pre_tile_sort_kernel(uint32_t* idx, ReadKey* keys, int64_t m,
-                                                                     ReadSet r) {
+                                                                     ReadSet r, const Ties ties) {
+    if (kWhole && !ties.many()) return;
     __shared__ uint32_t s[kTile];
     __shared__ ReadKey sk[kTile];
     const int64_t base = (int64_t)blockIdx.x * kTile;
@@ -297,10 +315,10 @@ __global__ void __launch_bounds__(kTileThreads) pre_tile_sort_kernel(uint32_t* i
 // position in the merged pair of runs, found by a binary search for the
 // number of smaller reads in the partner run (one load of a key per step
 // unless the reads have to be compared).
-template <bool kWhole>
 __global__ void pre_merge_kernel(const uint32_t* __restrict__ src, const ReadKey* __restrict__ skey,
                                  uint32_t* __restrict__ dst, ReadKey* __restrict__ dkey, int64_t m,
-                                 int64_t width, ReadSet r) {
+                                 int64_t width, ReadSet r, const Ties ties) {
+    const bool whole = ties.many();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const int64_t run = i / width;
@@ -320,7 +338,9 @@ __global__ void pre_merge_kernel(const uint32_t* __restrict__ src, const ReadKey
     }
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
-        if (key_less<kWhole>(r, skey[mid], src[mid], kx, x)) lo = mid + 1;
+        const ReadKey km = skey[mid];
+        const uint32_t xm = src[mid];
+        if (whole ? key_less<true>(r, km, xm, kx, x) : key_less<false>(r, km, xm, kx, x)) lo = mid + 1;
         else hi = mid;
     }
     const int64_t to = base + pos + (lo - p0);
@@ -332,7 +352,8 @@ __global__ void pre_merge_kernel(const uint32_t* __restrict__ src, const ReadKey
 // group's first position adds its comparisons to *work.
 constexpr unsigned kGroupMost = 4096;   // larger groups count as too much work
 __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, uint2* __restrict__ range,
-                                 unsigned long long* __restrict__ work) {
+                                 unsigned long long* __restrict__ work, const Ties ties) {
+    if (ties.many()) return;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -360,16 +381,20 @@ __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, ui
 }
 
 // Each read's place in its group: one warp counts the group's reads that come
-// before it.  Left undone (*work stays above the limit) where comparing within
-// the groups would cost more than the merges.
+// before it.  Left undone (*work is above the limit) where the estimate missed
+// groups so large that the merges are the better way after all.
 __global__ void pre_rank_kernel(const uint32_t* __restrict__ src, const uint2* __restrict__ range, int64_t m, ReadSet r,
                                 const unsigned long long* __restrict__ work, unsigned long long limit,
-                                uint32_t* __restrict__ dst) {
+                                uint32_t* __restrict__ dst, const Ties ties) {
     if (*work > limit) return;
     const int lane = threadIdx.x & 31;
     const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= m) return;
     const uint32_t x = src[p];
+    if (ties.many()) {          // sorted already
+        if (lane == 0) dst[p] = x;
+        return;
+    }
     const uint2 g = range[p];
     unsigned before = 0;
     if (g.y - g.x > 1)
@@ -618,12 +643,17 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
     CRISPY_TRY(ensure(ctx, j.range, (size_t)std::max<int64_t>(m, 1) * sizeof(uint2)));
     unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
-    const unsigned long long limit = 64ull * (unsigned long long)m + 4096;
+    unsigned long long* d_near = d_work + 1;
+    const unsigned long long limit = 256ull * (unsigned long long)m + 4096;
     const unsigned blocks = (unsigned)((m + 255) / 256), wblocks = (unsigned)((m + 7) / 8);
+    const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
     ReadKey* ka = nullptr;
     // keys first, reads of equal keys settled group by group; or, where the
     // groups are large (many copies of a read), the reads compared throughout
     auto sort_reads = [&](bool whole) {
+        // (60,000 reads: settling 64 comparisons a read costs about what the
+        // merges save)
+        const Ties ties{d_near, whole ? 1ull << 32 : tiles, whole ? 0ull : 64ull * (unsigned long long)m + 4096};
         a = j.idx.as<uint32_t>();
         b = j.idx_alt.as<uint32_t>();
         ka = j.keys.as<ReadKey>();
@@ -631,20 +661,18 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
         pre_key_kernel<<<blocks, 256, 0, s>>>(rs, a, m, ka);
         count_launch(ctx);
         if (m < 2) return;
-        const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
-        if (whole) pre_tile_sort_kernel<true><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs);
-        else pre_tile_sort_kernel<false><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs);
-        count_launch(ctx);
+        pre_tile_sort_kernel<false><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs, ties);
+        pre_neighbour_kernel<<<blocks, 256, 0, s>>>(ka, m, d_near);
+        pre_tile_sort_kernel<true><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs, ties);
+        count_launch(ctx, 3);
         for (int64_t w = kTile; w < m; w <<= 1) {
-            if (whole) pre_merge_kernel<true><<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs);
-            else pre_merge_kernel<false><<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs);
+            pre_merge_kernel<<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs, ties);
             count_launch(ctx);
             std::swap(a, b);
             std::swap(ka, kb);
         }
-        if (whole) return;
-        pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, j.range.as<uint2>(), d_work);
-        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, limit, b);
+        pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, j.range.as<uint2>(), d_work, ties);
+        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, whole ? ~0ull : limit, b, ties);
         count_launch(ctx, 2);
         std::swap(a, b);
     };
