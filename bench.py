@@ -392,6 +392,11 @@ def run_ours(args, dist, ws, rank, local):
     single_wf = n_pairs * mean_t / 1024
     kb, kf = st_k.get("kmer_bound_entries", 0), st_k.get("kmer_full_entries", 0)
     bound_pass = kb > 0
+    # K >= 5 at these cuts: the batched run bounds every pair with one 4-bit
+    # contraction on the tensor cores and counts the candidates (the tuner's
+    # report lists such read sets with the contraction's size)
+    filt = next((t for t in tune if t.get("kernel") == "kmer_filter_kernel" and t.get("reads") == n
+                 and t.get("k") == k), None)
     kmer_wf = (kb + kf) / 8 if bound_pass else single_wf
     work = (f"{kmer_wf / n_pairs:.4f} L1 wavefronts per k-mer pair: the level entries the bound pass "
             f"(section 0 of every column) and the full passes (the columns left alive) gather, "
@@ -402,6 +407,19 @@ def run_ours(args, dist, ws, rank, local):
               "frac": kmer_wf / kmer_s / 1e9 / lds_peak_gwf,
               "work_per_unit": work, "traffic": None,
               "peak_source": "measured: crispy_probe_lds128 (conflict-free 128-bit shared gathers), this run"}
+    if filt:
+        flops = 2.0 * filt["dims"] * filt["pairs"]
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        mhz = clk.get("sm_mhz") or 2070.0
+        peak = 2 * 16384 * sms * mhz * 1e6 / 1e12
+        roof_k = {"kernel": "kmer_filter_kernel (+ filter_verify_kernel and the passes between)",
+                  "bound": "tensor_fp4", "unit": "TFLOP/s",
+                  "achieved": flops / kmer_s / 1e12, "peak": peak, "frac": flops / kmer_s / 1e12 / peak,
+                  "work_per_unit": f"2 x {filt['dims']} 4-bit operations per bounded pair "
+                                   f"({filt['pairs']} pairs in tiles, {filt['candidates']} candidates counted exactly)",
+                  "traffic": None, "dims": filt["dims"], "candidates": filt["candidates"],
+                  "peak_source": "16,384 e2m1 multiply-adds per clock and SM (measured issue rate of the "
+                                 "128 x 224 x 64 MMA) x SMs x sampled SM clock"}
     if bound_pass:
         rg = (n + 127) // 128
         items = sum(n - 128 * r for r in range(rg))     # (128-row group, column) pairs
@@ -427,7 +445,8 @@ def run_ours(args, dist, ws, rank, local):
     roof_g = {"kernel": gen_kernel_name, "bound": "int32", "unit": "Gop/s",
               "achieved": gen_ops / gen_s / 1e9, "peak": int_peak_gops,
               "frac": gen_ops / gen_s / 1e9 / int_peak_gops,
-              "work_per_unit": "10 ops per band cell", "traffic": None,
+              "work_per_unit": "10 ops per cell of the whole band (narrow sweeps compute 0.46-0.76 of them)",
+              "traffic": None,
               "peak_source": "measured: crispy_probe_int32 (IADD3/LOP3 chains), this run"}
     # the dense count-vector formulation: 4^k/4 packed count words per read,
     # 2 ops per word and pair (a min and an add)
@@ -437,7 +456,7 @@ def run_ours(args, dist, ws, rank, local):
         "achieved": n_pairs * dense_ops / kmer_s / 1e9, "peak": int_peak_gops,
         "frac": n_pairs * dense_ops / kmer_s / 1e9 / int_peak_gops}
     dominant = roof_g if gen_s >= kmer_s else roof_k
-    _attach_traffic(roof_k, roof_g, n_pairs, cells, k)
+    _attach_traffic(roof_k if not filt else {}, roof_g, n_pairs, cells, k)
     _attach_hbm_view(roof_k, kmer_s)
     _attach_hbm_view(roof_g, gen_s)
 

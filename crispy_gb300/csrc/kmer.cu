@@ -3372,7 +3372,9 @@ int crispy_kmer_run(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* np
                          j.n >= kKmerTuneMinReads && kmer_autotune_enabled() && !kmer_split_env(nullptr);
     if (tunable && !kmer_filter_applies(j, thr)) CRISPY_TRY(kmer_tune_split(ctx, thr));
     CRISPY_TRY(kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr));
-    if (tunable && j.f_pairs > 0) kmer_note_filter(j);
+    if (mode == CRISPY_MODE_BATCHED && ctx->kmer_tune && j.n >= kKmerTuneMinReads && kmer_autotune_enabled() &&
+        j.f_pairs > 0)
+        kmer_note_filter(j);
     return CRISPY_OK;
 }
 
