@@ -626,11 +626,14 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
 // Pairs are binned by band slots; bin 0 is the wide-band kernel.  Bins are
 // fine where bands are common (kBand 31-79 at band 10 on 300-800 nt reads)
-// so that few slots of a pair sit outside its band.
-constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512};
+// so that few slots of a pair sit outside its band.  Up to 1,024 slots (kBand of
+// reads of 2,046 nt at band 2) a register shape takes them: one thread per pair
+// needs about a second for one pair (200 pairs of 1,200-1,600 nt at band 2:
+// 1,750 -> 1.5 ms; 15,000 at band 5: 1,122 -> 4.8 ms).
+constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512, 768, 1024};
 constexpr int kMaxSlots32 = 256;   // most slots of a 32-bit shape
 constexpr int kNumBins = sizeof(kBinSlots) / sizeof(kBinSlots[0]);
-__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512};
+__constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512, 768, 1024};
 // the sort key holds the order-bin (up to 2 * kNumBins) in 6 bits
 static_assert(2 * kNumBins < 64, "order-bins overflow the 18-bit sort key");
 
@@ -729,7 +732,7 @@ __global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, cons
 // bin of load window w (kNumBins = wide), [kStatWindows + 2w + 1] 1 when
 // the window holds a pair beyond the 16-bit range.
 constexpr int kOrderBits = 18;   // the sort key: order-bin << 12 | 4095 - sweep end / 2
-constexpr int kStatBins = 2, kStatWindows = 40;
+constexpr int kStatBins = 2, kStatWindows = 48;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
 // bands: the diagonals each pair is swept over (nullptr: all of its band);
@@ -794,7 +797,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     }
 }
 // untuned 32-bit shape per bin (the plain form always uses it)
-constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13, -1, -1};
+constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13, -1, -1, -1, -1};
 static_assert(kStatMaxSum16 < kStatWindows, "per-bin counters overlap the window slots");
 
 using WarpFn = void (*)(GenArgs);
@@ -858,7 +861,7 @@ int shape_slots(int shape) {
     return kShapes[shape].g * kShapes[shape].c;
 }
 // untuned 16-bit shape per bin (index into gen16's shapes), -1 = none
-constexpr int kDefault16[kNumBins] = {-1, 0, 1, 14, 2, 4, 5, 7, 8, 9, 10, 11, 12, 15, 13, 20, 21};
+constexpr int kDefault16[kNumBins] = {-1, 0, 1, 14, 2, 4, 5, 7, 8, 9, 10, 11, 12, 15, 13, 20, 21, 22, 23};
 int default_shape(int order_bin) {
     if (order_bin >= 1 && order_bin < kNumBins && kDefault16[order_bin] >= 0)
         return kNumShapes + kDefault16[order_bin];
@@ -1025,10 +1028,13 @@ bool gen16_ext_on() {
 // Whether a batched run sweeps narrow bands first: from about 1e9 band cells
 // (0.4 ms) on, where the saved slots outweigh the estimate, its read-back and
 // the second sweep's latency (about 100 us together; 7,000 pairs of 250 nt at
-// band 10 lost 180 us of 460).  CRISPY_GEN_NARROW=0 / 1 forces it off / on.
+// band 10 lost 180 us of 460); and whenever a whole band may be wider than any
+// register shape (the wide-band kernel takes about a second for one such pair).
+// CRISPY_GEN_NARROW=0 / 1 forces it off / on.
 bool narrow_pays(const GenJob& g, int64_t count, int band) {
     if (const char* e = std::getenv("CRISPY_GEN_NARROW")) return e[0] != '0';
     const double half = band >= 2 ? (double)g.max_len / band : (double)g.max_len;
+    if (half >= kBinSlots[kNumBins - 1]) return true;
     return (double)count * half * g.max_len >= 5e8;
 }
 
@@ -1814,15 +1820,17 @@ namespace crispy {
 
 // genDist over a cohort after kmer_run_cohort (server cross-job batching):
 // every job's survivors go through one classification and one set of
-// persistent bin launches (the jobs share every launch); then each job's
-// slice is thresholded, chunked and sorted on its own, with its own
-// threshold, and its chunks (in its own read indices) go to its sink.
+// persistent bin launches (the jobs share every launch); then every pair is
+// held against its job's threshold, one sort puts the survivors in order job
+// by job (gen_finish_cohort; a cohort with a job of more than one load window
+// goes job by job), and each job's chunks, in its own read indices, go to its
+// sink.
 namespace {
 
 // Threshold, sort and delivery of all of a cohort's jobs at once: one
 // compaction, one stable sort by (job, distance) and one read-back, where a
 // job by itself takes ten launches and two waits (27 jobs of 600 reads: about
-// 3 ms).  Each job has at most one load window of pairs, so one chunk.
+// 3 ms; a burst of 32 such jobs 8.5 -> 3.9 ms).  Each job has at most one load window of pairs, so one chunk.
 int gen_finish_cohort(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t total,
                       const std::vector<CohortJob>& jobs, const std::vector<int64_t>& counts,
                       std::vector<int64_t>& gen_counts) {

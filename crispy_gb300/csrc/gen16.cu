@@ -57,7 +57,9 @@
 // No such value can reach the score: the score's cell and every cell of its
 // path are untainted, ties included, and every tainted cell of the last row
 // or column lies below it.  Pairs whose score does not prove this are listed
-// and swept again over the whole band.
+// and swept again over the whole band.  About half the slots are left: 60,000
+// pairs of 250 nt at band 2 take 1.2 ms in place of 2.6, 591,000 pairs of
+// 300-500 nt at band 10 5.0 ms in place of 6.6.
 //
 // Layout.  G lanes per pair, R registers per lane: register r of lane l
 // holds slot l*R + r in its low half and slot G*R + l*R + r in its high
@@ -93,11 +95,13 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
+// (12 and 16 registers a lane, for bands of up to 1,024 slots, take 214 and 254
+// registers and no spills at two blocks per SM.)
 // Blocks per SM for the register budget, counted in warps per SM
 // sub-partition (16K registers each): 3 warps give a lane up to 168
 // registers, 4 up to 128.
 template <int R>
-constexpr int min_blocks16() { return R <= 3 ? 6 : (R == 4 ? 5 : 3); }
+constexpr int min_blocks16() { return R <= 3 ? 6 : R == 4 ? 5 : R <= 8 ? 3 : 2; }
 // A read in shared memory: two bit planes (bit 0 and bit 1 of each symbol's
 // code), 32 symbols per word, each behind kPlanePad zero words (positions
 // down to -192) and before 2 zero tail words.
@@ -125,7 +129,9 @@ static_assert(kBase % 4 == 0, "the score is read back as (K - 4s - kBase) / 4");
 // is below (kFloor - kBaseExt) / 4 - s, which values of at least -2 s reach
 // from s = kFloorFrom on.  A raised cell's path can still gain 5 per diagonal
 // move, (L1 + L2 - s) / 2 of them at the most, so (by the argument for narrow
-// sweeps) a score above floor_bound() is the true one.
+// sweeps) a score above floor_bound() is the true one; the others go to the
+// 32-bit kernel.  12,000 pairs of 1,800-2,048 nt at band 10, a whole
+// run: 10.2 ms in the 32-bit kernel, 5.3 here (with narrow sweeps).
 constexpr int kBaseExt = 65535 - 131 - 14 * (kGen16ExtSum + kSlack);
 constexpr uint32_t kFloor = 128u;
 constexpr int kFloorFrom = (kBaseExt - (int)kFloor) / 4;
@@ -674,14 +680,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
 
 constexpr Shape16 kShapes16[] = {{4, 1}, {4, 2}, {4, 4}, {8, 2}, {4, 5}, {4, 6}, {8, 3},
                                  {4, 7}, {8, 4}, {8, 5}, {8, 6}, {16, 4}, {16, 6}, {32, 4},
-                                 {4, 3}, {16, 7}, {16, 1}, {16, 2}, {32, 1}, {32, 2}, {32, 6}, {32, 8}};
+                                 {4, 3}, {16, 7}, {16, 1}, {16, 2}, {32, 1}, {32, 2}, {32, 6}, {32, 8}, {32, 12},
+                                 {32, 16}};
 constexpr int kNumShapes16 = sizeof(kShapes16) / sizeof(kShapes16[0]);
 constexpr bool shapes_within_max_r() {
     for (const Shape16& h : kShapes16)
-        if (h.r > kGen16MaxR) return false;
+        if (h.r > gen16_max_r(h.g * h.r * 2)) return false;
     return true;
 }
-static_assert(shapes_within_max_r(), "kGen16MaxR bounds every shape's registers");
+static_assert(shapes_within_max_r(), "gen16_max_r bounds every shape's registers");
 
 using Fn16 = void (*)(GenArgs);
 Fn16 fn16(int i) {
@@ -707,7 +714,9 @@ Fn16 fn16(int i) {
         case 18: return gen16_kernel<32, 1>;
         case 19: return gen16_kernel<32, 2>;
         case 20: return gen16_kernel<32, 6>;
-        default: return gen16_kernel<32, 8>;
+        case 21: return gen16_kernel<32, 8>;
+        case 22: return gen16_kernel<32, 12>;
+        default: return gen16_kernel<32, 16>;
     }
 }
 
@@ -722,6 +731,8 @@ Fn16 fn16_ext(int i) {
         case 15: return gen16_kernel<16, 7, true>;
         case 20: return gen16_kernel<32, 6, true>;
         case 21: return gen16_kernel<32, 8, true>;
+        case 22: return gen16_kernel<32, 12, true>;
+        case 23: return gen16_kernel<32, 16, true>;
         default: return nullptr;
     }
 }
@@ -745,8 +756,11 @@ int gen16_grid(crispy_ctx* ctx, int shape, int64_t count, bool ext) {
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ext ? fn16_ext(shape) : fn16(shape), kThreads, 0);
     const int64_t per_block = gen16_pairs_per_block(shape);
-    return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::max(1, per_sm) * ctx->sm_count,
-                                                       (count + per_block - 1) / per_block));
+    // (16 registers a lane on every SM would need a third more tag storage
+    // than any other shape does)
+    const int64_t most = std::min<int64_t>((int64_t)std::max(1, per_sm) * ctx->sm_count,
+                                           ctx->sm_count * gen16_lane_regs_per_sm() / (kThreads * kShapes16[shape].r));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(most, (count + per_block - 1) / per_block));
 }
 }  // namespace
 
@@ -754,6 +768,7 @@ int64_t gen16_lane_regs_per_sm() {
     static const int64_t v = [] {
         int64_t best = 0;
         for (int i = 0; i < kNumShapes16; ++i) {
+            if (kShapes16[i].r > gen16_max_r(0)) continue;   // their grids are held to this bound
             int per_sm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn16(i), kThreads, 0) != cudaSuccess) {
                 cudaGetLastError();

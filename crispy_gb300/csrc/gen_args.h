@@ -59,8 +59,9 @@ int gen16_num_shapes();
 Shape16 gen16_shape(int i);
 // Pairs per block of a shape (all its warps).
 int gen16_pairs_per_block(int i);
-// Registers per lane of the widest shape (bounds the tag storage).
-constexpr int kGen16MaxR = 8;
+// Registers per lane of the shapes a launch of up to `slots` band slots may
+// take, up to twice as wide as it needs (bounds the tag storage).
+constexpr int gen16_max_r(int slots) { return slots > 256 ? 16 : 8; }
 // 16-step blocks a pair's sweep runs at most, for pairs with L1 + L2 <= max_sum.
 inline int gen16_dir_blocks(int max_sum) { return (max_sum + 1) / 16 + 1; }
 // Words of choice storage a launch of shape i over `count` pairs needs.

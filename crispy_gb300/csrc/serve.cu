@@ -99,10 +99,11 @@ size_t estimate_base_bytes(const Job& j) {
 // of L1 + L2 <= 2 maxlen), and never more lanes than
 // 32 per possible pair plus a block.  It depends on the run, not the job:
 // a cohort counts it once.
-size_t tag_bytes(int maxlen, int64_t n, int sms) {
+size_t tag_bytes(int maxlen, int64_t n, int band, int sms) {
     const int64_t pairs = n * (n - 1) / 2;
+    const int slots = (band <= 0 ? maxlen / 2 : maxlen / band) + 1;   // (band 0: the default of 2)
     const int64_t lane_regs = std::min<int64_t>((int64_t)sms * crispy::gen16_lane_regs_per_sm(),
-                                                (32 * pairs + 128) * crispy::kGen16MaxR);
+                                                (32 * pairs + 128) * crispy::gen16_max_r(slots));
     const int64_t blocks = crispy::gen16_dir_blocks(2 * maxlen);
     return (size_t)(2 * lane_regs * 2 * blocks * 4);
 }
@@ -117,7 +118,7 @@ size_t run_bytes(const std::vector<Job*>& js, int sms) {
         maxlen = std::max(maxlen, j->maxlen);
         n += j->n;
     }
-    return base + tag_bytes(maxlen, n, sms);
+    return base + tag_bytes(maxlen, n, js.empty() ? 10 : js[0]->band, sms);
 }
 
 // K = 8: the same-key pass's queue of H sums, per block (one per SM) and
@@ -131,7 +132,7 @@ void set_estimate(Job& j, int sms) {
     j.maxlen = 0;
     for (int i = 0; i < j.n; ++i) j.maxlen = std::max(j.maxlen, j.len[i]);
     j.mem_base = estimate_base_bytes(j) + k8_queue_bytes(j, sms);
-    j.mem = j.mem_base + tag_bytes(j.maxlen, j.n, sms);
+    j.mem = j.mem_base + tag_bytes(j.maxlen, j.n, j.band, sms);
 }
 
 // SMs of a device for the estimates (a GB300's 152 when it cannot be read).

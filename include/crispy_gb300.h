@@ -59,9 +59,11 @@ extern "C" {
  * STAGED   the GB300 kernels (bit-sliced k-mer tiles, warp-cooperative
  *          anti-diagonal DP) launched the plain way: per stage / per window,
  *          one fixed band-tile shape per window.
- * BATCHED  the GB300 kernels as persistent work-queue kernels: row-group
- *          queue for kmerDist, pairs bucketed by band width and length with
- *          autotuned lanes-per-pair and band-tile shape for genDist, launch
+ * BATCHED  the GB300 kernels as persistent work-queue kernels: for kmerDist
+ *          (K >= 5, cuts up to 0.3) an upper bound of every pair on the
+ *          tensor cores and exact counts of the candidates it leaves, else a
+ *          row-group queue of the tile kernels; for genDist pairs bucketed by band width and length with
+ *          autotuned lanes-per-pair and band-tile shape, launch
  *          sequences replayed as CUDA graphs. */
 #define CRISPY_MODE_PLAIN    0
 #define CRISPY_MODE_BATCHED  1
@@ -347,7 +349,9 @@ int crispy_set_timing(crispy_ctx* ctx, int enable);
  * genDist bin (stage "gen": band, band slots, lanes per pair, slots per
  * lane, pairs per block, sample size, best and untuned times) and one per
  * read set whose k-mer bound-pass split was tuned (stage "kmer": reads, K,
- * split in 1/256, sampled row groups, best and default times).  Set
+ * split in 1/256, sampled row groups, best and default times) or that went
+ * through the candidate filter (dimensions, pairs bounded, candidates).
+ * Set
  * CRISPY_AUTOTUNE=0 in the environment to disable tuning.  No reference
  * counterpart. */
 int crispy_tune_report(char* buf, size_t len);
@@ -422,7 +426,8 @@ int crispy_server_cancel(crispy_server* srv, uint64_t job_id);
 int crispy_server_job_memory(crispy_server* srv, uint64_t job_id, size_t* reserved,
                              size_t* needed, int* cohort_size);
 /* The device bytes the server's admission reserves for a job of n reads of
- * these lengths at K = k (no device work). */
+ * these lengths at K = k (no device work; very small jobs whose bands are wider
+ * than 256 slots reserve somewhat more). */
 int crispy_server_job_bytes(const int32_t* lengths, int n, int k, size_t* bytes);
 /* Submit-to-finish latency percentiles (ms) over finished jobs, finished
  * job count and pairs processed (sum of n(n-1)/2). */

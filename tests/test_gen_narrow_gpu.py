@@ -155,3 +155,42 @@ def test_bands_beyond_256_slots(engine, monkeypatch, narrow_on):
     _check(engine, longr, _random_pairs(len(longr), 60, 48), (6, 4))
     short = synth.make_read_set(synth.ReadSetSpec(60, 3, 520, "uniform", 300, 500, 6, 882))
     _check(engine, short, _random_pairs(len(short), 300, 49), (1,))
+
+
+@pytest.mark.parametrize("narrow_on", ["0", "1", None])
+def test_bands_beyond_512_slots(engine, monkeypatch, narrow_on):
+    # kBand 500 to 1,023: the 768- and 1,024-slot shapes at their edges (a band
+    # of one slot more or less on either side of 768 and 1,024), and bands
+    # beyond them, which sweep narrow diagonals first unless told not to
+    if narrow_on is None:
+        monkeypatch.delenv("CRISPY_GEN_NARROW")
+    else:
+        monkeypatch.setenv("CRISPY_GEN_NARROW", narrow_on)
+    rng = np.random.default_rng(883)
+    base = rng.integers(0, 4, 1700)
+    fixed = []
+    for n in (510, 511, 512, 766, 767, 768, 769, 1022, 1023, 1024, 1025):
+        s = base[:n].copy()
+        hit = rng.random(n) < 0.04
+        s[hit] = rng.integers(0, 4, int(hit.sum()))
+        fixed.append(bytes(b"AGTC"[c] for c in s))
+    pairs = np.array([(i, j) for i in range(len(fixed)) for j in range(len(fixed)) if abs(i - j) <= 1], np.int32)
+    _check(engine, fixed, pairs, (1,))
+    reads = synth.make_read_set(synth.ReadSetSpec(60, 3, 1650, "uniform", 1200, 1600, 6, 884))
+    _check(engine, reads, _random_pairs(len(reads), 200, 50), (2,))
+    _check(engine, reads, _random_pairs(len(reads), 1, 51), (2, 1))
+    longr = synth.make_read_set(synth.ReadSetSpec(24, 1, 2100, "uniform", 1850, 2048, 6, 885))
+    _check(engine, longr, _random_pairs(len(longr), 40, 52), (3, 2))
+
+
+def test_server_estimate_wide_bands(monkeypatch):
+    # a few reads whose bands take the widest shapes: the run stays within the
+    # bytes it was admitted with
+    monkeypatch.delenv("CRISPY_GEN_NARROW")
+    reads = synth.make_read_set(synth.ReadSetSpec(40, 2, 1000, "uniform", 800, 1000, 6, 886))
+    buf, offs, lens = synth.pack_reads(reads)
+    with cg.Server(0, 0, 1) as srv:
+        jid = srv.submit(buf, offs, lens, 6, 1, 0.5, 0.5)
+        assert srv.wait(jid) == cg.JOB_DONE
+        mem = srv.job_memory(jid)
+        assert 0 < mem["needed"] <= mem["reserved"], mem
