@@ -8,7 +8,9 @@
 // min-sum  m = sum_k min(cnt_a[k], cnt_b[k]);  dist = 1 - m / min(Ta, Tb) in
 // single precision; a pair survives iff dist < thr or |dist - thr| < 1e-5.
 //
-// GB300 design (no tensor cores: a min-sum is not a dense contraction):
+// GB300 design.  The batched form at K >= 5 bounds the pairs on the tensor
+// cores and counts only the candidates (kmer_filter.cu).  The other forms, small
+// K, loose cuts and sets of reads nearly all alike take the tile kernels here:
 //   * min(a, b) = sum_{t>=1} [a >= t][b >= t].  Every read becomes a list of
 //     T "level entries" (t-1)*4^K + kmer, one per occurrence, where t is the
 //     occurrence rank of that K-mer in the read.  Then

@@ -642,14 +642,19 @@ __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float
 // An item is 128 row positions (a panel) against a run of 224-column tiles.  The rows'
 // signatures stay in shared memory for the whole item (up to 1,024
 // dimensions; longer signatures stream rows and columns together), the
-// columns' pass through a ring of 128-byte-wide TMA boxes.  One thread
-// issues the MMAs into one of two TMEM accumulators while four warps compare
+// columns' pass through two rings of 128-byte-wide TMA boxes, one for each
+// of the two TMEM accumulators and its issuing warp, while twelve warps compare
 // the other one with the rows' thresholds, 32 columns of 32 rows at a time.
 // All block scales are 1.
 //
 // Bound: the 4-bit MMA rate (a 128 x 224 tile of 768 dimensions is 1,344
 // cycles at 16,384 multiply-adds a cycle); the compare costs about 20
 // instructions per 32 x 32 values unless one of them is a candidate.
+// Measured, 99,999 reads of 300-500 nt at K = 6 (5.0e9 pairs, 768 dimensions,
+// 2.70 M candidates): 1.24 ms, 0.59 of that rate (0.97 ms with the compares
+// off, 1.87 ms with one issuing warp); the tile kernel took 7.26 ms.  Eight
+// compare warps 1.32 ms, sixteen 1.24 ms; clusters of one 1.23 ms but 69
+// against 63-70 us for 20,000 reads, of four 1.56 ms.
 template <bool kResident, int kCluster>
 __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const FilterArgs a) {
@@ -955,7 +960,9 @@ int rep_slots_for(int max_t) { return max_t <= 512 ? 256 : max_t <= 1536 ? 512 :
 // through the row's list, so its size costs nothing per row.
 //
 // Bound: the look-ups' shared-memory wavefronts (about 3 per 32 random
-// addresses) and issue slots.
+// addresses) and issue slots.  2.70 M candidates of 400 nt: 0.88 ms (1.3 ms
+// with every repeat looked up and bit marks; 8.5 ms with a hash table per
+// pair and no grouping by row).
 template <bool kBytes, bool kK8>
 __global__ void __launch_bounds__(kVerifyWarps * 32, kK8 ? 3 : 5) filter_verify_kernel(const VerifyArgs a) {
     extern __shared__ __align__(16) uint32_t vsmem[];

@@ -10,6 +10,10 @@
 //   * above: passes of at most 9 bits, as few as the key's bits allow and of
 //     equal width, each a histogram per 4,096-item tile, an exclusive scan
 //     (one warp per digit) and a stable scatter.
+// Bound: launches and their gaps at a few thousand items, L2 traffic above.  With
+// 4 to 7 passes of three launches whatever the size, sorts took 290 of the 708
+// us of kernel time for 1,000 reads; a whole call went from 592 to 460 us, one of
+// 200 alignments from 207 to 170, one of 20,000 reads from 2.09 to 1.94 ms.
 // Ranks come from warp matches on the digit, counted per warp over the warp's
 // own stretch of consecutive items.
 #include <cuda_runtime.h>
