@@ -1253,13 +1253,26 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
         base.ext = ext;
         CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));
         if (!retry) return CRISPY_OK;
-        uint32_t left = 0;
-        CRISPY_CK(ctx, cudaMemcpyAsync(&left, retry, 4, cudaMemcpyDeviceToHost, s));
-        CRISPY_CK(ctx, cudaStreamSynchronize(s));
-        if (left == 0) return CRISPY_OK;
-        CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, kGen16MaxSum, nullptr, retry + 1, st, &d_order));
-        return gen_run_bins(ctx, s, gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al), band,
-                            d_order, st);
+        // the pairs without proof over the whole band: beyond the 16-bit range
+        // in the extended form once more, then what that does not prove
+        bool again = ext && narrow;
+        for (;;) {
+            uint32_t left = 0;
+            CRISPY_CK(ctx, cudaMemcpyAsync(&left, retry, 4, cudaMemcpyDeviceToHost, s));
+            CRISPY_CK(ctx, cudaStreamSynchronize(s));
+            if (left == 0) return CRISPY_OK;
+            CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, again ? max_sum : kGen16MaxSum, nullptr,
+                                    retry + 1, st, &d_order));
+            base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
+            if (again) {
+                CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));   // the list is in d_order now
+                base.retry = retry;
+                base.ext = ext;
+            }
+            CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));
+            if (!again) return CRISPY_OK;
+            again = false;
+        }
     }
     CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, kGen16MaxSum, nullptr, nullptr, st, &d_order));
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;

@@ -129,12 +129,19 @@ static_assert(kBase % 4 == 0, "the score is read back as (K - 4s - kBase) / 4");
 // is below (kFloor - kBaseExt) / 4 - s, which values of at least -2 s reach
 // from s = kFloorFrom on.  A raised cell's path can still gain 5 per diagonal
 // move, (L1 + L2 - s) / 2 of them at the most, so (by the argument for narrow
-// sweeps) a score above floor_bound() is the true one; the others go to the
-// 32-bit kernel.  12,000 pairs of 1,800-2,048 nt at band 10, a whole
-// run: 10.2 ms in the 32-bit kernel, 5.3 here (with narrow sweeps).
+// sweeps) a score above floor_bound() is the true one.  Below that the sweep
+// must not have raised a cell: a cell's value is at least its diagonal
+// predecessor's - 4, so its key falls by at most 8 every two steps, and a
+// diagonal whose key is kFloorClear above the floor at the end of a block has
+// none raised in the next.  The pairs without either proof go to the 32-bit
+// kernel.  12,000 pairs of 1,800-2,048 nt at band 10, a whole
+// run: 10.2 ms in the 32-bit kernel, 5.0 here (with narrow sweeps).  500 pairs at
+// band 5, some unrelated: 1,433 ms with whole bands beyond 256 slots in the
+// wide-band kernel, 170 with only the score as proof, 1.0 with both.
 constexpr int kBaseExt = 65535 - 131 - 14 * (kGen16ExtSum + kSlack);
 constexpr uint32_t kFloor = 128u;
 constexpr int kFloorFrom = (kBaseExt - (int)kFloor) / 4;
+constexpr uint32_t kFloorClear = 128u;   // 8 diagonal moves of a block lose 64, tags and the stored base 34
 static_assert(kBaseExt % 4 == 0 && kBaseExt > (int)kFloor, "extended keys");
 __device__ __forceinline__ int floor_bound(int l1, int l2) {
     return -2 * kFloorFrom + (5 * max(0, l1 + l2 - kFloorFrom) + 1) / 2;
@@ -612,6 +619,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
             st.CP[0][r] = kOut2; st.CP[1][r] = kOut2;
         }
         Best16 col{kRefNegInf, -1}, row{kRefNegInf, -1};
+        uint32_t lowest = 0xFFFFFFFFu;   // of the in-band cells' bases, as blocks end (kExt)
         // the sweep ends at the last in-band cell of the last row or column
         int s_end = -1;
         if (valid) {
@@ -639,9 +647,19 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
                 block16<G, R, kTrack, kExt>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
             else
                 block16<G, R, kStart, kExt>(st, gl, s0, pc, mu, sel0, sel1, col, row, dst);
+            if (kExt && s0 + 2 * kBlock >= kFloorFrom) {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    lowest = __vminu2(lowest, __vminu2(st.K[0][r] | ~st.CP[0][r], st.K[1][r] | ~st.CP[1][r]));
+            }
         }
         col = group_best16<G>(col);
         row = group_best16<G>(row);
+        bool raised = false;   // a cell of the pair may have been raised to the floor
+        if (kExt) {
+            const bool low = (lowest & 0xFFFFu) < kFloor + kFloorClear || (lowest >> 16) < kFloor + kFloorClear;
+            raised = (__ballot_sync(0xffffffffu, low) >> (sub * G) & (0xFFFFFFFFu >> (32 - G))) != 0;
+        }
         const bool use_col = col.m > row.m;   // genKernel.cu:765-768
         const Best16 b = use_col ? col : row;
         // end cell E: last row (l2, at) or last column (at, l1)
@@ -670,7 +688,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
                 int most = INT_MIN / 8;
                 if (pc.lo < kb) most = min(pc.l1 - pc.lo - 1, pc.l2);
                 if (pc.hi < kb) most = max(most, min(pc.l2 - pc.hi - 1, pc.l1));
-                if (b.at < 0 || b.m <= 5 * most || (kExt && b.m <= floor_bound(pc.l1, pc.l2))) a.retry[1 + atomicAdd(a.retry, 1u)] = (uint32_t)p;
+                if (b.at < 0 || b.m <= 5 * most || (kExt && raised && b.m <= floor_bound(pc.l1, pc.l2)))
+                    a.retry[1 + atomicAdd(a.retry, 1u)] = (uint32_t)p;
             }
         }
         __syncwarp();

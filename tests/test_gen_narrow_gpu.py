@@ -194,3 +194,19 @@ def test_server_estimate_wide_bands(monkeypatch):
         assert srv.wait(jid) == cg.JOB_DONE
         mem = srv.job_memory(jid)
         assert 0 < mem["needed"] <= mem["reserved"], mem
+
+
+@pytest.mark.parametrize("narrow_on", ["0", "1"])
+def test_long_unrelated_reads(engine, monkeypatch, narrow_on):
+    # L1 + L2 > 3,600 and scores too low to prove anything: exact because no
+    # cell was raised to the floor, or left to the 32-bit kernel; among them
+    # reads without a symbol in common, whose scores fall the furthest
+    monkeypatch.setenv("CRISPY_GEN_NARROW", narrow_on)
+    rng = np.random.default_rng(887)
+    reads = [bytes(b"AGTC"[c] for c in rng.integers(0, 4, n)) for n in
+             (1801, 1850, 1903, 1957, 2000, 2031, 2047, 2048)]
+    reads += [b"A" * 1900, b"C" * 2048, b"G" * 1999, b"AC" * 1000, b"GT" * 1024, b"A" * 1024 + b"C" * 1024]
+    n = len(reads)
+    pairs = np.array([(i, j) for i in range(n) for j in range(n) if i != j], np.int32)
+    _check(engine, reads, pairs, (40, 10, 5))
+    _check(engine, reads, pairs[::7], (2,))
