@@ -381,17 +381,18 @@ __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, ui
 }
 
 // Each read's place in its group: one warp counts the group's reads that come
-// before it.  Left undone (*work is above the limit) where the estimate missed
-// groups so large that the merges are the better way after all.
+// before it.  Where the estimate missed groups so large that the merges are the
+// better way after all (*work is above the limit) the groups stay unsettled,
+// and dst is the order as it stands: the kernels that follow read it before
+// the host learns that it has to sort again.
 __global__ void pre_rank_kernel(const uint32_t* __restrict__ src, const uint2* __restrict__ range, int64_t m, ReadSet r,
                                 const unsigned long long* __restrict__ work, unsigned long long limit,
                                 uint32_t* __restrict__ dst, const Ties ties) {
-    if (*work > limit) return;
     const int lane = threadIdx.x & 31;
     const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= m) return;
     const uint32_t x = src[p];
-    if (ties.many()) {          // sorted already
+    if (ties.many() || *work > limit) {          // sorted already, or not to be settled here
         if (lane == 0) dst[p] = x;
         return;
     }

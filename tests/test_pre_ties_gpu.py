@@ -1,0 +1,59 @@
+"""preprocess on sets whose sort keys (length, first 28 bytes) tie in groups
+larger than the group-by-group settling takes: the sort has to start again
+from the reads themselves, and every kernel before that decision must see a
+valid order."""
+import numpy as np
+import pytest
+
+import crispy_gb300 as cg
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(eng, tmp_path, reads):
+    path = str(tmp_path / "raw.fa")
+    with open(path, "wb") as f:
+        for i, s in enumerate(reads):
+            f.write(b">r%d\n%b\n" % (i, s))
+    raw = cg.RawReads(path)
+    index, freq, _ = eng.preprocess(raw)
+    raw.close()
+    order = sorted(range(len(reads)), key=lambda i: (len(reads[i]), reads[i], i))
+    want, count = [], []
+    for q, i in enumerate(order):
+        if q and reads[order[q - 1]] == reads[i]:
+            want[-1], count[-1] = i, count[-1] + 1
+        else:
+            want.append(i)
+            count.append(1)
+    assert index.tolist() == want and freq.tolist() == count
+
+
+def _reads(n, kind):
+    rng = np.random.default_rng(n)
+    base = rng.choice(np.frombuffer(b"ACGT", np.uint8), 60)
+    if kind == "alike":
+        return [base.tobytes()] * n
+    out = []     # one key, told apart only behind the 28th byte
+    for _ in range(n):
+        s = base.copy()
+        s[28 + int(rng.integers(0, 31))] = b"ACGT"[int(rng.integers(0, 4))]
+        s[28 + int(rng.integers(0, 31))] = b"ACGTN"[int(rng.integers(0, 5))]
+        out.append(s.tobytes())
+    return out
+
+
+# one tile of 1,024: its groups' work, n * n, passes 256 n + 4,096 from n = 272
+@pytest.mark.parametrize("kind", ["alike", "behind"])
+@pytest.mark.parametrize("n", [2, 271, 272, 300, 1023, 1024, 1025])
+def test_one_group_of_ties(tmp_path, n, kind):
+    reads = _reads(n, kind)
+    eng = cg.Engine(0)          # nothing in its buffers yet
+    try:
+        _run(eng, tmp_path, reads)
+        # buffers that held a larger set's order
+        rng = np.random.default_rng(1)
+        _run(eng, tmp_path, [rng.choice(np.frombuffer(b"ACGT", np.uint8), 40).tobytes() for _ in range(3000)])
+        _run(eng, tmp_path, reads)
+    finally:
+        eng.close()
