@@ -260,11 +260,14 @@ __global__ void pre_primer_kernel(ReadSet r, int n, const uint8_t* __restrict__ 
 // Whether reads of equal keys are so many that comparing the reads throughout
 // costs less than settling them group by group: estimated from the equal
 // neighbours found inside the sorted tiles, of which `tiles` tiles taken
-// together hold about that many times more pairs.
+// together hold about that many times more pairs.  force: the reads are
+// compared throughout, whatever the estimate says (a tile may hold no two
+// equal keys although the set holds thousands of each).
 struct Ties {
     const unsigned long long* neighbours;
     unsigned long long tiles, limit;
-    __device__ bool many() const { return 2ull * *neighbours * tiles > limit; }
+    bool force;
+    __device__ bool many() const { return force || 2ull * *neighbours * tiles > limit; }
 };
 __global__ void pre_neighbour_kernel(const ReadKey* __restrict__ keys, int64_t m,
                                      unsigned long long* __restrict__ neighbours) {
@@ -351,6 +354,7 @@ __global__ void pre_merge_kernel(const uint32_t* __restrict__ src, const ReadKey
 // Groups of equal keys.  One warp per position finds its group's range; the
 // group's first position adds its comparisons to *work.
 constexpr unsigned kGroupMost = 4096;   // larger groups count as too much work
+constexpr unsigned long long kTooMuch = 1ull << 62;   // (the others' squares sum to 2^43 at the most)
 __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, uint2* __restrict__ range,
                                  unsigned long long* __restrict__ work, const Ties ties) {
     if (ties.many()) return;
@@ -375,7 +379,7 @@ __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, ui
     if (lane == 0) {
         range[p] = make_uint2((uint32_t)lo, (uint32_t)hi);
         const unsigned long long g = (unsigned long long)(hi - lo);
-        if (g >= kGroupMost) atomicAdd(work, 1ull << 40);
+        if (g >= kGroupMost) atomicOr(work, kTooMuch);
         else if (lo == p && g > 1) atomicAdd(work, g * g);
     }
 }
@@ -654,7 +658,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     auto sort_reads = [&](bool whole) {
         // (60,000 reads: settling 64 comparisons a read costs about what the
         // merges save)
-        const Ties ties{d_near, whole ? 1ull << 32 : tiles, whole ? 0ull : 64ull * (unsigned long long)m + 4096};
+        const Ties ties{d_near, tiles, 64ull * (unsigned long long)m + 4096, whole};
         a = j.idx.as<uint32_t>();
         b = j.idx_alt.as<uint32_t>();
         ka = j.keys.as<ReadKey>();
@@ -673,7 +677,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
             std::swap(ka, kb);
         }
         pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, j.range.as<uint2>(), d_work, ties);
-        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, whole ? ~0ull : limit, b, ties);
+        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, limit, b, ties);
         count_launch(ctx, 2);
         std::swap(a, b);
     };

@@ -57,3 +57,37 @@ def test_one_group_of_ties(tmp_path, n, kind):
         _run(eng, tmp_path, reads)
     finally:
         eng.close()
+
+
+def test_ties_apart_in_every_tile(tmp_path):
+    # 1,024 heads of 28 bases in turn, 4,200 times, each time with other tails:
+    # no tile of 1,024 holds two equal keys, so the estimate sees no tie, but
+    # every group is larger than those the settling knows the bounds of
+    kinds, copies = 1024, 4200
+    rng = np.random.default_rng(2)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    heads = np.unique(rng.integers(0, 4, (2 * kinds, 28)), axis=0)[:kinds]      # in order
+    turn = rng.permutation(kinds)
+    n = kinds * copies
+    tails = rng.integers(0, 4, (n, 4))
+    rows = np.empty((n, 35), np.uint8)
+    rows[:, :2] = np.frombuffer(b">\n", np.uint8)
+    rows[:, 2:30] = acgt[heads[np.tile(turn, copies)]]
+    rows[:, 30:34] = acgt[tails]
+    rows[:, 34] = 10
+    path = str(tmp_path / "raw.fa")
+    rows.tofile(path)
+    raw = cg.RawReads(path)
+    assert raw.n == n
+    eng = cg.Engine(0)
+    try:
+        index, freq, _ = eng.preprocess(raw)
+    finally:
+        eng.close()
+        raw.close()
+    code = np.tile(turn, copies) * 256 + tails @ np.array([64, 16, 4, 1])       # order of the bytes
+    last = np.zeros(kinds * 256, np.int64)
+    last[code] = np.arange(n)
+    count = np.bincount(code, minlength=kinds * 256)
+    assert np.array_equal(index, last[count > 0])
+    assert np.array_equal(freq, count[count > 0])
