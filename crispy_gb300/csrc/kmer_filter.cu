@@ -414,7 +414,6 @@ constexpr int kChunkA = kRows * 128;       // 256 dimensions of a tile's rows (b
 constexpr int kChunkB = kCols * 128;
 constexpr int kResidentChunks = 4;         // rows stay in shared memory up to 1,024 dimensions
 constexpr int kMaxDepth = 3;               // stages of each of the two rings
-constexpr int kCluster = 2;                // blocks that share the columns' boxes (TMA multicast)
 constexpr int kCandBuf = 96;               // candidates a warp holds before it writes them out
 constexpr int kEpilogueWarps = 12;         // for each quarter of the TMEM lanes:
 constexpr int kEpiPer = kEpilogueWarps / 4;
@@ -424,7 +423,7 @@ constexpr size_t kSmemLimit = 227 * 1024;
 constexpr long long kWaitCycles = 4000000000ll;   // about two seconds
 
 struct FilterArgs {
-    const int4* items;    // (panel group, first column tile, end column tile, -)
+    const int4* items;    // (panel, first column tile, end column tile, -)
     const int* segs;      // first item of each segment, and the end
     int nsegs;
     int chunks;           // 256-dimension chunks of a signature
@@ -493,15 +492,6 @@ __device__ __forceinline__ void tma_load(const CUtensorMap* map, uint32_t dst, i
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)) : "memory");
 }
-// The same box into every block of the cluster (the same offset there, and
-// the same barrier of each).
-__device__ __forceinline__ void tma_load_all(const CUtensorMap* map, uint32_t dst, int x, int y, uint64_t* bar,
-                                             uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
-        "[%0], [%1, {%2, %3}], [%4], %5;"
-        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)), "h"(mask) : "memory");
-}
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
     asm volatile(
@@ -510,10 +500,6 @@ __device__ __forceinline__ bool elect_one() {
         "selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
     return ok != 0;
 }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // K-major operand, 128-byte swizzle: 8-row groups of 1,024 bytes.
 __device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
@@ -533,11 +519,6 @@ __device__ __forceinline__ void mma_mxf4(uint32_t d, uint64_t a, uint64_t b, uin
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  ::"r"(smem_addr(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mma_commit_all(uint64_t* bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_addr(bar)), "h"(mask) : "memory");
 }
 
 #define TMEM_LD32(v, addr)                                                                                   \
@@ -636,7 +617,7 @@ __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float
 }
 
 // One persistent block per SM.  All tiles, panel after panel, are cut into
-// segments of equal length, and each cluster takes every so-many-th segment:
+// segments of equal length, and each block takes every so-many-th segment:
 // the same number of tiles for everyone, from several places of the triangle
 // (items of 64 tiles dealt in turn left the SMs idle for 14 % of the run).
 // An item is 128 row positions (a panel) against a run of 224-column tiles.  The rows'
@@ -653,9 +634,10 @@ __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float
 // Measured, 99,999 reads of 300-500 nt at K = 6 (5.0e9 pairs, 768 dimensions,
 // 2.70 M candidates): 1.24 ms, 0.59 of that rate (0.97 ms with the compares
 // off, 1.87 ms with one issuing warp); the tile kernel took 7.26 ms.  Eight
-// compare warps 1.32 ms, sixteen 1.24 ms; clusters of one 1.23 ms but 69
-// against 63-70 us for 20,000 reads, of four 1.56 ms.
-template <bool kResident, int kCluster>
+// compare warps 1.32 ms, sixteen 1.24 ms.  20,000 reads: 67 us.  Blocks stand
+// alone: pairs and fours that shared the columns' boxes took 1.24 and 1.56 ms
+// (63-70 us for 20,000 reads).
+template <bool kResident>
 __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const FilterArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -668,14 +650,11 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     uint8_t* tail = smem + bytes_a + 2 * a.depth * kStage;
     uint2* cbuf = reinterpret_cast<uint2*>(tail);
     Bars* bars = reinterpret_cast<Bars*>(tail + kEpilogueWarps * kCandBuf * sizeof(uint2));
-    // the cluster's blocks take adjacent panels and the same column tiles
-    const int rank = kCluster > 1 ? (int)(blockIdx.x % kCluster) : 0;
-    const int first = (int)(blockIdx.x / kCluster), stride = (int)(gridDim.x / kCluster);
-    constexpr uint16_t kAll = (uint16_t)((1u << kCluster) - 1u);
+    const int first = (int)blockIdx.x, stride = (int)gridDim.x;
     if (*reinterpret_cast<volatile uint32_t*>(&a.ctl->overflow)) return;   // an earlier round gave up
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2 * a.depth; ++s) { bar_init(&bars->full[s], 1); bar_init(&bars->empty[s], kCluster); }
+        for (int s = 0; s < 2 * a.depth; ++s) { bar_init(&bars->full[s], 1); bar_init(&bars->empty[s], 1); }
         bar_init(&bars->a_full, 1);
         bar_init(&bars->a_empty, 2);
         for (int b = 0; b < 2; ++b) { bar_init(&bars->acc_full[b], 1); bar_init(&bars->acc_empty[b], kEpilogueWarps); }
@@ -703,7 +682,6 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (kCluster > 1) cluster_sync();   // every block's barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (warp == 0) {
@@ -717,7 +695,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
             for (int sg = first; sg < a.nsegs && ok; sg += stride)
             for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
                 const int4 q = __ldg(a.items + it);
-                const int row0 = kRows * (kCluster * q.x + rank);
+                const int row0 = kRows * q.x;
                 if (kResident) {
                     if (!bar_wait(&bars->a_empty, (item & 1) ^ 1, bars, a.ctl)) { ok = false; break; }
                     bar_expect(&bars->a_full, (uint32_t)bytes_a);
@@ -735,20 +713,21 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
                         ++steps[g];
                         const uint32_t dst = ring + slot * kStage;
                         if (!kResident) tma_load(&map_rows, dst + kChunkB, 128 * k, row0, &bars->full[slot]);
-                        if (kCluster == 1) {
-                            tma_load(&map_cols, dst, 128 * k, kCols * t, &bars->full[slot]);
-                        } else {
-                            // this block's share of the columns, to all
-                            constexpr int kPart = kCols / kCluster;
-                            tma_load_all(&map_cols, dst + rank * kPart * 128, 128 * k, kCols * t + rank * kPart,
-                                         &bars->full[slot], kAll);
-                        }
+                        tma_load(&map_cols, dst, 128 * k, kCols * t, &bars->full[slot]);
                         if (++st == depth) { st = 0; ph ^= 1; }
                     }
                     stage[g] = st;
                     phase[g] = ph;
                 }
             }
+            // the tensor cores' last arrivals, which no stage waits for: the
+            // block's shared memory may be another's once it has ended
+            for (uint32_t g = 0; g < 2 && ok; ++g)
+                for (uint32_t s = 0; s < depth && ok; ++s) {
+                    const uint32_t uses = steps[g] / depth + (s < steps[g] % depth ? 1u : 0u);
+                    if (uses > 0) ok = bar_wait(&bars->empty[g * depth + s], (uses - 1) & 1, bars, a.ctl);
+                }
+            if (kResident && ok && item > 0) ok = bar_wait(&bars->a_empty, (item - 1) & 1, bars, a.ctl);
             if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
                 // the block gives up: let the copies in flight land first
                 const long long t0 = clock64();
@@ -792,8 +771,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
 #pragma unroll
                         for (int i = 0; i < 4; ++i)   // 64 dimensions (32 bytes) each
                             mma_mxf4(acc, da + 2 * i, db + 2 * i, scales, scales + 32, k + i > 0);
-                        if (kCluster == 1) mma_commit(&bars->empty[slot0 + stage]);
-                        else mma_commit_all(&bars->empty[slot0 + stage], kAll);
+                        mma_commit(&bars->empty[slot0 + stage]);
                         if (k == a.chunks - 1) mma_commit(&bars->acc_full[mine]);
                     }
                     __syncwarp();
@@ -820,7 +798,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         for (int sg = first; sg < a.nsegs && ok; sg += stride)
         for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it) {
             const int4 q = __ldg(a.items + it);
-            const int row = kRows * (kCluster * q.x + rank) + 32 * part + lane;
+            const int row = kRows * q.x + 32 * part + lane;
             const float rneed = row < a.n ? __ldg(a.need + row) : 1e9f;
             // half a count of slack: S is a multiple of 1/4
             const float rx = row < a.n ? (float)__ldg(a.excess + row) + 0.5f : 0.0f;
@@ -863,7 +841,6 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (kCluster > 1) cluster_sync();   // no block leaves while another may still write to it
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
@@ -1348,26 +1325,21 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     }
     const int plo = k == 8 ? 0 : olo / kRows, phi = k == 8 ? panels : (ohi + kRows - 1) / kRows;
     int64_t work = 0;
-    // groups of kCluster panels: from the first one's rows to the last one's end
-    const int glo = plo / kCluster, ghi = (phi + kCluster - 1) / kCluster;
-    auto first_tile = [&](int g) { return kRows * kCluster * g / kCols; };
-    auto end_tile = [&](int g) {
-        return pend.empty() ? tiles : (pend[std::min(panels, kCluster * (g + 1)) - 1] + kCols - 1) / kCols;
-    };
-    for (int g = glo; g < ghi; ++g) work += end_tile(g) - first_tile(g);
-    // rounds of at most 2^33 pairs; segments: four per cluster and round, at
+    auto first_tile = [&](int p) { return kRows * p / kCols; };
+    auto end_tile = [&](int p) { return pend.empty() ? tiles : (pend[p] + kCols - 1) / kCols; };
+    for (int p = plo; p < phi; ++p) work += end_tile(p) - first_tile(p);
+    // rounds of at most 2^33 pairs; segments: four per block and round, at
     // least one tile each
-    const int64_t pairs = work * kCluster * kRows * kCols;
+    const int64_t pairs = work * kRows * kCols;
     const int rounds = (int)std::min<int64_t>(kMaxRounds, std::max<int64_t>(1, (pairs + (1ll << 33) - 1) >> 33));
-    const int64_t nclusters = ctx->sm_count / kCluster;
-    const int64_t nsegs = std::max<int64_t>(1, std::min<int64_t>(work, 4 * nclusters * rounds));
+    const int64_t nsegs = std::max<int64_t>(1, std::min<int64_t>(work, 4ll * ctx->sm_count * rounds));
     std::vector<int4>& items = j.h_items;
     std::vector<int>& segs = j.h_segs;
     items.clear();
     segs.clear();
     int64_t done = 0;
-    for (int g = glo; g < ghi; ++g) {
-        for (int a = first_tile(g), e = end_tile(g); a < e;) {
+    for (int p = plo; p < phi; ++p) {
+        for (int a = first_tile(p), e = end_tile(p); a < e;) {
             const int64_t seg = (int64_t)segs.size();
             if (done == work * seg / nsegs) {
                 segs.push_back((int)items.size());
@@ -1375,7 +1347,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
             }
             const int64_t left = work * seg / nsegs - done;   // tiles to the end of the open segment
             const int c = (int)std::min<int64_t>(e - a, left);
-            items.push_back(make_int4(g, a, a + c, 0));
+            items.push_back(make_int4(p, a, a + c, 0));
             a += c;
             done += c;
         }
@@ -1401,26 +1373,11 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     const size_t stage = resident ? kChunkB : kChunkA + kChunkB;
     const int depth = (int)std::min<size_t>(kMaxDepth, (kSmemLimit - fixed - bytes_a) / (2 * stage));
     const size_t smem = fixed + bytes_a + 2 * depth * stage;
-    auto kern = resident ? kmer_filter_kernel<true, kCluster> : kmer_filter_kernel<false, kCluster>;
+    auto kern = resident ? kmer_filter_kernel<true> : kmer_filter_kernel<false>;
     CRISPY_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CUtensorMap map_rows, map_cols;
     CRISPY_TRY(signature_map(ctx, &map_rows, j.f_sig.ptr, j.f_dims / 2, n, kRows));
-    CRISPY_TRY(signature_map(ctx, &map_cols, j.f_sig.ptr, j.f_dims / 2, n, kCols / kCluster));
-    // clusters the device holds at once (an odd SM of a cluster of SMs stays idle)
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kCluster;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cfg.blockDim = dim3(kFilterThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.gridDim = dim3(ctx->sm_count / kCluster * kCluster);
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1)
-        clusters = ctx->sm_count / kCluster;
+    CRISPY_TRY(signature_map(ctx, &map_cols, j.f_sig.ptr, j.f_dims / 2, n, kCols));
 
     FilterArgs fa{};
     fa.chunks = chunks;
@@ -1478,8 +1435,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
         fa.segs = reinterpret_cast<const int*>(j.f_items.as<char>() + item_bytes) + i0;
         fa.nsegs = (int)(i1 - i0);
         fa.round = va.round = r;
-        cfg.gridDim = dim3((unsigned)(kCluster * std::min<int64_t>(clusters, i1 - i0)));
-        CRISPY_CK(ctx, cudaLaunchKernelEx(&cfg, kern, map_rows, map_cols, fa));
+        kern<<<(unsigned)std::min<int64_t>(ctx->sm_count, i1 - i0), kFilterThreads, smem, s>>>(map_rows, map_cols, fa);
         filter_count_kernel<<<cgrid, 256, 0, s>>>(va);
         filter_rows_kernel<<<(n + 255) / 256, 256, 0, s>>>(va);
         filter_scatter_kernel<<<cgrid, 256, 0, s>>>(va);
