@@ -205,6 +205,24 @@ double ev_sum_ms(StreamEvents& ev) {
 
 void count_launch(crispy_ctx* ctx, int n) { ctx->stats.kernels_launched += n; }
 
+int open_smem(crispy_ctx* ctx, const void* kernel) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, int> most;   // the device's room less the kernel's static share
+    int bytes = 0;
+    {
+        std::lock_guard<std::mutex> g(mu);
+        auto it = most.find({ctx->device, kernel});
+        if (it == most.end()) {
+            cudaFuncAttributes fa;
+            CRISPY_CK(ctx, cudaFuncGetAttributes(&fa, kernel));
+            it = most.emplace(std::make_pair(ctx->device, kernel), (int)(ctx->smem_optin - fa.sharedSizeBytes)).first;
+        }
+        bytes = it->second;
+    }
+    CRISPY_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    return CRISPY_OK;
+}
+
 void graph_clear(crispy_ctx* ctx) {
     for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second.exec);
     ctx->graphs.clear();

@@ -204,6 +204,14 @@ double ev_sum_ms(StreamEvents& ev);
 // kernel counter (every launch of this library increments it)
 void count_launch(crispy_ctx* ctx, int n = 1);
 
+// Opens a kernel's dynamic shared memory limit to all that its device gives a
+// block.  The limit belongs to the function and is shared by every thread of
+// the process, so it never depends on the job: one thread's smaller job would
+// make another's launch fail.
+int open_smem(crispy_ctx* ctx, const void* kernel);
+template <class F>
+int open_smem(crispy_ctx* ctx, F* kernel) { return open_smem(ctx, reinterpret_cast<const void*>(kernel)); }
+
 // Run a launch sequence through a CUDA graph: the first call with a key
 // enqueues it as it stands, the second captures `enqueue` (which must only
 // enqueue work on s: no host syncs, no allocation) and instantiates it; later

@@ -2748,7 +2748,7 @@ static int kmer_build_entries(crispy_ctx* ctx, int split = -1) {
     } else {
         auto prep = k == 8 ? kmer_prep_kernel<PrepHist12> : kmer_prep_kernel<PrepHist16>;
         const size_t hsmem = k == 8 ? PrepHist12::bytes(K4) : PrepHist16::bytes(K4);
-        CRISPY_CK(ctx, cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+        CRISPY_TRY(open_smem(ctx, prep));
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prep, kPrepThreads, hsmem);
         const int grid = std::min(n, ctx->sm_count * std::max(1, std::min(per_sm, 8)));
@@ -2900,21 +2900,21 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         }
         CRISPY_TRY(ensure(ctx, j.work, (size_t)j.ngroups + 16));
         CRISPY_CK(ctx, cudaMemcpyAsync(j.work.ptr, dense.data(), j.ngroups, cudaMemcpyHostToDevice, s));
-        if (fast) CRISPY_CK(ctx, cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+        if (fast) CRISPY_TRY(open_smem(ctx, tile));
         const char* split_env = std::getenv("CRISPY_KMER_K8_SPLIT");
         split8 = fast && K == 8 && mode == CRISPY_MODE_BATCHED && j.hkeys_ordered &&
                  !(split_env && std::strcmp(split_env, "0") == 0);
         if (split8) {
             tile_h = tile8h_fn_for(B);
-            CRISPY_CK(ctx, cudaFuncSetAttribute(tile_h, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
+            CRISPY_TRY(open_smem(ctx, tile_h));
         }
         const char* queue_env = std::getenv("CRISPY_KMER_K8_QUEUE");
         queue8 = split8 && !(queue_env && std::strcmp(queue_env, "0") == 0);
         if (queue8) {
             tile_s = tile8s_fn_for(B);
-            CRISPY_CK(ctx, cudaFuncSetAttribute(tile_s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem8));
+            CRISPY_TRY(open_smem(ctx, tile_s));
         }
-        CRISPY_CK(ctx, cudaFuncSetAttribute(kmer_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+        CRISPY_TRY(open_smem(ctx, kmer_dense_kernel));
         if (K == 8) {
             perm = j.perm.as<int32_t>();
             loff = j.offp.as<int64_t>();
@@ -3567,7 +3567,7 @@ int kmer_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, std::ve
     const int B = std::max(8, bits_for((uint64_t)j.max_t));
     TileFn tile = tile128_fn_for(B);
     const size_t tsmem = ((size_t)levels * K4 + 32) * (kRows128 / 8);
-    CRISPY_CK(ctx, cudaFuncSetAttribute(tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+    CRISPY_TRY(open_smem(ctx, tile));
     TileArgs ta{};
     ta.ent = j.ent.as<uint32_t>(); ta.gstart = j.gstart.as<int64_t>(); ta.gent = j.gent.as<int32_t>();
     ta.tent = j.tent.as<uint16_t>(); ta.tstart = j.tstart.as<int64_t>(); ta.tgent = j.tgent.as<int32_t>();

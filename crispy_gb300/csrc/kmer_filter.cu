@@ -1260,7 +1260,7 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
                                                         j.t0.as<int32_t>(), n, k, sample, j.f_hist.as<uint32_t>());
     filter_map_kernel<<<1, 1024, 0, s>>>(j.f_hist.as<uint32_t>(), K4, j.f_dims, j.f_map.as<uint16_t>());
     const size_t smem = (size_t)kSigWarps * j.f_dims * 2;
-    CRISPY_CK(ctx, cudaFuncSetAttribute(filter_sig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CRISPY_TRY(open_smem(ctx, filter_sig_kernel));
     filter_sig_kernel<<<std::min((n + kSigWarps - 1) / kSigWarps, ctx->sm_count * 8), kSigWarps * 32, smem, s>>>(
         j.f_packed.as<uint32_t>(), j.f_stride, t, perm, n, k, j.f_dims, j.f_map.as<uint16_t>(),
         j.f_sig.as<uint32_t>(), j.f_excess.as<uint16_t>(), k == 8 ? j.f_nh.as<uint16_t>() : nullptr);
@@ -1269,7 +1269,7 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
     const int words = direct ? K4 / 2 : 1 << slots_log2;
     const size_t lsmem = (size_t)kListWarps * words * 4;
     auto lists = direct ? filter_lists_kernel<true> : filter_lists_kernel<false>;
-    CRISPY_CK(ctx, cudaFuncSetAttribute(lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem));
+    CRISPY_TRY(open_smem(ctx, lists));
     lists<<<std::min((n + kListWarps - 1) / kListWarps, ctx->sm_count * 8), kListWarps * 32, lsmem, s>>>(
         j.f_packed.as<uint32_t>(), j.f_stride, t, perm, n, k, words, 32 - slots_log2, j.f_distinct.as<uint16_t>(),
         j.f_dstride, j.f_meta.as<int4>(), j.f_repeats.as<uint32_t>(), j.f_hist.as<uint32_t>() + K4);
@@ -1374,7 +1374,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     const int depth = (int)std::min<size_t>(kMaxDepth, (kSmemLimit - fixed - bytes_a) / (2 * stage));
     const size_t smem = fixed + bytes_a + 2 * depth * stage;
     auto kern = resident ? kmer_filter_kernel<true> : kmer_filter_kernel<false>;
-    CRISPY_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CRISPY_TRY(open_smem(ctx, kern));
     CUtensorMap map_rows, map_cols;
     CRISPY_TRY(signature_map(ctx, &map_rows, j.f_sig.ptr, j.f_dims / 2, n, kRows));
     CRISPY_TRY(signature_map(ctx, &map_cols, j.f_sig.ptr, j.f_dims / 2, n, kCols));
@@ -1422,7 +1422,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     const size_t vsmem = (size_t)kVerifyWarps * (map_words + va.rep_slots) * 4;
     auto verify = bytes ? filter_verify_kernel<true, false>
                         : k < 8 ? filter_verify_kernel<false, false> : filter_verify_kernel<false, true>;
-    CRISPY_CK(ctx, cudaFuncSetAttribute(verify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vsmem));
+    CRISPY_TRY(open_smem(ctx, verify));
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, verify, kVerifyWarps * 32, vsmem);
     per_sm = std::max(1, per_sm);

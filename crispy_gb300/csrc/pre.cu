@@ -626,7 +626,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
         int threads = (int)std::min<size_t>(256, (size_t)(96 * 1024) / per_thread);
         threads = std::max(32, threads / 32 * 32);
         const size_t smem = per_thread * threads;
-        CRISPY_CK(ctx, cudaFuncSetAttribute(pre_primer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CRISPY_TRY(open_smem(ctx, pre_primer_kernel));
         pre_primer_kernel<<<grid_for(n, threads, 4 * ctx->sm_count), threads, smem, s>>>(
             rs, n, j.primer.as<uint8_t>(), m_primer, o.max_mismatches, j.alive.as<uint8_t>(),
             j.counters.as<unsigned int>());
