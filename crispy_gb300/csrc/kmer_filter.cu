@@ -363,6 +363,13 @@ struct FilterCtl {
     uint32_t pad;
 };
 
+// True once a round's candidates outgrew the buffer or a wait ran out: the
+// kernels of the rounds that follow have nothing to do.
+__device__ __forceinline__ bool pass_ended(const FilterCtl* ctl) {
+    return (*reinterpret_cast<const volatile uint32_t*>(&ctl->overflow) |
+            *reinterpret_cast<const volatile uint32_t*>(&ctl->timeout)) != 0;
+}
+
 // Per position the smallest count that can pass with it as the shorter read
 // (smin), per 32 positions the smallest of these, and at K = 8 whether the
 // read is H-heavy: |H| >= mmin[T], without which no pair of reads with
@@ -436,6 +443,7 @@ struct FilterArgs {
     unsigned long long cap;
     int round;
     FilterCtl* ctl;
+    long long wait;       // cycles a wait may take
 };
 
 struct Bars {
@@ -468,23 +476,43 @@ __device__ __forceinline__ bool bar_try(uint64_t* b, uint32_t parity) {
         : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
     return ok != 0;
 }
-// A wait that gives up after kWaitCycles, or once another warp of the block
-// has: the block then leaves its loops and reports a timeout.
-__device__ __noinline__ bool bar_wait_slow(uint64_t* b, uint32_t parity, Bars* bars, FilterCtl* ctl) {
+// A wait that gives up after `limit` cycles (below 0: the loader's first one at
+// once), or once another thread of the block has: the block then leaves its
+// loops and the run reports a timeout.
+struct Waiter {
+    Bars* bars;
+    FilterCtl* ctl;
+    long long limit;
+};
+__device__ __noinline__ bool bar_wait_slow(uint64_t* b, uint32_t parity, const Waiter w) {
     const long long t0 = clock64();
-    for (uint32_t i = 1; !bar_try(b, parity); ++i) {
-        if (i & 31u) continue;
-        if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) return false;
-        if (clock64() - t0 > kWaitCycles) {
-            *reinterpret_cast<volatile uint32_t*>(&bars->abort) = 1u;
-            atomicOr(&ctl->timeout, 1u);
-            return false;
+    for (uint32_t i = 0;; ++i) {
+        if ((i & 31u) == 0) {
+            if (*reinterpret_cast<volatile uint32_t*>(&w.bars->abort)) return false;
+            if (clock64() - t0 > w.limit) {
+                *reinterpret_cast<volatile uint32_t*>(&w.bars->abort) = 1u;
+                atomicOr(&w.ctl->timeout, 1u);
+                return false;
+            }
         }
+        if (bar_try(b, parity)) return true;
     }
-    return true;
 }
-__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, Bars* bars, FilterCtl* ctl) {
-    return bar_try(b, parity) || bar_wait_slow(b, parity, bars, ctl);
+__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, const Waiter& w) {
+    return (w.limit >= 0 && bar_try(b, parity)) || bar_wait_slow(b, parity, w);
+}
+// The same for a whole warp, which goes on or gives up as one: one lane's
+// limit may run out as another's wait ends, and what follows a wait (elect,
+// TMEM loads) needs all lanes.
+__device__ __forceinline__ bool bar_wait_warp(uint64_t* b, uint32_t parity, const Waiter& w) {
+    uint32_t all;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "vote.sync.all.pred p, p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(all) : "r"(smem_addr(b)), "r"(parity) : "memory");
+    return all != 0 || __all_sync(0xffffffffu, bar_wait_slow(b, parity, w));
 }
 
 __device__ __forceinline__ void tma_load(const CUtensorMap* map, uint32_t dst, int x, int y, uint64_t* bar) {
@@ -632,7 +660,7 @@ __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float
 // cycles at 16,384 multiply-adds a cycle); the compare costs about 20
 // instructions per 32 x 32 values unless one of them is a candidate.
 // Measured, 99,999 reads of 300-500 nt at K = 6 (5.0e9 pairs, 768 dimensions,
-// 2.70 M candidates): 1.24 ms, 0.59 of that rate (0.97 ms with the compares
+// 2.70 M candidates): 1.25 ms, 0.59 of that rate (0.97 ms with the compares
 // off, 1.87 ms with one issuing warp); the tile kernel took 7.26 ms.  Eight
 // compare warps 1.32 ms, sixteen 1.24 ms.  20,000 reads: 67 us.  Blocks stand
 // alone: pairs and fours that shared the columns' boxes took 1.24 and 1.56 ms
@@ -651,7 +679,8 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     uint2* cbuf = reinterpret_cast<uint2*>(tail);
     Bars* bars = reinterpret_cast<Bars*>(tail + kEpilogueWarps * kCandBuf * sizeof(uint2));
     const int first = (int)blockIdx.x, stride = (int)gridDim.x;
-    if (*reinterpret_cast<volatile uint32_t*>(&a.ctl->overflow)) return;   // an earlier round gave up
+    // one thread looks: another block's wait may run out at any moment
+    if (__syncthreads_or(threadIdx.x == 0 && pass_ended(a.ctl))) return;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2 * a.depth; ++s) { bar_init(&bars->full[s], 1); bar_init(&bars->empty[s], 1); }
@@ -684,12 +713,14 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
+    const Waiter wt{bars, a.ctl, a.wait};
+    uint32_t steps[2] = {0, 0}, a_loads = 0;   // loads the loader has started
     if (warp == 0) {
         if (lane == 0) {
             // two rings of stages, for the even and the odd tiles: each ring
             // has one consumer, which meets every phase of its barriers
-            uint32_t stage[2] = {0, 0}, phase[2] = {1, 1}, steps[2] = {0, 0};
-            uint32_t item = 0, a_loads = 0, tile = 0;
+            uint32_t stage[2] = {0, 0}, phase[2] = {1, 1};
+            uint32_t item = 0, tile = 0;
             const uint32_t depth = (uint32_t)a.depth;
             bool ok = true;
             for (int sg = first; sg < a.nsegs && ok; sg += stride)
@@ -697,7 +728,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
                 const int4 q = __ldg(a.items + it);
                 const int row0 = kRows * q.x;
                 if (kResident) {
-                    if (!bar_wait(&bars->a_empty, (item & 1) ^ 1, bars, a.ctl)) { ok = false; break; }
+                    if (!bar_wait(&bars->a_empty, (item & 1) ^ 1, wt)) { ok = false; break; }
                     bar_expect(&bars->a_full, (uint32_t)bytes_a);
                     ++a_loads;
                     for (int k = 0; k < a.chunks; ++k)
@@ -708,7 +739,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
                     uint32_t st = stage[g], ph = phase[g];
                     for (int k = 0; k < a.chunks; ++k) {
                         const uint32_t slot = g * depth + st;
-                        if (!bar_wait(&bars->empty[slot], ph, bars, a.ctl)) { ok = false; break; }
+                        if (!bar_wait(&bars->empty[slot], ph, wt)) { ok = false; break; }
                         bar_expect(&bars->full[slot], kStage);
                         ++steps[g];
                         const uint32_t dst = ring + slot * kStage;
@@ -725,20 +756,9 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
             for (uint32_t g = 0; g < 2 && ok; ++g)
                 for (uint32_t s = 0; s < depth && ok; ++s) {
                     const uint32_t uses = steps[g] / depth + (s < steps[g] % depth ? 1u : 0u);
-                    if (uses > 0) ok = bar_wait(&bars->empty[g * depth + s], (uses - 1) & 1, bars, a.ctl);
+                    if (uses > 0) ok = bar_wait(&bars->empty[g * depth + s], (uses - 1) & 1, wt);
                 }
-            if (kResident && ok && item > 0) ok = bar_wait(&bars->a_empty, (item - 1) & 1, bars, a.ctl);
-            if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
-                // the block gives up: let the copies in flight land first
-                const long long t0 = clock64();
-                for (uint32_t g = 0; g < 2; ++g)
-                    for (uint32_t s = 0; s < depth; ++s) {
-                        const uint32_t uses = steps[g] / depth + (s < steps[g] % depth ? 1u : 0u);
-                        while (uses > 0 && !bar_try(&bars->full[g * depth + s], (uses - 1) & 1) &&
-                               clock64() - t0 < kWaitCycles) {}
-                    }
-                while (a_loads > 0 && !bar_try(&bars->a_full, (a_loads - 1) & 1) && clock64() - t0 < kWaitCycles) {}
-            }
+            if (kResident && ok && item > 0) ok = bar_wait(&bars->a_empty, (item - 1) & 1, wt);
         }
         __syncwarp();
     } else if (warp <= 2) {
@@ -756,14 +776,14 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         for (int sg = first; sg < a.nsegs && ok; sg += stride)
         for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
             const int4 q = __ldg(a.items + it);
-            if (kResident && !bar_wait(&bars->a_full, item & 1, bars, a.ctl)) { ok = false; break; }
+            if (kResident && !bar_wait_warp(&bars->a_full, item & 1, wt)) { ok = false; break; }
             for (int t = q.y; t < q.z && ok; ++t, ++tile) {
                 if ((tile & 1u) != mine) continue;
-                if (!bar_wait(&bars->acc_empty[mine], bphase, bars, a.ctl)) { ok = false; break; }
+                if (!bar_wait_warp(&bars->acc_empty[mine], bphase, wt)) { ok = false; break; }
                 bphase ^= 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int k = 0; k < a.chunks; ++k) {
-                    if (!bar_wait(&bars->full[slot0 + stage], phase, bars, a.ctl)) { ok = false; break; }
+                    if (!bar_wait_warp(&bars->full[slot0 + stage], phase, wt)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t db = desc_b + stage * (kStage >> 4);
                     const uint64_t da = kResident ? desc_a + k * (kChunkA >> 4) : db + (kChunkB >> 4);
@@ -780,12 +800,6 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
             }
             if (ok && kResident && elect_one()) mma_commit(&bars->a_empty);
             __syncwarp();
-        }
-        if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
-            if (elect_one()) mma_commit(&bars->drain);
-            __syncwarp();
-            const long long t0 = clock64();
-            while (!bar_try(&bars->drain, 0) && clock64() - t0 < kWaitCycles) {}
         }
         __syncwarp();
     } else {
@@ -811,8 +825,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
                     const int c = c0 + 32 * kEpiPer * k;
                     need[k] = c < a.n && row < a.n ? fminf(rneed, __ldg(a.cmin + (c >> 5))) - rx : 1e9f;
                 }
-                if (!bar_wait(&bars->acc_full[b], use & 1, bars, a.ctl)) { ok = false; break; }
-                __syncwarp();
+                if (!bar_wait_warp(&bars->acc_full[b], use & 1, wt)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + b * kCols + 32 * lead + ((uint32_t)(32 * part) << 16);
                 // one block of 32 columns on its way while the other is compared
@@ -837,6 +850,25 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         }
         __syncwarp();
         cand_flush(a, mine, (int)min(*reinterpret_cast<volatile uint32_t*>(held), (uint32_t)kCandBuf), lane);
+    }
+    __syncthreads();   // every warp has left its loops
+    if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
+        // the block gives up: let its copies land and its MMAs end first
+        const long long t0 = clock64();
+        if (threadIdx.x == 0) {
+            for (uint32_t g = 0; g < 2; ++g)
+                for (uint32_t s = 0; s < (uint32_t)a.depth; ++s) {
+                    const uint32_t uses = steps[g] / a.depth + (s < steps[g] % a.depth ? 1u : 0u);
+                    while (uses > 0 && !bar_try(&bars->full[g * a.depth + s], (uses - 1) & 1) &&
+                           clock64() - t0 < kWaitCycles) {}
+                }
+            while (a_loads > 0 && !bar_try(&bars->a_full, (a_loads - 1) & 1) && clock64() - t0 < kWaitCycles) {}
+        } else if (warp == 1 || warp == 2) {
+            if (elect_one()) mma_commit(&bars->drain);   // two arrivals
+            __syncwarp();
+            while (!bar_try(&bars->drain, 0) && clock64() - t0 < kWaitCycles) {}
+            __syncwarp();
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -873,9 +905,9 @@ struct VerifyArgs {
     int64_t out_cap;
 };
 
-// True when the round's candidates fit (else the pass has given up).
+// True when the round's candidates are there and fit.
 __device__ __forceinline__ bool round_fits(const VerifyArgs& a, unsigned long long found) {
-    if (*reinterpret_cast<volatile uint32_t*>(&a.ctl->overflow)) return false;
+    if (pass_ended(a.ctl)) return false;
     if (found <= a.cap) return true;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&a.ctl->overflow, 1u);
     return false;
@@ -1389,6 +1421,8 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     fa.cand = j.f_cand.as<uint2>();
     fa.cap = (unsigned long long)ccap;
     fa.ctl = ctl;
+    fa.wait = kWaitCycles;
+    if (const char* e = std::getenv("CRISPY_KMER_WAIT")) fa.wait = std::atoll(e);
     VerifyArgs va{};
     va.cand = fa.cand;
     va.cap = fa.cap;

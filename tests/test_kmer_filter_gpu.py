@@ -106,3 +106,31 @@ def test_filter_many_tiles(engine, monkeypatch, n, length):
     for pairs, d in got[1:]:
         assert np.array_equal(pairs, got[0][0])
         assert np.array_equal(d.view(np.uint32), got[0][1].view(np.uint32))
+
+
+# below 0: every block's loader gives up at its first wait; small limits: somewhere on
+# the way, with copies and matrix instructions in flight, or not at all
+@pytest.mark.parametrize("length", [250, 1400])
+@pytest.mark.parametrize("wait", [-1, 0, 300, 1000, 3000, 10000])
+def test_filter_wait_limit(engine, monkeypatch, wait, length):
+    n, cents = (4000, 100) if length == 250 else (1500, 40)
+    reads = _reads(n, 970 + length, root=length + 20, dist="uniform", a=length - 20, b=length, cents=cents)
+    buf, offs, lens = synth.pack_reads(reads)
+
+    def run():
+        engine.kmer_prepare(buf, offs, lens, 6)
+        return engine.kmer_fetch(engine.kmer_run(0.15, cg.MODE_BATCHED, True), True)
+
+    want = run()
+    monkeypatch.setenv("CRISPY_KMER_WAIT", str(wait))
+    for _ in range(3):
+        try:
+            got = run()
+        except cg.CrispyError as e:
+            assert e.code == cg.E_TIMEOUT
+        else:
+            assert wait >= 0
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    monkeypatch.delenv("CRISPY_KMER_WAIT")
+    got = run()         # the context is as usable as before
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
