@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -100,6 +101,8 @@ struct KmerJob {
     // signatures of the candidate filter (kmer_filter.cu).
     bool ent_ready = false;
     bool f_ready = false;
+    bool f_lists = false;            // the exact lists too
+    float f_gave_up = INFINITY;      // smallest cut at which these reads gave the filter up
     int f_dims = 0;                  // signature dimensions (4 bits each)
     int f_stride = 0;                // words per packed read
     int f_dstride = 0;               // distinct K-mers' room per read
@@ -108,7 +111,7 @@ struct KmerJob {
     DevBuf f_need, f_cmin, f_ctl, f_items, f_cand, f_candidx, f_sorted, f_rows;
     pinned_vector<int32_t> h_pend;
     std::vector<int4> h_items;
-    std::vector<int> h_segs;
+    std::vector<int2> h_segs;
     int64_t f_pairs = 0, f_found = 0;   // last run: pairs bounded, candidates left
 };
 

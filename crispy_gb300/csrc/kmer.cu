@@ -2571,6 +2571,7 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
     }
     j.ngroups = (n + 31) / 32;
     j.ent_ready = j.f_ready = false;
+    j.f_gave_up = INFINITY;
     CRISPY_TRY(ensure(ctx, j.off, (size_t)n * 8));
     CRISPY_TRY(ensure(ctx, j.t0, (size_t)n * 4));
     CRISPY_CK(ctx, cudaMemcpyAsync(j.t0.ptr, j.h_t.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -2830,9 +2831,12 @@ static int kmer_build_entries(crispy_ctx* ctx, int split = -1) {
 
 // sample > 0: a timing run of the batched tile kernel over every sample-th
 // row group (no graph, no dense-kernel rows, survivors left unsorted); its
-// duration goes to *sample_ms.
+// duration goes to *sample_ms.  *gave_up: nothing is done but an attempt of
+// the candidate filter, which these reads do not pay for at this cut (noted in
+// the job); the caller runs again with `again`, which keeps the attempt's
+// figures.
 static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* npairs, int sample,
-                         float* sample_ms) {
+                         float* sample_ms, bool* gave_up = nullptr, bool again = false) {
     if (!ctx) return CRISPY_E_INPUT;
     KmerJob& j = ctx->kmer;
     if (!j.ready) return fail(ctx, CRISPY_E_STATE, "kmer_run before kmer_prepare");
@@ -2841,9 +2845,11 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     if (A <= 0) return fail(ctx, CRISPY_E_UNSUPPORTED, "fewer than 10 reads: the reference has no tile size (arrayDim = 0)");
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
-    ctx->stats = crispy_stats{};
-    ctx->ev_kmer.used = 0;
-    CRISPY_CK(ctx, cudaEventRecord(ctx->t_begin, s));
+    if (!again) {
+        ctx->stats = crispy_stats{};
+        ctx->ev_kmer.used = 0;
+        CRISPY_CK(ctx, cudaEventRecord(ctx->t_begin, s));
+    }
     // the batched form bounds every pair on the tensor cores and counts the
     // candidates exactly, where that pays (kmer_filter.cu); the tile kernels
     // below take everything else, and a run whose candidates are too many
@@ -2935,11 +2941,16 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
         CRISPY_TRY(ensure(ctx, j.counter, 64));
         CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
         if (filter) {
-            bool gave_up = false;
-            CRISPY_TRY(kmer_filter_pass(ctx, olo, ohi, cap, A, sd, total_out, &gave_up));
-            if (!gave_up) return CRISPY_OK;
+            bool too_many = false;
+            CRISPY_TRY(kmer_filter_pass(ctx, olo, ohi, cap, A, sd, total_out, &too_many));
+            if (!too_many) return CRISPY_OK;
             filter = false;
             j.f_pairs = 0;
+            j.f_gave_up = thr;
+            if (olo == 0 && ohi == n && gave_up) {
+                *gave_up = true;
+                return CRISPY_OK;
+            }
             CRISPY_TRY(setup_tiles());
             CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
         }
@@ -3233,6 +3244,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     int64_t total = 0;
     j.spilled = false;
     CRISPY_TRY(run_pass(0, n, cap, &total));
+    if (gave_up && *gave_up) return CRISPY_OK;
     if (sample > 0) {
         j.nsurv = 0;
         return CRISPY_OK;
@@ -3240,6 +3252,7 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     if (total > cap && total <= dev_cap) {
         cap = std::min(dev_cap, total + total / 8 + 1024);
         CRISPY_TRY(run_pass(0, n, cap, &total));
+        if (gave_up && *gave_up) return CRISPY_OK;
         if (total > cap) return fail(ctx, CRISPY_E_STATE, "survivor count changed between passes");
     }
     if (total <= cap) {
@@ -3373,7 +3386,18 @@ int crispy_kmer_run(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* np
     const bool tunable = mode == CRISPY_MODE_BATCHED && ctx->kmer_tune && tile_rows_for(j.k) == kRows128 &&
                          j.n >= kKmerTuneMinReads && kmer_autotune_enabled() && !kmer_split_env(nullptr);
     if (tunable && !kmer_filter_applies(j, thr)) CRISPY_TRY(kmer_tune_split(ctx, thr));
-    CRISPY_TRY(kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr));
+    bool gave_up = false;
+    CRISPY_TRY(kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr, &gave_up));
+    if (gave_up) {
+        if (tunable) {
+            const crispy_stats attempt = ctx->stats;
+            const size_t events = ctx->ev_kmer.used;
+            CRISPY_TRY(kmer_tune_split(ctx, thr));
+            ctx->stats = attempt;
+            ctx->ev_kmer.used = events;
+        }
+        CRISPY_TRY(kmer_run_impl(ctx, thr, mode, dists, npairs, 0, nullptr, nullptr, true));
+    }
     if (mode == CRISPY_MODE_BATCHED && ctx->kmer_tune && j.n >= kKmerTuneMinReads && kmer_autotune_enabled() &&
         j.f_pairs > 0)
         kmer_note_filter(j);

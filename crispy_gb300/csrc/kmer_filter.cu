@@ -240,6 +240,32 @@ __global__ void __launch_bounds__(kSigWarps * 32) filter_sig_kernel(
     }
 }
 
+// Control block of a pass (device): candidate counts per round, then flags.
+constexpr int kMaxRounds = 72;
+struct FilterCtl {
+    unsigned long long cand[kMaxRounds];
+    uint32_t cursor[kMaxRounds];   // sorted candidates handed out, per round
+    uint32_t overflow;    // the candidates are too many
+    uint32_t timeout;     // a bounded wait ran out
+    uint32_t any_heavy;   // K = 8: a read is H-heavy
+    uint32_t pad;
+};
+
+// True once a round's candidates outgrew the buffer (or will) or a wait ran
+// out: the kernels that follow have nothing to do.
+__device__ __forceinline__ bool pass_ended(const FilterCtl* ctl) {
+    return (*reinterpret_cast<const volatile uint32_t*>(&ctl->overflow) |
+            *reinterpret_cast<const volatile uint32_t*>(&ctl->timeout)) != 0;
+}
+
+// After the probe: its candidates against what its share of the tiles may have.
+__device__ __forceinline__ bool probe_says_too_many(FilterCtl* ctl, unsigned long long most) {
+    const bool too_many = ctl->cand[0] > most;
+    if (too_many && blockIdx.x == 0 && threadIdx.x == 0) ctl->overflow = 1u;
+    return too_many;
+}
+__global__ void filter_probe_kernel(FilterCtl* ctl, unsigned long long most) { probe_says_too_many(ctl, most); }
+
 // ---- exact lists --------------------------------------------------------------
 // For the exact count every read is two lists: its distinct K-mers (16 bits
 // each, padded to a multiple of 8 with copies of the first) and its repeats,
@@ -251,6 +277,8 @@ constexpr uint32_t kSlotEmpty = 0xFFFFFFFFu;
 // One warp per position.  Occurrence ranks come from a counter table in
 // shared memory: direct (two 16-bit counters per word) up to K = 6, an
 // open-addressing table (K-mer << 16 | count, load at most 1/2) above.
+// The lists come between the probe and the rest of the pass and look at its
+// candidates, of which there may be `most`.
 // Repeats take the next free words of one array, whose size bounds them all;
 // up to kStaged of a read's are collected on the way (a second pass over the
 // read's distinct K-mers for them cost as much as the first).
@@ -259,7 +287,9 @@ template <bool kDirect>
 __global__ void __launch_bounds__(kListWarps * 32) filter_lists_kernel(
     const uint32_t* __restrict__ packed, int stride, const int32_t* __restrict__ tcount,
     const int32_t* __restrict__ perm, int n, int K, int words, int hshift, uint16_t* __restrict__ distinct,
-    int dstride, int4* __restrict__ meta, uint32_t* __restrict__ repeats, uint32_t* cursor) {
+    int dstride, int4* __restrict__ meta, uint32_t* __restrict__ repeats, uint32_t* cursor, FilterCtl* ctl,
+    unsigned long long most) {
+    if (probe_says_too_many(ctl, most) || pass_ended(ctl)) return;
     extern __shared__ __align__(16) uint32_t tables[];
     __shared__ uint32_t staged_all[kListWarps][kStaged];
     const unsigned full = 0xffffffffu;
@@ -352,24 +382,6 @@ __global__ void __launch_bounds__(kListWarps * 32) filter_lists_kernel(
     }
 }
 
-// Control block of a pass (device): candidate counts per round, then flags.
-constexpr int kMaxRounds = 72;
-struct FilterCtl {
-    unsigned long long cand[kMaxRounds];
-    uint32_t cursor[kMaxRounds];   // sorted candidates handed out, per round
-    uint32_t overflow;    // a round's candidates outgrew the buffer
-    uint32_t timeout;     // a bounded wait ran out
-    uint32_t any_heavy;   // K = 8: a read is H-heavy
-    uint32_t pad;
-};
-
-// True once a round's candidates outgrew the buffer or a wait ran out: the
-// kernels of the rounds that follow have nothing to do.
-__device__ __forceinline__ bool pass_ended(const FilterCtl* ctl) {
-    return (*reinterpret_cast<const volatile uint32_t*>(&ctl->overflow) |
-            *reinterpret_cast<const volatile uint32_t*>(&ctl->timeout)) != 0;
-}
-
 // Per position the smallest count that can pass with it as the shorter read
 // (smin), per 32 positions the smallest of these, and at K = 8 whether the
 // read is H-heavy: |H| >= mmin[T], without which no pair of reads with
@@ -431,7 +443,7 @@ constexpr long long kWaitCycles = 4000000000ll;   // about two seconds
 
 struct FilterArgs {
     const int4* items;    // (panel, first column tile, end column tile, -)
-    const int* segs;      // first item of each segment, and the end
+    const int2* segs;     // items of each segment: first, end
     int nsegs;
     int chunks;           // 256-dimension chunks of a signature
     int depth;            // stages of a ring
@@ -724,7 +736,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
             const uint32_t depth = (uint32_t)a.depth;
             bool ok = true;
             for (int sg = first; sg < a.nsegs && ok; sg += stride)
-            for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
+            for (int it = __ldg(&a.segs[sg].x), end = __ldg(&a.segs[sg].y); it < end && ok; ++it, ++item) {
                 const int4 q = __ldg(a.items + it);
                 const int row0 = kRows * q.x;
                 if (kResident) {
@@ -774,7 +786,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         const uint64_t desc_a = operand_desc(smem0), desc_b = operand_desc(ring + slot0 * kStage);
         const uint32_t acc = tmem + mine * kCols;
         for (int sg = first; sg < a.nsegs && ok; sg += stride)
-        for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it, ++item) {
+        for (int it = __ldg(&a.segs[sg].x), end = __ldg(&a.segs[sg].y); it < end && ok; ++it, ++item) {
             const int4 q = __ldg(a.items + it);
             if (kResident && !bar_wait_warp(&bars->a_full, item & 1, wt)) { ok = false; break; }
             for (int t = q.y; t < q.z && ok; ++t, ++tile) {
@@ -810,7 +822,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         uint32_t tile = 0;
         bool ok = true;
         for (int sg = first; sg < a.nsegs && ok; sg += stride)
-        for (int it = __ldg(a.segs + sg), end = __ldg(a.segs + sg + 1); it < end && ok; ++it) {
+        for (int it = __ldg(&a.segs[sg].x), end = __ldg(&a.segs[sg].y); it < end && ok; ++it) {
             const int4 q = __ldg(a.items + it);
             const int row = kRows * q.x + 32 * part + lane;
             const float rneed = row < a.n ? __ldg(a.need + row) : 1e9f;
@@ -1179,11 +1191,31 @@ int log2_bits(uint64_t v) {
 }  // namespace
 
 namespace {
-// Candidates a round may leave: 1/128 of its pairs and a base for small
-// sets.  Beyond that (sets whose reads are nearly all alike) counting one by
-// one costs more than the tile kernels: a candidate takes about 0.4 ns, the
-// tile kernels 1.5 ps (99,999 reads) to 20 ps (6,000 reads) per pair.
-int64_t candidate_room(int64_t pairs) { return std::min<int64_t>(1 << 24, pairs / 128 + (1 << 20)); }
+// Candidates a round may leave: 1/256 of its pairs and 3.1 M.  Beyond that (one
+// OTU holds a good part of the reads) counting one by one costs more than the
+// tile kernels.  Both cost the same at about 3.9 M candidates for 20,000 reads
+// of 250 nt, 9 M for 50,000, 23 M for 100,000 of 300-500 nt, 6 M for 30,000 of
+// them at K = 7 and 3 M for 12,000 at K = 5.  Whole kmerDist calls, filter
+// against tiles: 20,000 reads in Zipf's proportions (4.0 M) 1,543 and 1,888 us,
+// three tenths of them in one OTU (8.1 M) 2,864 and 2,110; 100,000 with 0.07 in
+// one (15 M) 8.0 and 10.6 ms, with 0.15 (54 M) 22.0 and 13.2.
+// (CRISPY_KMER_CAND sets the room, for tests.)
+int64_t candidate_room(int64_t pairs) {
+    if (const char* e = std::getenv("CRISPY_KMER_CAND")) return std::max(1ll, std::atoll(e));
+    return std::min<int64_t>(std::min<int64_t>(1 << 25, pairs / 256 + (3 << 20)), std::max<int64_t>(pairs, 1));
+}
+
+// Their buffer: a quarter more, so that a set which the probe lets pass by a
+// little does not fail at the end after all.
+int64_t candidate_buffer(int64_t room) { return room + room / 4; }
+
+// The probe: before the rest, one short run of tiles for each block, spread
+// evenly over all of them (it is the run's first work, none of it twice).  If
+// its candidates say that the room will not do, everything behind it ends at
+// once, the exact lists included, and the tile kernels take the reads.  Sets
+// of fewer tiles than this for each block are bounded without one: the whole
+// contraction takes no longer than the rest of the attempt.
+constexpr int64_t kProbeFrom = 16;
 
 // Bins of the fold, in chunks of 256: two per K-mer of a mean read for tight
 // cuts, three for loose ones.  Share of the pairs left as candidates, over
@@ -1212,16 +1244,17 @@ size_t kmer_filter_bytes(const int32_t* len, int n, int k) {
     }
     const int64_t read = 2 * (max_len / 16 + 5) * 4 + dims_for(tuples, n, k, kMostCut) / 2 + (most + 8) * 2 + 64;
     const int64_t pairs = (int64_t)n * (n + 512) / 2;
-    return (size_t)(n * read + tuples * 4 + candidate_room(pairs) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
+    return (size_t)(n * read + tuples * 4 + candidate_buffer(candidate_room(pairs)) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
 }
 
 // Rule: K >= 5 (K = 4 has 256 bins at most, and the bound leaves a third to
 // all of the pairs) and a cut of at most 0.3 (at 0.35 and above 7-30 % of
 // the pairs stay at K = 5, and counting those one by one costs more than the
 // tile kernels).  CRISPY_KMER_FILTER=0 turns
-// it off; so do the variables that pick the tile kernels' own forms.
+// it off; so do the variables that pick the tile kernels' own forms.  Reads
+// that gave it up once do so at every cut as loose while they stay prepared.
 bool kmer_filter_applies(const KmerJob& j, float thr) {
-    if (j.k < 5 || !(thr <= kMostCut) || j.max_t < 1) return false;
+    if (j.k < 5 || !(thr <= kMostCut) || j.max_t < 1 || thr >= j.f_gave_up) return false;
     const char* e = std::getenv("CRISPY_KMER_FILTER");
     if (e && e[0] == '0') return false;
     for (const char* v : {"CRISPY_KMER_SPLIT", "CRISPY_KMER_QFIRE", "CRISPY_KMER_PREP_WARP",
@@ -1230,7 +1263,8 @@ bool kmer_filter_applies(const KmerJob& j, float thr) {
     return true;
 }
 
-// Packed reads, K = 8 read order, fold and signatures of the prepared reads.
+// Packed reads, K = 8 read order, fold and signatures of the prepared reads;
+// their exact lists come with the first pass that needs them.
 int kmer_filter_build(crispy_ctx* ctx, float thr) {
     KmerJob& j = ctx->kmer;
     cudaStream_t s = ctx->stream;
@@ -1240,7 +1274,7 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
     for (int r = 0; r < n; ++r) tuples += j.h_t[r];
     const int dims = dims_for(tuples, n, k, thr);
     if (j.f_ready && j.f_dims == dims) return CRISPY_OK;
-    j.f_ready = false;
+    j.f_ready = j.f_lists = false;
     j.f_dims = dims;
     j.f_stride = ((j.max_len + 15) / 16 + 1 + 3) / 4 * 4;
     j.f_dstride = (j.max_t + 7) / 8 * 8;
@@ -1296,6 +1330,21 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
     filter_sig_kernel<<<std::min((n + kSigWarps - 1) / kSigWarps, ctx->sm_count * 8), kSigWarps * 32, smem, s>>>(
         j.f_packed.as<uint32_t>(), j.f_stride, t, perm, n, k, j.f_dims, j.f_map.as<uint16_t>(),
         j.f_sig.as<uint32_t>(), j.f_excess.as<uint16_t>(), k == 8 ? j.f_nh.as<uint16_t>() : nullptr);
+    count_launch(ctx, 3);
+    CRISPY_CK(ctx, cudaGetLastError());
+    j.f_ready = true;
+    return CRISPY_OK;
+}
+
+namespace {
+// The exact lists of the prepared reads, unless the pass has ended by then.
+int build_lists(crispy_ctx* ctx, FilterCtl* ctl, unsigned long long most) {
+    KmerJob& j = ctx->kmer;
+    cudaStream_t s = ctx->stream;
+    const int n = j.n, k = j.k;
+    const int K4 = 1 << (2 * k);
+    const int32_t* t = k == 8 ? j.f_t.as<int32_t>() : j.t0.as<int32_t>();
+    const int32_t* perm = k == 8 ? j.f_perm.as<int32_t>() : nullptr;
     const bool direct = k <= 6;
     const int slots_log2 = j.max_t <= 512 ? 10 : j.max_t <= 1024 ? 11 : 12;
     const int words = direct ? K4 / 2 : 1 << slots_log2;
@@ -1304,17 +1353,17 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
     CRISPY_TRY(open_smem(ctx, lists));
     lists<<<std::min((n + kListWarps - 1) / kListWarps, ctx->sm_count * 8), kListWarps * 32, lsmem, s>>>(
         j.f_packed.as<uint32_t>(), j.f_stride, t, perm, n, k, words, 32 - slots_log2, j.f_distinct.as<uint16_t>(),
-        j.f_dstride, j.f_meta.as<int4>(), j.f_repeats.as<uint32_t>(), j.f_hist.as<uint32_t>() + K4);
-    count_launch(ctx, 4);
+        j.f_dstride, j.f_meta.as<int4>(), j.f_repeats.as<uint32_t>(), j.f_hist.as<uint32_t>() + K4, ctl, most);
+    count_launch(ctx);
     CRISPY_CK(ctx, cudaGetLastError());
-    j.f_ready = true;
     return CRISPY_OK;
 }
+}  // namespace
 
 // One pass over the pairs whose lower read ID lies in [olo, ohi): survivors
 // in j.keys / j.vals (up to cap), their count in j.counter (cleared by the
-// caller) and *total.  *gave_up: a round's candidates outgrew their buffer;
-// the caller then runs the tile kernels instead.  The threshold tables must
+// caller) and *total.  *gave_up: the candidates are more than their buffer
+// takes; the caller then runs the tile kernels instead.  The threshold tables must
 // be in j.mmin / j.smin.
 int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int sd, int64_t* total,
                      bool* gave_up) {
@@ -1366,32 +1415,46 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     const int rounds = (int)std::min<int64_t>(kMaxRounds, std::max<int64_t>(1, (pairs + (1ll << 33) - 1) >> 33));
     const int64_t nsegs = std::max<int64_t>(1, std::min<int64_t>(work, 4ll * ctx->sm_count * rounds));
     std::vector<int4>& items = j.h_items;
-    std::vector<int>& segs = j.h_segs;
+    std::vector<int2>& segs = j.h_segs;   // the probe's, then the rounds'
     items.clear();
     segs.clear();
-    int64_t done = 0;
+    const int64_t room = candidate_room((pairs + rounds - 1) / rounds), ccap = candidate_buffer(room);
+    const bool probe = work >= kProbeFrom * ctx->sm_count && room * rounds < (int64_t)n * (n - 1) / 2;
+    const int64_t nprobe = probe ? ctx->sm_count : 0;
+    const int64_t probe_run = std::min<int64_t>(8, std::max<int64_t>(1, work / (128ll * ctx->sm_count)));
+    segs.resize(nprobe);
+    int64_t done = 0, probed = 0, probe_tiles = 0;
+    bool open = false;   // the open segment's first tiles go to the probe
     for (int p = plo; p < phi; ++p) {
         for (int a = first_tile(p), e = end_tile(p); a < e;) {
-            const int64_t seg = (int64_t)segs.size();
+            const int64_t seg = (int64_t)segs.size() - nprobe;
             if (done == work * seg / nsegs) {
-                segs.push_back((int)items.size());
+                if (seg > 0) segs.back().y = (int)items.size();
+                segs.push_back(make_int2((int)items.size(), 0));
+                open = probed < nprobe && probed < (seg + 1) * nprobe / nsegs;
                 continue;
             }
             const int64_t left = work * seg / nsegs - done;   // tiles to the end of the open segment
-            const int c = (int)std::min<int64_t>(e - a, left);
+            int c = (int)std::min<int64_t>(e - a, left);
+            if (open) {
+                c = (int)std::min<int64_t>(c, probe_run);
+                segs[probed++] = make_int2((int)items.size(), (int)items.size() + 1);
+                segs.back().x = (int)items.size() + 1;
+                probe_tiles += c;
+                open = false;
+            }
             items.push_back(make_int4(p, a, a + c, 0));
             a += c;
             done += c;
         }
     }
-    segs.push_back((int)items.size());
     if (items.empty()) return CRISPY_OK;
+    segs.back().y = (int)items.size();
     const size_t item_bytes = items.size() * sizeof(int4);
-    CRISPY_TRY(ensure(ctx, j.f_items, item_bytes + segs.size() * sizeof(int)));
+    CRISPY_TRY(ensure(ctx, j.f_items, item_bytes + segs.size() * sizeof(int2)));
     CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.ptr, items.data(), item_bytes, cudaMemcpyHostToDevice, s));
-    CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.as<char>() + item_bytes, segs.data(), segs.size() * sizeof(int),
+    CRISPY_CK(ctx, cudaMemcpyAsync(j.f_items.as<char>() + item_bytes, segs.data(), segs.size() * sizeof(int2),
                                    cudaMemcpyHostToDevice, s));
-    const int64_t ccap = candidate_room((pairs + rounds - 1) / rounds);
     CRISPY_TRY(ensure(ctx, j.f_cand, (size_t)ccap * sizeof(uint2)));
     CRISPY_TRY(ensure(ctx, j.f_candidx, (size_t)ccap * 4));
     CRISPY_TRY(ensure(ctx, j.f_sorted, (size_t)ccap * sizeof(uint2)));
@@ -1463,10 +1526,25 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     ev_begin(ctx, ctx->ev_kmer, s);
     fa.items = j.f_items.as<int4>();
     const int cgrid = std::min((n + 63) / 64, ctx->sm_count * 8);
+    const int2* d_segs = reinterpret_cast<const int2*>(j.f_items.as<char>() + item_bytes);
+    if (probe) {
+        fa.segs = d_segs;
+        fa.nsegs = (int)nprobe;
+        fa.round = 0;
+        kern<<<(unsigned)nprobe, kFilterThreads, smem, s>>>(map_rows, map_cols, fa);
+        count_launch(ctx);
+    }
+    const unsigned long long most = probe ? (unsigned long long)((double)room * rounds * probe_tiles / work) : ~0ull;
+    if (!j.f_lists) {
+        CRISPY_TRY(build_lists(ctx, ctl, most));
+    } else if (probe) {
+        filter_probe_kernel<<<1, 1, 0, s>>>(ctl, most);
+        count_launch(ctx);
+    }
     for (int r = 0; r < rounds; ++r) {
         const int64_t i0 = nsegs * r / rounds, i1 = nsegs * (r + 1) / rounds;
         if (i1 <= i0) continue;
-        fa.segs = reinterpret_cast<const int*>(j.f_items.as<char>() + item_bytes) + i0;
+        fa.segs = d_segs + nprobe + i0;
         fa.nsegs = (int)(i1 - i0);
         fa.round = va.round = r;
         kern<<<(unsigned)std::min<int64_t>(ctx->sm_count, i1 - i0), kFilterThreads, smem, s>>>(map_rows, map_cols, fa);
@@ -1486,11 +1564,10 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
     *total = (int64_t)found;
     if (h.timeout) return fail(ctx, CRISPY_E_TIMEOUT, "k-mer filter: a device-side wait ran out");
+    *gave_up = h.overflow != 0;
+    if (!*gave_up) j.f_lists = true;
     int64_t cand = 0;
-    for (int r = 0; r < rounds; ++r) {
-        cand += (int64_t)h.cand[r];
-        *gave_up |= h.cand[r] > fa.cap;
-    }
+    for (int r = 0; r < rounds; ++r) cand += (int64_t)h.cand[r];
     j.f_pairs += pairs;
     j.f_found += cand;
     return CRISPY_OK;

@@ -1,0 +1,123 @@
+"""Read sets whose candidates are too many for the tensor-core filter: the tile
+kernels take them, with the same survivors.  CRISPY_KMER_CAND sets the room for
+candidates, so that small sets reach every way the filter is given up: by the
+probe before the rest, by a round whose candidates outgrow the room, and in a
+later range of a run whose survivors spill.  kmer_launches counts the rounds of
+the attempt and the tile launch behind it."""
+import numpy as np
+import pytest
+
+import crispy_gb300 as cg
+import oracle
+from crispy_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _reads(n, k, seed, cents, length=250):
+    spec = synth.ReadSetSpec(n + n // 8 + 8, cents, length + 10, "normal", length, 15, k, seed)
+    return synth.make_read_set(spec)[:n]
+
+
+def _run(engine, thr):
+    got = engine.kmer_fetch(engine.kmer_run(thr, cg.MODE_BATCHED, True), True)
+    return got, engine.stats()
+
+
+def _same(got, want):
+    assert np.array_equal(got[0], want[0])
+    assert np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("k", [5, 6, 7, 8])
+def test_round_outgrows_its_room(engine, monkeypatch, k):
+    # fewer tiles than the probe is for: the one round overflows
+    reads = _reads(900, k, 80 + k, 6)
+    buf, offs, lens = synth.pack_reads(reads)
+    want = oracle.kmer_all(buf, offs, lens, k, 0.2)
+    engine.kmer_prepare(buf, offs, lens, k)
+    got, st = _run(engine, 0.2)
+    _same(got, want)
+    assert st["kmer_launches"] == 1                     # the filter alone
+    engine.kmer_prepare(buf, offs, lens, k)
+    monkeypatch.setenv("CRISPY_KMER_CAND", str(max(1, len(want[0]) // 2)))
+    got, st = _run(engine, 0.2)
+    _same(got, want)
+    assert st["kmer_launches"] == 2                     # an attempt, then the tiles
+    got, st = _run(engine, 0.25)                        # looser: no second attempt
+    _same(got, oracle.kmer_all(buf, offs, lens, k, 0.25))
+    assert st["kmer_launches"] == 1
+    monkeypatch.delenv("CRISPY_KMER_CAND")
+    got, st = _run(engine, 0.05)                        # tighter: another attempt
+    _same(got, oracle.kmer_all(buf, offs, lens, k, 0.05))
+    engine.kmer_prepare(buf, offs, lens, k)             # new reads: as at first
+    got, st = _run(engine, 0.2)
+    _same(got, want)
+    assert st["kmer_launches"] == 1
+
+
+@pytest.mark.parametrize("k", [6, 8])
+def test_probe_gives_up(engine, monkeypatch, k):
+    # k = 8: runs of equal H keys wide enough for as many tiles
+    n = 12000 if k == 6 else 14000
+    reads = _reads(n, k, 90 + k, 60 if k == 6 else 2)
+    buf, offs, lens = synth.pack_reads(reads)
+    thr = 0.1 if k == 6 else 0.05
+    monkeypatch.setenv("CRISPY_KMER_FILTER", "0")
+    engine.kmer_prepare(buf, offs, lens, k)
+    want, _ = _run(engine, thr)
+    monkeypatch.setenv("CRISPY_KMER_FILTER", "1")
+    for room in (50, len(want[0]) // 2, 1 << 22):
+        monkeypatch.setenv("CRISPY_KMER_CAND", str(room))
+        engine.kmer_prepare(buf, offs, lens, k)
+        got, st = _run(engine, thr)
+        _same(got, want)
+        if room < len(want[0]):
+            assert st["kmer_launches"] == 2
+        # genDist behind either: its reads come packed or not
+        engine.gen_prepare_from_kmer()
+    assert len(want[0]) > n
+
+
+@pytest.mark.parametrize("k", [6, 8])
+def test_second_range_gives_up(engine, monkeypatch, k):
+    # survivors beyond the device share, the second half of the reads in one
+    # OTU: a range of stage rows may overflow where those before it did not
+    reads = _reads(1400, k, 100 + k, 60)
+    dense = _reads(700, k, 110 + k, 1)
+    reads = synth.preprocess_order(reads) + synth.preprocess_order(dense)
+    buf, offs, lens = synth.pack_reads(reads)
+    thr = 0.15
+    want = oracle.kmer_all(buf, offs, lens, k, thr)
+    monkeypatch.setenv("CRISPY_KMER_DEVICE_PAIRS", str(len(want[0]) // 2))
+    for room in (len(want[0]) // 2, len(want[0]) * 3 // 4, 1 << 22):
+        monkeypatch.setenv("CRISPY_KMER_CAND", str(room))
+        engine.kmer_prepare(buf, offs, lens, k)
+        got, st = _run(engine, thr)
+        assert st["kmer_spilled"] == 1
+        _same(got, want)
+
+
+def test_tuner_behind_a_gave_up_filter(engine, monkeypatch):
+    # the bound pass's split is tuned from the second batched run on, as for
+    # sets the filter never takes
+    monkeypatch.delenv("CRISPY_AUTOTUNE", raising=False)
+    monkeypatch.setenv("CRISPY_KMER_CAND", "1000")
+    reads = _reads(8900, 6, 120, 100)
+    buf, offs, lens = synth.pack_reads(reads)
+
+    def tuned():
+        return [e for e in cg.tune_report()
+                if e.get("stage") == "kmer" and e["reads"] == len(reads) and "candidates" not in e]
+
+    want = None
+    for i in range(3):
+        engine.kmer_prepare(buf, offs, lens, 6)
+        got, st = _run(engine, 0.1)
+        assert st["kmer_launches"] == 2 and (i or st["kmer_bound_entries"] > 0)   # (a tuned split may be 0)
+        want = want or got
+        _same(got, want)
+        assert len(tuned()) == (1 if i else 0)
+    monkeypatch.setenv("CRISPY_KMER_FILTER", "0")
+    engine.kmer_prepare(buf, offs, lens, 6)
+    _same(_run(engine, 0.1)[0], want)
