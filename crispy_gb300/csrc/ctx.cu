@@ -124,18 +124,43 @@ int ensure(crispy_ctx* ctx, DevBuf& b, size_t bytes) {
     if (bytes <= b.bytes && b.ptr) return CRISPY_OK;
     release(ctx, b);
     size_t want = bytes < 256 ? 256 : bytes;
-    if (ctx && ctx->mem_cap && ctx->mem_in_use + want > ctx->mem_cap)
-        return fail(ctx, CRISPY_E_OOM, "device allocation of %zu bytes exceeds the context cap (%zu of %zu in use)",
-                    want, ctx->mem_in_use, ctx->mem_cap);
-    cudaError_t e = cudaMalloc(&b.ptr, want);
+    auto over = [&] { return ctx && ctx->mem_cap && ctx->mem_in_use + want > ctx->mem_cap; };
+    cudaError_t e = over() ? cudaErrorMemoryAllocation : cudaMalloc(&b.ptr, want);
+    if (e == cudaErrorMemoryAllocation && ctx && (ctx->filter_users == 0 || ctx->gen_users == 0)) {
+        // what earlier steps hold and nothing needs any more goes first
+        cudaGetLastError();
+        cudaStreamSynchronize(ctx->stream);
+        if (ctx->filter_users == 0) kmer_filter_release(ctx);
+        if (ctx->gen_users == 0) gen_scratch_release(ctx);
+        e = over() ? cudaErrorMemoryAllocation : cudaMalloc(&b.ptr, want);
+    }
     if (e != cudaSuccess) {
+        cudaGetLastError();
         b.ptr = nullptr;
+        if (over())
+            return fail(ctx, CRISPY_E_OOM, "device allocation of %zu bytes exceeds the context cap (%zu of %zu in use)",
+                        want, ctx->mem_in_use, ctx->mem_cap);
         return fail(ctx, CRISPY_E_OOM, "device allocation of %zu bytes failed: %s", want,
                     cudaGetErrorString(e));
     }
     b.bytes = want;
     if (ctx) ctx->mem_in_use += want;
     return CRISPY_OK;
+}
+
+void kmer_filter_release(crispy_ctx* ctx) {
+    KmerJob& k = ctx->kmer;
+    k.f_ready = k.f_lists = false;
+    for (DevBuf* b : {&k.f_packed, &k.f_hist, &k.f_map, &k.f_sig, &k.f_excess, &k.f_perm, &k.f_t,
+                      &k.f_hkey, &k.f_nh, &k.f_heavy, &k.f_pend, &k.f_need, &k.f_cmin, &k.f_ctl,
+                      &k.f_items, &k.f_cand, &k.f_candidx, &k.f_sorted, &k.f_rows, &k.f_distinct, &k.f_meta,
+                      &k.f_repeats})
+        release(ctx, *b);
+}
+
+void gen_scratch_release(crispy_ctx* ctx) {
+    GenJob& g = ctx->gen;
+    for (DevBuf* b : {&g.bands, &g.retry, &g.dirs, &g.buckets, &g.tune_sample}) release(ctx, *b);
 }
 
 void release(crispy_ctx* ctx, DevBuf& b) {
@@ -320,11 +345,9 @@ int crispy_ctx_trim(crispy_ctx* ctx) {
     for (DevBuf* b : {&k.seq, &k.off, &k.len, &k.t, &k.gstart, &k.gent, &k.ent, &k.cntmax,
                       &k.hinfo, &k.keys, &k.keys_alt, &k.vals, &k.vals_alt, &k.pairs, &k.dists,
                       &k.counter, &k.mmin, &k.smin, &k.work, &k.sort_tmp, &k.tstart, &k.tgent,
-                      &k.tent, &k.bcnt, &k.tgentL, &k.nsec, &k.t0, &k.offp, &k.perm, &k.sq,
-                      &k.f_packed, &k.f_hist, &k.f_map, &k.f_sig, &k.f_excess, &k.f_perm, &k.f_t,
-                      &k.f_hkey, &k.f_nh, &k.f_heavy, &k.f_pend, &k.f_need, &k.f_cmin, &k.f_ctl,
-                      &k.f_items, &k.f_cand, &k.f_candidx, &k.f_sorted, &k.f_rows, &k.f_distinct, &k.f_meta, &k.f_repeats})
+                      &k.tent, &k.bcnt, &k.tgentL, &k.nsec, &k.t0, &k.offp, &k.perm, &k.sq})
         release(ctx, *b);
+    kmer_filter_release(ctx);
     release_host(k.h_spill_pairs);
     release_host(k.h_spill_dists);
     k.spilled = false;

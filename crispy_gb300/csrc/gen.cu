@@ -631,7 +631,8 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 // needs about a second for one pair (200 pairs of 1,200-1,600 nt at band 2:
 // 1,750 -> 1.5 ms; 15,000 at band 5: 1,122 -> 4.8 ms).
 constexpr int kBinSlots[] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512, 768, 1024};
-constexpr int kMaxSlots32 = 256;   // most slots of a 32-bit shape
+constexpr int kMaxSlots32 = 256;    // most slots of a 32-bit shape
+constexpr int kMaxSlots16 = 1024;   // of a 16-bit one (kMaxSlots32 in lean runs)
 constexpr int kNumBins = sizeof(kBinSlots) / sizeof(kBinSlots[0]);
 __constant__ int c_bin_slots[kNumBins] = {0, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 192, 224, 256, 384, 512, 768, 1024};
 // the sort key holds the order-bin (up to 2 * kNumBins) in 6 bits
@@ -738,7 +739,7 @@ constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
 // bands: the diagonals each pair is swept over (nullptr: all of its band);
 // list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
-                                    const int32_t* __restrict__ len, int band, int nbins, int max_sum,
+                                    const int32_t* __restrict__ len, int band, int nbins, int max_sum, int most_slots,
                                     const uint32_t* __restrict__ bands, const uint32_t* __restrict__ list,
                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                     unsigned long long* __restrict__ stats) {
@@ -762,7 +763,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         for (int b = 1; b < nbins; ++b)
             if (c_bin_slots[b] >= (lo + hi) / 2 + 1) { bin = b; break; }
         lng = l1 + l2 > kGen16MaxSum ? 1 : 0;
-        if (l1 + l2 > max_sum && c_bin_slots[bin] > kMaxSlots32) bin = 0;   // the 32-bit kernel's widest shape
+        if (c_bin_slots[bin] > (l1 + l2 > max_sum ? kMaxSlots32 : most_slots)) bin = 0;   // no register shape
         if (bin != 0 && l1 + l2 <= max_sum) sum_reg = l1 + l2;
         wb = bin == 0 ? nbins : bin;
         ob = bin == 0 ? 2 * nbins : bin + lng * nbins;   // wide pairs sort last
@@ -921,7 +922,7 @@ __global__ void gather_stride_kernel(const uint32_t* __restrict__ src, int64_t n
 int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs& a,
                const uint32_t* d_order, int64_t n_items, DevBuf& sample_buf, DevBuf& queue_buf,
                DevBuf& dirs_buf, int* out) {
-    const int few = latency_shape(bin, n_items, ctx->sm_count);
+    const int few = ctx->lean ? -1 : latency_shape(bin, n_items, ctx->sm_count);
     const int dflt = few >= 0 ? few : default_shape(bin);
     *out = dflt;
     if (!autotune_enabled() || n_items < 4096) return CRISPY_OK;
@@ -932,10 +933,11 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tuned.find(key);
         if (it != g_tuned.end()) {
-            *out = it->second.shape;
+            if (!ctx->lean || shape_slots(it->second.shape) <= kMaxSlots32) *out = it->second.shape;
             return CRISPY_OK;
         }
     }
+    if (ctx->lean) return CRISPY_OK;
     // strided sample of the bin (keeps its length spread), taken on the device
     const int64_t want = std::min<int64_t>(n_items, 24576);
     CRISPY_TRY(ensure(ctx, sample_buf, (size_t)want * 4));
@@ -1057,7 +1059,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
     auto classify = [&]() -> int {
         CRISPY_CK(ctx, cudaMemsetAsync(d_stats, 0, (size_t)nstats * 8, s));
         gen_classify_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, max_sum, bands, list,
+            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, max_sum, ctx->lean ? kMaxSlots32 : kMaxSlots16, bands, list,
             sorted ? g.ckeys.as<uint32_t>() : nullptr, sorted ? g.cvals.as<uint32_t>() : nullptr, d_stats);
         count_launch(ctx);
         if (sorted) {
@@ -1075,7 +1077,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
             (uint64_t)(uintptr_t)g.len.ptr, (uint64_t)(uintptr_t)d_stats, (uint64_t)(uintptr_t)g.ckeys.ptr,
             (uint64_t)(uintptr_t)g.ckeys_alt.ptr, (uint64_t)(uintptr_t)g.cvals.ptr,
             (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr, (uint64_t)(uintptr_t)bands,
-            (uint64_t)(uintptr_t)list, (uint64_t)max_sum});
+            (uint64_t)(uintptr_t)list, (uint64_t)max_sum, (uint64_t)ctx->lean});
         CRISPY_TRY(graph_run(ctx, s, key, classify));
         *d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
     } else {
@@ -1128,7 +1130,7 @@ int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band,
         // a bin too small to fill the chip joins the next one of the same
         // kernel, up to twice its slots: two short launches side by side cost
         // more than one (1,300 and 5,200 pairs of 250 nt: 330 -> 230 us a run)
-        if (!runs.empty() && runs.back().n < kSmallBin && ob != kWideOrderBin &&
+        if (!ctx->lean && !runs.empty() && runs.back().n < kSmallBin && ob != kWideOrderBin &&
             (runs.back().ob < kNumBins) == (ob < kNumBins)) {
             const int a = runs.back().ob, base_bin = ob < kNumBins ? 0 : kNumBins;
             if (kBinSlots[ob - base_bin] <= 2 * kBinSlots[a - base_bin]) {
@@ -1212,18 +1214,17 @@ int gen_run_bins(crispy_ctx* ctx, cudaStream_t s, const GenArgs& base, int band,
 // diagonals it is likely to need first and the few pairs whose score does not
 // prove the result over the whole band after that.
 // kdist (may be nullptr): the pairs' K-mer distances at K = kdist_k.
-int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count,
-                      int band, int mode, float* d_dist, int32_t* d_score, int32_t* d_ml,
-                      int32_t* d_al, const float* kdist = nullptr, int kdist_k = 0) {
+static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count,
+                             int band, int mode, float* d_dist, int32_t* d_score, int32_t* d_ml,
+                             int32_t* d_al, const float* kdist, int kdist_k) {
     GenJob& g = ctx->gen;
-    if (count <= 0) return CRISPY_OK;
     std::vector<unsigned long long> st;
     uint32_t* d_order = nullptr;
     if (mode == CRISPY_MODE_BATCHED) {
         // (a forced shape sweeps whole bands, up to the shape's full width)
-        const bool narrow = forced_shape() < 0 && narrow_pays(g, count, band);
+        const bool narrow = !ctx->lean && forced_shape() < 0 && narrow_pays(g, count, band);
         // pairs beyond the 16-bit range: its extended form first
-        const bool ext = forced_shape() < 0 && 2 * g.max_len > kGen16MaxSum && gen16_ext_on();
+        const bool ext = !ctx->lean && forced_shape() < 0 && 2 * g.max_len > kGen16MaxSum && gen16_ext_on();
         const int max_sum = ext ? kGen16ExtSum : kGen16MaxSum;
         uint32_t *bands = nullptr, *retry = nullptr;
         if (narrow || ext) {
@@ -1317,6 +1318,32 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
     }
     CRISPY_CK(ctx, cudaGetLastError());
     return CRISPY_OK;
+}
+
+// The same, once more in the lean forms where memory does not do for the others.
+int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count,
+                      int band, int mode, float* d_dist, int32_t* d_score, int32_t* d_ml,
+                      int32_t* d_al, const float* kdist = nullptr, int kdist_k = 0) {
+    if (count <= 0) return CRISPY_OK;
+    const crispy_stats before = ctx->stats;
+    const size_t events = ctx->ev_gen.used;
+    auto run = [&]() -> int {
+        ++ctx->gen_users;
+        const int rc = gen_dispatch_form(ctx, s, d_pairs, count, band, mode, d_dist, d_score, d_ml, d_al, kdist, kdist_k);
+        --ctx->gen_users;
+        return rc;
+    };
+    int rc = run();
+    if (rc != CRISPY_E_OOM || ctx->lean) return rc;
+    for (int k = 0; k < 2; ++k) CRISPY_CK(ctx, cudaStreamSynchronize(ctx->side[k]));
+    CRISPY_CK(ctx, cudaStreamSynchronize(s));
+    gen_scratch_release(ctx);
+    ctx->stats = before;
+    ctx->ev_gen.used = events;
+    ctx->lean = true;
+    rc = run();
+    ctx->lean = false;
+    return rc;
 }
 
 }  // namespace crispy
@@ -1481,16 +1508,27 @@ int crispy_gen_prepare_from_kmer(crispy_ctx* ctx) {
     g.ready = false;
     const int n = j.n;
     g.n = n;
-    if (j.f_ready) {
-        // the k-mer run left the reads packed, a fixed stride each: a copy,
-        // and lengths and offsets written on the device
+    // the k-mer run may have left the reads packed, a fixed stride each
+    const size_t fwords = (size_t)n * j.f_stride;
+    auto packed_room = [&]() -> int {
+        CRISPY_TRY(ensure(ctx, g.len, (size_t)n * 4));
+        CRISPY_TRY(ensure(ctx, g.woff, (size_t)(n + 1) * 8));
+        return ensure(ctx, g.packed, (fwords + 4) * 4);
+    };
+    bool copy = j.f_ready;
+    if (copy) {
+        ++ctx->filter_users;
+        const int rc = packed_room();
+        --ctx->filter_users;
+        if (rc == CRISPY_E_OOM) copy = false;
+        else CRISPY_TRY(rc);
+    }
+    if (copy) {
+        // a copy, and lengths and offsets written on the device
         if (j.min_len <= 0) return fail(ctx, CRISPY_E_INPUT, "a read is empty");
         g.max_len = j.max_len;
         cudaStream_t s = ctx->stream;
-        const size_t words = (size_t)n * j.f_stride;
-        CRISPY_TRY(ensure(ctx, g.len, (size_t)n * 4));
-        CRISPY_TRY(ensure(ctx, g.woff, (size_t)(n + 1) * 8));
-        CRISPY_TRY(ensure(ctx, g.packed, (words + 4) * 4));
+        const size_t words = fwords;
         CRISPY_CK(ctx, cudaMemcpyAsync(g.packed.ptr, j.f_packed.ptr, words * 4, cudaMemcpyDeviceToDevice, s));
         gen_stride_kernel<<<(n + 256) / 256, 256, 0, s>>>(j.t0.as<int32_t>(), n, j.k, j.f_stride,
                                                           g.len.as<int32_t>(), g.woff.as<int64_t>());

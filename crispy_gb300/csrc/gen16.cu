@@ -704,7 +704,7 @@ constexpr Shape16 kShapes16[] = {{4, 1}, {4, 2}, {4, 4}, {8, 2}, {4, 5}, {4, 6},
 constexpr int kNumShapes16 = sizeof(kShapes16) / sizeof(kShapes16[0]);
 constexpr bool shapes_within_max_r() {
     for (const Shape16& h : kShapes16)
-        if (h.r > gen16_max_r(h.g * h.r * 2)) return false;
+        if (h.r > gen16_max_r(h.g * h.r * 2) || (h.g * h.r * 2 <= 256 && h.r > kGen16LeanR)) return false;
     return true;
 }
 static_assert(shapes_within_max_r(), "gen16_max_r bounds every shape's registers");
@@ -778,16 +778,17 @@ int gen16_grid(crispy_ctx* ctx, int shape, int64_t count, bool ext) {
     // (16 registers a lane on every SM would need a third more tag storage
     // than any other shape does)
     const int64_t most = std::min<int64_t>((int64_t)std::max(1, per_sm) * ctx->sm_count,
-                                           ctx->sm_count * gen16_lane_regs_per_sm() / (kThreads * kShapes16[shape].r));
+                                           ctx->sm_count * gen16_lane_regs_per_sm(1024) / (kThreads * kShapes16[shape].r));
     return (int)std::max<int64_t>(1, std::min<int64_t>(most, (count + per_block - 1) / per_block));
 }
 }  // namespace
 
-int64_t gen16_lane_regs_per_sm() {
-    static const int64_t v = [] {
+int64_t gen16_lane_regs_per_sm(int slots) {
+    auto most = [](int slots) {
         int64_t best = 0;
         for (int i = 0; i < kNumShapes16; ++i) {
             if (kShapes16[i].r > gen16_max_r(0)) continue;   // their grids are held to this bound
+            if (2 * kShapes16[i].g * kShapes16[i].r > slots) continue;
             int per_sm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn16(i), kThreads, 0) != cudaSuccess) {
                 cudaGetLastError();
@@ -796,8 +797,9 @@ int64_t gen16_lane_regs_per_sm() {
             best = std::max<int64_t>(best, (int64_t)per_sm * kThreads * kShapes16[i].r);
         }
         return best;
-    }();
-    return v;
+    };
+    static const int64_t all = most(1024), narrow = most(256);
+    return slots > 256 ? all : narrow;
 }
 
 int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks, bool ext) {

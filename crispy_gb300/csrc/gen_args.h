@@ -64,13 +64,15 @@ int gen16_pairs_per_block(int i);
 constexpr int gen16_max_r(int slots) { return slots > 256 ? 16 : 8; }
 // 16-step blocks a pair's sweep runs at most, for pairs with L1 + L2 <= max_sum.
 inline int gen16_dir_blocks(int max_sum) { return (max_sum + 1) / 16 + 1; }
+constexpr int kGen16LeanR = 7;   // of the shapes of up to 256 slots
 // Words of choice storage a launch of shape i over `count` pairs needs.
 int64_t gen16_dir_words(crispy_ctx* ctx, int shape, int64_t count, int dir_blocks, bool ext = false);
 // Narrowest shape with an extended form that covers the slots, -1: none.
 int gen16_ext_shape(int slots);
-// Largest resident threads x registers per lane of one SM over the shapes:
-// a launch holds at most this many tag words per SM and sub-block.
-int64_t gen16_lane_regs_per_sm();
+// Largest resident threads x registers per lane of one SM over the shapes of
+// up to `slots` band slots: a launch holds at most this many tag words per SM
+// and sub-block.
+int64_t gen16_lane_regs_per_sm(int slots);
 // Launch shape i over a.count pairs: persistent grid sized by occupancy.
 int gen16_launch(crispy_ctx* ctx, cudaStream_t s, int shape, const GenArgs& a, bool timed);
 

@@ -179,6 +179,12 @@ struct crispy_ctx {
     // server's contexts: every job is a new read set, and tuning one costs
     // more than it saves)
     bool kmer_tune = true;
+    // runs take the forms that need least device memory: no candidate filter,
+    // whole bands, no 16-bit shapes beyond 256 slots or for pairs beyond the
+    // 16-bit range (server jobs that would not fit the budget otherwise)
+    bool lean = false;
+    int filter_users = 0;    // > 0: the candidate filter's buffers are in use
+    int gen_users = 0;       // > 0: genDist's scratch is
     size_t mem_cap = 0;      // 0 = unlimited
     size_t mem_in_use = 0;   // bytes held by DevBuf allocations
     // device bytes the current run has asked for (each buffer's largest
@@ -194,6 +200,11 @@ namespace crispy {
 int fail(crispy_ctx* ctx, int code, const char* fmt, ...);
 int cuda_fail(crispy_ctx* ctx, cudaError_t e, const char* what, const char* file, int line);
 int ensure(crispy_ctx* ctx, DevBuf& b, size_t bytes);
+// Gives back the candidate filter's buffers (the next run that wants them
+// builds them again).
+void kmer_filter_release(crispy_ctx* ctx);
+// The same for the scratch of genDist's launches.
+void gen_scratch_release(crispy_ctx* ctx);
 int ensure_host(crispy_ctx* ctx, HostBuf& b, size_t bytes);
 void release(DevBuf& b);
 void release(crispy_ctx* ctx, DevBuf& b);

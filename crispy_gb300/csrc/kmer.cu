@@ -2853,15 +2853,42 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     // the batched form bounds every pair on the tensor cores and counts the
     // candidates exactly, where that pays (kmer_filter.cu); the tile kernels
     // below take everything else, and a run whose candidates are too many
-    bool filter = mode == CRISPY_MODE_BATCHED && sample == 0 && kmer_filter_applies(j, thr);
+    bool filter = mode == CRISPY_MODE_BATCHED && sample == 0 && !ctx->lean && kmer_filter_applies(j, thr);
     j.f_pairs = j.f_found = 0;
-    if (filter) CRISPY_TRY(kmer_filter_build(ctx, thr));
+    // Without room for the filter's buffers, or for others beside them, the
+    // tile kernels take the reads.
+    struct Hold {
+        crispy_ctx* c;
+        bool on;
+        Hold(crispy_ctx* ctx, bool hold) : c(ctx), on(hold) { if (on) ++c->filter_users; }
+        ~Hold() { drop(); }
+        void drop() { if (on) --c->filter_users; on = false; }
+    } hold(ctx, filter);
+    auto drop_filter = [&]() -> int {
+        CRISPY_CK(ctx, cudaStreamSynchronize(s));
+        hold.drop();
+        kmer_filter_release(ctx);
+        filter = false;
+        j.f_pairs = 0;
+        return CRISPY_OK;
+    };
+    auto want = [&](DevBuf& b, size_t bytes) -> int {
+        const int rc = ensure(ctx, b, bytes);
+        if (rc != CRISPY_E_OOM || !filter) return rc;
+        CRISPY_TRY(drop_filter());
+        return ensure(ctx, b, bytes);
+    };
+    if (filter) {
+        const int rc = kmer_filter_build(ctx, thr);
+        if (rc == CRISPY_E_OOM) CRISPY_TRY(drop_filter());
+        else CRISPY_TRY(rc);
+    }
     const int sd = (n + A - 1) / A;
 
     std::vector<uint16_t> mmin, smin;
     build_mmin(thr, j.max_t, mmin, smin);
-    CRISPY_TRY(ensure(ctx, j.mmin, mmin.size() * 2));
-    CRISPY_TRY(ensure(ctx, j.smin, smin.size() * 2));
+    CRISPY_TRY(want(j.mmin, mmin.size() * 2));
+    CRISPY_TRY(want(j.smin, smin.size() * 2));
     CRISPY_CK(ctx, cudaMemcpyAsync(j.mmin.ptr, mmin.data(), mmin.size() * 2, cudaMemcpyHostToDevice, s));
     CRISPY_CK(ctx, cudaMemcpyAsync(j.smin.ptr, smin.data(), smin.size() * 2, cudaMemcpyHostToDevice, s));
 
@@ -2893,7 +2920,10 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     TileFn tile_h = nullptr, tile_s = tile;
     const int32_t* perm = nullptr;
     const int64_t* loff = j.off.as<int64_t>();
+    bool tiles_ready = false;
     auto setup_tiles = [&]() -> int {
+        if (tiles_ready) return CRISPY_OK;
+        tiles_ready = true;
         CRISPY_TRY(kmer_build_entries(ctx));
         dense.assign(j.ngroups, 0);
         for (int rg = 0; rg < nrg; ++rg) {
@@ -2934,26 +2964,31 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     // *total.  Without a read order the kernels cover the rows [olo, ohi);
     // with one they cover every row and emit() keeps the range.
     auto run_pass = [&](int olo, int ohi, int64_t cap, int64_t* total_out) -> int {
-        CRISPY_TRY(ensure(ctx, j.keys, (size_t)cap * 8));
-        CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)cap * 8));
-        CRISPY_TRY(ensure(ctx, j.vals, (size_t)cap * 4));
-        CRISPY_TRY(ensure(ctx, j.vals_alt, (size_t)cap * 4));
-        CRISPY_TRY(ensure(ctx, j.counter, 64));
+        CRISPY_TRY(want(j.keys, (size_t)cap * 8));
+        CRISPY_TRY(want(j.keys_alt, (size_t)cap * 8));
+        CRISPY_TRY(want(j.vals, (size_t)cap * 4));
+        CRISPY_TRY(want(j.vals_alt, (size_t)cap * 4));
+        CRISPY_TRY(want(j.counter, 64));
         CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
         if (filter) {
             bool too_many = false;
-            CRISPY_TRY(kmer_filter_pass(ctx, olo, ohi, cap, A, sd, total_out, &too_many));
-            if (!too_many) return CRISPY_OK;
+            const int rc = kmer_filter_pass(ctx, olo, ohi, cap, A, sd, total_out, &too_many);
+            if (rc == CRISPY_OK && !too_many) return CRISPY_OK;
+            if (rc == CRISPY_E_OOM) CRISPY_TRY(drop_filter());
+            else CRISPY_TRY(rc);
             filter = false;
             j.f_pairs = 0;
-            j.f_gave_up = thr;
-            if (olo == 0 && ohi == n && gave_up) {
-                *gave_up = true;
-                return CRISPY_OK;
+            if (too_many) {
+                j.f_gave_up = thr;
+                if (olo == 0 && ohi == n && gave_up) {
+                    *gave_up = true;
+                    return CRISPY_OK;
+                }
             }
-            CRISPY_TRY(setup_tiles());
+            hold.drop();
             CRISPY_CK(ctx, cudaMemsetAsync(j.counter.ptr, 0, 64, s));
         }
+        CRISPY_TRY(setup_tiles());
         const int rlo = perm ? 0 : olo, rhi = perm ? n : ohi;
 
         TileArgs ta{};
@@ -3224,9 +3259,9 @@ static int kmer_run_impl(crispy_ctx* ctx, float thr, int mode, int dists, int64_
     };
     // sort + decode the j.nsurv keys of the last pass into j.pairs / j.dists
     auto finish_pass = [&]() -> int {
-        CRISPY_TRY(ensure(ctx, j.pairs, (size_t)std::max<int64_t>(j.nsurv, 1) * 8));
-        CRISPY_TRY(ensure(ctx, j.dists, (size_t)std::max<int64_t>(j.nsurv, 1) * 4));
-        CRISPY_TRY(ensure(ctx, j.sort_tmp, sort_tmp_bytes(j.nsurv)));
+        CRISPY_TRY(want(j.pairs, (size_t)std::max<int64_t>(j.nsurv, 1) * 8));
+        CRISPY_TRY(want(j.dists, (size_t)std::max<int64_t>(j.nsurv, 1) * 4));
+        CRISPY_TRY(want(j.sort_tmp, sort_tmp_bytes(j.nsurv)));
         if (mode == CRISPY_MODE_BATCHED && j.nsurv > 0) {
             const std::string key = "ksort," + key_of({(uint64_t)j.nsurv, (uint64_t)key_bits,
                 (uint64_t)n, (uint64_t)(uintptr_t)j.keys.ptr, (uint64_t)(uintptr_t)j.keys_alt.ptr,

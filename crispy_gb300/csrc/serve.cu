@@ -59,6 +59,7 @@ struct Job {
     int n = 0, k = 6, band = 10;
     float kthr = -1, gthr = -1;
     int maxlen = 0;
+    bool lean = false;     // in the forms that need least memory: the others do not fit the budget
     size_t mem_base = 0;   // estimate without the genDist cell tags
     size_t mem = 0;        // estimate of a lone run
     int state = CRISPY_JOB_QUEUED;
@@ -76,7 +77,8 @@ struct Job {
 };
 
 // Device bytes a job needs at its peak apart from the genDist cell tags
-// (generous; the server only uses it for admission).
+// (generous; the server only uses it for admission), in its lean forms
+// without the candidate filter and narrow sweeps.
 size_t estimate_base_bytes(const Job& j) {
     size_t reads = j.bases.size() + (size_t)j.n * 16;
     int64_t t = 0;
@@ -86,25 +88,25 @@ size_t estimate_base_bytes(const Job& j) {
     const size_t groups = (size_t)(j.n + 31) / 32;
     const size_t entries = (size_t)(2 * t + 32LL * (16 + 40) * groups) * 4 + (size_t)j.n * 136;
     const size_t survivors = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * 24;
-    const size_t gen = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * 56 + reads;
+    const size_t gen = (size_t)std::max<int64_t>(1 << 20, 16LL * j.n) * (j.lean ? 48 : 56) + reads;
     // the candidate filter's buffers, beside the entries a run that gives it
     // up needs as well
-    const size_t filter = crispy::kmer_filter_bytes(j.len.data(), j.n, j.k);
+    const size_t filter = j.lean ? 0 : crispy::kmer_filter_bytes(j.len.data(), j.n, j.k);
     return 2 * reads + entries + filter + survivors + gen + (8u << 20);
 }
 
 // Bytes of the 16-bit DP's cell tags a run over n reads of at most maxlen
 // symbols may ask for: two launches in flight, each holding one word per
 // resident lane, register and sub-block (two per 16-step block, for pairs
-// of L1 + L2 <= 2 maxlen), and never more lanes than
-// 32 per possible pair plus a block.  It depends on the run, not the job:
-// a cohort counts it once.
-size_t tag_bytes(int maxlen, int64_t n, int band, int sms) {
+// of L1 + L2 <= 2 maxlen, kGen16MaxSum in the lean forms), and never more
+// lanes than 32 per possible pair plus a block.  It depends on the run, not
+// the job: a cohort counts it once.
+size_t tag_bytes(int maxlen, int64_t n, int band, bool lean, int sms) {
     const int64_t pairs = n * (n - 1) / 2;
     const int slots = (band <= 0 ? maxlen / 2 : maxlen / band) + 1;   // (band 0: the default of 2)
-    const int64_t lane_regs = std::min<int64_t>((int64_t)sms * crispy::gen16_lane_regs_per_sm(),
-                                                (32 * pairs + 128) * crispy::gen16_max_r(slots));
-    const int64_t blocks = crispy::gen16_dir_blocks(2 * maxlen);
+    const int64_t lane_regs = std::min<int64_t>((int64_t)sms * crispy::gen16_lane_regs_per_sm(lean ? 256 : 1024),
+                                                (32 * pairs + 128) * (lean ? crispy::kGen16LeanR : crispy::gen16_max_r(slots)));
+    const int64_t blocks = crispy::gen16_dir_blocks(lean ? std::min(2 * maxlen, crispy::kGen16MaxSum) : 2 * maxlen);
     return (size_t)(2 * lane_regs * 2 * blocks * 4);
 }
 
@@ -118,7 +120,7 @@ size_t run_bytes(const std::vector<Job*>& js, int sms) {
         maxlen = std::max(maxlen, j->maxlen);
         n += j->n;
     }
-    return base + tag_bytes(maxlen, n, js.empty() ? 10 : js[0]->band, sms);
+    return base + tag_bytes(maxlen, n, js.empty() ? 10 : js[0]->band, !js.empty() && js[0]->lean, sms);
 }
 
 // K = 8: the same-key pass's queue of H sums, per block (one per SM) and
@@ -132,7 +134,7 @@ void set_estimate(Job& j, int sms) {
     j.maxlen = 0;
     for (int i = 0; i < j.n; ++i) j.maxlen = std::max(j.maxlen, j.len[i]);
     j.mem_base = estimate_base_bytes(j) + k8_queue_bytes(j, sms);
-    j.mem = j.mem_base + tag_bytes(j.maxlen, j.n, j.band, sms);
+    j.mem = j.mem_base + tag_bytes(j.maxlen, j.n, j.band, j.lean, sms);
 }
 
 // SMs of a device for the estimates (a GB300's 152 when it cannot be read).
@@ -185,7 +187,7 @@ struct crispy_server {
     }
 
     bool cohort_member(const Job* j) const {
-        return cohorts_enabled() && j->k >= 2 && j->k <= 6 && j->n >= 10 && j->n <= kCohortJobReads;
+        return cohorts_enabled() && !j->lean && j->k >= 2 && j->k <= 6 && j->n >= 10 && j->n <= kCohortJobReads;
     }
 
     // With `first` taken: the other queued jobs that can share its run.
@@ -259,6 +261,7 @@ struct crispy_server {
     void run_jobs(crispy_ctx* c, const std::vector<Job*>& js) {
         c->run_epoch++;
         c->run_need = 0;
+        c->lean = js[0]->lean;
         const size_t reserved = run_bytes(js, sms);
         bool done = false;
         if (js.size() > 1) {
@@ -401,6 +404,10 @@ int crispy_server_submit(crispy_server* s, const char* seqbuf, const int64_t* of
     set_estimate(*j, s->sms);
     j->t_submit = clock_type::now();
     std::lock_guard<std::mutex> g(s->mu);
+    if (j->mem > s->budget) {
+        j->lean = true;
+        set_estimate(*j, s->sms);
+    }
     if (j->mem > s->budget) {
         s->err = "job needs more device memory than the server budget";
         delete j;

@@ -110,12 +110,14 @@ int crispy_array_dim(int n);
 
 /* Upload reads and build the per-read k-mer structures on the device
  * (replaces formTuples/sortTuples, kmerMain.cpp:117-159, and the texture
- * upload of kmerCUDA.cu:37-71).  seqbuf holds the reads back to back. */
+ * upload of kmerCUDA.cu:37-71).  seqbuf holds the reads back to back.  The
+ * k-mer structures are built by the first run that needs them, and their
+ * memory is asked for there. */
 int crispy_kmer_prepare(crispy_ctx* ctx, const char* seqbuf,
                         const int64_t* offsets, const int32_t* lengths,
                         int n, int k);
 
-/* Re-run the device-side K-mer structure build from the reads uploaded by
+/* The next run builds its K-mer structures again from the reads uploaded by
  * the last crispy_kmer_prepare (no host transfer).  Part of formTuples in
  * the reference (kmerMain.cpp:117-159). */
 int crispy_kmer_rebuild(crispy_ctx* ctx);
@@ -319,8 +321,10 @@ int crispy_sparsecut(const char* in_base, int num_reads, const float* cutoffs, i
 
 /* ---- timing of the last run (CUDA events on the context's stream) ---- */
 typedef struct crispy_stats {
-    double kmer_kernel_ms;     /* summed duration of the k-mer tile kernel launches */
-    int64_t kmer_launches;
+    double kmer_kernel_ms;     /* summed duration of the k-mer kernels that bound and
+                                  count pairs */
+    int64_t kmer_launches;     /* rounds of the candidate filter and tile launches: both,
+                                  where the filter gave the reads up */
     double gen_kernel_ms;      /* summed duration of the DP kernel launches */
     int64_t gen_launches;
     double total_ms;           /* whole call, device side */
@@ -335,7 +339,8 @@ typedef struct crispy_stats {
                                   share and were gathered in pinned host memory */
     /* bound pass of the batched 128-row tile kernel (K <= 6): level entries
      * gathered by bound passes (section 0) and by full passes, the (row
-     * group, column) items counted in full and the full-pass rounds */
+     * group, column) items counted in full and the full-pass rounds (0 for runs
+ * that the candidate filter took) */
     int64_t kmer_bound_entries;
     int64_t kmer_full_entries;
     int64_t kmer_full_columns;
@@ -369,8 +374,8 @@ int crispy_probe_lds128(crispy_ctx* ctx, double* wavefronts_per_s);
 
 /* ---- memory cap of one context (device bytes); 0 = unlimited.  An
  *      allocation that would exceed it fails with CRISPY_E_OOM, exactly as
- *      an exhausted device would.  The server gives every slot a share of
- *      its HBM budget this way. ---- */
+ *      an exhausted device would, once the run has tried the forms that need
+ *      least memory (tile kernels for every pair, whole bands). ---- */
 int crispy_ctx_set_mem_cap(crispy_ctx* ctx, size_t bytes);
 int crispy_ctx_mem_in_use(const crispy_ctx* ctx, size_t* bytes);
 /* Release every device buffer the context holds (its jobs stay valid only
@@ -427,7 +432,9 @@ int crispy_server_job_memory(crispy_server* srv, uint64_t job_id, size_t* reserv
                              size_t* needed, int* cohort_size);
 /* The device bytes the server's admission reserves for a job of n reads of
  * these lengths at K = k (no device work; very small jobs whose bands are wider
- * than 256 slots reserve somewhat more). */
+ * than 256 slots reserve somewhat more).  A job that fits the budget only in
+ * the forms that need least memory (tile kernels, whole bands) runs in those
+ * and reserves less. */
 int crispy_server_job_bytes(const int32_t* lengths, int n, int k, size_t* bytes);
 /* Submit-to-finish latency percentiles (ms) over finished jobs, finished
  * job count and pairs processed (sum of n(n-1)/2). */
