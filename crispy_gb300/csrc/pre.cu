@@ -50,13 +50,14 @@ struct ReadSet {
 
 __device__ __forceinline__ uint32_t be32(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
-// strcmp-style order of two reads of equal length L (unsigned bytes).
-__device__ __forceinline__ int cmp_bytes(const ReadSet& r, uint32_t a, uint32_t b, int L) {
+// strcmp-style order of two reads of equal length L (unsigned bytes) whose
+// first `first` 16-byte words are equal.
+__device__ __forceinline__ int cmp_bytes(const ReadSet& r, uint32_t a, uint32_t b, int L, int first = 0) {
     const uint4* pa = r.pad + r.woff[a];
     const uint4* pb = r.pad + r.woff[b];
     const int nw = (L + 15) >> 4;
     // four words of each on their way at a time: duplicates compare to the end
-    for (int w0 = 0; w0 < nw; w0 += 4) {
+    for (int w0 = first; w0 < nw; w0 += 4) {
         uint4 xs[4], ys[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -96,13 +97,23 @@ struct ReadKey {
     unsigned long long hi, lo;
 };
 __device__ __forceinline__ bool key_equal(const ReadKey& a, const ReadKey& b) { return a.hi == b.hi && a.lo == b.lo; }
+// Order of two reads of this key: their length is known, and where no range
+// is among the first 16 classes (odd ones) so are their first 16 bytes.
+__device__ __forceinline__ int tie_cmp(const ReadSet& r, const ReadKey& k, uint32_t a, uint32_t b) {
+    const int L = (int)(k.hi >> 48);
+    const bool exact = (k.hi & 0x0000111111111111ull) == 0 && (k.lo & 0x1111000000000000ull) == 0;
+    return cmp_bytes(r, a, b, L, exact ? 1 : 0);
+}
 // kWhole: reads whose keys agree are compared; otherwise they keep the record
 // order, to be settled group by group afterwards.
 template <bool kWhole>
 __device__ __forceinline__ bool key_less(const ReadSet& r, const ReadKey& ka, uint32_t a, const ReadKey& kb, uint32_t b) {
     if (ka.hi != kb.hi) return ka.hi < kb.hi;
     if (ka.lo != kb.lo) return ka.lo < kb.lo;
-    return kWhole ? read_less(r, a, b) : a < b;
+    if (!kWhole) return a < b;
+    if (a == kNone || b == kNone || (ka.hi >> 48) == 0xFFFFull) return read_less(r, a, b);
+    const int c = tie_cmp(r, ka, a, b);
+    return c ? c < 0 : a < b;
 }
 __device__ __forceinline__ uint32_t byte_class(uint32_t c) {
     if (c == 0) return 0;
@@ -258,23 +269,48 @@ __global__ void pre_primer_kernel(ReadSet r, int n, const uint8_t* __restrict__ 
 }
 
 // Whether reads of equal keys are so many that comparing the reads throughout
-// costs less than settling them group by group: estimated from the equal
-// neighbours found inside the sorted tiles, of which `tiles` tiles taken
-// together hold about that many times more pairs.  force: the reads are
-// compared throughout, whatever the estimate says (a tile may hold no two
-// equal keys although the set holds thousands of each).
+// costs less than settling them group by group.  force: the reads are compared
+// throughout, whatever the estimate says.
 struct Ties {
-    const unsigned long long* neighbours;
-    unsigned long long tiles, limit;
+    const unsigned long long* too_many;   // pre_sample_kernel
     bool force;
-    __device__ bool many() const { return force || 2ull * *neighbours * tiles > limit; }
+    __device__ bool many() const { return force || *too_many != 0; }
 };
-__global__ void pre_neighbour_kernel(const ReadKey* __restrict__ keys, int64_t m,
-                                     unsigned long long* __restrict__ neighbours) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool tie = p + 1 < m && (p + 1) % kTile != 0 && key_equal(keys[p], keys[p + 1]);
-    const int c = __popc(__ballot_sync(0xffffffffu, tie));
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(neighbours, (unsigned long long)c);
+
+// The estimate: pairs of equal keys among up to 1,024 reads spread over the
+// set (found in a table of hashes), and as many more in the whole set as it
+// has more pairs.  One block, before the sort (5 us): looking at sorted tiles
+// instead costs sets with many ties a tile sort more (28 us).  Whole calls of
+// 60,000 reads of 250 nt, reads compared throughout without keys, and now: no
+// common head 642 and 556 us, a common head of 20 bases 695 and 652, of 40
+// bases 714 and 674, all of one length 739 and 650.
+constexpr int kSample = 1024, kSampleSlots = 4096;
+__global__ void __launch_bounds__(kSample) pre_sample_kernel(const ReadKey* __restrict__ keys, int64_t m, double limit,
+                                                             unsigned long long* __restrict__ too_many) {
+    __shared__ unsigned long long slot[kSampleSlots];
+    __shared__ unsigned count[kSampleSlots];
+    __shared__ unsigned pairs;
+    const int t = threadIdx.x;
+    for (int q = t; q < kSampleSlots; q += kSample) { slot[q] = 0; count[q] = 0; }
+    if (t == 0) pairs = 0;
+    __syncthreads();
+    const int64_t step = m / kSample;   // 0: every read
+    if (step > 0 || t < m) {
+        const int64_t p = step > 0 ? t * step + (int64_t)((uint32_t)t * 0x9E3779B1u >> 8) % step : t;
+        const ReadKey k = keys[p];
+        const unsigned long long h = ((k.hi ^ (k.lo << 1 | k.lo >> 63)) * 0x9E3779B97F4A7C15ull ^ k.lo * 0xC2B2AE3D27D4EB4Full) | 1ull;
+        for (unsigned q = (unsigned)(h >> 40) % kSampleSlots;; q = (q + 1) % kSampleSlots) {
+            const unsigned long long old = atomicCAS(&slot[q], 0ull, h);
+            if (old == 0 || old == h) {
+                const unsigned before = atomicAdd(&count[q], 1u);
+                if (before) atomicAdd(&pairs, before);
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    const double more = step > 0 ? (double)m / kSample : 1.0;
+    if (t == 0) *too_many = 2.0 * pairs * more * more > limit ? 1ull : 0ull;
 }
 
 // Bitonic sort of one tile: keys and indices in shared memory.  With kWhole
@@ -284,7 +320,7 @@ __global__ void pre_neighbour_kernel(const ReadKey* __restrict__ keys, int64_t m
 template <bool kWhole>
 __global__ void __launch_bounds__(kTileThreads) pre_tile_sort_kernel(uint32_t* idx, ReadKey* keys, int64_t m,
                                                                      ReadSet r, const Ties ties) {
-    if (kWhole && !ties.many()) return;
+    if (kWhole != ties.many()) return;
     __shared__ uint32_t s[kTile];
     __shared__ ReadKey sk[kTile];
     const int64_t base = (int64_t)blockIdx.x * kTile;
@@ -392,14 +428,15 @@ __global__ void pre_group_kernel(const ReadKey* __restrict__ keys, int64_t m, ui
 __global__ void pre_rank_kernel(const uint32_t* __restrict__ src, const uint2* __restrict__ range, int64_t m, ReadSet r,
                                 const unsigned long long* __restrict__ work, unsigned long long limit,
                                 uint32_t* __restrict__ dst, const Ties ties) {
+    if (ties.many() || *work > limit) {          // sorted already, or not to be settled here
+        const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (q < m) dst[q] = src[q];
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= m) return;
     const uint32_t x = src[p];
-    if (ties.many() || *work > limit) {          // sorted already, or not to be settled here
-        if (lane == 0) dst[p] = x;
-        return;
-    }
     const uint2 g = range[p];
     unsigned before = 0;
     if (g.y - g.x > 1)
@@ -417,7 +454,7 @@ __global__ void pre_last_kernel(const uint32_t* __restrict__ sorted, const ReadK
     if (p + 1 < m && key_equal(keys[p], keys[p + 1])) {
         const uint32_t a = sorted[p], b = sorted[p + 1];
         const int la = r.len[a];
-        last = la != r.len[b] || cmp_bytes(r, a, b, la) != 0;
+        last = la != r.len[b] || (la < 0xFFFF ? tie_cmp(r, keys[p], a, b) : cmp_bytes(r, a, b, la)) != 0;
     }
     flag[p] = last ? 1 : 0;
 }
@@ -648,7 +685,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
     CRISPY_TRY(ensure(ctx, j.range, (size_t)std::max<int64_t>(m, 1) * sizeof(uint2)));
     unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
-    unsigned long long* d_near = d_work + 1;
+    unsigned long long* d_many = d_work + 1;
     const unsigned long long limit = 256ull * (unsigned long long)m + 4096;
     const unsigned blocks = (unsigned)((m + 255) / 256), wblocks = (unsigned)((m + 7) / 8);
     const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
@@ -656,20 +693,20 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     // keys first, reads of equal keys settled group by group; or, where the
     // groups are large (many copies of a read), the reads compared throughout
     auto sort_reads = [&](bool whole) {
-        // (60,000 reads: settling 64 comparisons a read costs about what the
-        // merges save)
-        const Ties ties{d_near, tiles, 64ull * (unsigned long long)m + 4096, whole};
+        const Ties ties{d_many, whole};
         a = j.idx.as<uint32_t>();
         b = j.idx_alt.as<uint32_t>();
         ka = j.keys.as<ReadKey>();
         ReadKey* kb = j.keys_alt.as<ReadKey>();
         pre_key_kernel<<<blocks, 256, 0, s>>>(rs, a, m, ka);
-        count_launch(ctx);
+        // (60,000 reads: settling 64 comparisons a read costs about what the
+        // merges save)
+        pre_sample_kernel<<<1, kSample, 0, s>>>(ka, m, 64.0 * (double)m + 4096.0, d_many);
+        count_launch(ctx, 2);
         if (m < 2) return;
         pre_tile_sort_kernel<false><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs, ties);
-        pre_neighbour_kernel<<<blocks, 256, 0, s>>>(ka, m, d_near);
         pre_tile_sort_kernel<true><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs, ties);
-        count_launch(ctx, 3);
+        count_launch(ctx, 2);
         for (int64_t w = kTile; w < m; w <<= 1) {
             pre_merge_kernel<<<blocks, 256, 0, s>>>(a, ka, b, kb, m, w, rs, ties);
             count_launch(ctx);

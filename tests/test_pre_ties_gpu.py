@@ -91,3 +91,35 @@ def test_ties_apart_in_every_tile(tmp_path):
     count = np.bincount(code, minlength=kinds * 256)
     assert np.array_equal(index, last[count > 0])
     assert np.array_equal(freq, count[count > 0])
+
+
+# most reads tie in their keys: a shared head, with and without a byte among
+# its first 16 that only has a range, reads that end before, at and behind the
+# 16th and 28th byte, one length, one read in many copies
+@pytest.mark.parametrize("n", [700, 1024, 6000])
+@pytest.mark.parametrize("kind", ["head", "range early", "range late", "short", "copies"])
+def test_sets_of_many_ties(tmp_path, n, kind):
+    rng = np.random.default_rng(n)
+    head = rng.choice(np.frombuffer(b"ACGT", np.uint8), 40)
+    if kind == "range early":
+        head[3] = ord("R")
+    if kind == "range late":
+        head[20] = ord("K")
+    lo, hi = (12, 33) if kind == "short" else (60, 64)
+    reads = []
+    for _ in range(n):
+        tail = rng.choice(np.frombuffer(b"ACGTN", np.uint8), hi - 40 if hi > 40 else 1)
+        s = np.concatenate([head, tail])[:int(rng.integers(lo, hi))].copy()
+        if kind.startswith("range"):        # told apart behind the range byte, before and after the 16th
+            s[int(rng.choice([5, 14, 25]))] = b"ACGT"[int(rng.integers(0, 4))]
+        if kind == "short":
+            s[int(rng.integers(0, len(s)))] = b"ACGT"[int(rng.integers(0, 4))]
+        s[-1] = b"ACGT"[int(rng.integers(0, 4))]
+        reads.append(s.tobytes())
+    if kind == "copies":
+        reads = [reads[int(rng.integers(0, 5))] if i % 3 else reads[i] for i in range(n)]
+    eng = cg.Engine(0)
+    try:
+        _run(eng, tmp_path, reads)
+    finally:
+        eng.close()
