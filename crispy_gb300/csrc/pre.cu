@@ -681,9 +681,25 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     // sort by (length, bytes, record index)
     uint32_t* a = j.idx.as<uint32_t>();
     uint32_t* b = j.idx_alt.as<uint32_t>();
-    CRISPY_TRY(ensure(ctx, j.keys, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
-    CRISPY_TRY(ensure(ctx, j.keys_alt, (size_t)std::max<int64_t>(m, 1) * sizeof(ReadKey)));
-    CRISPY_TRY(ensure(ctx, j.range, (size_t)std::max<int64_t>(m, 1) * sizeof(uint2)));
+    // keys and group ranges where the raw reads were (the padded ones stay),
+    // as far as they reach: 40 bytes a read
+    size_t carved = 0;
+    auto carve = [&](DevBuf& own, size_t bytes, void** out) -> int {
+        bytes = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+        if (carved + bytes <= j.seq.bytes) {
+            *out = j.seq.as<uint8_t>() + carved;
+            carved += bytes;
+            return CRISPY_OK;
+        }
+        CRISPY_TRY(ensure(ctx, own, bytes));
+        *out = own.ptr;
+        return CRISPY_OK;
+    };
+    void *keys0, *keys1, *ranges;
+    CRISPY_TRY(carve(j.keys, (size_t)m * sizeof(ReadKey), &keys0));
+    CRISPY_TRY(carve(j.keys_alt, (size_t)m * sizeof(ReadKey), &keys1));
+    CRISPY_TRY(carve(j.range, (size_t)m * sizeof(uint2), &ranges));
+    uint2* d_range = static_cast<uint2*>(ranges);
     unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
     unsigned long long* d_many = d_work + 1;
     const unsigned long long limit = 256ull * (unsigned long long)m + 4096;
@@ -696,8 +712,8 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
         const Ties ties{d_many, whole};
         a = j.idx.as<uint32_t>();
         b = j.idx_alt.as<uint32_t>();
-        ka = j.keys.as<ReadKey>();
-        ReadKey* kb = j.keys_alt.as<ReadKey>();
+        ka = static_cast<ReadKey*>(keys0);
+        ReadKey* kb = static_cast<ReadKey*>(keys1);
         pre_key_kernel<<<blocks, 256, 0, s>>>(rs, a, m, ka);
         // (60,000 reads: settling 64 comparisons a read costs about what the
         // merges save)
@@ -713,8 +729,8 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
             std::swap(a, b);
             std::swap(ka, kb);
         }
-        pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, j.range.as<uint2>(), d_work, ties);
-        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, j.range.as<uint2>(), m, rs, d_work, limit, b, ties);
+        pre_group_kernel<<<wblocks, 256, 0, s>>>(ka, m, d_range, d_work, ties);
+        pre_rank_kernel<<<wblocks, 256, 0, s>>>(a, d_range, m, rs, d_work, limit, b, ties);
         count_launch(ctx, 2);
         std::swap(a, b);
     };

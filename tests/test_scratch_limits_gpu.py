@@ -98,3 +98,25 @@ def test_server_admits_lean_jobs(kind):
         with pytest.raises(cg.CrispyError) as e:
             srv.submit(buf, offs, lens, k=k, band=band)
         assert e.value.code == cg.E_OOM
+
+
+@pytest.mark.parametrize("length", [30, 250])
+def test_preprocess_needs_no_more_than_before_the_keys(tmp_path, length):
+    # the sort keys lie where the raw reads were: beside reads, padded reads and
+    # the index lists (43 bytes a record) there is nothing of any size
+    n = 20000
+    rng = np.random.default_rng(length)
+    rows = np.full((n, length + 3), 10, np.uint8)
+    rows[:, 0] = ord(">")
+    rows[:, 2:-1] = rng.choice(np.frombuffer(b"ACGT", np.uint8), (n, length))
+    path = str(tmp_path / "raw.fa")
+    rows.tofile(path)
+    raw = cg.RawReads(path)
+    with cg.Engine(0) as eng:
+        index, _, _ = eng.preprocess(raw)
+        used = eng.mem_in_use()
+    raw.close()
+    seqs = [r.tobytes() for r in rows[:, 2:-1]]
+    assert index.tolist() == sorted({s: i for i, s in enumerate(seqs)}.values(), key=lambda i: seqs[i])
+    short = max(0, 40 - length + 8) * n          # reads of under 40 bytes leave too little room
+    assert used <= n * (length + (length + 15) // 16 * 16 + 43) + short + (1 << 16)
