@@ -3395,11 +3395,12 @@ static int kmer_tune_split(crispy_ctx* ctx, float thr) {
 }
 
 // Read sets whose batched runs the candidate filter took twice or more, for
-// crispy_tune_report: the filter's dimensions and what it left, and the split
-// the tile kernels would start from.
+// crispy_tune_report: the filter's dimensions and what it left, and at K <= 6
+// the split that the tile kernels would take for them (tuned or default).
 struct KmerFilterNote {
     int n, k, dims, runs;
     int64_t pairs, found;
+    uint64_t fp;
 };
 static std::map<std::string, KmerFilterNote> g_kfilter;   // guarded by g_ktune_mu
 
@@ -3410,7 +3411,7 @@ static void kmer_note_filter(const KmerJob& j) {
     std::lock_guard<std::mutex> g(g_ktune_mu);
     if (g_kfilter.size() >= 256 && !g_kfilter.count(key)) g_kfilter.clear();
     KmerFilterNote& e = g_kfilter[key];
-    e = KmerFilterNote{j.n, j.k, j.f_dims, e.runs + 1, j.f_pairs, j.f_found};
+    e = KmerFilterNote{j.n, j.k, j.f_dims, e.runs + 1, j.f_pairs, j.f_found, kmer_fingerprint(j)};
 }
 
 int crispy_kmer_run(crispy_ctx* ctx, float thr, int mode, int dists, int64_t* npairs) {
@@ -3528,10 +3529,15 @@ std::string kmer_tune_json() {
         char item[256];
         snprintf(item, sizeof item,
                  ", {\"stage\": \"kmer\", \"kernel\": \"kmer_filter_kernel\", \"reads\": %d, \"k\": %d, "
-                 "\"split\": %d, \"dims\": %d, \"pairs\": %lld, \"candidates\": %lld}",
-                 kv.second.n, kv.second.k, kSplitDefault, kv.second.dims, (long long)kv.second.pairs,
-                 (long long)kv.second.found);
+                 "\"dims\": %d, \"pairs\": %lld, \"candidates\": %lld",
+                 kv.second.n, kv.second.k, kv.second.dims, (long long)kv.second.pairs, (long long)kv.second.found);
         out += item;
+        if (tile_rows_for(kv.second.k) == kRows128) {
+            const auto t = g_ktuned.find(kv.second.fp);
+            snprintf(item, sizeof item, ", \"split\": %d", t == g_ktuned.end() ? kSplitDefault : t->second.split);
+            out += item;
+        }
+        out += "}";
     }
     return out;
 }
