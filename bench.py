@@ -302,6 +302,7 @@ def run_ours(args, dist, ws, rank, local):
     if not all(identical.values()):
         print(f"bench: forms disagree: {identical}", file=sys.stderr)
     cells = st_g["gen_cells"]
+    swept = st_g["gen_swept_cells"]
     mean_t = float(np.mean(np.maximum(np.array(lens) - k + 1, 0)))
 
     step_s = _max_over_ranks(dist, float(np.mean(ms_b)) / 1e3)
@@ -377,7 +378,7 @@ def run_ours(args, dist, ws, rank, local):
         tune = []
     gen_kernel_name = ("gen16_kernel" if any(t.get("kernel") == "gen16_kernel" for t in tune)
                        else "gen_warp_kernel")
-    gen_ops = cells * 10                        # frozen: 10 per band cell
+    gen_ops = swept * 10                        # frozen: 10 per cell swept
     tile_kernel = ("kmer_tile8h_kernel + kmer_tile8_kernel" if k == 8 else "kmer_tile_kernel" if k == 7
                    else "kmer_tile128_kernel")
     # The tile kernels are bound by the L1 data pipe: one conflict-free
@@ -445,8 +446,13 @@ def run_ours(args, dist, ws, rank, local):
     roof_g = {"kernel": gen_kernel_name, "bound": "int32", "unit": "Gop/s",
               "achieved": gen_ops / gen_s / 1e9, "peak": int_peak_gops,
               "frac": gen_ops / gen_s / 1e9 / int_peak_gops,
-              "work_per_unit": "10 ops per cell of the whole band (narrow sweeps compute 0.46-0.76 of them)",
-              "traffic": None,
+              "work_per_unit": f"10 ops per band cell swept ({swept / max(1, cells):.3f} of the whole bands' cells: "
+                               "narrow sweeps, and the pairs swept twice)",
+              "traffic": None, "swept_cells": swept,
+              "whole_band_view": {
+                  "achieved": cells * 10 / gen_s / 1e9, "unit": "Gop/s",
+                  "note": "operations of the whole bands over the same time: above the kernel's own rate by the "
+                          "cells that narrow sweeps leave out, and not a roofline"},
               "peak_source": "measured: crispy_probe_int32 (IADD3/LOP3 chains), this run"}
     # the dense count-vector formulation: 4^k/4 packed count words per read,
     # 2 ops per word and pair (a min and an add)
@@ -456,7 +462,7 @@ def run_ours(args, dist, ws, rank, local):
         "achieved": n_pairs * dense_ops / kmer_s / 1e9, "peak": int_peak_gops,
         "frac": n_pairs * dense_ops / kmer_s / 1e9 / int_peak_gops}
     dominant = roof_g if gen_s >= kmer_s else roof_k
-    _attach_traffic(roof_k if not filt else {}, roof_g, n_pairs, cells, k)
+    _attach_traffic(roof_k, roof_g, n_pairs, swept, k, bool(filt))
     _attach_hbm_view(roof_k, kmer_s)
     _attach_hbm_view(roof_g, gen_s)
 
@@ -791,9 +797,10 @@ def _attach_hbm_view(roof, seconds):
                         "peak_source": "measured: MEASURED_PEAKS.json hbm_gbs"}
 
 
-def _attach_traffic(roof_k, roof_g, n_pairs, cells, k):
+def _attach_traffic(roof_k, roof_g, n_pairs, cells, k, filtered):
     """DRAM bytes per launch from a committed ncu summary, scaled by units
-    (k = 8 has kmerDist figures of its own, from the stress set)."""
+    (the candidate filter and the tile kernels have kmerDist figures of their
+    own, the latter also at k = 8, from the stress set)."""
     p = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if not os.path.exists(p):
         return
@@ -801,7 +808,8 @@ def _attach_traffic(roof_k, roof_g, n_pairs, cells, k):
         t = json.load(open(p))
     except (OSError, ValueError):
         return
-    tk = t.get("k8", t) if k == 8 else t
+    # (the filter's k = 8 form covers same-key ranges only: no figures of its own)
+    tk = ({} if k == 8 else t.get("kmer_filter", {})) if filtered else t.get("k8", t) if k == 8 else t
     if "kmer_bytes_per_pair" in tk:
         roof_k["traffic"] = tk["kmer_bytes_per_pair"] * n_pairs
         roof_k["traffic_source"] = tk.get("source")

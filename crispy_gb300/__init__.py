@@ -121,6 +121,7 @@ PROTOTYPES = {
                                   C.c_char_p, C.c_char_p, C.POINTER(ClustStats)]),
     "crispy_sparsecut": (C.c_int, [C.c_char_p, C.c_int, _P, C.c_int, C.POINTER(ClustStats)]),
     "crispy_get_stats": (C.c_int, [_P, C.POINTER(Stats)]),
+    "crispy_gen_swept_cells": (C.c_int, [_P, C.POINTER(C.c_int64)]),
     "crispy_set_timing": (C.c_int, [_P, C.c_int]),
     "crispy_probe_int32": (C.c_int, [_P, C.POINTER(C.c_double)]),
     "crispy_probe_lds128": (C.c_int, [_P, C.POINTER(C.c_double)]),
@@ -321,7 +322,9 @@ class Engine:
     def stats(self) -> dict:
         s = Stats()
         self._check(self.lib.crispy_get_stats(self.h, C.byref(s)))
-        return s.as_dict()
+        swept = C.c_int64()
+        self._check(self.lib.crispy_gen_swept_cells(self.h, C.byref(swept)))
+        return {**s.as_dict(), "gen_swept_cells": swept.value}
 
     # ---- kmerDist ----
     def kmer_prepare(self, buf: np.ndarray, offs: np.ndarray, lens: np.ndarray, k: int = 6):

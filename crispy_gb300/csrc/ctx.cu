@@ -421,6 +421,12 @@ int crispy_get_stats(const crispy_ctx* ctx, crispy_stats* out) {
     return CRISPY_OK;
 }
 
+int crispy_gen_swept_cells(const crispy_ctx* ctx, int64_t* cells) {
+    if (!ctx || !cells) return CRISPY_E_INPUT;
+    *cells = ctx->gen_swept;
+    return CRISPY_OK;
+}
+
 int crispy_probe_int32(crispy_ctx* ctx, double* gops) {
     if (!ctx || !gops) return CRISPY_E_INPUT;
     cudaSetDevice(ctx->device);

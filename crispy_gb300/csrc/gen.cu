@@ -599,20 +599,23 @@ __global__ void gen_poskeys_kernel(const float* __restrict__ dist, int64_t count
     vals[i] = (uint32_t)i;
 }
 
-// Band cells of one pair in O(1): rows i = 1..l2 hold columns
-// max(1, i-kb)..min(l1, i+kb), non-empty for i <= min(l2, l1 + kb).
-__host__ __device__ inline int64_t band_cells_of(int l1, int l2, int band) {
-    const int64_t kb = band >= 2 ? (l1 + l2) / (2 * band) : (l1 > l2 ? l1 : l2);
+// Cells of one pair on diagonals -lo .. hi (row - column) in O(1): rows i =
+// 1..l2 hold columns max(1, i-hi)..min(l1, i+lo), non-empty for i <= min(l2,
+// l1 + hi).
+__host__ __device__ inline int64_t swept_cells_of(int l1, int l2, int64_t lo, int64_t hi) {
     if (l1 <= 0 || l2 <= 0) return 0;
-    const int64_t I = l2 < l1 + kb ? l2 : l1 + kb;
-    int64_t a = l1 - kb > 0 ? l1 - kb : 0;
+    const int64_t I = l2 < l1 + hi ? l2 : l1 + hi;
+    int64_t a = l1 - lo > 0 ? l1 - lo : 0;
     a = a < I ? a : I;
-    const int64_t sum_hi = a * (a + 1) / 2 + a * kb + (I - a) * l1;
-    const int64_t b = kb + 1 < I ? kb + 1 : I;
-    const int64_t sum_lo = b + (I * (I + 1) / 2 - b * (b + 1) / 2) - kb * (I - b);
+    const int64_t sum_hi = a * (a + 1) / 2 + a * lo + (I - a) * l1;
+    const int64_t b = hi + 1 < I ? hi + 1 : I;
+    const int64_t sum_lo = b + (I * (I + 1) / 2 - b * (b + 1) / 2) - hi * (I - b);
     return sum_hi - sum_lo + I;
 }
-
+__host__ __device__ inline int64_t band_cells_of(int l1, int l2, int band) {
+    const int64_t kb = band >= 2 ? (l1 + l2) / (2 * band) : (l1 > l2 ? l1 : l2);
+    return swept_cells_of(l1, l2, kb, kb);
+}
 
 // Register-resident shapes (sub-group lanes G, band slots per lane C).
 // Every one serves a pair with kBand + 1 <= G * C.
@@ -736,6 +739,7 @@ constexpr int kOrderBits = 18;   // the sort key: order-bin << 12 | 4095 - sweep
 constexpr int kStatBins = 2, kStatWindows = 48;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
+constexpr int kStatSwept = kStatMaxSum16 + 1;   // cells this launch's sweeps hold
 // bands: the diagonals each pair is swept over (nullptr: all of its band);
 // list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
@@ -747,7 +751,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     const int lane = threadIdx.x & 31;
     const bool ok = at < count;
     const int64_t p = ok && list ? (int64_t)list[at] : at;
-    unsigned long long cells = 0;
+    unsigned long long cells = 0, swept = 0;
     int kb = 0, ob = -1, wb = -1, lng = 0;
     int sum_reg = 0;   // L1 + L2 of a pair for the register kernels' 16-bit form
     if (ok) {
@@ -774,15 +778,20 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
             keys[at] = ((uint32_t)ob << 12) | (uint32_t)(4095 - min((se + (lo & 1)) >> 1, 4095));
             vals[at] = (uint32_t)p;
         }
-        if (!list) cells = (unsigned long long)band_cells_of(l1, l2, band);
+        cells = (unsigned long long)swept_cells_of(l1, l2, kb, kb);
+        // (the wide-band kernel knows whole bands only)
+        swept = bands && bin != 0 ? (unsigned long long)swept_cells_of(l1, l2, lo, hi) : cells;
+        if (list) cells = 0;
     }
     // one atomic per warp and counter: the counters are few and shared by
     // every pair, so per-pair atomics would serialise
     cells = __reduce_add_sync(0xffffffffu, (unsigned)cells) + 0ull;   // cells < 2^32 per warp
+    swept = __reduce_add_sync(0xffffffffu, (unsigned)swept) + 0ull;
     const unsigned kbw = __reduce_max_sync(0xffffffffu, (unsigned)kb);
     const unsigned sum16 = __reduce_max_sync(0xffffffffu, (unsigned)sum_reg);
     if (lane == 0) {
         if (cells) atomicAdd(&stats[0], cells);
+        if (swept) atomicAdd(&stats[kStatSwept], swept);
         atomicMax(&stats[1], (unsigned long long)kbw);
         if (sum16) atomicMax(&stats[kStatMaxSum16], (unsigned long long)sum16);
     }
@@ -799,7 +808,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
 }
 // untuned 32-bit shape per bin (the plain form always uses it)
 constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13, -1, -1, -1, -1};
-static_assert(kStatMaxSum16 < kStatWindows, "per-bin counters overlap the window slots");
+static_assert(kStatSwept < kStatWindows, "per-bin counters overlap the window slots");
 
 using WarpFn = void (*)(GenArgs);
 WarpFn shape_fn(int shape) {
@@ -1086,6 +1095,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
     st.resize(nstats);
     CRISPY_CK(ctx, cudaMemcpyAsync(st.data(), d_stats, (size_t)nstats * 8, cudaMemcpyDeviceToHost, s));
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
+    ctx->gen_swept += (int64_t)st[kStatSwept];
     return CRISPY_OK;
 }
 
@@ -1326,6 +1336,7 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
                       int32_t* d_al, const float* kdist = nullptr, int kdist_k = 0) {
     if (count <= 0) return CRISPY_OK;
     const crispy_stats before = ctx->stats;
+    const int64_t swept = ctx->gen_swept;
     const size_t events = ctx->ev_gen.used;
     auto run = [&]() -> int {
         ++ctx->gen_users;
@@ -1339,6 +1350,7 @@ int gen_dispatch_impl(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int6
     CRISPY_CK(ctx, cudaStreamSynchronize(s));
     gen_scratch_release(ctx);
     ctx->stats = before;
+    ctx->gen_swept = swept;
     ctx->ev_gen.used = events;
     ctx->lean = true;
     rc = run();
@@ -1627,6 +1639,7 @@ int crispy_gen_align(crispy_ctx* ctx, const int32_t* pairs, int64_t npairs, int 
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     ctx->stats = crispy_stats{};
+    ctx->gen_swept = 0;
     ctx->ev_gen.used = 0;
     if (npairs == 0) return CRISPY_OK;
     CRISPY_TRY(ensure(ctx, g.pairs, (size_t)npairs * 8));
@@ -1761,6 +1774,7 @@ int crispy_gen_run(crispy_ctx* ctx, const int32_t* pairs, int64_t npairs, int ba
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     ctx->stats = crispy_stats{};
+    ctx->gen_swept = 0;
     ctx->ev_gen.used = 0;
     CRISPY_CK(ctx, cudaEventRecord(ctx->t_begin, s));
     int64_t ns = 0;
@@ -1837,6 +1851,7 @@ int crispy_gen_run_from_kmer(crispy_ctx* ctx, int band, float thr, int mode, cri
     const int64_t npairs = k.nsurv;
     const crispy_stats kst = ctx->stats;
     ctx->stats = crispy_stats{};
+    ctx->gen_swept = 0;
     ctx->ev_gen.used = 0;
     CRISPY_CK(ctx, cudaEventRecord(ctx->t_begin, s));
     int64_t ns = 0;
@@ -1970,6 +1985,7 @@ int gen_run_cohort(crispy_ctx* ctx, const std::vector<CohortJob>& jobs, const st
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     ctx->stats = crispy_stats{};
+    ctx->gen_swept = 0;
     ctx->ev_gen.used = 0;
     gen_counts.assign(jobs.size(), 0);
     if (total > 0) {

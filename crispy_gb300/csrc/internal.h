@@ -168,6 +168,7 @@ struct crispy_ctx {
     bool timing = false;
     std::string err;
     crispy_stats stats{};
+    int64_t gen_swept = 0;   // band cells the last genDist run computed
     crispy::KmerJob kmer;
     crispy::GenJob gen;
     crispy::PreJob pre;
