@@ -650,22 +650,45 @@ static_assert(2 * kNumBins < 64, "order-bins overflow the 18-bit sort key");
 // 1,400 nt; a mismatch takes 9 from the score and about 8 8-mers), and leaves
 // 0.76 (99,999 reads of 300-500 nt, band 10), 0.74 (20,000 of 250 nt), 0.46
 // (band 5) and 0.28 (band 2) of the band's slots; at 0.35 it is 98 %, whose
-// second sweep costs more than the slots saved.  One warp
-// per pair: the longer read's 8-mers in a hashed bitmap, the shorter's looked
-// up in it.
+// second sweep costs more than the slots saved.  Beyond 0.6 of the 8-mers (a
+// divergence of 0.11, 1 - 0.6 = (1 - 0.11)^8) two mismatches take the same
+// 8-mers and the count no longer tells how many there are: such pairs keep
+// their whole band where a register shape has it (unrelated reads of 250 nt at
+// band 2: 0.88 of the slots swept to no end, 60,000 pairs 5.4 ms for 2.9).
+// One warp per pair: the longer read's 8-mers in a hashed bitmap, the
+// shorter's looked up in it.
+//
+// Large lists (kSample): first the slots a sample of the pairs would save, in
+// probe[0] of probe[1].  Where that is under a sixteenth nothing is estimated
+// for the others (40 us for 60,000 pairs of 250 nt).
 constexpr int kBandWarps = 8;
 constexpr int kBandBits = 14;
+constexpr int kBandSample = 1024;          // pairs
+constexpr int64_t kBandSampleFrom = 16384;
+template <bool kSample>
 __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32_t* __restrict__ packed,
                                                                     const int64_t* __restrict__ woff,
                                                                     const int32_t* __restrict__ len,
                                                                     const int2* __restrict__ pairs, int64_t count,
                                                                     int band, int max_sum,
-                                                                    uint32_t* __restrict__ bands) {
+                                                                    uint32_t* __restrict__ bands,
+                                                                    unsigned long long* __restrict__ probe) {
     __shared__ __align__(16) uint32_t bitmap[kBandWarps][1 << (kBandBits - 5)];
     const int lane = threadIdx.x & 31;
     uint32_t* bm = bitmap[threadIdx.x >> 5];
     const int64_t nw = (int64_t)gridDim.x * kBandWarps;
-    for (int64_t p = (int64_t)blockIdx.x * kBandWarps + (threadIdx.x >> 5); p < count; p += nw) {
+    if (!kSample && probe && probe[0] * 16 < probe[1]) {
+        for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < count; p += nw * 32) {
+            const int2 pr = pairs[p];
+            const int l1 = len[pr.x], l2 = len[pr.y];
+            const uint32_t kb = (uint32_t)(band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2));
+            bands[p] = kb | kb << 16;
+        }
+        return;
+    }
+    const int64_t todo = kSample ? kBandSample : count;
+    for (int64_t i = (int64_t)blockIdx.x * kBandWarps + (threadIdx.x >> 5); i < todo; i += nw) {
+        const int64_t p = kSample ? i * count / kBandSample : i;
         const int2 pr = pairs[p];
         const int l1 = len[pr.x], l2 = len[pr.y];
         const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
@@ -695,26 +718,36 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
             }
             miss = __reduce_add_sync(0xffffffffu, miss);
             const int e = miss * 13 / 32 + 3;
-            lo = min(kb, e + max(0, l1 - l2));
-            hi = min(kb, e + max(0, l2 - l1));
+            if (5 * miss <= 3 * ts || kb >= kMaxSlots16) {
+                lo = min(kb, e + max(0, l1 - l2));
+                hi = min(kb, e + max(0, l2 - l1));
+            }
         }
-        if (lane == 0) bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+        if (kSample) {
+            if (lane == 0) {
+                atomicAdd(&probe[0], (unsigned long long)(2 * kb - lo - hi));
+                atomicAdd(&probe[1], (unsigned long long)(2 * kb + 2));
+            }
+        } else if (lane == 0) {
+            bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+        }
         __syncwarp();
     }
 }
 
 // The same estimate from kmerDist's own count: of the shorter read's T K-mers
-// T * distance find no partner, so 8 / K times that stands for the 8-mers.
+// T * distance find no partner, so 8 / K times that stands for the 8-mers
+// (up to the share of K-mers that the same divergence takes, most_dist).
 __global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, const int2* __restrict__ pairs,
-                                           const float* __restrict__ kdist, int K, int64_t count, int band,
-                                           int max_sum, uint32_t* __restrict__ bands) {
+                                           const float* __restrict__ kdist, int K, float most_dist, int64_t count,
+                                           int band, int max_sum, uint32_t* __restrict__ bands) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= count) return;
     const int2 pr = pairs[p];
     const int l1 = len[pr.x], l2 = len[pr.y];
     const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
     int lo = kb, hi = kb;
-    if (l1 + l2 <= max_sum && kb >= 16) {
+    if (l1 + l2 <= max_sum && kb >= 16 && (kdist[p] <= most_dist || kb >= kMaxSlots16)) {
         const float miss = kdist[p] * (float)(min(l1, l2) - K + 1);
         const int e = (int)fminf(miss * 3.25f / (float)K, 4096.0f) + 3;
         lo = min(kb, e + max(0, l1 - l2));
@@ -740,6 +773,7 @@ constexpr int kStatBins = 2, kStatWindows = 48;
 constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
 constexpr int kStatSwept = kStatMaxSum16 + 1;   // cells this launch's sweeps hold
+constexpr int kStatNarrow = kStatSwept + 1;     // pairs swept over part of their band
 // bands: the diagonals each pair is swept over (nullptr: all of its band);
 // list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
@@ -752,6 +786,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
     const bool ok = at < count;
     const int64_t p = ok && list ? (int64_t)list[at] : at;
     unsigned long long cells = 0, swept = 0;
+    bool swept_part = false;
     int kb = 0, ob = -1, wb = -1, lng = 0;
     int sum_reg = 0;   // L1 + L2 of a pair for the register kernels' 16-bit form
     if (ok) {
@@ -782,6 +817,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         // (the wide-band kernel knows whole bands only)
         swept = bands && bin != 0 ? (unsigned long long)swept_cells_of(l1, l2, lo, hi) : cells;
         if (list) cells = 0;
+        swept_part = lo < kb || hi < kb;
     }
     // one atomic per warp and counter: the counters are few and shared by
     // every pair, so per-pair atomics would serialise
@@ -795,6 +831,8 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         atomicMax(&stats[1], (unsigned long long)kbw);
         if (sum16) atomicMax(&stats[kStatMaxSum16], (unsigned long long)sum16);
     }
+    const unsigned part = __ballot_sync(0xffffffffu, swept_part);
+    if (lane == 0 && part) atomicAdd(&stats[kStatNarrow], (unsigned long long)__popc(part));
     const unsigned same_bin = __match_any_sync(0xffffffffu, ob);
     if (ok && lane == __ffs(same_bin) - 1) atomicAdd(&stats[kStatBins + ob], (unsigned long long)__popc(same_bin));
     const int64_t win = ok ? at / CRISPY_GEN_WINDOW : -1;
@@ -808,7 +846,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
 }
 // untuned 32-bit shape per bin (the plain form always uses it)
 constexpr int kDefaultShape[kNumBins] = {-1, 0, 3, 4, 4, 14, 5, 15, 6, 16, 7, 11, 12, 13, 13, -1, -1, -1, -1};
-static_assert(kStatSwept < kStatWindows, "per-bin counters overlap the window slots");
+static_assert(kStatNarrow < kStatWindows, "per-bin counters overlap the window slots");
 
 using WarpFn = void (*)(GenArgs);
 WarpFn shape_fn(int shape) {
@@ -889,7 +927,7 @@ int latency_shape(int order_bin, int64_t n_items, int sms) {
     int best = -1;
     for (int i = 0; i < gen16_num_shapes(); ++i) {
         const Shape16 h = gen16_shape(i);
-        if (2 * h.g * h.r < need || h.r > 2) continue;
+        if (2 * h.g * h.r < need || h.r > (need > 128 ? 4 : 2)) continue;
         if (n_items * h.g > 32ll * 12 * sms) continue;   // at most 12 warps per SM
         if (best < 0 || h.r < gen16_shape(best).r || (h.r == gen16_shape(best).r && h.g < gen16_shape(best).g)) best = i;
     }
@@ -980,6 +1018,7 @@ int pick_shape(crispy_ctx* ctx, cudaStream_t s, int band, int bin, const GenArgs
             t.dirs = dirs_buf.as<uint32_t>();
             t.dirs_words = dir_words;
             t.retry = nullptr;   // a timing run proves nothing
+            t.retry_most = 0;
             t.queue = queue_buf.as<unsigned int>() + (qslot++ % 64);
             CRISPY_CK(ctx, cudaMemsetAsync(t.queue, 0, 4, s));
             cudaEventRecord(e0, s);
@@ -1243,15 +1282,27 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
             CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));
         }
         if (narrow) {
-            CRISPY_TRY(ensure(ctx, g.bands, (size_t)count * 4));
+            const size_t probe_at = ((size_t)count * 4 + 15) / 16 * 16;
+            CRISPY_TRY(ensure(ctx, g.bands, probe_at + 16));
             bands = g.bands.as<uint32_t>();
             if (kdist && kdist_k >= 5) {
+                const float most = 1.0f - std::pow(0.4f, (float)kdist_k / 8.0f);
                 gen_bands_from_kmer_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, count, band, max_sum, bands);
+                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, most, count, band, max_sum, bands);
             } else {
+                unsigned long long* probe = nullptr;
+                if (count >= kBandSampleFrom) {
+                    probe = reinterpret_cast<unsigned long long*>(g.bands.as<char>() + probe_at);
+                    CRISPY_CK(ctx, cudaMemsetAsync(probe, 0, 16, s));
+                    gen_bands_kernel<true><<<kBandSample / kBandWarps, kBandWarps * 32, 0, s>>>(
+                        g.packed.as<uint32_t>(), g.woff.as<int64_t>(), g.len.as<int32_t>(), d_pairs, count, band, max_sum,
+                        bands, probe);
+                    count_launch(ctx);
+                }
                 const int blocks = (int)std::min<int64_t>((count + kBandWarps - 1) / kBandWarps, 8ll * ctx->sm_count);
-                gen_bands_kernel<<<blocks, kBandWarps * 32, 0, s>>>(g.packed.as<uint32_t>(), g.woff.as<int64_t>(),
-                                                                   g.len.as<int32_t>(), d_pairs, count, band, max_sum, bands);
+                gen_bands_kernel<false><<<blocks, kBandWarps * 32, 0, s>>>(
+                    g.packed.as<uint32_t>(), g.woff.as<int64_t>(), g.len.as<int32_t>(), d_pairs, count, band, max_sum,
+                    bands, probe);
             }
             count_launch(ctx);
         }
@@ -1259,8 +1310,13 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
         ctx->stats.gen_cells += (int64_t)st[0];
         ctx->stats.gen_pairs += count;
         GenArgs base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
-        base.bands = bands;
+        if (!ext && st[kStatNarrow] == 0) retry = nullptr;   // whole bands all of them
+        // a list that the estimate fails is swept in part once for an eighth of
+        // it, and then whole
+        const uint32_t retry_most = (uint32_t)std::max<int64_t>(1024, count / 8);
+        base.bands = retry ? bands : nullptr;
         base.retry = retry;
+        base.retry_most = retry ? retry_most : 0;
         base.ext = ext;
         CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));
         if (!retry) return CRISPY_OK;
@@ -1278,6 +1334,7 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
             if (again) {
                 CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));   // the list is in d_order now
                 base.retry = retry;
+                base.retry_most = std::max<uint32_t>(1024, left / 8);
                 base.ext = ext;
             }
             CRISPY_TRY(gen_run_bins(ctx, s, base, band, d_order, st));

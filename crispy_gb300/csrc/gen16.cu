@@ -574,6 +574,18 @@ __global__ void __launch_bounds__(kThreads, min_blocks16<R>()) gen16_kernel(GenA
         if (base >= a.count) break;
         const int64_t item = base + sub;
         const bool valid = item < a.count;
+        if (a.retry_most) {
+            // the estimate fails these reads: another sweep of part of the
+            // band would be lost too
+            uint32_t listed = lane == 0 ? *reinterpret_cast<volatile uint32_t*>(a.retry) : 0u;
+            listed = __shfl_sync(0xffffffffu, listed, 0);
+            if (listed > a.retry_most) {
+                if (gl == 0 && valid)
+                    a.retry[1 + atomicAdd(a.retry, 1u)] = a.order ? a.order[item] : (uint32_t)item;
+                if (!a.queue) base += stride;
+                continue;
+            }
+        }
         int64_t p = -1;
         Pair16 pc{0, 0, 0, 0, 0, {INT_MIN / 2, INT_MIN / 2, INT_MIN / 2, INT_MIN / 2}};
         int2 pr = make_int2(0, 0);

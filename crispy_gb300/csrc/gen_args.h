@@ -34,6 +34,9 @@ struct GenArgs {
     // whose result that does not prove ([0] their count, then pair indices)
     const uint32_t* bands;
     uint32_t* retry;
+    // once more pairs than this are listed, the rest go to the list unswept
+    // (0: no limit)
+    uint32_t retry_most;
     int ext;                 // pairs beyond kGen16MaxSum: the extended form of the shape
     // All 1.  Adds written as multiply-adds by these run on the FMA pipe;
     // distinct multipliers keep the compiler from factoring a common

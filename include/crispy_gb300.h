@@ -347,8 +347,8 @@ typedef struct crispy_stats {
     int64_t kmer_rounds;
 } crispy_stats;
 int crispy_get_stats(const crispy_ctx* ctx, crispy_stats* out);
-/* Cells the sweeps of the last genDist run held: narrow sweeps leave part of
- * a pair's band out, a pair without proof is swept twice (gen_cells counts
+/* Cells of the sweeps the last genDist run planned: narrow sweeps leave part
+ * of a pair's band out, a pair without proof is swept twice (gen_cells counts
  * every pair's whole band once). */
 int crispy_gen_swept_cells(const crispy_ctx* ctx, int64_t* cells);
 /* Enable per-launch event timing (adds events around the hot kernels). */
