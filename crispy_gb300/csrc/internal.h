@@ -60,6 +60,7 @@ template <class T> using pinned_vector = std::vector<T, PinnedAlloc<T>>;
 struct KmerJob {
     bool ready = false;
     int n = 0, k = 0, max_len = 0, min_len = 0, max_t = 0;
+    int64_t sum_t = 0;          // tuples of all reads
     int ngroups = 0;            // 32-read groups
     int64_t nent = 0;           // entries in the interleaved level-entry array
     pinned_vector<int32_t> h_t;   // tuples per read (L - K + 1)

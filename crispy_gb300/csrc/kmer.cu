@@ -2559,6 +2559,7 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
     j.max_len = 0;
     j.min_len = CRISPY_MAX_READ_LEN;
     j.max_t = 0;
+    j.sum_t = 0;
     for (int r = 0; r < n; ++r) {
         if (lengths[r] > CRISPY_MAX_READ_LEN)
             return fail(ctx, CRISPY_E_UNSUPPORTED, "read %d length %d > %d", r, lengths[r], CRISPY_MAX_READ_LEN);
@@ -2568,6 +2569,7 @@ int kmer_layout(crispy_ctx* ctx, const int32_t* lengths, int n, int k) {
         j.max_len = std::max(j.max_len, (int)lengths[r]);
         j.min_len = std::min(j.min_len, (int)lengths[r]);
         j.max_t = std::max(j.max_t, j.h_t[r]);
+        j.sum_t += j.h_t[r];
     }
     j.ngroups = (n + 31) / 32;
     j.ent_ready = j.f_ready = false;
@@ -3405,9 +3407,7 @@ struct KmerFilterNote {
 static std::map<std::string, KmerFilterNote> g_kfilter;   // guarded by g_ktune_mu
 
 static void kmer_note_filter(const KmerJob& j) {
-    int64_t sum = 0;
-    for (int r = 0; r < j.n; ++r) sum += j.h_t[r];
-    const std::string key = key_of({(uint64_t)j.n, (uint64_t)j.k, (uint64_t)sum, (uint64_t)j.max_t});
+    const std::string key = key_of({(uint64_t)j.n, (uint64_t)j.k, (uint64_t)j.sum_t, (uint64_t)j.max_t});
     std::lock_guard<std::mutex> g(g_ktune_mu);
     if (g_kfilter.size() >= 256 && !g_kfilter.count(key)) g_kfilter.clear();
     KmerFilterNote& e = g_kfilter[key];

@@ -591,14 +591,17 @@ __device__ __forceinline__ void tmem_fill32(uint32_t addr, uint32_t x) {
         ::"r"(addr), "r"(x) : "memory");
 }
 
-// Candidates of one warp: kept in shared memory, written out in runs.
-__device__ __forceinline__ void cand_flush(const FilterArgs& a, const uint2* buf, int count, int lane) {
+// Candidates of one warp: kept in shared memory, written out in runs.  Once
+// one does not fit any more the warp takes no others (*stuffed): the pass has
+// given up, and where every pair is a candidate taking them is most of its time.
+__device__ __forceinline__ void cand_flush(const FilterArgs& a, const uint2* buf, int count, int lane, bool* stuffed) {
     if (count == 0) return;
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(&a.ctl->cand[a.round], (unsigned long long)count);
     base = __shfl_sync(0xffffffffu, base, 0);
     for (int i = lane; i < count; i += 32)
         if (base + i < a.cap) a.cand[base + i] = buf[i];
+    *stuffed = base + count > a.cap;
 }
 
 __device__ __forceinline__ float max3(float x, float y, float z) {
@@ -609,7 +612,8 @@ __device__ __forceinline__ float max3(float x, float y, float z) {
 
 // One 32 x 32 block of bounds: lane = row, v = 32 columns from c0 on.
 __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float (&v)[32], float thr, int row,
-                                                int c0, uint2* buf, uint32_t* held, int lane) {
+                                                int c0, uint2* buf, uint32_t* held, int lane, bool* stuffed) {
+    if (*stuffed) return;
     float mx[4];
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -649,7 +653,7 @@ __device__ __forceinline__ void take_candidates(const FilterArgs& a, const float
     __syncwarp();
     const uint32_t n = *reinterpret_cast<volatile uint32_t*>(held);
     if (n > (uint32_t)kCandBuf / 2) {
-        cand_flush(a, buf, (int)min(n, (uint32_t)kCandBuf), lane);
+        cand_flush(a, buf, (int)min(n, (uint32_t)kCandBuf), lane, stuffed);
         __syncwarp();
         if (lane == 0) *held = 0;
         __syncwarp();
@@ -820,7 +824,7 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
         uint2* mine = cbuf + (warp - 3) * kCandBuf;
         uint32_t* held = &bars->held[warp - 3];
         uint32_t tile = 0;
-        bool ok = true;
+        bool ok = true, stuffed = false;
         for (int sg = first; sg < a.nsegs && ok; sg += stride)
         for (int it = __ldg(&a.segs[sg].x), end = __ldg(&a.segs[sg].y); it < end && ok; ++it) {
             const int4 q = __ldg(a.items + it);
@@ -855,13 +859,13 @@ __global__ void __launch_bounds__(kFilterThreads, 1) kmer_filter_kernel(
                             __syncwarp();
                             if (lane == 0) bar_arrive(&bars->acc_empty[b]);
                         }
-                        take_candidates(a, v[k & 1], need[k], row, c0 + 32 * kEpiPer * k, mine, held, lane);
+                        take_candidates(a, v[k & 1], need[k], row, c0 + 32 * kEpiPer * k, mine, held, lane, &stuffed);
                     }
                 }
             }
         }
         __syncwarp();
-        cand_flush(a, mine, (int)min(*reinterpret_cast<volatile uint32_t*>(held), (uint32_t)kCandBuf), lane);
+        cand_flush(a, mine, (int)min(*reinterpret_cast<volatile uint32_t*>(held), (uint32_t)kCandBuf), lane, &stuffed);
     }
     __syncthreads();   // every warp has left its loops
     if (*reinterpret_cast<volatile uint32_t*>(&bars->abort)) {
@@ -898,6 +902,9 @@ struct VerifyArgs {
     uint32_t* rowcnt;
     uint32_t* rowoff;
     unsigned long long cap;
+    const uint32_t* repeated; // repeats of all reads
+    float tuples;             // tuples of all reads
+    double most;              // candidates worth counting, were none dearer than usual
     int round;
     FilterCtl* ctl;
     const uint16_t* distinct;
@@ -917,10 +924,13 @@ struct VerifyArgs {
     int64_t out_cap;
 };
 
-// True when the round's candidates are there and fit.
+// True when the round's candidates are there, fit and are worth counting: a
+// candidate costs more where most of a read's K-mers are repeats (reads of few
+// bases: 1.7 ns for 0.3 with 0.88 of them; 0.06 to 0.28 are usual).
 __device__ __forceinline__ bool round_fits(const VerifyArgs& a, unsigned long long found) {
     if (pass_ended(a.ctl)) return false;
-    if (found <= a.cap) return true;
+    const float dearer = 1.0f + 8.0f * fmaxf(0.0f, (float)*a.repeated / a.tuples - 0.3f);
+    if (found <= a.cap && (dearer == 1.0f || (double)found * dearer <= a.most)) return true;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&a.ctl->overflow, 1u);
     return false;
 }
@@ -966,10 +976,17 @@ __global__ void __launch_bounds__(256) filter_scatter_kernel(const VerifyArgs a)
 
 constexpr int kVerifyWarps = 8;
 
-// Slots of the table of a row's repeats: a read of 400 nt has about 20 at
-// K = 6, one of 1,400 about 220.  Rows with more than half as many repeats
-// (long runs of few bases) search the row's list instead.
-int rep_slots_for(int max_t) { return max_t <= 512 ? 256 : max_t <= 1536 ? 512 : 1024; }
+// Slots of the table of a row's repeats, filled to a half at the most: five
+// times the repeats that a read of max_t random K-mers has (21 of 394 at K = 6,
+// 213 of 1,400), since reads are not random.  Rows with more (few bases over and
+// over) fill it part by part.
+int rep_slots_for(int k, int max_t) {
+    const double kinds = (double)(1 << (2 * k));
+    const double repeats = max_t - kinds * (1.0 - std::exp(-max_t / kinds));
+    int slots = 256;
+    while (slots < 1024 && slots < 5.0 * repeats) slots *= 2;
+    return slots;
+}
 
 // A warp takes up to 32 consecutive candidates of the sorted list.  Per row
 // (about 4 to 30 candidates each) it marks the row's distinct K-mers in a map
@@ -1019,6 +1036,13 @@ __global__ void __launch_bounds__(kVerifyWarps * 32, kK8 ? 3 : 5) filter_verify_
                     map[w >> 21] = 0;
                 }
             }
+        }
+    };
+    auto put_repeats = [&](int first, int count) {
+        for (int q = lane; q < count; q += 32) {
+            const uint32_t e = a.repeats[first + q];
+            uint32_t h = (e * 0x9E3779B1u) >> rshift;
+            while (atomicCAS(&rt[h], kSlotEmpty, e) != kSlotEmpty) h = (h + 1u) & rmask;
         }
     };
     const int64_t total = (int64_t)found;
@@ -1071,13 +1095,7 @@ __global__ void __launch_bounds__(kVerifyWarps * 32, kK8 ? 3 : 5) filter_verify_
                 cur = r;
                 mr = a.meta[r];
                 mark(reinterpret_cast<const uint4*>(a.distinct + (int64_t)r * a.dstride), mr.x, true);
-                if (mr.y <= rep_most) {
-                    for (int q = lane; q < mr.y; q += 32) {
-                        const uint32_t e = a.repeats[mr.z + q];
-                        uint32_t h = (e * 0x9E3779B1u) >> rshift;
-                        while (atomicCAS(&rt[h], kSlotEmpty, e) != kSlotEmpty) h = (h + 1u) & rmask;
-                    }
-                }
+                if (mr.y <= rep_most) put_repeats(mr.z, mr.y);
                 __syncwarp();
             }
             const int nd = (int)(sz & 0xFFFFu), nr = (int)(sz >> 16);
@@ -1116,17 +1134,23 @@ __global__ void __launch_bounds__(kVerifyWarps * 32, kK8 ? 3 : 5) filter_verify_
             if (nr > 0 && m + (uint32_t)min(nr, mr.y) >= __shfl_sync(full, lim, i)) {
                 const uint32_t rep = __shfl_sync(full, first_rep, i);
                 uint32_t more = 0;
-                for (int q = lane; q < nr; q += 32) {
-                    const uint32_t e = a.repeats[rep + q];
-                    if (!both && !(e & 0x8000u)) continue;
-                    if (mr.y <= rep_most) {
+                // a row with more repeats than the table takes at once fills it
+                // part by part
+                for (int k0 = 0; k0 < mr.y; k0 += rep_most) {
+                    if (mr.y > rep_most) {
+                        __syncwarp();
+                        for (int q = lane; q < a.rep_slots; q += 32) rt[q] = kSlotEmpty;
+                        __syncwarp();
+                        put_repeats(mr.z + k0, min(rep_most, mr.y - k0));
+                        __syncwarp();
+                    }
+                    for (int q = lane; q < nr; q += 32) {
+                        const uint32_t e = a.repeats[rep + q];
+                        if (!both && !(e & 0x8000u)) continue;
                         uint32_t h = (e * 0x9E3779B1u) >> rshift;
                         uint32_t v;
                         while ((v = rt[h]) != kSlotEmpty && v != e) h = (h + 1u) & rmask;
                         more += v == e;
-                    } else {
-                        for (int k = 0; k < mr.y; ++k)
-                            if (a.repeats[mr.z + k] == e) { ++more; break; }
                     }
                 }
                 m += __reduce_add_sync(full, more);
@@ -1191,18 +1215,24 @@ int log2_bits(uint64_t v) {
 }  // namespace
 
 namespace {
-// Candidates a round may leave: 1/256 of its pairs and 3.1 M.  Beyond that (one
-// OTU holds a good part of the reads) counting one by one costs more than the
-// tile kernels.  Both cost the same at about 3.9 M candidates for 20,000 reads
-// of 250 nt, 9 M for 50,000, 23 M for 100,000 of 300-500 nt, 6 M for 30,000 of
-// them at K = 7 and 3 M for 12,000 at K = 5.  Whole kmerDist calls, filter
-// against tiles: 20,000 reads in Zipf's proportions (4.0 M) 1,543 and 1,888 us,
-// three tenths of them in one OTU (8.1 M) 2,864 and 2,110; 100,000 with 0.07 in
-// one (15 M) 8.0 and 10.6 ms, with 0.15 (54 M) 22.0 and 13.2.
-// (CRISPY_KMER_CAND sets the room, for tests.)
-int64_t candidate_room(int64_t pairs) {
+// Candidates a round may leave: 1/256 of its pairs and 3.1 M at K = 6, less
+// where the tile kernels are faster (K = 7 and 8) or a candidate dearer (K = 5:
+// more repeats).  Beyond that (one OTU holds a good part of the reads) counting
+// one by one costs more than the tile kernels.  Both cost the same at about
+// 3.9 M candidates for 20,000 reads of 250 nt, 9 M for 50,000, 4.2 M for 12,000
+// of 300-500 nt, 23 M for 100,000, 2.9 M for 11,000 at K = 5, 2.4 M for 12,000
+// and 6 M for 30,000 at K = 7, 1.8 M for 20,000 of 250 nt at K = 8.  Whole
+// kmerDist calls, filter against tiles: 20,000 reads in Zipf's proportions
+// (4.0 M) 1,543 and 1,888 us, three tenths of them in one OTU (8.1 M) 2,864 and
+// 2,110; 100,000 with 0.07 in one (15 M) 8.0 and 10.6 ms, with 0.15 (54 M) 22.0
+// and 13.2.  (CRISPY_KMER_CAND sets the room, for tests.)
+int64_t candidates_worth(int64_t pairs, int k) {
     if (const char* e = std::getenv("CRISPY_KMER_CAND")) return std::max(1ll, std::atoll(e));
-    return std::min<int64_t>(std::min<int64_t>(1 << 25, pairs / 256 + (3 << 20)), std::max<int64_t>(pairs, 1));
+    const int64_t base = (int64_t)(k <= 5 ? 11 : k == 6 ? 12 : k == 7 ? 9 : 6) << 18;
+    return std::min<int64_t>(1 << 25, pairs / 256 + base);
+}
+int64_t candidate_room(int64_t pairs, int k) {
+    return std::min<int64_t>(candidates_worth(pairs, k), std::max<int64_t>(pairs, 1));
 }
 
 // Their buffer: a quarter more, so that a set which the probe lets pass by a
@@ -1223,11 +1253,23 @@ constexpr int64_t kProbeFrom = 16;
 // 2 T bins 2 to 5 times at cuts up to 0.15 but 4 to 12 times at 0.3, at 3 T
 // bins 1.5 to 4 times at 0.3; 1.3 T bins leave 6 to 15 times at 0.12.
 constexpr float kMostCut = 0.3f;
-int dims_for(int64_t tuples, int n, int k, float thr) {
+int dims_wanted(int64_t tuples, int n, float thr) {
     const int mean = (int)(tuples / std::max(1, n));
-    const int most = std::min(1 << (2 * k), 4096);
     const int halves = thr <= 0.15f ? 4 : thr <= 0.25f ? 5 : 6;
-    return std::min(most, std::max(1, (halves * mean / 2 + 128) / 256) * 256);
+    return halves * mean / 2;
+}
+int dims_for(int64_t tuples, int n, int k, float thr) {
+    const int most = std::min(1 << (2 * k), 4096);
+    return std::min(most, std::max(1, (dims_wanted(tuples, n, thr) + 128) / 256) * 256);
+}
+// Whether 4^K bins are enough of those (K = 5 has 1,024): kmerDist calls,
+// filter against tiles, at 2.0 times as many wanted 1,073 and 2,256 us (15,000
+// reads of 1,000 nt, cut 0.05) but 2,418 and 1,954 (6,000, cut 0.15), at 1.7
+// times 1,118 and 1,704 (6,000 of 850 nt, cut 0.15) but 2,478 and 1,456 (6,000
+// of 600 nt, cut 0.3), at 1.5 times 1,338 and 1,363 (6,000 of 500 nt, cut 0.3).
+bool dims_do(int64_t tuples, int n, int k, float thr) {
+    const float most = thr <= 0.08f ? 2.0f : thr <= 0.15f ? 1.7f : 1.5f;
+    return (float)dims_wanted(tuples, n, thr) <= most * (float)std::min(1 << (2 * k), 4096);
 }
 }  // namespace
 
@@ -1244,17 +1286,18 @@ size_t kmer_filter_bytes(const int32_t* len, int n, int k) {
     }
     const int64_t read = 2 * (max_len / 16 + 5) * 4 + dims_for(tuples, n, k, kMostCut) / 2 + (most + 8) * 2 + 64;
     const int64_t pairs = (int64_t)n * (n + 512) / 2;
-    return (size_t)(n * read + tuples * 4 + candidate_buffer(candidate_room(pairs)) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
+    return (size_t)(n * read + tuples * 4 + candidate_buffer(candidate_room(pairs, k)) * 20 + pairs / (kRows * kCols) * 16 + (1 << 20));
 }
 
 // Rule: K >= 5 (K = 4 has 256 bins at most, and the bound leaves a third to
 // all of the pairs) and a cut of at most 0.3 (at 0.35 and above 7-30 % of
 // the pairs stay at K = 5, and counting those one by one costs more than the
-// tile kernels).  CRISPY_KMER_FILTER=0 turns
+// tile kernels), with bins enough for the reads' length.  CRISPY_KMER_FILTER=0 turns
 // it off; so do the variables that pick the tile kernels' own forms.  Reads
 // that gave it up once do so at every cut as loose while they stay prepared.
 bool kmer_filter_applies(const KmerJob& j, float thr) {
     if (j.k < 5 || !(thr <= kMostCut) || j.max_t < 1 || thr >= j.f_gave_up) return false;
+    if (!dims_do(j.sum_t, j.n, j.k, thr)) return false;
     const char* e = std::getenv("CRISPY_KMER_FILTER");
     if (e && e[0] == '0') return false;
     for (const char* v : {"CRISPY_KMER_SPLIT", "CRISPY_KMER_QFIRE", "CRISPY_KMER_PREP_WARP",
@@ -1270,8 +1313,7 @@ int kmer_filter_build(crispy_ctx* ctx, float thr) {
     cudaStream_t s = ctx->stream;
     const int n = j.n, k = j.k;
     const int K4 = 1 << (2 * k);
-    int64_t tuples = 0;
-    for (int r = 0; r < n; ++r) tuples += j.h_t[r];
+    const int64_t tuples = j.sum_t;
     const int dims = dims_for(tuples, n, k, thr);
     if (j.f_ready && j.f_dims == dims) return CRISPY_OK;
     j.f_ready = j.f_lists = false;
@@ -1418,7 +1460,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     std::vector<int2>& segs = j.h_segs;   // the probe's, then the rounds'
     items.clear();
     segs.clear();
-    const int64_t room = candidate_room((pairs + rounds - 1) / rounds), ccap = candidate_buffer(room);
+    const int64_t room = candidate_room((pairs + rounds - 1) / rounds, k), ccap = candidate_buffer(room);
     const bool probe = work >= kProbeFrom * ctx->sm_count && room * rounds < (int64_t)n * (n - 1) / 2;
     const int64_t nprobe = probe ? ctx->sm_count : 0;
     const int64_t probe_run = std::min<int64_t>(8, std::max<int64_t>(1, work / (128ll * ctx->sm_count)));
@@ -1504,7 +1546,10 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     va.mmin = j.mmin.as<uint16_t>();
     va.n = n;
     va.K = k;
-    va.rep_slots = rep_slots_for(j.max_t);
+    va.rep_slots = rep_slots_for(k, j.max_t);
+    va.repeated = j.f_hist.as<uint32_t>() + (1 << (2 * k));
+    va.tuples = (float)std::max<int64_t>(j.sum_t, 1);
+    va.most = (double)candidates_worth((pairs + rounds - 1) / rounds, k);
     va.olo = olo;
     va.ohi = ohi;
     va.A = A;
@@ -1514,7 +1559,7 @@ int kmer_filter_pass(crispy_ctx* ctx, int olo, int ohi, int64_t cap, int A, int 
     va.vals = j.vals.as<uint32_t>();
     va.out_cap = cap;
     // byte marks where they leave room for five blocks per SM
-    const bool bytes = k <= 6 && va.rep_slots == 256;
+    const bool bytes = k <= 6 && (size_t)kVerifyWarps * ((1 << (2 * k)) + va.rep_slots * 4) <= kSmemLimit / 5;
     const int map_words = bytes ? 1 << (2 * k - 2) : 1 << (2 * k - 5);
     const size_t vsmem = (size_t)kVerifyWarps * (map_words + va.rep_slots) * 4;
     auto verify = bytes ? filter_verify_kernel<true, false>

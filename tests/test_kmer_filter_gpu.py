@@ -134,3 +134,21 @@ def test_filter_wait_limit(engine, monkeypatch, wait, length):
     monkeypatch.delenv("CRISPY_KMER_WAIT")
     got = run()         # the context is as usable as before
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+# reads of few bases over and over: more repeats than the count's table takes
+# at once (128, 256 or 512 entries), so that it is filled part by part
+@pytest.mark.parametrize("k,length", [(5, 450), (6, 300), (6, 900), (7, 500), (7, 2048), (8, 700), (8, 2048)])
+def test_filter_rows_of_many_repeats(engine, monkeypatch, k, length):
+    rng = np.random.default_rng(k + length)
+    reads = []
+    for unit in (1, 2, 3, 5, 9, 40):
+        base = np.resize(rng.choice(np.frombuffer(b"ACGT", np.uint8), unit), length)
+        for _ in range(30):
+            s = base[:int(rng.integers(length - length // 8, length + 1))].copy()
+            for p in rng.integers(0, len(s), int(rng.integers(0, 6))):
+                s[p] = b"ACGT"[int(rng.integers(0, 4))]
+            reads.append(s.tobytes())
+    reads = [reads[i] for i in rng.permutation(len(reads))]
+    for thr in (0.05, 0.3):
+        assert _check(engine, monkeypatch, reads, k, thr) > 100
