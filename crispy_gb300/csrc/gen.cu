@@ -658,13 +658,30 @@ static_assert(2 * kNumBins < 64, "order-bins overflow the 18-bit sort key");
 // One warp per pair: the longer read's 8-mers in a hashed bitmap, the
 // shorter's looked up in it.
 //
-// Large lists (kSample): first the slots a sample of the pairs would save, in
-// probe[0] of probe[1].  Where that is under a sixteenth nothing is estimated
-// for the others (40 us for 60,000 pairs of 250 nt).
+// The slots saved, of all slots, go to probe[0] and probe[1]: of every pair, or
+// of a sample of the pairs first (kSample).  Where they are less than
+// min_share of them nothing is estimated for the others (40 us for 60,000 pairs
+// of 250 nt) and nothing swept in part (gen_classify_kernel).
 constexpr int kBandWarps = 8;
 constexpr int kBandBits = 14;
 constexpr int kBandSample = 1024;          // pairs
-constexpr int64_t kBandSampleFrom = 16384;
+constexpr int64_t kBandSampleFrom = 2048;
+// Adds a block's sums to probe (every thread of the block calls it; the sums
+// of lane 0 count).
+__device__ __forceinline__ void add_saved(unsigned long long saved, unsigned long long slots, unsigned long long* probe) {
+    __shared__ unsigned long long sum[2];
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sum[0], saved);
+        atomicAdd(&sum[1], slots);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && sum[threadIdx.x]) atomicAdd(&probe[threadIdx.x], sum[threadIdx.x]);
+}
+__device__ __forceinline__ bool too_little_saved(const unsigned long long* probe, float min_share) {
+    return (double)probe[0] < (double)min_share * (double)probe[1];
+}
 template <bool kSample>
 __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32_t* __restrict__ packed,
                                                                     const int64_t* __restrict__ woff,
@@ -672,12 +689,13 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
                                                                     const int2* __restrict__ pairs, int64_t count,
                                                                     int band, int max_sum,
                                                                     uint32_t* __restrict__ bands,
-                                                                    unsigned long long* __restrict__ probe) {
+                                                                    unsigned long long* probe, bool sampled,
+                                                                    float min_share) {
     __shared__ __align__(16) uint32_t bitmap[kBandWarps][1 << (kBandBits - 5)];
     const int lane = threadIdx.x & 31;
     uint32_t* bm = bitmap[threadIdx.x >> 5];
     const int64_t nw = (int64_t)gridDim.x * kBandWarps;
-    if (!kSample && probe && probe[0] * 16 < probe[1]) {
+    if (!kSample && sampled && too_little_saved(probe, min_share)) {
         for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < count; p += nw * 32) {
             const int2 pr = pairs[p];
             const int l1 = len[pr.x], l2 = len[pr.y];
@@ -686,6 +704,7 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
         }
         return;
     }
+    unsigned long long saved = 0, slots = 0;
     const int64_t todo = kSample ? kBandSample : count;
     for (int64_t i = (int64_t)blockIdx.x * kBandWarps + (threadIdx.x >> 5); i < todo; i += nw) {
         const int64_t p = kSample ? i * count / kBandSample : i;
@@ -723,16 +742,12 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
                 hi = min(kb, e + max(0, l2 - l1));
             }
         }
-        if (kSample) {
-            if (lane == 0) {
-                atomicAdd(&probe[0], (unsigned long long)(2 * kb - lo - hi));
-                atomicAdd(&probe[1], (unsigned long long)(2 * kb + 2));
-            }
-        } else if (lane == 0) {
-            bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
-        }
+        saved += (unsigned long long)(2 * kb - lo - hi);
+        slots += (unsigned long long)(2 * kb + 2);
+        if (!kSample && lane == 0) bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
         __syncwarp();
     }
+    if (kSample || !sampled) add_saved(saved, slots, probe);
 }
 
 // The same estimate from kmerDist's own count: of the shorter read's T K-mers
@@ -740,20 +755,23 @@ __global__ void __launch_bounds__(kBandWarps * 32) gen_bands_kernel(const uint32
 // (up to the share of K-mers that the same divergence takes, most_dist).
 __global__ void gen_bands_from_kmer_kernel(const int32_t* __restrict__ len, const int2* __restrict__ pairs,
                                            const float* __restrict__ kdist, int K, float most_dist, int64_t count,
-                                           int band, int max_sum, uint32_t* __restrict__ bands) {
+                                           int band, int max_sum, uint32_t* __restrict__ bands,
+                                           unsigned long long* __restrict__ probe) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= count) return;
-    const int2 pr = pairs[p];
-    const int l1 = len[pr.x], l2 = len[pr.y];
+    const int2 pr = p < count ? pairs[p] : make_int2(0, 0);
+    const int l1 = p < count ? len[pr.x] : 0, l2 = p < count ? len[pr.y] : 0;
     const int kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
     int lo = kb, hi = kb;
-    if (l1 + l2 <= max_sum && kb >= 16 && (kdist[p] <= most_dist || kb >= kMaxSlots16)) {
+    if (p < count && l1 + l2 <= max_sum && kb >= 16 && (kdist[p] <= most_dist || kb >= kMaxSlots16)) {
         const float miss = kdist[p] * (float)(min(l1, l2) - K + 1);
         const int e = (int)fminf(miss * 3.25f / (float)K, 4096.0f) + 3;
         lo = min(kb, e + max(0, l1 - l2));
         hi = min(kb, e + max(0, l2 - l1));
     }
-    bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+    if (p < count) bands[p] = (uint32_t)lo | (uint32_t)hi << 16;
+    const unsigned saved = __reduce_add_sync(0xffffffffu, (unsigned)(2 * kb - lo - hi));
+    const unsigned slots = __reduce_add_sync(0xffffffffu, p < count ? (unsigned)(2 * kb + 2) : 0u);
+    add_saved(saved, slots, probe);
 }
 
 // Per-pair classification for the launch plan, on the device.  Order-bin
@@ -774,11 +792,13 @@ constexpr int kWideOrderBin = 2 * kNumBins;
 constexpr int kStatMaxSum16 = kStatBins + kWideOrderBin + 1;
 constexpr int kStatSwept = kStatMaxSum16 + 1;   // cells this launch's sweeps hold
 constexpr int kStatNarrow = kStatSwept + 1;     // pairs swept over part of their band
-// bands: the diagonals each pair is swept over (nullptr: all of its band);
+// bands: the diagonals each pair is swept over (nullptr: all of its band, and
+// so where they save too little of the slots);
 // list: the pairs to take (nullptr: all), whose cells then stay uncounted.
 __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t count,
                                     const int32_t* __restrict__ len, int band, int nbins, int max_sum, int most_slots,
-                                    const uint32_t* __restrict__ bands, const uint32_t* __restrict__ list,
+                                    const uint32_t* __restrict__ bands, const unsigned long long* __restrict__ probe,
+                                    float min_share, const uint32_t* __restrict__ list,
                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                     unsigned long long* __restrict__ stats) {
     const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -794,7 +814,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         const int l1 = len[pr.x], l2 = len[pr.y];
         kb = band >= 2 ? (l1 + l2) / (2 * band) : max(l1, l2);
         int lo = kb, hi = kb;
-        if (bands) {
+        if (bands && !too_little_saved(probe, min_share)) {
             lo = (int)(bands[p] & 0xFFFFu);
             hi = (int)(bands[p] >> 16);
         }
@@ -815,7 +835,7 @@ __global__ void gen_classify_kernel(const int2* __restrict__ pairs, int64_t coun
         }
         cells = (unsigned long long)swept_cells_of(l1, l2, kb, kb);
         // (the wide-band kernel knows whole bands only)
-        swept = bands && bin != 0 ? (unsigned long long)swept_cells_of(l1, l2, lo, hi) : cells;
+        swept = bin != 0 ? (unsigned long long)swept_cells_of(l1, l2, lo, hi) : cells;
         if (list) cells = 0;
         swept_part = lo < kb || hi < kb;
     }
@@ -1075,24 +1095,42 @@ bool gen16_ext_on() {
     return !(e && e[0] == '0');
 }
 
-// Whether a batched run sweeps narrow bands first: from about 1e9 band cells
-// (0.4 ms) on, where the saved slots outweigh the estimate, its read-back and
-// the second sweep's latency (about 100 us together; 7,000 pairs of 250 nt at
-// band 10 lost 180 us of 460); and whenever a whole band may be wider than any
-// register shape (the wide-band kernel takes about a second for one such pair).
+// Whether a batched run sweeps narrow bands first, and the least share of the
+// slots that they have to save (known on the device only): from about 1e9 band
+// cells (0.4 ms) on, where they save more than they cost.  That is the
+// read-back and the second launches (80 us), the estimate where the pairs come
+// without K-mer distances (list; 0.8 ns a pair of 250 nt), and the chain of
+// anti-diagonals of the pairs swept again (three times beyond the 16-bit range).
+// Measured, whole bands against narrow ones: 117,000 pairs of 250 nt at band 10
+// (0.07 of the slots saved) 1,049 and 1,228 us, 22,000 of 300-500 nt at band 5
+// (0.26) 926 and 1,040, 3,000 of 1,200-1,600 nt at band 10 (0.08) 1,135 and 1,403;
+// 117,000 of 250 nt at band 5 (0.32) 1,815 and 1,546, 60,000 at band 2 (0.66)
+// 2,560 and 1,200.  Whenever a whole band may be wider than any register shape:
+// the wide-band kernel takes about a second for one such pair.
 // CRISPY_GEN_NARROW=0 / 1 forces it off / on.
-bool narrow_pays(const GenJob& g, int64_t count, int band) {
-    if (const char* e = std::getenv("CRISPY_GEN_NARROW")) return e[0] != '0';
+struct NarrowPlan {
+    bool on;
+    float min_share;
+};
+NarrowPlan narrow_plan(const GenJob& g, int64_t count, int band, bool list) {
+    constexpr float least = 1.0f / 16;
+    if (const char* e = std::getenv("CRISPY_GEN_NARROW")) return {e[0] != '0', least};
     const double half = band >= 2 ? (double)g.max_len / band : (double)g.max_len;
-    if (half >= kBinSlots[kNumBins - 1]) return true;
-    return (double)count * half * g.max_len >= 5e8;
+    if (half >= kBinSlots[kNumBins - 1]) return {true, 0.0f};
+    if ((double)count * half * g.max_len < 5e8) return {false, 0.0f};
+    const double mean = (double)g.sum_len / std::max(1, g.n);
+    const double whole_us = count * mean * mean * (band >= 2 ? 2.0 / band : 1.0) / 2.4e6;
+    const double cost_us = 80.0 + (list ? count * mean * 3.2e-6 : 0.0) +
+                           (2 * g.max_len > kGen16MaxSum ? 3 : 1) * 0.12 * mean;
+    const double share = 1.2 * cost_us / whole_us;
+    return {share < 0.75, std::max(least, (float)share)};
 }
 
 // Classification of `count` pairs (all, or those of `list`): statistics to
 // the host and, for the batched form, the launch order.
 int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t count, int band, bool sorted,
-                 int max_sum, const uint32_t* bands, const uint32_t* list, std::vector<unsigned long long>& st,
-                 uint32_t** d_order) {
+                 int max_sum, const uint32_t* bands, const unsigned long long* probe, float min_share,
+                 const uint32_t* list, std::vector<unsigned long long>& st, uint32_t** d_order) {
     GenJob& g = ctx->gen;
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
     const int nstats = kStatWindows + 2 * (int)nwin;
@@ -1107,7 +1145,7 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
     auto classify = [&]() -> int {
         CRISPY_CK(ctx, cudaMemsetAsync(d_stats, 0, (size_t)nstats * 8, s));
         gen_classify_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, max_sum, ctx->lean ? kMaxSlots32 : kMaxSlots16, bands, list,
+            d_pairs, count, g.len.as<int32_t>(), band, kNumBins, max_sum, ctx->lean ? kMaxSlots32 : kMaxSlots16, bands, probe, min_share, list,
             sorted ? g.ckeys.as<uint32_t>() : nullptr, sorted ? g.cvals.as<uint32_t>() : nullptr, d_stats);
         count_launch(ctx);
         if (sorted) {
@@ -1121,11 +1159,13 @@ int gen_classify(crispy_ctx* ctx, cudaStream_t s, const int2* d_pairs, int64_t c
     };
     if (sorted) {
         CRISPY_TRY(ensure(ctx, g.scan, sort_tmp_bytes(count)));
+        uint32_t share_bits = 0;
+        std::memcpy(&share_bits, &min_share, 4);
         const std::string key = "gclass," + key_of({(uint64_t)count, (uint64_t)band, (uint64_t)(uintptr_t)d_pairs,
             (uint64_t)(uintptr_t)g.len.ptr, (uint64_t)(uintptr_t)d_stats, (uint64_t)(uintptr_t)g.ckeys.ptr,
             (uint64_t)(uintptr_t)g.ckeys_alt.ptr, (uint64_t)(uintptr_t)g.cvals.ptr,
             (uint64_t)(uintptr_t)g.cvals_alt.ptr, (uint64_t)(uintptr_t)g.scan.ptr, (uint64_t)(uintptr_t)bands,
-            (uint64_t)(uintptr_t)list, (uint64_t)max_sum, (uint64_t)ctx->lean});
+            (uint64_t)(uintptr_t)list, (uint64_t)max_sum, (uint64_t)ctx->lean, (uint64_t)(uintptr_t)probe, (uint64_t)share_bits});
         CRISPY_TRY(graph_run(ctx, s, key, classify));
         *d_order = sort_lands_in_alt(count, kOrderBits) ? g.cvals_alt.as<uint32_t>() : g.cvals.as<uint32_t>();
     } else {
@@ -1271,11 +1311,14 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
     uint32_t* d_order = nullptr;
     if (mode == CRISPY_MODE_BATCHED) {
         // (a forced shape sweeps whole bands, up to the shape's full width)
-        const bool narrow = !ctx->lean && forced_shape() < 0 && narrow_pays(g, count, band);
+        const bool list = !(kdist && kdist_k >= 5);
+        const NarrowPlan plan = narrow_plan(g, count, band, list);
+        const bool narrow = !ctx->lean && forced_shape() < 0 && plan.on;
         // pairs beyond the 16-bit range: its extended form first
         const bool ext = !ctx->lean && forced_shape() < 0 && 2 * g.max_len > kGen16MaxSum && gen16_ext_on();
         const int max_sum = ext ? kGen16ExtSum : kGen16MaxSum;
         uint32_t *bands = nullptr, *retry = nullptr;
+        unsigned long long* probe = nullptr;
         if (narrow || ext) {
             CRISPY_TRY(ensure(ctx, g.retry, (size_t)(count + 1) * 4));
             retry = g.retry.as<uint32_t>();
@@ -1285,28 +1328,28 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
             const size_t probe_at = ((size_t)count * 4 + 15) / 16 * 16;
             CRISPY_TRY(ensure(ctx, g.bands, probe_at + 16));
             bands = g.bands.as<uint32_t>();
-            if (kdist && kdist_k >= 5) {
+            probe = reinterpret_cast<unsigned long long*>(g.bands.as<char>() + probe_at);
+            CRISPY_CK(ctx, cudaMemsetAsync(probe, 0, 16, s));
+            if (!list) {
                 const float most = 1.0f - std::pow(0.4f, (float)kdist_k / 8.0f);
                 gen_bands_from_kmer_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(
-                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, most, count, band, max_sum, bands);
+                    g.len.as<int32_t>(), d_pairs, kdist, kdist_k, most, count, band, max_sum, bands, probe);
             } else {
-                unsigned long long* probe = nullptr;
-                if (count >= kBandSampleFrom) {
-                    probe = reinterpret_cast<unsigned long long*>(g.bands.as<char>() + probe_at);
-                    CRISPY_CK(ctx, cudaMemsetAsync(probe, 0, 16, s));
+                const bool sampled = count >= kBandSampleFrom;
+                if (sampled) {
                     gen_bands_kernel<true><<<kBandSample / kBandWarps, kBandWarps * 32, 0, s>>>(
                         g.packed.as<uint32_t>(), g.woff.as<int64_t>(), g.len.as<int32_t>(), d_pairs, count, band, max_sum,
-                        bands, probe);
+                        bands, probe, sampled, plan.min_share);
                     count_launch(ctx);
                 }
                 const int blocks = (int)std::min<int64_t>((count + kBandWarps - 1) / kBandWarps, 8ll * ctx->sm_count);
                 gen_bands_kernel<false><<<blocks, kBandWarps * 32, 0, s>>>(
                     g.packed.as<uint32_t>(), g.woff.as<int64_t>(), g.len.as<int32_t>(), d_pairs, count, band, max_sum,
-                    bands, probe);
+                    bands, probe, sampled, plan.min_share);
             }
             count_launch(ctx);
         }
-        CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, true, max_sum, bands, nullptr, st, &d_order));
+        CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, true, max_sum, bands, probe, plan.min_share, nullptr, st, &d_order));
         ctx->stats.gen_cells += (int64_t)st[0];
         ctx->stats.gen_pairs += count;
         GenArgs base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
@@ -1314,7 +1357,7 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
         // a list that the estimate fails is swept in part once for an eighth of
         // it, and then whole
         const uint32_t retry_most = (uint32_t)std::max<int64_t>(1024, count / 8);
-        base.bands = retry ? bands : nullptr;
+        base.bands = retry && st[kStatNarrow] != 0 ? bands : nullptr;
         base.retry = retry;
         base.retry_most = retry ? retry_most : 0;
         base.ext = ext;
@@ -1322,14 +1365,14 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
         if (!retry) return CRISPY_OK;
         // the pairs without proof over the whole band: beyond the 16-bit range
         // in the extended form once more, then what that does not prove
-        bool again = ext && narrow;
+        bool again = ext && base.bands != nullptr;
         for (;;) {
             uint32_t left = 0;
             CRISPY_CK(ctx, cudaMemcpyAsync(&left, retry, 4, cudaMemcpyDeviceToHost, s));
             CRISPY_CK(ctx, cudaStreamSynchronize(s));
             if (left == 0) return CRISPY_OK;
-            CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, again ? max_sum : kGen16MaxSum, nullptr,
-                                    retry + 1, st, &d_order));
+            CRISPY_TRY(gen_classify(ctx, s, d_pairs, left, band, true, again ? max_sum : kGen16MaxSum, nullptr, nullptr,
+                                    0.0f, retry + 1, st, &d_order));
             base = gen_base_args(ctx, d_pairs, band, st, d_dist, d_score, d_ml, d_al);
             if (again) {
                 CRISPY_CK(ctx, cudaMemsetAsync(retry, 0, 4, s));   // the list is in d_order now
@@ -1342,7 +1385,7 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
             again = false;
         }
     }
-    CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, kGen16MaxSum, nullptr, nullptr, st, &d_order));
+    CRISPY_TRY(gen_classify(ctx, s, d_pairs, count, band, false, kGen16MaxSum, nullptr, nullptr, 0.0f, nullptr, st, &d_order));
     const int64_t nwin = (count + CRISPY_GEN_WINDOW - 1) / CRISPY_GEN_WINDOW;
     const int kbmax = (int)st[1];
     ctx->stats.gen_cells += (int64_t)st[0];
@@ -1538,6 +1581,7 @@ int crispy_gen_prepare(crispy_ctx* ctx, const char* seqbuf, const int64_t* offse
     g.h_woff.resize(n + 1);
     int64_t end = 0, words = 0;
     g.max_len = 0;
+    g.sum_len = 0;
     for (int r = 0; r < n; ++r) {
         if (lengths[r] > CRISPY_MAX_READ_LEN)
             return fail(ctx, CRISPY_E_UNSUPPORTED, "read %d length %d > %d", r, lengths[r], CRISPY_MAX_READ_LEN);
@@ -1546,6 +1590,7 @@ int crispy_gen_prepare(crispy_ctx* ctx, const char* seqbuf, const int64_t* offse
         words += (lengths[r] + 15) / 16;
         end = std::max(end, offsets[r] + lengths[r]);
         g.max_len = std::max(g.max_len, (int)lengths[r]);
+        g.sum_len += lengths[r];
     }
     g.h_woff[n] = words;
     cudaStream_t s = ctx->stream;
@@ -1596,6 +1641,7 @@ int crispy_gen_prepare_from_kmer(crispy_ctx* ctx) {
         // a copy, and lengths and offsets written on the device
         if (j.min_len <= 0) return fail(ctx, CRISPY_E_INPUT, "a read is empty");
         g.max_len = j.max_len;
+        g.sum_len = j.sum_t + (int64_t)n * (j.k - 1);
         cudaStream_t s = ctx->stream;
         const size_t words = fwords;
         CRISPY_CK(ctx, cudaMemcpyAsync(g.packed.ptr, j.f_packed.ptr, words * 4, cudaMemcpyDeviceToDevice, s));
@@ -1611,6 +1657,7 @@ int crispy_gen_prepare_from_kmer(crispy_ctx* ctx) {
     g.h_woff.resize(n + 1);
     int64_t words = 0;
     g.max_len = 0;
+    g.sum_len = 0;
     for (int r = 0; r < n; ++r) {
         const int L = j.h_t[r] + j.k - 1;
         if (L <= 0) return fail(ctx, CRISPY_E_INPUT, "read %d is empty", r);
@@ -1618,6 +1665,7 @@ int crispy_gen_prepare_from_kmer(crispy_ctx* ctx) {
         g.h_woff[r] = words;
         words += (L + 15) / 16;
         g.max_len = std::max(g.max_len, L);
+        g.sum_len += L;
     }
     g.h_woff[n] = words;
     cudaStream_t s = ctx->stream;
@@ -1657,12 +1705,14 @@ int crispy_gen_prepare_from_pre(crispy_ctx* ctx, const crispy_raw* raw) {
     g.h_woff.resize(n + 1);
     int64_t words = 0;
     g.max_len = 0;
+    g.sum_len = 0;
     for (int r = 0; r < n; ++r) {
         if (len[r] > CRISPY_MAX_READ_LEN)
             return fail(ctx, CRISPY_E_UNSUPPORTED, "read %d length %d > %d", r, len[r], CRISPY_MAX_READ_LEN);
         g.h_woff[r] = words;
         words += (len[r] + 15) / 16;
         g.max_len = std::max(g.max_len, len[r]);
+        g.sum_len += len[r];
     }
     g.h_woff[n] = words;
     cudaStream_t s = ctx->stream;

@@ -120,6 +120,7 @@ struct KmerJob {
 struct GenJob {
     bool ready = false;
     int n = 0, max_len = 0;
+    int64_t sum_len = 0;    // of all reads
     pinned_vector<int32_t> h_len;
     pinned_vector<int64_t> h_woff;     // first packed word of each read
     pinned_vector<uint32_t> h_tiles;   // survivors per compaction tile (chunk boundaries)
