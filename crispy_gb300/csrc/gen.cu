@@ -1311,7 +1311,9 @@ static int gen_dispatch_form(crispy_ctx* ctx, cudaStream_t s, const int2* d_pair
     uint32_t* d_order = nullptr;
     if (mode == CRISPY_MODE_BATCHED) {
         // (a forced shape sweeps whole bands, up to the shape's full width)
-        const bool list = !(kdist && kdist_k >= 5);
+        // (long reads find K-mers of few kinds by chance: 1,400 nt at K = 5 left
+        // 0.5 of the pairs without proof)
+        const bool list = !(kdist && kdist_k >= 5 && 2 * g.sum_len <= (int64_t)g.n << (2 * kdist_k));
         const NarrowPlan plan = narrow_plan(g, count, band, list);
         const bool narrow = !ctx->lean && forced_shape() < 0 && plan.on;
         // pairs beyond the 16-bit range: its extended form first
