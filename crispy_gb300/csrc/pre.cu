@@ -268,6 +268,16 @@ __global__ void pre_primer_kernel(ReadSet r, int n, const uint8_t* __restrict__ 
     }
 }
 
+// Comparisons inside groups of equal keys up to which settling them costs less
+// than comparing reads in every merge: 4 million, whatever the number of reads
+// (20,000 reads of 250 nt settled with 2.5 M in 430 us and compared throughout
+// in 499, with 4.5 M 539 and 513; 60,000 with 3.3 M 622 and 632, with 18 M 864
+// and 658; 150,000 with 4.9 M 1,026 and 983, of 120 nt with 6.2 M 930 and 808).
+// An estimate that was wrong by more than four times is given up for the other
+// form.
+constexpr double kSettleWorth = 4e6;
+constexpr unsigned long long kSettleMost = 1ull << 24;
+
 // Whether reads of equal keys are so many that comparing the reads throughout
 // costs less than settling them group by group.  force: the reads are compared
 // throughout, whatever the estimate says.
@@ -702,7 +712,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
     uint2* d_range = static_cast<uint2*>(ranges);
     unsigned long long* d_work = j.counters.as<unsigned long long>() + 4;
     unsigned long long* d_many = d_work + 1;
-    const unsigned long long limit = 256ull * (unsigned long long)m + 4096;
+    const unsigned long long limit = kSettleMost;
     const unsigned blocks = (unsigned)((m + 255) / 256), wblocks = (unsigned)((m + 7) / 8);
     const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
     ReadKey* ka = nullptr;
@@ -715,9 +725,7 @@ extern "C" int crispy_preprocess(crispy_ctx* ctx, const char* seqbuf, const int6
         ka = static_cast<ReadKey*>(keys0);
         ReadKey* kb = static_cast<ReadKey*>(keys1);
         pre_key_kernel<<<blocks, 256, 0, s>>>(rs, a, m, ka);
-        // (60,000 reads: settling 64 comparisons a read costs about what the
-        // merges save)
-        pre_sample_kernel<<<1, kSample, 0, s>>>(ka, m, 64.0 * (double)m + 4096.0, d_many);
+        pre_sample_kernel<<<1, kSample, 0, s>>>(ka, m, kSettleWorth, d_many);
         count_launch(ctx, 2);
         if (m < 2) return;
         pre_tile_sort_kernel<false><<<tiles, kTileThreads, 0, s>>>(a, ka, m, rs, ties);
