@@ -135,7 +135,7 @@ static_assert(kBase % 4 == 0, "the score is read back as (K - 4s - kBase) / 4");
 // diagonal whose key is kFloorClear above the floor at the end of a block has
 // none raised in the next.  The pairs without either proof go to the 32-bit
 // kernel.  12,000 pairs of 1,800-2,048 nt at band 10, a whole
-// run: 10.2 ms in the 32-bit kernel, 5.0 here (with narrow sweeps).  500 pairs at
+// run: 10.2 ms in the 32-bit kernel, 4.5 here.  500 pairs at
 // band 5, some unrelated: 1,433 ms with whole bands beyond 256 slots in the
 // wide-band kernel, 170 with only the score as proof, 1.0 with both.
 constexpr int kBaseExt = 65535 - 131 - 14 * (kGen16ExtSum + kSlack);
