@@ -1225,9 +1225,13 @@ namespace {
 // kmerDist calls, filter against tiles: 20,000 reads in Zipf's proportions
 // (4.0 M) 1,543 and 1,888 us, three tenths of them in one OTU (8.1 M) 2,864 and
 // 2,110; 100,000 with 0.07 in one (15 M) 8.0 and 10.6 ms, with 0.15 (54 M) 22.0
-// and 13.2.  (CRISPY_KMER_CAND sets the room, for tests.)
+// and 13.2.  (CRISPY_KMER_CAND sets the room, for tests: N, or below 0 one in -N of
+// the pairs.)
 int64_t candidates_worth(int64_t pairs, int k) {
-    if (const char* e = std::getenv("CRISPY_KMER_CAND")) return std::max(1ll, std::atoll(e));
+    if (const char* e = std::getenv("CRISPY_KMER_CAND")) {
+        const int64_t v = std::atoll(e);
+        return std::max<int64_t>(1, v < 0 ? pairs / -v : v);
+    }
     const int64_t base = (int64_t)(k <= 5 ? 11 : k == 6 ? 12 : k == 7 ? 9 : 6) << 18;
     return std::min<int64_t>(1 << 25, pairs / 256 + base);
 }

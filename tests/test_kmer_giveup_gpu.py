@@ -81,21 +81,32 @@ def test_probe_gives_up(engine, monkeypatch, k):
 
 @pytest.mark.parametrize("k", [6, 8])
 def test_second_range_gives_up(engine, monkeypatch, k):
-    # survivors beyond the device share, the second half of the reads in one
-    # OTU: a range of stage rows may overflow where those before it did not
-    reads = _reads(1400, k, 100 + k, 60)
-    dense = _reads(700, k, 110 + k, 1)
-    reads = synth.preprocess_order(reads) + synth.preprocess_order(dense)
+    # survivors beyond the device share, the last reads all of one OTU: the
+    # first pass and the first ranges of stage rows have few candidates for
+    # their pairs, the last range many
+    sparse = _reads(2000, k, 100 + k, 1000)
+    dense = _reads(620, k, 110 + k, 1, 270)      # longer: behind the others
+    reads = [r for r in sparse if len(r) < 262] + [r for r in synth.preprocess_order(dense) if len(r) > 262]
     buf, offs, lens = synth.pack_reads(reads)
     thr = 0.15
     want = oracle.kmer_all(buf, offs, lens, k, thr)
-    monkeypatch.setenv("CRISPY_KMER_DEVICE_PAIRS", str(len(want[0]) // 2))
-    for room in (len(want[0]) // 2, len(want[0]) * 3 // 4, 1 << 22):
-        monkeypatch.setenv("CRISPY_KMER_CAND", str(room))
+    monkeypatch.setenv("CRISPY_KMER_DEVICE_PAIRS", str(len(want[0]) * 9 // 10))
+    launches = {}
+    # room for any number; for one in 20 of a pass's pairs, which the last
+    # reads' own rows outgrow; for one in 1,000, which the first pass does
+    for room in ("100000000", "-20", "-1000"):
+        monkeypatch.setenv("CRISPY_KMER_CAND", room)
         engine.kmer_prepare(buf, offs, lens, k)
         got, st = _run(engine, thr)
         assert st["kmer_spilled"] == 1
         _same(got, want)
+        launches[room] = st["kmer_launches"]
+    passes = launches["100000000"]               # the filter in every pass
+    assert passes >= 3
+    # one attempt more than passes, after which no other pass tries (at K = 8
+    # every pass bounds all pairs: what the first one fits fits the others)
+    assert launches["-20"] == (passes + 1 if k == 6 else passes)
+    assert launches["-1000"] == passes + 1
 
 
 def test_tuner_behind_a_gave_up_filter(engine, monkeypatch):
