@@ -1391,6 +1391,8 @@ int build_lists(crispy_ctx* ctx, FilterCtl* ctl, unsigned long long most) {
     const int K4 = 1 << (2 * k);
     const int32_t* t = k == 8 ? j.f_t.as<int32_t>() : j.t0.as<int32_t>();
     const int32_t* perm = k == 8 ? j.f_perm.as<int32_t>() : nullptr;
+    // (a pass that gave up or ran out of time may have built them already)
+    CRISPY_CK(ctx, cudaMemsetAsync(j.f_hist.as<uint32_t>() + K4, 0, 4, s));
     const bool direct = k <= 6;
     const int slots_log2 = j.max_t <= 512 ? 10 : j.max_t <= 1024 ? 11 : 12;
     const int words = direct ? K4 / 2 : 1 << slots_log2;

@@ -132,3 +132,25 @@ def test_tuner_behind_a_gave_up_filter(engine, monkeypatch):
     monkeypatch.setenv("CRISPY_KMER_FILTER", "0")
     engine.kmer_prepare(buf, offs, lens, 6)
     _same(_run(engine, 0.1)[0], want)
+
+
+@pytest.mark.parametrize("k,length", [(5, 300), (6, 500), (8, 400)])
+def test_lists_built_again_after_giving_up(engine, monkeypatch, k, length):
+    # reads over two bases: nearly every K-mer is a repeat, so the lists of
+    # repeats fill their room; a round gives up behind them, and tighter cuts
+    # with as many dimensions build them again, time after time
+    rng = np.random.default_rng(k)
+    base = rng.choice(np.frombuffer(b"TC", np.uint8), length)
+    reads = []
+    for _ in range(400):
+        s = base[:int(rng.integers(length - 20, length + 1))].copy()
+        for p in rng.integers(0, len(s), int(rng.integers(0, 4))):
+            s[p] = b"TC"[int(rng.integers(0, 2))]
+        reads.append(s.tobytes())
+    buf, offs, lens = synth.pack_reads(synth.preprocess_order(reads))
+    engine.kmer_prepare(buf, offs, lens, k)
+    for i, thr in enumerate((0.15, 0.14, 0.13, 0.12, 0.11, 0.1, 0.09)):
+        # given up at all cuts but the last (the room is what it is for them)
+        monkeypatch.setenv("CRISPY_KMER_CAND", "50" if i < 6 else "100000000")
+        got, _ = _run(engine, thr)
+        _same(got, oracle.kmer_all(buf, offs, lens, k, thr))
