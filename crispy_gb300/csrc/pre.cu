@@ -294,7 +294,8 @@ struct Ties {
 // 60,000 reads of 250 nt, reads compared throughout without keys, and now: no
 // common head 642 and 556 us, a common head of 20 bases 695 and 652, of 40
 // bases 714 and 674, all of one length 739 and 650.
-constexpr int kSample = 1024, kSampleSlots = 4096;
+constexpr int kSample = 1024, kSampleSlots = 2048;
+static_assert(kSampleSlots >= 2 * kSample && kSampleSlots * 12 + 16 <= 48 * 1024, "a free slot for every read, in static shared memory");
 __global__ void __launch_bounds__(kSample) pre_sample_kernel(const ReadKey* __restrict__ keys, int64_t m, double limit,
                                                              unsigned long long* __restrict__ too_many) {
     __shared__ unsigned long long slot[kSampleSlots];
